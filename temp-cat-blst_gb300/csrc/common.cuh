@@ -107,10 +107,10 @@ struct MsmWork {
 };
 
 struct FftWork {
-    DevBuf values, roots, glv, scratch, meta;
+    DevBuf values, roots, glv, scratch, prod, meta;
     void release()
     {
-        for (DevBuf* b : {&values, &roots, &glv, &scratch, &meta}) b->release();
+        for (DevBuf* b : {&values, &roots, &glv, &scratch, &prod, &meta}) b->release();
     }
 };
 

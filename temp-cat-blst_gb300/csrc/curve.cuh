@@ -187,6 +187,51 @@ __device__ __forceinline__ void xyzz_add(xyzz& p, const xyzz& q)
     fp_mul2(p.y, U1, R, S1, PPP); // Y3 = R (Q - X3) - S1 PPP, one reduction
 }
 
+// d = p - q, p += q, sharing everything but the two R's (12M + 3S for both
+// against 24M + 4S); exceptional operands take the general additions.
+__device__ __forceinline__ void xyzz_add_sub(xyzz& p, xyzz& d, const xyzz& q)
+{
+    fp U1, S1, P, S2;
+    fp_mul(U1, p.x, q.zz);
+    fp_mul(P, q.x, p.zz);
+    fp_sub(P, P, U1);
+    if (xyzz_is_inf(p) || xyzz_is_inf(q) || fp_is_zero(P)) {
+        xyzz n = q;
+        fp_neg(n.y, n.y);
+        d = p;
+        xyzz_add(d, n);
+        xyzz_add(p, q);
+        return;
+    }
+    fp_mul(S1, p.y, q.zzz);
+    fp_mul(S2, q.y, p.zzz);
+    fp PP, PPP, t, R;
+    fp_sqr(PP, P);
+    fp_mul(PPP, PP, P);
+    fp_mul(t, p.zz, q.zz);
+    fp_mul(p.zz, t, PP);
+    fp_mul(t, p.zzz, q.zzz);
+    fp_mul(p.zzz, t, PPP);
+    d.zz = p.zz;
+    d.zzz = p.zzz;
+    fp_mul(U1, U1, PP);           // Q = U1 PP
+    fp_neg(P, PPP);
+    fp_sub(P, P, U1);
+    fp_sub(P, P, U1);             // -PPP - 2Q
+    fp_neg(PPP, PPP);
+    fp_sub(R, S2, S1);
+    fp_sqr(t, R);
+    fp_add(p.x, t, P);
+    fp_sub(t, U1, p.x);
+    fp_mul2(p.y, t, R, S1, PPP);  // Y3 = R (Q - X3) - S1 PPP
+    fp_add(R, S2, S1);
+    fp_neg(R, R);
+    fp_sqr(t, R);
+    fp_add(d.x, t, P);
+    fp_sub(t, U1, d.x);
+    fp_mul2(d.y, t, R, S1, PPP);
+}
+
 __device__ __forceinline__ void xyzz_neg(xyzz& p) { fp_neg(p.y, p.y); }
 
 // Jacobian (X, Y, Z) = (x*zz, y*zzz, zz); reference point.cpp:2109
@@ -305,145 +350,6 @@ __device__ __constant__ static const uint32_t FP_BETA[12] = {
     0x8671f071u, 0xcd03c9e4u, 0x1fcda5d2u, 0x5dab2246u, 0xd3851b95u, 0x587042afu,
     0x01bacb9eu, 0x8eb60ebeu, 0x83d050d2u, 0x03f97d6eu, 0x54638741u, 0x18f02065u};
 
-// Signed fixed-window digits of a value below 2^128 (4 little-endian words):
-// 26 digits d_i in [-15, 16] with value = sum_i d_i 32^i (window recoding
-// with carry, as the MSM's digit recoding).  Every value uses the same 26
-// windows, so lanes of a warp working on different scalars add at the same
-// positions.  5-bit windows against 4-bit: 125 doublings and ~50 additions
-// instead of 128 and ~62, for a 16-entry table (7% faster FFTs measured).
-__device__ __forceinline__ void booth5_128(int8_t* d, const uint32_t* k)
-{
-    uint32_t carry = 0;
-#pragma unroll
-    for (int i = 0; i < 26; i++) {
-        const uint32_t bit = 5 * i, word = bit >> 5, sh = bit & 31;
-        uint32_t raw = word < 4 ? k[word] >> sh : 0u;
-        if (sh > 27 && word + 1 < 4) raw |= k[word + 1] << (32 - sh);
-        raw &= 31u;
-        int v = (int)(raw + carry);
-        if (v > 16) { v -= 32; carry = 1; }
-        else carry = 0;
-        d[i] = (int8_t)v;
-    }
-}
-static __device__ __noinline__ void jac_mult_glv(jac& out, const jac& P, const uint32_t* k1, const uint32_t* k2)
-{
-    int8_t d1[26], d2[26];
-    booth5_128(d1, k1);
-    booth5_128(d2, k2);
-    jac T[16];                                   // T[i] = (i + 1) P
-    T[0] = P;
-    T[1] = P; jac_dbl(T[1]);
-#pragma unroll 1
-    for (int i = 2; i < 16; i++) {
-        if (i & 1) { T[i] = T[i / 2]; jac_dbl(T[i]); }         // (i+1) even: 2 ((i+1)/2) P
-        else { T[i] = T[i - 1]; jac_add(T[i], P); }
-    }
-    fp beta;
-#pragma unroll
-    for (int i = 0; i < 12; i++) beta.v[i] = FP_BETA[i];
-    jac acc;
-    jac_set_inf(acc);
-    for (int i = 25; i >= 0; i--) {
-        if (i < 25) {
-            jac_dbl(acc); jac_dbl(acc); jac_dbl(acc); jac_dbl(acc); jac_dbl(acc);
-        }
-        const int a = d1[i], b = d2[i];
-        if (a) {
-            jac t = T[(a > 0 ? a : -a) - 1];
-            if (a < 0) jac_neg(t);
-            jac_add(acc, t);
-        }
-        if (b) {
-            jac t = T[(b > 0 ? b : -b) - 1];
-            fp_mul(t.x, t.x, beta);
-            if (b < 0) jac_neg(t);
-            jac_add(acc, t);
-        }
-    }
-    out = acc;
-}
-
-// Width-5 NAF of a value below 2^128 (4 little-endian words): digits d_i in
-// {0, +-1, +-3, ..., +-15} with value = sum_i d_i 2^i and at most one nonzero
-// digit in any five consecutive positions (density ~1/6).  Returns the number
-// of digits, at most 129: subtracting a negative digit can carry the value
-// past 2^128 once, after which every step halves it.
-__device__ __forceinline__ int wnaf5_128(int8_t* d, const uint32_t* k)
-{
-    uint32_t w0 = k[0], w1 = k[1], w2 = k[2], w3 = k[3], w4 = 0;
-    int len = 0;
-#pragma unroll 1
-    for (int i = 0; i < 130 && (w0 | w1 | w2 | w3 | w4); i++) {
-        int v = 0;
-        if (w0 & 1u) {
-            v = (int)(w0 & 31u);
-            if (v > 16) v -= 32;
-            if (v > 0) {
-                w0 -= (uint32_t)v;                   // the low five bits are v: no borrow
-            } else {
-                uint64_t s = (uint64_t)w0 + (uint32_t)(-v);
-                w0 = (uint32_t)s;
-                s = (s >> 32) + w1; w1 = (uint32_t)s;
-                s = (s >> 32) + w2; w2 = (uint32_t)s;
-                s = (s >> 32) + w3; w3 = (uint32_t)s;
-                w4 += (uint32_t)(s >> 32);
-            }
-        }
-        d[i] = (int8_t)v;
-        len = i + 1;
-        w0 = (w0 >> 1) | (w1 << 31);
-        w1 = (w1 >> 1) | (w2 << 31);
-        w2 = (w2 >> 1) | (w3 << 31);
-        w3 = (w3 >> 1) | (w4 << 31);
-        w4 >>= 1;
-    }
-    return len;
-}
-
-// jac_mult_glv for lanes that all multiply by one scalar (k1, k2): each half
-// in width-5 NAF over the odd multiples P, 3P, ..., 15P (one doubling and
-// seven additions) and phi of them, ~129 doublings and ~50 additions against
-// 133 and ~57 for the fixed windows.  The digit positions depend on the
-// scalar, so lanes with different scalars would diverge at every addition;
-// jac_mult_glv serves those.
-static __device__ __noinline__ void jac_mult_glv_shared(jac& out, const jac& P, const uint32_t* k1,
-                                                        const uint32_t* k2)
-{
-    int8_t d1[130], d2[130];
-    const int n1 = wnaf5_128(d1, k1), n2 = wnaf5_128(d2, k2);
-    jac T[8];                                    // T[i] = (2 i + 1) P
-    jac P2 = P;
-    jac_dbl(P2);
-    T[0] = P;
-#pragma unroll 1
-    for (int i = 1; i < 8; i++) {
-        T[i] = T[i - 1];
-        jac_add(T[i], P2);
-    }
-    fp beta;
-#pragma unroll
-    for (int i = 0; i < 12; i++) beta.v[i] = FP_BETA[i];
-    jac acc;
-    jac_set_inf(acc);
-    for (int i = max(n1, n2) - 1; i >= 0; i--) {
-        jac_dbl(acc);
-        const int a = i < n1 ? d1[i] : 0, b = i < n2 ? d2[i] : 0;
-        if (a) {
-            jac t = T[(a > 0 ? a : -a) >> 1];
-            if (a < 0) jac_neg(t);
-            jac_add(acc, t);
-        }
-        if (b) {
-            jac t = T[(b > 0 ? b : -b) >> 1];
-            fp_mul(t.x, t.x, beta);
-            if (b < 0) jac_neg(t);
-            jac_add(acc, t);
-        }
-    }
-    out = acc;
-}
-
 // ---------------------------------------------------------------------------
 // Quad point operations: four consecutive lanes (a quad) hold the same
 // operands and perform one XYZZ addition or doubling together.  At each step
@@ -542,110 +448,6 @@ __device__ __forceinline__ void xyzz_add_quad(xyzz& p, const xyzz& o, const quad
     const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
     p.zzz = fp_bcast(r, 2, q);
     fp_sub(p.y, a, b);
-}
-
-// dbl-2009-l as jac_dbl: X^2, Y^2, Y Z | B^2, (X + B)^2, E^2 | E (D - X3).
-__device__ __forceinline__ void jac_dbl_quad(jac& p, const quad_lane& q)
-{
-    if (jac_is_inf(p)) return;
-    fp r = fp_mul_call(fp_pick(q.k, p.x, p.y, p.y, p.y), fp_pick(q.k, p.x, p.y, p.z, p.z));
-    const fp A = fp_bcast(r, 0, q), B = fp_bcast(r, 1, q), YZ = fp_bcast(r, 2, q);
-    fp XB, E, t, D;
-    fp_add(XB, p.x, B);
-    fp_dbl(E, A);
-    fp_add(E, E, A);
-    r = fp_mul_call(fp_pick(q.k, B, XB, E, E), fp_pick(q.k, B, XB, E, E));
-    const fp C = fp_bcast(r, 0, q), T = fp_bcast(r, 1, q), F = fp_bcast(r, 2, q);
-    fp_sub(t, T, A);
-    fp_sub(t, t, C);
-    fp_dbl(D, t);
-    fp_sub(t, F, D);
-    fp_sub(p.x, t, D);
-    fp_sub(t, D, p.x);
-    fp_dbl(p.z, YZ);
-    r = fp_mul_call(E, t);                      // the same product on every lane
-    fp C8;
-    fp_dbl(C8, C);
-    fp_dbl(C8, C8);
-    fp_dbl(C8, C8);
-    fp_sub(p.y, r, C8);
-}
-
-// p += o as jac_add: Z1^2, Z2^2, Y1 Z2, Y2 Z1 | U1, U2, S1, S2 | H^2, R^2,
-// Z1 Z2 | U1 HH, H HH, Z1 Z2 H | R (V - X3), S1 HHH.
-__device__ __forceinline__ void jac_add_quad(jac& p, const jac& o, const quad_lane& q)
-{
-    if (jac_is_inf(o)) return;
-    if (jac_is_inf(p)) {
-        p = o;
-        return;
-    }
-    fp r = fp_mul_call(fp_pick(q.k, p.z, o.z, p.y, o.y), fp_pick(q.k, p.z, o.z, o.z, p.z));
-    const fp z1z1 = fp_bcast(r, 0, q), z2z2 = fp_bcast(r, 1, q), s1a = fp_bcast(r, 2, q), ra = fp_bcast(r, 3, q);
-    r = fp_mul_call(fp_pick(q.k, p.x, o.x, s1a, ra), fp_pick(q.k, z2z2, z1z1, z2z2, z1z1));
-    const fp u1 = fp_bcast(r, 0, q), s1 = fp_bcast(r, 2, q);
-    fp h = fp_bcast(r, 1, q), R = fp_bcast(r, 3, q);
-    fp_sub(h, h, u1);
-    fp_sub(R, R, s1);
-    if (fp_is_zero(h)) {
-        if (fp_is_zero(R)) jac_dbl_quad(p, q);
-        else jac_set_inf(p);
-        return;
-    }
-    r = fp_mul_call(fp_pick(q.k, h, R, p.z, p.z), fp_pick(q.k, h, R, o.z, o.z));
-    const fp HH = fp_bcast(r, 0, q), RR = fp_bcast(r, 1, q), Z12 = fp_bcast(r, 2, q);
-    r = fp_mul_call(fp_pick(q.k, u1, h, Z12, Z12), fp_pick(q.k, HH, HH, h, h));
-    const fp V = fp_bcast(r, 0, q), HHH = fp_bcast(r, 1, q);
-    p.z = fp_bcast(r, 2, q);
-    fp t;
-    fp_sub(t, RR, HHH);
-    fp_sub(t, t, V);
-    fp_sub(p.x, t, V);
-    fp_sub(t, V, p.x);
-    r = fp_mul_call(fp_pick(q.k, R, s1, s1, s1), fp_pick(q.k, t, HHH, HHH, HHH));
-    const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
-    fp_sub(p.y, a, b);
-}
-
-// jac_mult_glv with quad operations: every lane of the quad passes the same
-// point and scalar and ends with the product.
-static __device__ __noinline__ void jac_mult_glv_quad(jac& out, const jac& P, const uint32_t* k1, const uint32_t* k2,
-                                                      const quad_lane q)
-{
-    int8_t d1[26], d2[26];
-    booth5_128(d1, k1);
-    booth5_128(d2, k2);
-    jac T[16];                                   // T[i] = (i + 1) P
-    T[0] = P;
-    T[1] = P;
-    jac_dbl_quad(T[1], q);
-#pragma unroll 1
-    for (int i = 2; i < 16; i++) {
-        if (i & 1) { T[i] = T[i / 2]; jac_dbl_quad(T[i], q); }
-        else { T[i] = T[i - 1]; jac_add_quad(T[i], P, q); }
-    }
-    fp beta;
-#pragma unroll
-    for (int i = 0; i < 12; i++) beta.v[i] = FP_BETA[i];
-    jac acc;
-    jac_set_inf(acc);
-    for (int i = 25; i >= 0; i--) {
-        if (i < 25)
-            for (int k = 0; k < 5; k++) jac_dbl_quad(acc, q);
-        const int a = d1[i], b = d2[i];
-        if (a) {
-            jac t = T[(a > 0 ? a : -a) - 1];
-            if (a < 0) jac_neg(t);
-            jac_add_quad(acc, t, q);
-        }
-        if (b) {
-            jac t = T[(b > 0 ? b : -b) - 1];
-            fp_mul(t.x, t.x, beta);
-            if (b < 0) jac_neg(t);
-            jac_add_quad(acc, t, q);
-        }
-    }
-    out = acc;
 }
 
 }  // namespace catmsm

@@ -3,37 +3,38 @@
 // Drop-in for blst_p1_fft / blst_p1_fft_with_domain /
 // blst_p1_ifft_unscaled_with_domain (reference fft_c_api.cpp:51-103,
 // fft/ctFft.h:32-124, fft/context.h:182-215).  The transform is the same
-// radix-2 decimation-in-time schedule with the same root indexing
+// radix-2 decimation-in-time network with the same root indexing
 // (root j * n/len, or n - j * n/len when the inverse reads forward roots), so
 // outputs equal the reference's for any root table the caller supplies.
 //
-// Device layout: the Jacobian points (blst_p1 bytes, 144 B) of one or many
-// transforms, concatenated in HBM; a job descriptor per transform.
-//   k_roots_prepare    per root index: Montgomery Fr -> canonical -> GLV
-//                      halves (k = k1 + lambda k2), stored as 8 words.
-//   k_bitrev_multi     out-of-place bit-reversal permutation of every job.
-//   k_fft_stage_multi  one launch per stage level for ALL jobs that have the
-//                      level (a batch of transforms fills the GPU where one
-//                      small transform cannot); inside a job, threads map
-//                      first onto the non-trivial butterflies (j >= 1, one
-//                      GLV scalar multiplication each), then onto the
-//                      j == 0 butterflies, so a warp rarely mixes the two.
-//                      Early stages (32 or more active groups) put the lanes
-//                      of a warp on one root (width-5 NAF halves); later
-//                      ones on consecutive roots (signed 5-bit fixed
-//                      windows, the same digit positions for every root).
-//                      Launches small enough to fit one wave at four lanes
-//                      per butterfly use quad point operations.
-//   k_fft_finish_multi the inverse 1/n scale (one GLV multiplication per
-//                      element of scaled jobs) and canonical coordinates.
-// Each butterfly is ~1.7k Fp multiplications (~1M IMAD) against 576 bytes of
-// traffic, so large stages are IMAD-bound and read/write straight from
-// HBM/L2; staging tiles in shared memory would save nothing measurable.
+// Device layout: the points of one or many transforms, concatenated, as XYZZ
+// (192 B) between the passes; a job descriptor per transform.
+//   k_bitrev_multi     Jacobian input -> XYZZ in bit-reversed order.
+//   then passes over the levels, each chosen by fft_plan for the whole batch:
+//   k_fft_stage_multi  one level, one lane per butterfly, for batches that fill
+//                      the GPU: the multiply pipe bounds it (~80% busy), so it
+//                      takes the fewest multiplications: n/2 scalar
+//                      multiplications a level.
+//   k_fft_items + k_fft_combine  q levels at once, for batches that do not:
+//                      there a level lasts as long as ONE scalar multiplication
+//                      (~0.7 ms), whatever its count, so q levels are rewritten as
+//                      sums over products of roots.  Every output of a 2^q-point
+//                      block is sum_m +- (root product) x_m, each product
+//                      of a point by a root product is an item of its own
+//                      ((4^q - 1) / 3 of them per block, all independent), and
+//                      the combine adds them up.  Twice (q = 2) to 2.7 times (q = 4) the
+//                      scalar multiplications per level, q times fewer in sequence.
+//   k_fft_finish_multi Jacobian, canonical coordinates.
+// The inverse's 1/n scale is multiplied into the roots of a job's last pass.
+// Each butterfly is ~1.5k Fp multiplications (~0.9M IMAD) against 768 bytes of
+// traffic, so memory never binds.
 #include "common.cuh"
 #include "curve.cuh"
 #include "fr.cuh"
+#include "glv_mult.cuh"
 #include "catmsm_internal.h"
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -69,6 +70,26 @@ __global__ void k_roots_prepare(const uint32_t* __restrict__ roots_mont, uint32_
     fr_glv_split(out + 8 * i, out + 8 * i + 4, c);
 }
 
+// The scaled roots of a job's last level: out[j] = root(j) * scale, j < n / 2
+// (root(j) = w^j, or entry n - j when the inverse reads forward roots), and
+// out[n / 2] = scale, as GLV halves.
+__global__ void k_roots_prepare_scaled(const uint32_t* __restrict__ roots_mont, const uint32_t* __restrict__ scale,
+                                       uint32_t n, int inv_from_fwd, uint32_t* __restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > n / 2) return;
+    uint32_t m[8], c[8];
+    for (int k = 0; k < 8; k++) m[k] = scale[k];
+    if (i != 0 && i != n / 2) {
+        const size_t idx = inv_from_fwd ? n - i : i;
+        uint32_t r[8];
+        for (int k = 0; k < 8; k++) r[k] = roots_mont[8 * idx + k];
+        fr_mul(m, m, r);
+    }
+    fr_from_mont(c, m);
+    fr_glv_split(out + 8 * (size_t)i, out + 8 * (size_t)i + 4, c);
+}
+
 // powers of a Montgomery root: out[i] = w^i (Montgomery)
 __global__ void k_root_powers(const uint32_t* __restrict__ w, uint32_t n, uint32_t* __restrict__ out)
 {
@@ -80,16 +101,16 @@ __global__ void k_root_powers(const uint32_t* __restrict__ w, uint32_t n, uint32
     for (int k = 0; k < 8; k++) out[8 * i + k] = o[k];
 }
 
-// A batch of transforms shares one launch per stage level.  Job descriptor:
+// A batch of transforms shares the launches of every pass.  Job descriptor:
 struct FftJob {
     uint32_t val_off;    // first element of this transform in the values buffer
     uint32_t n, logn;
-    uint32_t glv_off;    // first prepared root (8 words each); glv_off + n: the scale
+    uint32_t glv_off;    // first prepared root (8 words each); glv_off + n: the scaled roots of the last level
     int32_t inv_from_fwd;
-    int32_t scaled;
     uint32_t xn;         // inputs [xn, n) are the identity: stage s runs only the
                          // min(xn, n / 2^s) groups holding a non-identity input
-    uint32_t pad;
+    const uint32_t* roots;   // the n Montgomery roots
+    const uint32_t* scale;   // Montgomery scale of every output, or null
 };
 
 // thread t of a launch over per-job ranges: find the job whose range holds t
@@ -105,7 +126,7 @@ __device__ __forceinline__ uint32_t find_range(const uint32_t* __restrict__ pre,
     return lo;
 }
 
-__global__ void k_bitrev_multi(const jac* __restrict__ in, jac* __restrict__ out, const FftJob* __restrict__ jobs,
+__global__ void k_bitrev_multi(const jac* __restrict__ in, xyzz* __restrict__ out, const FftJob* __restrict__ jobs,
                                const uint32_t* __restrict__ pre, uint32_t njobs, uint32_t total)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -115,24 +136,34 @@ __global__ void k_bitrev_multi(const jac* __restrict__ in, jac* __restrict__ out
     const uint32_t r = J.logn ? (__brev(i) >> (32 - J.logn)) : 0;
     jac p;
     load_jac(p, in + t);
-    store_jac(out + J.val_off + r, p);
+    xyzz o;
+    jac_to_xyzz(o, p);
+    store_xyzz(out + J.val_off + r, o);
 }
 
-// Stage `len` over every job with n >= len.  lst: for this stage, pairs of
-// (job id, exclusive prefix of n/2 butterflies), `cnt` entries.  Quad = true:
-// a quad of lanes per butterfly (quad point operations), for stages with too
-// few butterflies to fill the GPU, where the ~0.9M-cycle chain of one scalar
-// multiplication, not the multiplier throughput, sets the stage time.
-template <bool Quad>
-__global__ void __launch_bounds__(64) k_fft_stage_multi(jac* __restrict__ a, const FftJob* __restrict__ jobs,
+// Group g of a level with `groups` groups, `active` of them holding a
+// non-identity input (bit-reversed positions: the bit reversals of
+// 0 .. active - 1).
+__device__ __forceinline__ uint32_t active_group(uint32_t g, uint32_t active, uint32_t groups)
+{
+    return active < groups ? __brev(g) >> (32 - (31 - __clz(groups))) : g;
+}
+
+// Stage `len` over every job with n >= len, one lane per butterfly.  lst: for
+// this stage, pairs of (job id, exclusive prefix of n/2 butterflies), `cnt`
+// entries.  Threads map first onto the non-trivial butterflies (j >= 1), then
+// onto the j == 0 ones, so a warp rarely mixes the two.  MinBlocks: resident
+// blocks per SM the registers are limited for.  4 (255 registers) is 3% faster
+// while one wave holds the launch; above that, 6 (168 registers) shortens the
+// last wave: 46080 butterflies 3.5 -> 3.1 ms a level.
+template <int MinBlocks>
+__global__ void __launch_bounds__(64, MinBlocks) k_fft_stage_multi(xyzz* __restrict__ a, const FftJob* __restrict__ jobs,
                                                         const uint32_t* __restrict__ lst_job,
                                                         const uint32_t* __restrict__ lst_pre, uint32_t cnt,
                                                         uint32_t total, uint32_t len, const uint32_t* __restrict__ glv)
 {
-    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t t = Quad ? gt >> 2 : gt;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const quad_lane ql = quad_of(threadIdx.x & 31);
     const uint32_t e = find_range(lst_pre, cnt, t);
     const FftJob J = jobs[lst_job[e]];
     const uint32_t b = t - lst_pre[e];
@@ -147,7 +178,7 @@ __global__ void __launch_bounds__(64) k_fft_stage_multi(jac* __restrict__ a, con
     uint32_t g, j;
     bool shared = false;
     if (b < nontriv) {
-        if (!Quad && (active & 31u) == 0) {
+        if ((active & 31u) == 0) {
             j = 1 + b / active;
             g = b % active;
             shared = true;
@@ -159,75 +190,211 @@ __global__ void __launch_bounds__(64) k_fft_stage_multi(jac* __restrict__ a, con
         g = b - nontriv;
         j = 0;
     }
-    // After the bit-reversal permutation, position p holds input bitrev(p);
-    // group g of this stage (positions g len .. g len + len - 1) holds a
-    // non-identity input iff bitrev(g) over log2(groups) bits is below xn, so
-    // the active groups are the bit reversals of 0 .. active - 1.
-    if (active < groups) g = __brev(g) >> (32 - (J.logn - (31 - __clz(len))));
-    jac* base = a + J.val_off;
+    g = active_group(g, active, groups);
+    xyzz* base = a + J.val_off;
     const uint32_t i0 = g * len + j, i1 = i0 + half;
-    jac u, v;
-    load_jac(u, base + i0);
-    load_jac(v, base + i1);
-    if (j) {
-        uint32_t idx = j * (J.n / len);
-        if (J.inv_from_fwd) idx = J.n - idx;
+    xyzz u, v;
+    load_xyzz(v, base + i1);
+    const bool scaled = J.scale && len == J.n;       // the job's last level: roots times the scale
+    if (j || scaled) {
+        uint32_t idx = J.n + j;
+        if (!scaled) {
+            idx = j * groups;
+            if (J.inv_from_fwd) idx = J.n - idx;
+        }
         const uint32_t* r = glv + 8 * (size_t)(J.glv_off + idx);
-        if (Quad) jac_mult_glv_quad(v, v, r, r + 4, ql);
-        else if (shared) jac_mult_glv_shared(v, v, r, r + 4);
-        else jac_mult_glv(v, v, r, r + 4);
+        if (shared) xyzz_mult_glv_shared(v, v, r, r + 4);
+        else xyzz_mult_glv(v, v, r, r + 4);
     }
-    jac s = u;
-    if (Quad) {
-        jac_add_quad(s, v, ql);
-        jac_neg(v);
-        jac_add_quad(u, v, ql);
-        if (ql.k == 0) store_jac(base + i0, s);
-        if (ql.k == 1) store_jac(base + i1, u);
-    } else {
-        jac_add(s, v);
-        jac_neg(v);
-        jac_add(u, v);
-        store_jac(base + i0, s);
-        store_jac(base + i1, u);
+    load_xyzz(u, base + i0);
+    if (scaled) {
+        const uint32_t* r = glv + 8 * (size_t)(J.glv_off + J.n + half);
+        xyzz_mult_glv_shared(u, u, r, r + 4);        // one scale per job, shared by its lanes
     }
+    xyzz d;
+    xyzz_add_sub(u, d, v);
+    store_xyzz(base + i0, u);
+    store_xyzz(base + i1, d);
 }
 
-// inverse scale (jobs with scaled != 0) and canonicalisation of every element
-template <bool Quad>
-__global__ void __launch_bounds__(64) k_fft_finish_multi(jac* __restrict__ a, const FftJob* __restrict__ jobs,
-                                                         const uint32_t* __restrict__ pre, uint32_t njobs,
-                                                         uint32_t total, const uint32_t* __restrict__ glv,
-                                                         int do_scale)
+// ---------------------------------------------------------------- q levels at once
+// Levels s0 + 1 .. s0 + q of a job over its blocks of 2^q h positions (h =
+// 2^s0): position j + m h (j < h) of a block holds x_m, and output k of the
+// butterfly (block, j) is
+//   sum_m (-1)^popc(m & k) C(m, k) x_m,
+//   C = product over the set bits i of m of the root of level i at position
+//       j + h (k mod 2^i) of its half-block.
+// C depends on k only below m's top bit t, so the products of x_m are the 2^t
+// items (m, k mod 2^t).  Item 0 is x_0 itself.  Item 1 + (4^t - 1) / 3 +
+// (m - 2^t) 2^t + (k mod 2^t) is the product (m, k), so a butterfly has
+// 1 + (4^q - 1) / 3 items.
+__host__ __device__ __forceinline__ uint32_t pass_items(uint32_t q) { return 1 + ((1u << (2 * q)) - 1) / 3; }
+
+__device__ __forceinline__ uint32_t item_of(uint32_t m, uint32_t k)
 {
+    if (m == 0) return 0;
+    const uint32_t t = 31 - __clz(m), top = 1u << t;
+    return 1 + (top * top - 1) / 3 + (m - top) * top + (k & (top - 1));
+}
+
+// A pass of one job: its q, blocks and butterflies.
+struct PassGeom {
+    uint32_t q, groups, active, bf;
+};
+
+__device__ __forceinline__ PassGeom pass_geom(const FftJob& J, uint32_t s0, uint32_t q)
+{
+    PassGeom g;
+    g.q = min(q, J.logn - s0);
+    g.groups = J.n >> (s0 + g.q);
+    g.active = min(g.groups, J.xn);
+    g.bf = g.active << s0;
+    return g;
+}
+
+// The products of a pass: item-major per job (all items of one kind are
+// adjacent, so trivial ones do not share warps with multiplications).
+// Quad: a quad of lanes per item.
+template <bool Quad>
+__global__ void __launch_bounds__(64) k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod,
+                                                  const FftJob* __restrict__ jobs,
+                                                  const uint32_t* __restrict__ lst_job,
+                                                  const uint32_t* __restrict__ lst_pre, uint32_t cnt, uint32_t total,
+                                                  uint32_t s0, uint32_t q)
+{
+    __shared__ quad_table tabs[Quad ? 16 : 1];
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t t = Quad ? gt >> 2 : gt;
     if (t >= total) return;
     const quad_lane ql = quad_of(threadIdx.x & 31);
-    const FftJob J = jobs[find_range(pre, njobs, t)];
-    jac v;
-    load_jac(v, a + t);
-    if (do_scale && J.scaled) {
-        const uint32_t* r = glv + 8 * (size_t)(J.glv_off + J.n);
-        if (Quad) jac_mult_glv_quad(v, v, r, r + 4, ql);
-        else jac_mult_glv_shared(v, v, r, r + 4);        // one scale per job, shared by its lanes
+    const uint32_t e = find_range(lst_pre, cnt, t);
+    const FftJob J = jobs[lst_job[e]];
+    const PassGeom G = pass_geom(J, s0, q);
+    const uint32_t b = t - lst_pre[e];
+    const uint32_t it = b / G.bf, bf = b % G.bf;
+    const uint32_t h = 1u << s0, j = bf & (h - 1);
+    const uint32_t g = active_group(bf >> s0, G.active, G.groups);
+    uint32_t m = 0, k = 0;
+    if (it) {
+        uint32_t top = 1, rem = it - 1;              // rem in [0, top^2) at top = 2^t
+        while (rem >= top * top) {
+            rem -= top * top;
+            top <<= 1;
+        }
+        m = top + rem / top;
+        k = rem & (top - 1);
     }
-    if (jac_is_inf(v)) {
-        jac_set_inf(v);
-    } else {
-        fp_canon(v.x, v.x);
-        fp_canon(v.y, v.y);
-        fp_canon(v.z, v.z);
+    xyzz v;
+    load_xyzz(v, a + J.val_off + ((size_t)g << (s0 + G.q)) + j + m * h);
+    // the coefficient: Montgomery roots multiplied up (root 0 is never read:
+    // a j = 0 butterfly has no multiplication)
+    uint32_t c[8];
+    bool one = true;
+    if (J.scale && s0 + G.q == J.logn) {
+        for (int w = 0; w < 8; w++) c[w] = J.scale[w];
+        one = false;
     }
-    if (!Quad || ql.k == 0) store_jac(a + t, v);
+    for (uint32_t i = 0; i < G.q; i++) {
+        if (!((m >> i) & 1u)) continue;
+        const uint32_t pos = j + h * (k & ((1u << i) - 1));
+        if (pos == 0) continue;
+        uint32_t idx = pos * (J.n >> (s0 + i + 1));
+        if (J.inv_from_fwd) idx = J.n - idx;
+        uint32_t r[8];
+        for (int w = 0; w < 8; w++) r[w] = J.roots[8 * (size_t)idx + w];
+        if (one) {
+            for (int w = 0; w < 8; w++) c[w] = r[w];
+            one = false;
+        } else {
+            fr_mul(c, c, r);
+        }
+    }
+    if (!one) {
+        uint32_t kc[8], k12[8];
+        fr_from_mont(kc, c);
+        fr_glv_split(k12, k12 + 4, kc);
+        if (Quad) xyzz_mult_glv_quad(v, v, k12, k12 + 4, tabs + (threadIdx.x >> 2), ql);
+        else xyzz_mult_glv(v, v, k12, k12 + 4);
+    }
+    if (!Quad || ql.k == 0) store_xyzz(prod + t, v);
 }
 
-// Launches with at most this many scalar multiplications use quads: four
-// lanes each still fit in one wave of resident threads, and the stage time is
-// one multiplication's latency, which quads cut ~1.8x.  Larger launches are
-// throughput-bound and keep one lane per butterfly (quads cost ~1.6x the
-// multiplier work).
-static size_t fft_quad_max()
+// The sums of a pass: `width` = 4 * 2^(q - 1) lanes per output, each quad adds
+// two products, then a tree over the output's quads.
+__global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ prod, xyzz* __restrict__ a,
+                                                     const FftJob* __restrict__ jobs,
+                                                     const uint32_t* __restrict__ lst_job,
+                                                     const uint32_t* __restrict__ lst_pre,
+                                                     const uint32_t* __restrict__ lst_out, uint32_t cnt,
+                                                     uint32_t total, uint32_t s0, uint32_t q)
+{
+    const uint32_t lw = q + 1;                       // log2 of the lanes per output
+    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t o = gt >> lw;
+    const bool valid = o < total;
+    const quad_lane ql = quad_of(threadIdx.x & 31);
+    const uint32_t qi = (gt & ((1u << lw) - 1)) >> 2;
+    uint32_t dst = 0;
+    xyzz acc, v;
+    xyzz_set_inf(acc);
+    if (valid) {
+        const uint32_t e = find_range(lst_out, cnt, o);
+        const FftJob J = jobs[lst_job[e]];
+        const PassGeom G = pass_geom(J, s0, q);
+        const uint32_t b = o - lst_out[e];
+        const uint32_t k = b / G.bf, bf = b % G.bf;
+        const uint32_t h = 1u << s0;
+        dst = J.val_off + (active_group(bf >> s0, G.active, G.groups) << (s0 + G.q)) + (bf & (h - 1)) + k * h;
+        const xyzz* p = prod + lst_pre[e] + bf;
+        if (2 * qi < (1u << G.q)) {
+            const uint32_t m0 = 2 * qi, m1 = m0 + 1;
+            load_xyzz(acc, p + (size_t)item_of(m0, k) * G.bf);
+            load_xyzz(v, p + (size_t)item_of(m1, k) * G.bf);
+            if (__popc(m0 & k) & 1) xyzz_neg(acc);
+            if (__popc(m1 & k) & 1) xyzz_neg(v);
+            xyzz_add_quad(acc, v, ql);
+        }
+    }
+    for (uint32_t d = 4; d < (1u << lw); d <<= 1) {
+        __syncwarp();
+        const uint32_t* pv = reinterpret_cast<const uint32_t*>(&acc);
+        uint32_t* po = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+        for (int w = 0; w < 48; w++) po[w] = __shfl_down_sync(0xffffffffu, pv[w], d);
+        if (((4 * qi) & (2 * d - 1)) == 0) xyzz_add_quad(acc, v, ql);
+    }
+    if (valid && (gt & ((1u << lw) - 1)) == 0) store_xyzz(a + dst, acc);
+}
+
+// Jacobian with canonical coordinates; one-point jobs are scaled here (they
+// have no pass).
+__global__ void __launch_bounds__(64) k_fft_finish_multi(const xyzz* __restrict__ a, jac* __restrict__ out,
+                                                         const FftJob* __restrict__ jobs,
+                                                         const uint32_t* __restrict__ pre, uint32_t njobs,
+                                                         uint32_t total)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const FftJob J = jobs[find_range(pre, njobs, t)];
+    xyzz v;
+    load_xyzz(v, a + t);
+    if (J.logn == 0 && J.scale) {
+        uint32_t c[8], kc[8], k12[8];
+        for (int w = 0; w < 8; w++) c[w] = J.scale[w];
+        fr_from_mont(kc, c);
+        fr_glv_split(k12, k12 + 4, kc);
+        xyzz_mult_plain(v, v, k12, k12 + 4);
+    }
+    jac o;
+    xyzz_to_jac(o, v);
+    fp_canon(o.x, o.x);
+    fp_canon(o.y, o.y);
+    fp_canon(o.z, o.z);
+    store_jac(out + t, o);
+}
+
+// Scalar multiplications that run at once as quads (one wave of k_fft_items<true>).
+static size_t fft_quad_wave()
 {
     static std::atomic<size_t> by_dev[64];          // shared by every calling thread
     int dev = 0;
@@ -238,10 +405,93 @@ static size_t fft_quad_max()
     }
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_stage_multi<true>, 64, 0);
-    size_t v = (sms > 0 && per_sm > 0) ? (size_t)sms * per_sm * 64 / 4 : (size_t)device_sms() * 64;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_items<true>, 64, 0);
+    size_t v = (sms > 0 && per_sm > 0) ? (size_t)sms * per_sm * 16 : (size_t)device_sms() * 64;
     if (dev >= 0 && dev < 64) by_dev[dev].store(v, std::memory_order_relaxed);
     return v;
+}
+
+// One pass: levels s0 + 1 .. s0 + q.
+struct FftPass {
+    uint32_t s0 = 0, q = 1;
+    enum { kStage, kQuads, kLanes } kind = kStage;
+    uint32_t off = 0, cnt = 0;          // its entries of the job lists
+    uint32_t items = 0, outputs = 0;
+};
+
+// Items and outputs of a pass over every job that has its first level.
+static void pass_counts(const std::vector<FftJob>& jobs, uint32_t s0, uint32_t q, size_t& items, size_t& outputs)
+{
+    items = outputs = 0;
+    for (const FftJob& J : jobs) {
+        if (J.logn <= s0) continue;
+        const uint32_t qe = std::min(q, J.logn - s0);
+        const size_t bf = (size_t)std::min(J.n >> (s0 + qe), J.xn) << s0;
+        items += bf * pass_items(qe);
+        outputs += bf << qe;
+    }
+}
+
+// The cheapest sequence of passes by a model of their times (ms), fitted on
+// GB300 (wave = 9728 quads, 4 blocks of 16 on each of 152 SMs; four waves' worth of
+// lanes are resident at once).  Both forms last one multiplication's latency as
+// long as a warp has its scheduler to itself, more when two share it, and
+// add up beyond a wave; a sum costs kSumMs per product.
+static double quads_ms(size_t items, size_t wave)
+{
+    const size_t rem = items % wave;
+    return 1.05 * (double)(items / wave) + (rem == 0 ? 0.0 : rem <= 3 * wave / 10 ? 0.76 : 1.05);
+}
+
+static double lanes_ms(size_t items, size_t wave)
+{
+    const size_t rem = items % (4 * wave);
+    return 2.4 * (double)(items / (4 * wave)) + (rem == 0 ? 0.0 : rem <= 2 * wave ? 1.65 : 1.95);
+}
+
+static double stage_ms(size_t butterflies, size_t wave)
+{
+    if (butterflies <= 4 * wave) return lanes_ms(butterflies, wave);
+    return 0.5 + 2.3 * (double)butterflies / (double)(4 * wave);
+}
+
+static std::vector<FftPass> fft_plan(const std::vector<FftJob>& jobs, uint32_t maxlog)
+{
+    constexpr double kSumMs = 0.8e-6, kLaunchMs = 0.02;
+    constexpr uint32_t kMaxQ = 4;
+    constexpr size_t kMaxItems = size_t(1) << 18;    // 50 MB of products
+    const size_t wave = fft_quad_wave();
+    std::vector<double> best(maxlog + 1, 1e300);
+    std::vector<FftPass> via(maxlog + 1);
+    best[0] = 0;
+    for (uint32_t s = 0; s < maxlog; s++) {
+        for (uint32_t q = 1; q <= kMaxQ && s + q <= maxlog; q++) {
+            size_t items, outputs;
+            pass_counts(jobs, s, q, items, outputs);
+            FftPass p;
+            p.s0 = s;
+            p.q = q;
+            double ms = q == 1 ? stage_ms(outputs / 2, wave) : 1e300;
+            if (items <= kMaxItems) {
+                const size_t products = items - (outputs >> q);      // item 0 is a copy
+                const double sums = kLaunchMs * q + kSumMs * (double)outputs * (1u << q);
+                const double quads = quads_ms(products, wave) + sums;
+                const double lanes = lanes_ms(products, wave) + sums;
+                if (std::min(quads, lanes) < ms) {
+                    p.kind = quads <= lanes ? FftPass::kQuads : FftPass::kLanes;
+                    ms = std::min(quads, lanes);
+                }
+            }
+            if (best[s] + ms < best[s + q]) {
+                best[s + q] = best[s] + ms;
+                via[s + q] = p;
+            }
+        }
+    }
+    std::vector<FftPass> plan;
+    for (uint32_t s = maxlog; s > 0; s = via[s].s0) plan.push_back(via[s]);
+    std::reverse(plan.begin(), plan.end());
+    return plan;
 }
 
 // Runs every job of `specs` over the concatenated values in d_values
@@ -254,7 +504,6 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
     std::vector<uint32_t> vpre(count + 1);
     size_t total = 0, glv_total = 0;
     uint32_t maxlog = 0;
-    bool any_scale = false;
     for (size_t i = 0; i < count; i++) {
         const size_t n = specs[i].n;
         uint32_t lg = 0;
@@ -263,85 +512,101 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
         jobs[i].n = (uint32_t)n;
         jobs[i].logn = lg;
         jobs[i].inv_from_fwd = specs[i].inv_from_fwd ? 1 : 0;
-        jobs[i].scaled = specs[i].scale_mont ? 1 : 0;
         jobs[i].glv_off = (uint32_t)glv_total;
         jobs[i].xn = (uint32_t)(specs[i].xn && specs[i].xn < n ? specs[i].xn : n);
-        jobs[i].pad = 0;
+        jobs[i].roots = specs[i].roots_mont;
+        jobs[i].scale = specs[i].scale_mont;
         vpre[i] = (uint32_t)total;
         total += n;
-        glv_total += n + 1;
+        glv_total += n + n / 2 + 1;
         maxlog = lg > maxlog ? lg : maxlog;
-        any_scale |= specs[i].scale_mont != nullptr;
     }
     vpre[count] = (uint32_t)total;
     if (total >= 0x7fffffffu) return cudaErrorInvalidValue;
-    // per-stage (job, prefix) lists
-    std::vector<uint32_t> lst_job, lst_pre, st_off(maxlog + 2), st_cnt(maxlog + 2), st_tot(maxlog + 2);
-    for (uint32_t s = 1; s <= maxlog; s++) {
-        st_off[s] = (uint32_t)lst_job.size();
-        uint32_t acc = 0;
+    std::vector<FftPass> plan = fft_plan(jobs, maxlog);
+    // per-pass lists of (job, first item, first output)
+    std::vector<uint32_t> lst_job, lst_item, lst_out;
+    size_t max_items = 0;
+    bool stages = false;
+    for (FftPass& p : plan) {
+        p.off = (uint32_t)lst_job.size();
         for (size_t i = 0; i < count; i++) {
-            if (jobs[i].logn >= s) {
-                lst_job.push_back((uint32_t)i);
-                lst_pre.push_back(acc);
-                const uint32_t groups = jobs[i].n >> s;
-                acc += (groups < jobs[i].xn ? groups : jobs[i].xn) << (s - 1);
-            }
+            const FftJob& J = jobs[i];
+            if (J.logn <= p.s0) continue;
+            const uint32_t qe = std::min(p.q, J.logn - p.s0);
+            const uint32_t bf = std::min(J.n >> (p.s0 + qe), J.xn) << p.s0;
+            lst_job.push_back((uint32_t)i);
+            lst_item.push_back(p.items);
+            lst_out.push_back(p.outputs);
+            p.items += p.kind == FftPass::kStage ? bf : bf * pass_items(qe);
+            p.outputs += bf << qe;
         }
-        st_cnt[s] = (uint32_t)lst_job.size() - st_off[s];
-        st_tot[s] = acc;
+        p.cnt = (uint32_t)lst_job.size() - p.off;
+        if (p.kind == FftPass::kStage) stages = true;
+        else max_items = std::max(max_items, (size_t)p.items);
     }
-    const size_t meta_words = count * (sizeof(FftJob) / 4) + (count + 1) + 2 * lst_job.size() + 8;
-    jac* tmp = (jac*)W.scratch.get(total * sizeof(jac));
-    uint32_t* glv = (uint32_t*)W.glv.get(glv_total * 32);
+    const size_t meta_words = count * (sizeof(FftJob) / 4) + (count + 1) + 3 * lst_job.size() + 8;
+    xyzz* tmp = (xyzz*)W.scratch.get(total * sizeof(xyzz));
+    xyzz* prod = (xyzz*)W.prod.get(max_items * sizeof(xyzz));
+    uint32_t* glv = (uint32_t*)W.glv.get(stages ? glv_total * 32 : 0);
     uint32_t* meta = (uint32_t*)W.meta.get(meta_words * 4);
     uint32_t* hmeta = (uint32_t*)ctx->h_meta.get(meta_words * 4);
-    if (!tmp || !glv || !meta || !hmeta) return cudaErrorMemoryAllocation;
+    if (!tmp || !prod || !glv || !meta || !hmeta) return cudaErrorMemoryAllocation;
     uint32_t* hp = hmeta;
     std::memcpy(hp, jobs.data(), count * sizeof(FftJob));
     hp += count * (sizeof(FftJob) / 4);
     std::memcpy(hp, vpre.data(), (count + 1) * 4);
     hp += count + 1;
-    if (!lst_job.empty()) {
-        std::memcpy(hp, lst_job.data(), lst_job.size() * 4);
-        std::memcpy(hp + lst_job.size(), lst_pre.data(), lst_pre.size() * 4);
+    for (const std::vector<uint32_t>* l : {&lst_job, &lst_item, &lst_out}) {
+        if (!l->empty()) std::memcpy(hp, l->data(), l->size() * 4);
+        hp += l->size();
     }
     CATMSM_CHECK(cudaMemcpyAsync(meta, hmeta, meta_words * 4, cudaMemcpyHostToDevice, st));
     const FftJob* d_jobs = reinterpret_cast<const FftJob*>(meta);
     const uint32_t* d_vpre = meta + count * (sizeof(FftJob) / 4);
     const uint32_t* d_lst_job = d_vpre + count + 1;
-    const uint32_t* d_lst_pre = d_lst_job + lst_job.size();
+    const uint32_t* d_lst_item = d_lst_job + lst_job.size();
+    const uint32_t* d_lst_out = d_lst_item + lst_job.size();
     // prepared roots per job (jobs sharing a root table share the work only
     // through the L2; preparation is O(n) next to O(n log n) scalar mults)
-    for (size_t i = 0; i < count; i++) {
+    for (size_t i = 0; stages && i < count; i++) {
         k_roots_prepare<<<div_up(jobs[i].n, 256), 256, 0, st>>>(specs[i].roots_mont, jobs[i].n, glv + 8 * (size_t)jobs[i].glv_off);
         if (specs[i].scale_mont)
-            k_roots_prepare<<<1, 32, 0, st>>>(specs[i].scale_mont, 1, glv + 8 * (size_t)(jobs[i].glv_off + jobs[i].n));
+            k_roots_prepare_scaled<<<div_up(jobs[i].n / 2 + 1, 256), 256, 0, st>>>(
+                specs[i].roots_mont, specs[i].scale_mont, jobs[i].n, jobs[i].inv_from_fwd,
+                glv + 8 * (size_t)(jobs[i].glv_off + jobs[i].n));
         g_stats.launches += 1 + (specs[i].scale_mont ? 1 : 0);
     }
-    k_bitrev_multi<<<div_up(total, 256), 256, 0, st>>>((const jac*)d_values, tmp, d_jobs, d_vpre, (uint32_t)count,
+    k_bitrev_multi<<<div_up(total, 128), 128, 0, st>>>((const jac*)d_values, tmp, d_jobs, d_vpre, (uint32_t)count,
                                                        (uint32_t)total);
     g_stats.launches++;
-    const size_t qmax = fft_quad_max();
-    for (uint32_t s = 1; s <= maxlog; s++) {
-        if (st_tot[s] <= qmax)
-            k_fft_stage_multi<true><<<div_up(4 * (size_t)st_tot[s], 64), 64, 0, st>>>(
-                tmp, d_jobs, d_lst_job + st_off[s], d_lst_pre + st_off[s], st_cnt[s], st_tot[s], 1u << s, glv);
+    for (const FftPass& p : plan) {
+        const uint32_t* lj = d_lst_job + p.off;
+        const uint32_t* li = d_lst_item + p.off;
+        if (p.kind == FftPass::kStage) {
+            if (p.items <= 4 * fft_quad_wave())
+                k_fft_stage_multi<4><<<div_up(p.items, 64), 64, 0, st>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
+                                                                         2u << p.s0, glv);
+            else
+                k_fft_stage_multi<6><<<div_up(p.items, 64), 64, 0, st>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
+                                                                         2u << p.s0, glv);
+            g_stats.launches++;
+            continue;
+        }
+        if (p.kind == FftPass::kQuads)
+            k_fft_items<true><<<div_up(4 * (size_t)p.items, 64), 64, 0, st>>>(tmp, prod, d_jobs, lj, li, p.cnt,
+                                                                              p.items, p.s0, p.q);
         else
-            k_fft_stage_multi<false><<<div_up(st_tot[s], 64), 64, 0, st>>>(
-                tmp, d_jobs, d_lst_job + st_off[s], d_lst_pre + st_off[s], st_cnt[s], st_tot[s], 1u << s, glv);
-        g_stats.launches++;
+            k_fft_items<false><<<div_up(p.items, 64), 64, 0, st>>>(tmp, prod, d_jobs, lj, li, p.cnt, p.items, p.s0,
+                                                                   p.q);
+        k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1), 128), 128, 0, st>>>(
+            prod, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q);
+        g_stats.launches += 2;
     }
-    if (any_scale && total <= qmax)
-        k_fft_finish_multi<true><<<div_up(4 * total, 64), 64, 0, st>>>(tmp, d_jobs, d_vpre, (uint32_t)count,
-                                                                       (uint32_t)total, glv, 1);
-    else
-        k_fft_finish_multi<false><<<div_up(total, 64), 64, 0, st>>>(tmp, d_jobs, d_vpre, (uint32_t)count,
-                                                                    (uint32_t)total, glv, any_scale ? 1 : 0);
+    k_fft_finish_multi<<<div_up(total, 64), 64, 0, st>>>(tmp, (jac*)d_values, d_jobs, d_vpre, (uint32_t)count,
+                                                         (uint32_t)total);
     g_stats.launches++;
-    CATMSM_CHECK(cudaGetLastError());
-    CATMSM_CHECK(cudaMemcpyAsync(d_values, tmp, total * sizeof(jac), cudaMemcpyDeviceToDevice, st));
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 
 // single transform: d_values n Jacobian points; d_roots_mont the n

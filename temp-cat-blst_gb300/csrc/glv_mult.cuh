@@ -1,0 +1,513 @@
+// Scalar multiplication of a variable G1 point by a GLV-split scalar
+// k = k1 + lambda k2 (k1, k2 < 2^128): k P = k1 P + k2 phi(P).
+//
+// Both halves walk one chain of ~128 doublings and add multiples of P and of
+// phi(P) from an 8-entry table.  What bounds it: in a full launch the multiply
+// pipe (additions were half of the work), in a small one the chain.  The table is
+// "effective affine": P is read as the affine point (X, Y) of the isomorphic
+// curve y^2 = x^3 + 4 Z^6 (the a = 0 formulas never use the constant), the
+// multiples are built with mixed additions, and their z ratios bring all of
+// them to one common z without an inversion.  The main loop's additions are then
+// mixed (8M + 3S) instead of general Jacobian ones (12M + 4S, about a third more), and the
+// common z is multiplied in once at the end.  Inverting to real affine tables
+// instead cost as much as it saved (a serial chain per thread).
+//
+// Points are XYZZ in and out: the next pass adds them without a square per
+// addition, and the quad form (below) keeps them so throughout.
+#pragma once
+#include "curve.cuh"
+
+namespace catmsm {
+
+// Signed fixed 4-bit windows of a value below 2^128: 33 digits in [-7, 8].
+// Lanes of a warp on different scalars add at the same positions.  Against 5-bit
+// windows: ~61 additions instead of ~50 for a table of 8 entries instead of
+// 16 (seven mixed additions and a rescaling each), the same work in total
+// and half the local memory.
+__device__ __forceinline__ void booth4_128(int8_t* d, const uint32_t* k)
+{
+    uint32_t carry = 0;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        int v = (int)(((k[i >> 3] >> (4 * (i & 7))) & 15u) + carry);
+        carry = v > 8 ? 1u : 0u;
+        d[i] = (int8_t)(v - (int)(carry << 4));
+    }
+    d[32] = (int8_t)carry;
+}
+
+// Width-5 NAF of a value below 2^128 (4 little-endian words): digits d_i in
+// {0, +-1, +-3, ..., +-15} with value = sum_i d_i 2^i and at most one nonzero
+// digit in any five consecutive positions (density ~1/6).  Returns the number
+// of digits, at most 129: subtracting a negative digit can carry the value
+// past 2^128 once, after which every step halves it.
+__device__ __forceinline__ int wnaf5_128(int8_t* d, const uint32_t* k)
+{
+    uint32_t w0 = k[0], w1 = k[1], w2 = k[2], w3 = k[3], w4 = 0;
+    int len = 0;
+#pragma unroll 1
+    for (int i = 0; i < 130 && (w0 | w1 | w2 | w3 | w4); i++) {
+        int v = 0;
+        if (w0 & 1u) {
+            v = (int)(w0 & 31u);
+            if (v > 16) v -= 32;
+            if (v > 0) {
+                w0 -= (uint32_t)v;                   // the low five bits are v: no borrow
+            } else {
+                uint64_t s = (uint64_t)w0 + (uint32_t)(-v);
+                w0 = (uint32_t)s;
+                s = (s >> 32) + w1; w1 = (uint32_t)s;
+                s = (s >> 32) + w2; w2 = (uint32_t)s;
+                s = (s >> 32) + w3; w3 = (uint32_t)s;
+                w4 += (uint32_t)(s >> 32);
+            }
+        }
+        d[i] = (int8_t)v;
+        len = i + 1;
+        w0 = (w0 >> 1) | (w1 << 31);
+        w1 = (w1 >> 1) | (w2 << 31);
+        w2 = (w2 >> 1) | (w3 << 31);
+        w3 = (w3 >> 1) | (w4 << 31);
+        w4 >>= 1;
+    }
+    return len;
+}
+
+// p += (ax, ay), Jacobian + affine (madd with the a = 0 special cases)
+__device__ __forceinline__ void jac_madd(jac& p, const fp& ax, const fp& ay)
+{
+    if (jac_is_inf(p)) {
+        p.x = ax; p.y = ay;
+        fp_set_one(p.z);
+        return;
+    }
+    fp zz, h, r, t;
+    fp_sqr(zz, p.z);
+    fp_mul(h, ax, zz);
+    fp_sub(h, h, p.x);
+    fp_mul(zz, zz, p.z);
+    fp_mul(r, ay, zz);
+    fp_sub(r, r, p.y);
+    if (fp_is_zero(h)) {
+        if (fp_is_zero(r)) jac_dbl(p);
+        else jac_set_inf(p);
+        return;
+    }
+    fp_mul(p.z, p.z, h);
+    fp_sqr(t, h);
+    fp_mul(zz, p.x, t);           // V = X1 HH
+    fp_mul(t, t, h);              // HHH
+    fp_sqr(h, r);
+    fp_sub(h, h, t);
+    fp_sub(h, h, zz);
+    fp_sub(p.x, h, zz);           // X3 = R^2 - HHH - 2V
+    fp_sub(zz, zz, p.x);
+    fp_neg(t, t);
+    fp_mul2(p.y, zz, r, p.y, t);  // Y3 = R (V - X3) - Y1 HHH, one reduction
+}
+
+// Eight multiples of the point with Jacobian x, y (z read as 1) on a common z:
+// (tx[i], ty[i]) = (2i + 1) P (Odd) or (i + 1) P, and bx[i] = beta tx[i], the x
+// of phi.  zg: the common z, zero if a multiple met an exceptional case (a
+// point of small order).
+template <bool Odd>
+__device__ __forceinline__ void glv_table(fp* tx, fp* ty, fp* bx, fp& zg, const fp& X, const fp& Y)
+{
+    fp rat[8];                    // z of entry i over z of entry i - 1
+    fp ax, ay, z, V, W, S, M, t;
+    // 2 (X, Y) as xyzz_dbl_affine: zz = U^2, z = U = 2Y
+    fp_dbl(z, Y);
+    fp_sqr(V, z);
+    fp_mul(W, V, z);
+    fp_mul(S, X, V);
+    fp_sqr(M, X);
+    fp_dbl(t, M);
+    fp_add(M, t, M);
+    fp_sqr(t, M);
+    fp_sub(t, t, S);
+    fp_sub(t, t, S);              // x of 2P
+    fp_sub(V, S, t);
+    fp_mul(M, M, V);
+    fp_mul(W, W, Y);
+    fp_sub(M, M, W);              // y of 2P
+    zg = z;
+    fp x, y;
+    int i0;
+    if (Odd) {
+        // on the curve scaled by U, 2P is affine and P = (X U^2, Y U^3)
+        ax = t; ay = M;
+        x = S; y = W;
+        fp_set_one(z);
+        i0 = 1;
+    } else {
+        ax = X; ay = Y;
+        tx[0] = X; ty[0] = Y;
+        rat[1] = z;
+        x = t; y = M;
+        i0 = 2;
+    }
+    tx[i0 - 1] = x; ty[i0 - 1] = y;
+#pragma unroll 1
+    for (int i = i0; i < 8; i++) {
+        fp zz, h, r;
+        fp_sqr(zz, z);
+        fp_mul(h, ax, zz);
+        fp_sub(h, h, x);
+        fp_mul(zz, zz, z);
+        fp_mul(r, ay, zz);
+        fp_sub(r, r, y);
+        fp_mul(z, z, h);
+        rat[i] = h;
+        fp_sqr(t, h);
+        fp_mul(zz, x, t);
+        fp_mul(t, t, h);
+        fp_sqr(h, r);
+        fp_sub(h, h, t);
+        fp_sub(h, h, zz);
+        fp_sub(x, h, zz);
+        fp_sub(zz, zz, x);
+        fp_neg(t, t);
+        fp_mul2(y, zz, r, y, t);
+        tx[i] = x; ty[i] = y;
+    }
+    fp beta;
+#pragma unroll
+    for (int k = 0; k < 12; k++) beta.v[k] = FP_BETA[k];
+    fp_mul(bx[7], tx[7], beta);
+    fp s = rat[7];
+#pragma unroll 1
+    for (int i = 6; i >= 0; i--) {
+        if (i < 6) fp_mul(s, s, rat[i + 1]);
+        fp s2;
+        fp_sqr(s2, s);
+        fp_mul(t, tx[i], s2);
+        tx[i] = t;
+        fp_mul(bx[i], t, beta);
+        fp_mul(s2, s2, s);
+        fp_mul(ty[i], ty[i], s2);
+    }
+    if (Odd) fp_mul(zg, zg, s);
+    else zg = s;
+}
+
+// k1 P + k2 phi(P) by double and add with the complete additions: points of small
+// order only, whose table has no common z.
+static __device__ __noinline__ void xyzz_mult_plain(xyzz& out, const xyzz& P, const uint32_t* k1, const uint32_t* k2)
+{
+    xyzz Q = P, acc;
+    fp beta;
+#pragma unroll
+    for (int k = 0; k < 12; k++) beta.v[k] = FP_BETA[k];
+    fp_mul(Q.x, Q.x, beta);
+    xyzz_set_inf(acc);
+#pragma unroll 1
+    for (int i = 127; i >= 0; i--) {
+        xyzz_dbl(acc);
+        if ((k1[i >> 5] >> (i & 31)) & 1u) xyzz_add(acc, P);
+        if ((k2[i >> 5] >> (i & 31)) & 1u) xyzz_add(acc, Q);
+    }
+    out = acc;
+}
+
+// acc on the table's curve -> out with P's own z and the table's common z
+__device__ __forceinline__ void glv_finish(xyzz& out, const jac& acc, const fp& zg, const xyzz& P)
+{
+    if (jac_is_inf(acc)) {
+        xyzz_set_inf(out);
+        return;
+    }
+    fp z, zz;
+    fp_mul(z, acc.z, zg);
+    fp_sqr(zz, z);
+    fp_mul(z, zz, z);
+    const fp pzz = P.zz, pzzz = P.zzz;
+    out.x = acc.x;
+    out.y = acc.y;
+    fp_mul(out.zz, zz, pzz);
+    fp_mul(out.zzz, z, pzzz);
+}
+
+// Lanes with scalars of their own: fixed windows.
+static __device__ __noinline__ void xyzz_mult_glv(xyzz& out, const xyzz& P, const uint32_t* k1, const uint32_t* k2)
+{
+    if (xyzz_is_inf(P)) {
+        xyzz_set_inf(out);
+        return;
+    }
+    fp tx[8], ty[8], bx[8], zg;
+    glv_table<false>(tx, ty, bx, zg, P.x, P.y);
+    if (fp_is_zero(zg)) {
+        xyzz_mult_plain(out, P, k1, k2);
+        return;
+    }
+    int8_t d1[33], d2[33];
+    booth4_128(d1, k1);
+    booth4_128(d2, k2);
+    jac acc;
+    jac_set_inf(acc);
+#pragma unroll 1
+    for (int i = 32; i >= 0; i--) {
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) jac_dbl(acc);
+#pragma unroll 1
+        for (int hh = 0; hh < 2; hh++) {
+            const int a = hh ? d2[i] : d1[i];
+            if (a) {
+                const int e = (a > 0 ? a : -a) - 1;
+                fp y = ty[e];
+                if (a < 0) fp_neg(y, y);
+                jac_madd(acc, hh ? bx[e] : tx[e], y);
+            }
+        }
+    }
+    glv_finish(out, acc, zg, P);
+}
+
+// Lanes that all multiply by one scalar: width-5 NAF halves over the odd
+// multiples (~43 additions against ~61); the digit positions depend on the scalar.
+static __device__ __noinline__ void xyzz_mult_glv_shared(xyzz& out, const xyzz& P, const uint32_t* k1,
+                                                         const uint32_t* k2)
+{
+    if (xyzz_is_inf(P)) {
+        xyzz_set_inf(out);
+        return;
+    }
+    fp tx[8], ty[8], bx[8], zg;
+    glv_table<true>(tx, ty, bx, zg, P.x, P.y);
+    if (fp_is_zero(zg)) {
+        xyzz_mult_plain(out, P, k1, k2);
+        return;
+    }
+    int8_t d1[130], d2[130];
+    const int n1 = wnaf5_128(d1, k1), n2 = wnaf5_128(d2, k2);
+    jac acc;
+    jac_set_inf(acc);
+#pragma unroll 1
+    for (int i = max(n1, n2) - 1; i >= 0; i--) {
+        jac_dbl(acc);
+#pragma unroll 1
+        for (int hh = 0; hh < 2; hh++) {
+            const int a = hh ? (i < n2 ? d2[i] : 0) : (i < n1 ? d1[i] : 0);
+            if (a) {
+                const int e = (a > 0 ? a : -a) >> 1;
+                fp y = ty[e];
+                if (a < 0) fp_neg(y, y);
+                jac_madd(acc, hh ? bx[e] : tx[e], y);
+            }
+        }
+    }
+    glv_finish(out, acc, zg, P);
+}
+
+// ---------------------------------------------------------------------------
+// The quad form: four lanes on one multiplication (see the quad point
+// operations), for launches whose time is the chain of one of them.  XYZZ
+// throughout: a doubling is 3 dependent products and a mixed addition 4.  zz
+// lives in lane 2 and zzz in lane 3 only, the lanes that multiply them, so
+// neither is ever exchanged and most operands are the same expression in
+// several lanes: an operation broadcasts 7 or 8 products where the general quad
+// operations broadcast 9 or 10, and picks operands with a third of the selects.  The
+// table lives in shared memory, one copy per quad.
+struct quad_table {
+    fp x[8], y[8], bx[8], ny[8];  // ny: -y; while the table is built, the z ratios and their suffix products
+};
+
+struct quad_acc {
+    fp x, y;    // every lane
+    fp z;       // lane 2: zz, lane 3: zzz (other lanes: unused)
+    bool inf;
+};
+
+// m ? b : a, word by word (m all ones or zero)
+__device__ __forceinline__ fp fp_sel(const fp& a, const fp& b, uint32_t m)
+{
+    fp r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = (a.v[i] & ~m) | (b.v[i] & m);
+    return r;
+}
+
+// dbl-2008-s: U^2, X^2 | U V, X V, ZZ V, M^2 | M (S - X3), Y W, -, ZZZ W
+__device__ __forceinline__ void qacc_dbl(quad_acc& p, const quad_lane& q)
+{
+    const uint32_t odd = 0u - (q.k & 1u), l2 = 0u - (q.k == 2), l3 = 0u - (q.k == 3);
+    fp U, M, t, r;
+    fp_dbl(U, p.y);
+    t = fp_sel(U, p.x, odd);
+    r = fp_mul_call(t, t);
+    const fp V = fp_bcast(r, 0, q);
+    M = fp_bcast(r, 1, q);
+    fp_dbl(t, M);
+    fp_add(M, t, M);
+    r = fp_mul_call(fp_sel(fp_sel(fp_sel(U, p.x, odd), p.z, l2), M, l3), fp_sel(V, M, l3));
+    p.z = fp_sel(p.z, r, l2);
+    const fp W = fp_bcast(r, 0, q), S = fp_bcast(r, 1, q);
+    t = fp_bcast(r, 3, q);
+    fp_sub(t, t, S);
+    fp_sub(p.x, t, S);
+    fp_sub(t, S, p.x);
+    r = fp_mul_call(fp_sel(fp_sel(M, p.y, odd), p.z, l3), fp_sel(t, W, odd));
+    p.z = fp_sel(p.z, r, l3);
+    const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
+    fp_sub(p.y, a, b);
+}
+
+// The part of a mixed addition after the differences P = U2 - X1 and R = S2 -
+// Y1: P^2, R^2 | P PP, X1 PP, ZZ PP | R (Q - X3), Y1 PPP, -, ZZZ PPP
+__device__ __forceinline__ void qacc_madd_core(quad_acc& p, const fp& P, const fp& R, const quad_lane& q)
+{
+    const uint32_t odd = 0u - (q.k & 1u), l2 = 0u - (q.k == 2), l3 = 0u - (q.k == 3);
+    fp t = fp_sel(P, R, odd);
+    fp r = fp_mul_call(t, t);
+    const fp PP = fp_bcast(r, 0, q), RR = fp_bcast(r, 1, q);
+    r = fp_mul_call(fp_sel(fp_sel(P, p.x, odd), p.z, l2), PP);
+    p.z = fp_sel(p.z, r, l2);
+    const fp PPP = fp_bcast(r, 0, q), Q = fp_bcast(r, 1, q);
+    fp_sub(t, RR, PPP);
+    fp_sub(t, t, Q);
+    fp_sub(p.x, t, Q);
+    fp_sub(t, Q, p.x);
+    r = fp_mul_call(fp_sel(fp_sel(R, p.y, odd), p.z, l3), fp_sel(t, PPP, odd));
+    p.z = fp_sel(p.z, r, l3);
+    const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
+    fp_sub(p.y, a, b);
+}
+
+// The differences of (ax, ay) and p: lanes 2 and 3 multiply by zz and zzz.
+__device__ __forceinline__ void qacc_diff(fp& P, fp& R, const quad_acc& p, const fp& ax, const fp& ay,
+                                          const quad_lane& q)
+{
+    const fp r = fp_mul_call(fp_sel(ax, ay, 0u - (q.k & 1u)), p.z);
+    P = fp_bcast(r, 2, q);
+    R = fp_bcast(r, 3, q);
+    fp_sub(P, P, p.x);
+    fp_sub(R, R, p.y);
+}
+
+__device__ __forceinline__ void qacc_set(quad_acc& p, const fp& ax, const fp& ay)
+{
+    p.x = ax;
+    p.y = ay;
+    fp_set_one(p.z);
+    p.inf = false;
+}
+
+__device__ __forceinline__ void qacc_madd(quad_acc& p, const fp& ax, const fp& ay, const quad_lane& q)
+{
+    if (p.inf) {
+        qacc_set(p, ax, ay);
+        return;
+    }
+    fp P, R;
+    qacc_diff(P, R, p, ax, ay, q);
+    if (fp_is_zero(P)) {
+        if (fp_is_zero(R)) qacc_dbl(p, q);
+        else p.inf = true;
+        return;
+    }
+    qacc_madd_core(p, P, R, q);
+}
+
+// Every lane of the quad passes the same point and scalar and ends with the product.
+static __device__ __noinline__ void xyzz_mult_glv_quad(xyzz& out, const xyzz& P, const uint32_t* k1,
+                                                       const uint32_t* k2, quad_table* tab, const quad_lane q)
+{
+    if (xyzz_is_inf(P)) {
+        xyzz_set_inf(out);
+        return;
+    }
+    // multiples 1 .. 8 of the affine (X, Y), z ratios to tab->ny
+    quad_acc c;
+    qacc_set(c, P.x, P.y);
+    fp h;
+    fp_dbl(h, P.y);               // z of 2 (X, Y)
+    qacc_dbl(c, q);
+    if (q.k == 0) {
+        tab->x[0] = P.x; tab->y[0] = P.y;
+        tab->x[1] = c.x; tab->y[1] = c.y;
+        tab->ny[1] = h;
+    }
+#pragma unroll 1
+    for (int i = 2; i < 8; i++) {
+        fp R;
+        qacc_diff(h, R, c, P.x, P.y, q);
+        qacc_madd_core(c, h, R, q);
+        if (q.k == 0) {
+            tab->x[i] = c.x; tab->y[i] = c.y;
+            tab->ny[i] = h;
+        }
+    }
+    __syncwarp(q.mask);
+    if (fp_is_zero(fp_bcast(c.z, 2, q))) {       // zz of 8 P: zero if any ratio is
+        xyzz_mult_plain(out, P, k1, k2);
+        return;
+    }
+    // suffix products: ny[i] = product of the ratios i + 1 .. 7 (i < 7)
+    fp s = tab->ny[7];
+#pragma unroll 1
+    for (int i = 5; i >= 0; i--) {
+        fp t;
+        fp_mul(t, s, tab->ny[i + 1]);
+        __syncwarp(q.mask);
+        if (q.k == 0) tab->ny[i + 1] = s;
+        s = t;
+    }
+    if (q.k == 0) tab->ny[0] = s;
+    __syncwarp(q.mask);
+    fp beta;
+#pragma unroll
+    for (int k = 0; k < 12; k++) beta.v[k] = FP_BETA[k];
+    // lane k rescales entries k and k + 4 (entry 7 has the common z already)
+#pragma unroll 1
+    for (uint32_t i = q.k; i < 8; i += 4) {
+        fp one;
+        fp_set_one(one);
+        const fp si = i < 7 ? tab->ny[i] : one;
+        fp s2, x;
+        fp_sqr(s2, si);
+        fp_mul(x, tab->x[i], s2);
+        tab->x[i] = x;
+        fp_mul(x, x, beta);
+        tab->bx[i] = x;
+        fp_mul(s2, s2, si);
+        fp_mul(x, tab->y[i], s2);
+        tab->y[i] = x;
+        fp_neg(x, x);
+        tab->ny[i] = x;
+    }
+    __syncwarp(q.mask);
+    int8_t d1[33], d2[33];
+    booth4_128(d1, k1);
+    booth4_128(d2, k2);
+    quad_acc acc;
+    qacc_set(acc, P.x, P.y);
+    acc.inf = true;
+#pragma unroll 1
+    for (int i = 32; i >= 0; i--) {
+        if (!acc.inf) {
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) qacc_dbl(acc, q);
+        }
+#pragma unroll 1
+        for (int hh = 0; hh < 2; hh++) {
+            const int a = hh ? d2[i] : d1[i];
+            if (a) {
+                const int e = (a > 0 ? a : -a) - 1;
+                qacc_madd(acc, hh ? tab->bx[e] : tab->x[e], a > 0 ? tab->y[e] : tab->ny[e], q);
+            }
+        }
+    }
+    if (acc.inf) {
+        xyzz_set_inf(out);
+        return;
+    }
+    // common z of the table (lanes 2 and 3 hold its zz and zzz), then P's own
+    fp r = fp_mul_call(acc.z, c.z);
+    r = fp_mul_call(r, fp_sel(P.zz, P.zzz, 0u - (q.k & 1u)));
+    out.x = acc.x;
+    out.y = acc.y;
+    out.zz = fp_bcast(r, 2, q);
+    out.zzz = fp_bcast(r, 3, q);
+}
+
+}  // namespace catmsm
