@@ -35,7 +35,7 @@ def build(ref=False):
     """Compile liboracle.so (and the reference .so if asked and the reference
     sources are present)."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
-    if ref and os.path.isdir(REFERENCE_DIR):
+    if ref and os.path.isdir(os.path.join(REFERENCE_DIR, "blst")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "-j8", "REF=" + REFERENCE_DIR], check=True)
 
 
