@@ -23,13 +23,12 @@
 // One round is three launches:
 //   forward   each thread walks its pairs from first to last, storing the
 //             running product of the denominators before each pair (its
-//             prefix) and ending with its total; the block multiplies its
-//             threads' totals in a shared-memory tree;
-//   invert    one thread per block inverts the block's product
+//             prefix) and ending with its total; groups of 16 lanes multiply
+//             their totals by shuffles;
+//   invert    one thread per group inverts the group's product
 //             (fp_inv_vartime: tens of microseconds, not Fermat's ~0.45 ms);
-//   backward  the block re-forms the tree, pushes the inverse down to a
-//             per-thread inverse of its total, and each thread walks its
-//             pairs from last to first: inv(d_j) = prefix_j * I, I *= d_j,
+//   backward  a thread's inverse is the group's times the other lanes'
+//             product, and each thread walks its pairs from last to first: inv(d_j) = prefix_j * I, I *= d_j,
 //             then the affine sum.  The same kernel then runs the next
 //             round's forward pass, or, after the last round, folds the
 //             remaining list into the chunk's bucket / head / tail exactly as
@@ -46,6 +45,7 @@
 namespace catmsm {
 
 constexpr int kAffThreads = 128;
+constexpr uint32_t kAffGroup = 16;      // lanes that share an inversion
 // Resident blocks per SM the round kernels are compiled for (register limit
 // 65536 / (128 x this)).
 #ifndef CATMSM_AFF_MIN_BLOCKS
@@ -100,11 +100,13 @@ struct SrcSorted {
     const uint32_t* sorted_key;
     size_t base;
     __device__ __forceinline__ uint32_t key(uint32_t i) const { return sorted_key[base + i]; }
-    __device__ __forceinline__ Row row(uint32_t i) const
+    // the item's token: one load, made a pair or two before the row is needed
+    __device__ __forceinline__ uint32_t token(uint32_t i) const { return sorted_pt[base + i]; }
+    __device__ __forceinline__ Row row_of(uint32_t v) const
     {
-        const uint32_t v = sorted_pt[base + i];
         return Row{reinterpret_cast<const uint4*>(pts + (v & 0x7fffffffu)), (v >> 31) != 0};
     }
+    __device__ __forceinline__ Row row(uint32_t i) const { return row_of(token(i)); }
 };
 
 // A thread's private arrays (lists, pair positions, prefix products) are
@@ -124,10 +126,12 @@ struct SrcList {
     const uint32_t* keys;
     Slots sl;
     __device__ __forceinline__ uint32_t key(uint32_t i) const { return keys[sl.at(i)]; }
-    __device__ __forceinline__ Row row(uint32_t i) const
+    __device__ __forceinline__ uint32_t token(uint32_t i) const { return i; }
+    __device__ __forceinline__ Row row_of(uint32_t i) const
     {
         return Row{reinterpret_cast<const uint4*>(pts + sl.at(i)), false};
     }
+    __device__ __forceinline__ Row row(uint32_t i) const { return row_of(i); }
 };
 
 template <class Src>
@@ -234,19 +238,28 @@ __device__ __forceinline__ fp aff_forward(const Src& src, uint32_t cnt, affine* 
     fp q;
     fp_set_one(q);
     if (np == 0) return q;
+    // pair j: a, b its tokens; an, bn those of pair j + 1; ip2 the position of pair j + 2
     uint32_t ip = pairpos[ps.at(0)] >> 16;
-    Row ra = src.row(ip), rb = src.row(ip + 1);
+    uint32_t a = src.token(ip), b = src.token(ip + 1), an = a, bn = b, ip2 = 0;
+    if (np > 1) {
+        ip = pairpos[ps.at(1)] >> 16;
+        an = src.token(ip);
+        bn = src.token(ip + 1);
+    }
+    if (np > 2) ip2 = pairpos[ps.at(2)] >> 16;
     for (uint32_t j = 0; j < np; j++) {
+        const Row ra = src.row_of(a), rb = src.row_of(b);
         fp x1, x2, d;
         row_x<Src>(ra, x1);
         row_x<Src>(rb, x2);
-        const Row ca = ra, cb = rb;
-        if (j + 1 < np) {
-            ip = pairpos[ps.at(j + 1)] >> 16;
-            ra = src.row(ip);
-            rb = src.row(ip + 1);
+        a = an;
+        b = bn;
+        if (j + 2 < np) {
+            an = src.token(ip2);
+            bn = src.token(ip2 + 1);
         }
-        pair_den<Src>(ca, cb, x1, x2, d);
+        if (j + 3 < np) ip2 = pairpos[ps.at(j + 3)] >> 16;
+        pair_den<Src>(ra, rb, x1, x2, d);
         stg_fp(prefix + ps.at(j), q);
         fp_mul(q, q, d);
     }
@@ -262,24 +275,29 @@ __device__ __forceinline__ void aff_backward(const Src& src, uint32_t np, affine
                                              const uint32_t* pairpos, const fp* prefix, Slots ps, fp I)
 {
     if (np == 0) return;
-    uint32_t pp = pairpos[ps.at(np - 1)];
-    Row ra = src.row(pp >> 16), rb = src.row((pp >> 16) + 1);
+    // pair j: pp its positions, a, b its tokens; pn, an, bn those of pair j - 1
+    uint32_t pp = pairpos[ps.at(np - 1)], pn = 0, an = 0, bn = 0;
+    uint32_t a = src.token(pp >> 16), b = src.token((pp >> 16) + 1);
+    if (np > 1) pn = pairpos[ps.at(np - 2)];
     for (uint32_t j = np; j-- > 0;) {
+        const Row ra = src.row_of(a), rb = src.row_of(b);
         fp x1, y1, x2, y2, d;
         row_x<Src>(ra, x1);
         row_x<Src>(rb, x2);
         row_y<Src>(ra, y1);
         row_y<Src>(rb, y2);
-        const Row ca = ra, cb = rb;
         const uint32_t o = pp & 0xffffu;
         if (j > 0) {
-            pp = pairpos[ps.at(j - 1)];
-            ra = src.row(pp >> 16);
-            rb = src.row((pp >> 16) + 1);
+            an = src.token(pn >> 16);
+            bn = src.token((pn >> 16) + 1);
         }
-        const uint32_t kind = pair_den<Src>(ca, cb, x1, x2, d);
+        const uint32_t kind = pair_den<Src>(ra, rb, x1, x2, d);
         fp inv;
         fp_mul(inv, ldg_fp<true>(prefix + ps.at(j)), I);   // rewritten by the next forward pass
+        pp = pn;
+        if (j > 1) pn = pairpos[ps.at(j - 2)];
+        a = an;
+        b = bn;
         fp_mul(I, I, d);
         affine r;
         if (kind == kPairAdd || kind == kPairDbl) {
@@ -312,41 +330,27 @@ __device__ __forceinline__ void aff_backward(const Src& src, uint32_t np, affine
     }
 }
 
-// Product of the block's leaves in a shared-memory tree nd[1 .. 2T) (leaf of
-// thread i at T + i, node n = nd[2n] * nd[2n + 1]); returns the root.
-__device__ __forceinline__ fp block_product(fp* nd, const fp& leaf)
+// The lanes of a group share one inversion.  Multiplies their totals by a
+// butterfly of shuffles: every lane ends with the group's product (returned) and
+// with the product of the other lanes' totals (`rest`), so that the inverse of
+// the product times `rest` is the inverse of the lane's own total.  7 dependent
+// products for 16 lanes and no barrier; a shared-memory tree over the block's
+// 128 threads, formed again by the next launch, was 28 and held 12 KB of the L1.
+// Groups of 16: twice the inversions of whole warps (one launch of them lasts
+// as long: a warp per scheduler at 2^20 points) and two products fewer.
+__device__ __forceinline__ fp group_product(const fp& total, fp& rest)
 {
-    const uint32_t T = kAffThreads, tid = threadIdx.x;
-    nd[T + tid] = leaf;
-    __syncthreads();
-    for (uint32_t s = T / 2; s > 0; s >>= 1) {
-        if (tid < s) fp_mul(nd[s + tid], nd[2 * (s + tid)], nd[2 * (s + tid) + 1]);
-        __syncthreads();
+    fp p = total;
+#pragma unroll
+    for (uint32_t d = 1; d < kAffGroup; d <<= 1) {
+        fp o;
+#pragma unroll
+        for (int k = 0; k < 12; k++) o.v[k] = __shfl_xor_sync(0xffffffffu, p.v[k], d);
+        if (d == 1) rest = o;
+        else fp_mul(rest, rest, o);
+        fp_mul(p, p, o);
     }
-    return nd[1];
-}
-
-// With the tree of block_product in nd and the root's inverse: each node's
-// inverse times its sibling is the sibling's inverse, top down; returns the
-// inverse of this thread's leaf.
-__device__ __forceinline__ fp block_leaf_inverse(fp* nd, const fp& root_inv)
-{
-    const uint32_t T = kAffThreads, tid = threadIdx.x;
-    if (tid == 0) nd[1] = root_inv;
-    __syncthreads();
-    for (uint32_t s = 1; s < T; s <<= 1) {
-        if (tid < s) {
-            const uint32_t n = s + tid;
-            const fp v = nd[n], a = nd[2 * n], b = nd[2 * n + 1];
-            fp ia, ib;
-            fp_mul(ia, v, b);
-            fp_mul(ib, v, a);
-            nd[2 * n] = ia;
-            nd[2 * n + 1] = ib;
-        }
-        __syncthreads();
-    }
-    return nd[T + tid];
+    return p;
 }
 
 // k_accumulate's fold over the thread's final list: runs of equal keys are
@@ -397,20 +401,27 @@ struct AffArgs {
     uint32_t* meta;               // per thread: pairs | output items << 16 of the round in flight
     uint32_t* pairpos;            // pair j of thread t at j T + t: input position << 16 | output slot
     fp* prefix;                   // pair j of thread t at j T + t: its prefix product
-    fp* ttot;                     // per thread: product of its denominators
-    fp* btot;                     // per block: product of its threads' products, then its inverse
+    fp* rest;                     // per thread: product of the other lanes' denominators in its group
+    fp* gtot;                     // per group: product of its denominators, then its inverse
     xyzz* buckets;
     xyzz* head;
     xyzz* tail;
     uint32_t block0;              // first block of this launch (the rounds run as two halves)
 };
 
+// Ends a forward pass: the thread's total goes into its group's product.
+__device__ __forceinline__ void aff_totals(const AffArgs& A, uint32_t t, const fp& tot)
+{
+    fp rest;
+    const fp g = group_product(tot, rest);
+    stg_fp(A.rest + t, rest);
+    if (t % kAffGroup == 0) stg_fp(A.gtot + t / kAffGroup, g);
+}
+
 // Round 1's forward pass, over the sorted entries.
 __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_first(AffArgs A)
 {
-    __shared__ fp nd[2 * kAffThreads];
-    const uint32_t blk = A.block0 + blockIdx.x;
-    const uint32_t t = blk * blockDim.x + threadIdx.x;
+    const uint32_t t = (A.block0 + blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t E = *A.total_ptr;
     const size_t start = (size_t)t * A.L;
     const uint32_t cnt = start < E ? (uint32_t)min((size_t)A.L, (size_t)E - start) : 0;
@@ -419,20 +430,18 @@ __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_firs
     const Slots sl{t, A.T};
     const fp tot = aff_forward(src, cnt, A.list_pts[0], A.list_key[0], sl, A.pairpos, A.prefix, sl, &np, &co);
     A.meta[t] = np | (co << 16);
-    stg_fp(A.ttot + t, tot);
-    const fp root = block_product(nd, tot);
-    if (threadIdx.x == 0) stg_fp(A.btot + blk, root);
+    aff_totals(A, t, tot);
 }
 
-// One thread per block product: its inverse, in place (one inversion's
+// One thread per group product: its inverse, in place (about one inversion's
 // latency for the whole launch).
-__global__ void k_aff_invert(fp* __restrict__ btot, uint32_t nb)
+__global__ void k_aff_invert(fp* __restrict__ gtot, uint32_t n)
 {
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < nb) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
         fp r;
-        fp_inv_vartime(r, ldg_fp<true>(btot + b));   // overwritten below
-        stg_fp(btot + b, r);
+        fp_inv_vartime(r, ldg_fp<true>(gtot + i));   // overwritten below
+        stg_fp(gtot + i, r);
     }
 }
 
@@ -442,16 +451,15 @@ __global__ void k_aff_invert(fp* __restrict__ btot, uint32_t nb)
 template <bool First, bool Last>
 __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_round(AffArgs A, uint32_t r)
 {
-    __shared__ fp nd[2 * kAffThreads];
-    const uint32_t blk = A.block0 + blockIdx.x;
-    const uint32_t t = blk * blockDim.x + threadIdx.x;
+    const uint32_t t = (A.block0 + blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t E = *A.total_ptr;
     const size_t start = (size_t)t * A.L;
     const Slots sl{t, A.T};
     const uint32_t m = A.meta[t];
     const uint32_t np = m & 0xffffu, co = m >> 16;
-    block_product(nd, ldg_fp<true>(A.ttot + t));                  // both rewritten at the end of this launch
-    const fp I = block_leaf_inverse(nd, ldg_fp<true>(A.btot + blk));
+    fp I;                                                         // both rewritten at the end of this launch
+    fp_mul(I, ldg_fp<true>(A.rest + t), ldg_fp<true>(A.gtot + t / kAffGroup));
+    __syncwarp();                                                 // the group's inverse is read before lane 0 rewrites it
     const uint32_t out = (r - 1) & 1, in = r & 1;
     if (First) {
         const SrcSorted src{A.pts, A.sorted_pt, A.sorted_key, start};
@@ -468,10 +476,7 @@ __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_roun
         const fp tot = aff_forward(list, co, A.list_pts[in], A.list_key[in], sl, A.pairpos, A.prefix, sl, &np2,
                                    &co2);
         A.meta[t] = np2 | (co2 << 16);
-        stg_fp(A.ttot + t, tot);
-        __syncthreads();                      // every leaf inverse of this round is read
-        const fp root = block_product(nd, tot);
-        if (threadIdx.x == 0) stg_fp(A.btot + blk, root);
+        aff_totals(A, t, tot);
     }
 }
 
@@ -523,13 +528,13 @@ cudaError_t msm_accumulate_affine(Ctx* ctx, const void* pts, const uint32_t* sor
     A.meta = (uint32_t*)W.aff_meta.get(threads * 4);
     A.pairpos = (uint32_t*)W.aff_pairpos.get(threads * H * 4);
     A.prefix = (fp*)W.aff_prefix.get(threads * H * sizeof(fp));
-    A.ttot = (fp*)W.aff_ttot.get(threads * sizeof(fp));
-    A.btot = (fp*)W.aff_btot.get((size_t)grid * sizeof(fp));
+    A.rest = (fp*)W.aff_rest.get(threads * sizeof(fp));
+    A.gtot = (fp*)W.aff_gtot.get(threads / kAffGroup * sizeof(fp));
     A.buckets = (xyzz*)buckets;
     A.head = (xyzz*)head;
     A.tail = (xyzz*)tail;
     if (!A.list_pts[0] || !A.list_pts[1] || !A.list_key[0] || !A.list_key[1] || !A.meta || !A.pairpos ||
-        !A.prefix || !A.ttot || !A.btot)
+        !A.prefix || !A.rest || !A.gtot)
         return cudaErrorMemoryAllocation;
     if (!ctx->aff_stream) {
         int prio = 0;
@@ -543,6 +548,7 @@ cudaError_t msm_accumulate_affine(Ctx* ctx, const void* pts, const uint32_t* sor
     const uint32_t blk0[2] = {0, half0};
     cudaStream_t sts[2] = {st, ctx->aff_stream};
     const int halves = nblk[1] ? 2 : 1;
+    constexpr uint32_t kGroups = kAffThreads / kAffGroup;      // per block
     if (halves == 2) {
         CATMSM_CHECK(cudaEventRecord(ctx->aff_fork, st));
         CATMSM_CHECK(cudaStreamWaitEvent(sts[1], ctx->aff_fork, 0));
@@ -554,7 +560,8 @@ cudaError_t msm_accumulate_affine(Ctx* ctx, const void* pts, const uint32_t* sor
     for (uint32_t r = 1; r <= rounds; r++) {
         const bool first = r == 1, last = r == rounds;
         for (int h = 0; h < halves; h++)
-            k_aff_invert<<<div_up(nblk[h], 32), 32, 0, sts[h]>>>(A.btot + blk0[h], nblk[h]);
+            k_aff_invert<<<div_up(nblk[h] * kGroups, 32), 32, 0, sts[h]>>>(A.gtot + (size_t)blk0[h] * kGroups,
+                                                                         nblk[h] * kGroups);
         for (int h = 0; h < halves; h++) {
             A.block0 = blk0[h];
             if (first && last) k_aff_round<true, true><<<nblk[h], kAffThreads, 0, sts[h]>>>(A, r);

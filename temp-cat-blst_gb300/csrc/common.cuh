@@ -95,13 +95,13 @@ struct MsmWork {
     DevBuf points, scalars, digits, ranks, counts, offsets, block_sums, sorted_pt, sorted_key,
         buckets, head, tail, seg, wins, total, status, misc, glv_pts, glv_sc, glv_sign;
     // batch-affine accumulation rounds (bucket_affine.cu)
-    DevBuf aff_pts0, aff_pts1, aff_key0, aff_key1, aff_meta, aff_pairpos, aff_prefix, aff_ttot, aff_btot;
+    DevBuf aff_pts0, aff_pts1, aff_key0, aff_key1, aff_meta, aff_pairpos, aff_prefix, aff_rest, aff_gtot;
     void release()
     {
         for (DevBuf* b : {&points, &scalars, &digits, &ranks, &counts, &offsets, &block_sums, &sorted_pt,
                           &sorted_key, &buckets, &head, &tail, &seg, &wins, &total, &status, &misc, &glv_pts,
                           &glv_sc, &glv_sign, &aff_pts0, &aff_pts1, &aff_key0, &aff_key1, &aff_meta, &aff_pairpos,
-                          &aff_prefix, &aff_ttot, &aff_btot})
+                          &aff_prefix, &aff_rest, &aff_gtot})
             b->release();
     }
 };

@@ -1001,15 +1001,17 @@ static uint32_t accumulate_chunk(size_t nD)
 
 // Batch-affine rounds for nD bucket entries over M buckets.  A round pairs
 // entries of one bucket inside one chunk, so it pays only when buckets hold
-// many entries; each round costs three launches per half and one inversion
-// per block.  Measured on GB300 (accumulate stage, ms, rounds 0 / 2 / 3 / 4):
-// 2^20 points 5.38 / 5.03 / 4.89 / 4.93; 2^22 18.45 / 17.48 / 17.10 / 17.15;
-// 2^18 1.43 / 1.51 / 1.61 / 1.72 (fewer entries per bucket: no gain).
+// many entries; each round costs three launches per half and the latency of one
+// inversion (65 us, partly overlapped with the other half).  Measured on GB300
+// (whole MSM, ms, rounds 0 / 1 / 2 / 3; entries): 2^18 points 2.26 / 2.25 / 2.29 / 2.38
+// (4.2 M); 300007 2.49 / 2.43 / 2.47 / 2.58 (4.8 M); 2^19 3.68 / 3.55 / 3.39 / 3.45
+// (8.4 M); 700001 4.63 / 4.38 / 4.17 / 4.22 (11.2 M); 2^20 6.51 / 6.18 / 5.75 / 5.65
+// (16.8 M); 2^22 22.5 / 22.2 / 20.6 / 20.3 (58.7 M); a fourth round is slower at all.
 uint32_t msm_affine_rounds(size_t nD, size_t M)
 {
     const double per = (double)nD / (double)(M ? M : 1);
-    if (nD < (size_t(1) << 24) || per < 16) return 0;
-    return 3;
+    if (nD < (size_t(1) << 22) || per < 16) return 0;
+    return nD < 7 * (size_t(1) << 20) ? 1 : nD < (size_t(1) << 24) ? 2 : 3;
 }
 
 static bool use_glv(const Ctx* ctx, size_t n, uint32_t nbits)
