@@ -42,6 +42,8 @@
 #include "fpinv.cuh"
 #include "catmsm_internal.h"
 
+#include <algorithm>
+
 namespace catmsm {
 
 constexpr int kAffThreads = 128;
@@ -395,7 +397,7 @@ struct AffArgs {
     const uint32_t* sorted_key;
     const uint32_t* total_ptr;    // E, the number of sorted entries
     uint32_t L, H;                // chunk length, pair slots per thread (ceil(L / 2))
-    size_t T;                     // threads of the whole grid (both halves): the slot-major stride
+    size_t T;                     // threads of a slice: the slot-major stride
     affine* list_pts[2];          // per-thread lists: slot i of thread t at i T + t
     uint32_t* list_key[2];
     uint32_t* meta;               // per thread: pairs | output items << 16 of the round in flight
@@ -406,8 +408,21 @@ struct AffArgs {
     xyzz* buckets;
     xyzz* head;
     xyzz* tail;
-    uint32_t block0;              // first block of this launch (the rounds run as two halves)
+    uint32_t slice, slices;       // this slice's block b holds the chunks of block b slices + slice
 };
+
+// Whether no chunk of the slice's block b holds an entry (a batch's launches
+// cover full MSMs, whatever the batch holds).
+__device__ __forceinline__ bool aff_idle(const AffArgs& A, uint32_t b, uint32_t E)
+{
+    return ((size_t)b * A.slices + A.slice) * kAffThreads * A.L >= E;
+}
+
+// The chunk of this thread.
+__device__ __forceinline__ uint32_t aff_chunk(const AffArgs& A)
+{
+    return (blockIdx.x * A.slices + A.slice) * kAffThreads + threadIdx.x;
+}
 
 // Ends a forward pass: the thread's total goes into its group's product.
 __device__ __forceinline__ void aff_totals(const AffArgs& A, uint32_t t, const fp& tot)
@@ -421,9 +436,10 @@ __device__ __forceinline__ void aff_totals(const AffArgs& A, uint32_t t, const f
 // Round 1's forward pass, over the sorted entries.
 __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_first(AffArgs A)
 {
-    const uint32_t t = (A.block0 + blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t E = *A.total_ptr;
-    const size_t start = (size_t)t * A.L;
+    if (aff_idle(A, blockIdx.x, E)) return;
+    const size_t start = (size_t)aff_chunk(A) * A.L;
     const uint32_t cnt = start < E ? (uint32_t)min((size_t)A.L, (size_t)E - start) : 0;
     const SrcSorted src{A.pts, A.sorted_pt, A.sorted_key, start};
     uint32_t np = 0, co = 0;
@@ -435,14 +451,13 @@ __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_firs
 
 // One thread per group product: its inverse, in place (about one inversion's
 // latency for the whole launch).
-__global__ void k_aff_invert(fp* __restrict__ gtot, uint32_t n)
+__global__ void k_aff_invert(AffArgs A, uint32_t n)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        fp r;
-        fp_inv_vartime(r, ldg_fp<true>(gtot + i));   // overwritten below
-        stg_fp(gtot + i, r);
-    }
+    if (i >= n || aff_idle(A, i / (kAffThreads / kAffGroup), *A.total_ptr)) return;
+    fp r;
+    fp_inv_vartime(r, ldg_fp<true>(A.gtot + i));     // overwritten below
+    stg_fp(A.gtot + i, r);
 }
 
 // Backward pass of round r (inputs: the sorted entries if First, else list
@@ -451,9 +466,10 @@ __global__ void k_aff_invert(fp* __restrict__ gtot, uint32_t n)
 template <bool First, bool Last>
 __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_round(AffArgs A, uint32_t r)
 {
-    const uint32_t t = (A.block0 + blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t E = *A.total_ptr;
-    const size_t start = (size_t)t * A.L;
+    if (aff_idle(A, blockIdx.x, E)) return;
+    const size_t start = (size_t)aff_chunk(A) * A.L;
     const Slots sl{t, A.T};
     const uint32_t m = A.meta[t];
     const uint32_t np = m & 0xffffu, co = m >> 16;
@@ -470,7 +486,7 @@ __global__ void __launch_bounds__(kAffThreads, CATMSM_AFF_MIN_BLOCKS) k_aff_roun
     }
     const SrcList list{A.list_pts[out], A.list_key[out], sl};
     if (Last) {
-        aff_fold(list, co, A.sorted_key, start, E, A.L, t, A.buckets, A.head, A.tail);
+        aff_fold(list, co, A.sorted_key, start, E, A.L, aff_chunk(A), A.buckets, A.head, A.tail);
     } else {
         uint32_t np2 = 0, co2 = 0;
         const fp tot = aff_forward(list, co, A.list_pts[in], A.list_key[in], sl, A.pairpos, A.prefix, sl, &np2,
@@ -497,85 +513,113 @@ cudaError_t fp_inv_test_device(Ctx* ctx, const uint64_t* d_a, uint64_t* d_out, s
     return cudaGetLastError();
 }
 
-// Rounds of batch-affine additions over the sorted entries, then the fold
-// into the chunk's bucket / head / tail (the output contract of
-// k_accumulate: the fixup stage joins chunk carries unchanged).  rounds >= 1.
-// The blocks run as two independent halves, the first on st and the second
-// on the context's second stream: an inversion launch (one inversion's
-// latency, a few SMs busy) of one half overlaps the other half's round
-// kernel instead of idling the GPU.
-cudaError_t msm_accumulate_affine(Ctx* ctx, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
-                                  const uint32_t* total, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
-                                  void* head, void* tail, cudaStream_t st)
+// The chunks run in slices of blocks, alternating between the pipeline's stream
+// and the workspace's second one: an inversion launch (one inversion's latency,
+// few warps) of one slice overlaps the other stream's round kernel instead of
+// idling the GPU.  At most four waves and 2^25 entries a slice (~8 GB of lists
+// and prefix products per stream), an even number of slices.  A slice takes every
+// count-th block, so all have the same share of the entries however few of
+// the chunks a batch fills.  (Two waves a slice: 2^22 points 20.3 -> 20.5 ms.)
+struct AffSlices {
+    uint32_t count, blocks;     // slices, most blocks of one
+};
+
+static AffSlices aff_slices(uint32_t L, uint32_t grid)
+{
+    if (grid <= 1) return {1, 1};
+    const uint32_t waves = 4 * CATMSM_AFF_MIN_BLOCKS * (uint32_t)device_sms();
+    const uint32_t most = std::max(1u, std::min(waves, (1u << 25) / (kAffThreads * L)));
+    const uint32_t n = 2 * ((grid + 2 * most - 1) / (2 * most));
+    return {n, (grid + n - 1) / n};
+}
+
+cudaError_t aff_prepare(AffWork& W, uint32_t L, size_t chunks, cudaStream_t st)
+{
+    if (L == 0 || L > 0xffffu) return cudaErrorInvalidValue;
+    const size_t T = (size_t)aff_slices(L, div_up(chunks, kAffThreads)).blocks * kAffThreads;
+    const size_t H = (L + 1) / 2;
+    for (AffWork::Set& w : W.set) {
+        if (!w.pts0.get(T * L * sizeof(affine)) || !w.pts1.get(T * L * sizeof(affine)) || !w.key0.get(T * L * 4) ||
+            !w.key1.get(T * L * 4) || !w.meta.get(T * 4) || !w.pairpos.get(T * H * 4) ||
+            !w.prefix.get(T * H * sizeof(fp)) || !w.rest.get(T * sizeof(fp)) ||
+            !w.gtot.get(T / kAffGroup * sizeof(fp)))
+            return cudaErrorMemoryAllocation;
+    }
+    if (!W.stream) {
+        int prio = 0;
+        CATMSM_CHECK(cudaStreamGetPriority(st, &prio));     // the second stream runs at the pipeline stream's priority
+        CATMSM_CHECK(cudaStreamCreateWithPriority(&W.stream, cudaStreamNonBlocking, prio));
+    }
+    if (!W.fork) CATMSM_CHECK(cudaEventCreateWithFlags(&W.fork, cudaEventDisableTiming));
+    if (!W.join) CATMSM_CHECK(cudaEventCreateWithFlags(&W.join, cudaEventDisableTiming));
+    return cudaSuccess;
+}
+
+cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
+                           const uint32_t* total, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
+                           void* head, void* tail, cudaStream_t st, int* launches)
 {
     if (rounds == 0 || L == 0 || L > 0xffffu) return cudaErrorInvalidValue;
-    MsmWork& W = ctx->msm;
-    const uint32_t H = (L + 1) / 2;
     const uint32_t grid = div_up(chunks, kAffThreads);
-    const size_t threads = (size_t)grid * kAffThreads;
-    AffArgs A;
-    A.pts = (const affine*)pts;
-    A.sorted_pt = sorted_pt;
-    A.sorted_key = sorted_key;
-    A.total_ptr = total;
-    A.L = L;
-    A.H = H;
-    A.T = threads;
-    A.list_pts[0] = (affine*)W.aff_pts0.get(threads * L * sizeof(affine));
-    A.list_pts[1] = (affine*)W.aff_pts1.get(threads * L * sizeof(affine));
-    A.list_key[0] = (uint32_t*)W.aff_key0.get(threads * L * 4);
-    A.list_key[1] = (uint32_t*)W.aff_key1.get(threads * L * 4);
-    A.meta = (uint32_t*)W.aff_meta.get(threads * 4);
-    A.pairpos = (uint32_t*)W.aff_pairpos.get(threads * H * 4);
-    A.prefix = (fp*)W.aff_prefix.get(threads * H * sizeof(fp));
-    A.rest = (fp*)W.aff_rest.get(threads * sizeof(fp));
-    A.gtot = (fp*)W.aff_gtot.get(threads / kAffGroup * sizeof(fp));
-    A.buckets = (xyzz*)buckets;
-    A.head = (xyzz*)head;
-    A.tail = (xyzz*)tail;
-    if (!A.list_pts[0] || !A.list_pts[1] || !A.list_key[0] || !A.list_key[1] || !A.meta || !A.pairpos ||
-        !A.prefix || !A.rest || !A.gtot)
-        return cudaErrorMemoryAllocation;
-    if (!ctx->aff_stream) {
-        int prio = 0;
-        CATMSM_CHECK(cudaStreamGetPriority(st, &prio));     // the second half runs at the pipeline stream's priority
-        CATMSM_CHECK(cudaStreamCreateWithPriority(&ctx->aff_stream, cudaStreamNonBlocking, prio));
-        CATMSM_CHECK(cudaEventCreateWithFlags(&ctx->aff_fork, cudaEventDisableTiming));
-        CATMSM_CHECK(cudaEventCreateWithFlags(&ctx->aff_join, cudaEventDisableTiming));
-    }
-    const uint32_t half0 = (grid + 1) / 2;
-    const uint32_t nblk[2] = {half0, grid - half0};
-    const uint32_t blk0[2] = {0, half0};
-    cudaStream_t sts[2] = {st, ctx->aff_stream};
-    const int halves = nblk[1] ? 2 : 1;
+    const AffSlices S = aff_slices(L, grid);
     constexpr uint32_t kGroups = kAffThreads / kAffGroup;      // per block
-    if (halves == 2) {
-        CATMSM_CHECK(cudaEventRecord(ctx->aff_fork, st));
-        CATMSM_CHECK(cudaStreamWaitEvent(sts[1], ctx->aff_fork, 0));
+    AffArgs A[2];
+    cudaStream_t sts[2] = {st, W.stream};
+    for (int h = 0; h < 2; h++) {
+        const AffWork::Set& w = W.set[h];
+        A[h].pts = (const affine*)pts;
+        A[h].sorted_pt = sorted_pt;
+        A[h].sorted_key = sorted_key;
+        A[h].total_ptr = total;
+        A[h].L = L;
+        A[h].H = (L + 1) / 2;
+        A[h].T = (size_t)S.blocks * kAffThreads;
+        A[h].list_pts[0] = (affine*)w.pts0.p;
+        A[h].list_pts[1] = (affine*)w.pts1.p;
+        A[h].list_key[0] = (uint32_t*)w.key0.p;
+        A[h].list_key[1] = (uint32_t*)w.key1.p;
+        A[h].meta = (uint32_t*)w.meta.p;
+        A[h].pairpos = (uint32_t*)w.pairpos.p;
+        A[h].prefix = (fp*)w.prefix.p;
+        A[h].rest = (fp*)w.rest.p;
+        A[h].gtot = (fp*)w.gtot.p;
+        A[h].buckets = (xyzz*)buckets;
+        A[h].head = (xyzz*)head;
+        A[h].tail = (xyzz*)tail;
+        A[h].slice = 0;
+        A[h].slices = S.count;
     }
-    for (int h = 0; h < halves; h++) {
-        A.block0 = blk0[h];
-        k_aff_first<<<nblk[h], kAffThreads, 0, sts[h]>>>(A);
+    if (S.count > 1) {
+        CATMSM_CHECK(cudaEventRecord(W.fork, st));
+        CATMSM_CHECK(cudaStreamWaitEvent(W.stream, W.fork, 0));
     }
-    for (uint32_t r = 1; r <= rounds; r++) {
-        const bool first = r == 1, last = r == rounds;
-        for (int h = 0; h < halves; h++)
-            k_aff_invert<<<div_up(nblk[h] * kGroups, 32), 32, 0, sts[h]>>>(A.gtot + (size_t)blk0[h] * kGroups,
-                                                                         nblk[h] * kGroups);
-        for (int h = 0; h < halves; h++) {
-            A.block0 = blk0[h];
-            if (first && last) k_aff_round<true, true><<<nblk[h], kAffThreads, 0, sts[h]>>>(A, r);
-            else if (first) k_aff_round<true, false><<<nblk[h], kAffThreads, 0, sts[h]>>>(A, r);
-            else if (last) k_aff_round<false, true><<<nblk[h], kAffThreads, 0, sts[h]>>>(A, r);
-            else k_aff_round<false, false><<<nblk[h], kAffThreads, 0, sts[h]>>>(A, r);
+    for (uint32_t s0 = 0; s0 < S.count; s0 += 2) {
+        uint32_t nblk[2];
+        for (uint32_t h = 0; h < 2; h++) {
+            A[h].slice = s0 + h;
+            nblk[h] = s0 + h < grid ? (grid - (s0 + h) + S.count - 1) / S.count : 0;
+            if (!nblk[h]) continue;
+            k_aff_first<<<nblk[h], kAffThreads, 0, sts[h]>>>(A[h]);
+            ++*launches;
         }
-        g_stats.launches += 2 * halves;
+        for (uint32_t r = 1; r <= rounds; r++) {
+            const bool first = r == 1, last = r == rounds;
+            for (uint32_t h = 0; h < 2; h++)
+                if (nblk[h]) k_aff_invert<<<div_up(nblk[h] * kGroups, 32), 32, 0, sts[h]>>>(A[h], nblk[h] * kGroups);
+            for (uint32_t h = 0; h < 2; h++) {
+                if (!nblk[h]) continue;
+                if (first && last) k_aff_round<true, true><<<nblk[h], kAffThreads, 0, sts[h]>>>(A[h], r);
+                else if (first) k_aff_round<true, false><<<nblk[h], kAffThreads, 0, sts[h]>>>(A[h], r);
+                else if (last) k_aff_round<false, true><<<nblk[h], kAffThreads, 0, sts[h]>>>(A[h], r);
+                else k_aff_round<false, false><<<nblk[h], kAffThreads, 0, sts[h]>>>(A[h], r);
+                *launches += 2;
+            }
+        }
     }
-    g_stats.launches += halves;
     CATMSM_CHECK(cudaGetLastError());
-    if (halves == 2) {
-        CATMSM_CHECK(cudaEventRecord(ctx->aff_join, sts[1]));
-        CATMSM_CHECK(cudaStreamWaitEvent(st, ctx->aff_join, 0));
+    if (S.count > 1) {
+        CATMSM_CHECK(cudaEventRecord(W.join, W.stream));
+        CATMSM_CHECK(cudaStreamWaitEvent(st, W.join, 0));
     }
     return cudaSuccess;
 }

@@ -28,15 +28,14 @@ static void ctx_destroy(Ctx* c)
     if (cudaSetDevice(c->device) == cudaSuccess) {
         if (c->stream) cudaStreamSynchronize(c->stream);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
-        if (c->aff_stream) cudaStreamSynchronize(c->aff_stream);
+        if (c->msm.aff.stream) cudaStreamSynchronize(c->msm.aff.stream);
         c->msm.release();
         c->fft.release();
         for (PinnedBuf* b : {&c->h_points, &c->h_scalars, &c->h_out, &c->h_values, &c->h_meta}) b->release();
         for (cudaEvent_t e : c->prof.ev)
             if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {c->points_ready, c->aff_fork, c->aff_join})
-            if (e) cudaEventDestroy(e);
-        for (cudaStream_t st : {c->stream, c->copy_stream, c->aff_stream})
+        if (c->points_ready) cudaEventDestroy(c->points_ready);
+        for (cudaStream_t st : {c->stream, c->copy_stream})
             if (st) cudaStreamDestroy(st);
     }
     delete c;

@@ -52,14 +52,17 @@ void fixup_giants(const void* hot_list, const uint32_t* hot_count, const uint32_
 void msm_reduce_pair(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outA, void* outQ,
                      cudaStream_t st);
 
-// Bucket accumulation with `rounds` rounds of batch-affine additions
-// (Montgomery batch inversion per block and round) before the XYZZ fold;
-// same outputs as k_accumulate (buckets / head / tail per chunk of L sorted
-// entries), so the fixup stage is unchanged.
-cudaError_t msm_accumulate_affine(Ctx* ctx, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
-                                  const uint32_t* total, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
-                                  void* head, void* tail, cudaStream_t st);
-// Rounds the plain MSM uses for nD bucket entries over M buckets (0: the
+// Bucket accumulation with `rounds` (>= 1) rounds of batch-affine additions
+// (Montgomery batch inversion) before the XYZZ fold; same outputs as
+// k_accumulate (buckets / head / tail per chunk of L sorted entries), so the
+// fixup stage is unchanged.  aff_prepare sizes W for up to `chunks` chunks
+// (bounded: the chunks run in slices); aff_accumulate only launches, so it can
+// be captured.  *launches is increased by the kernels launched.
+cudaError_t aff_prepare(AffWork& W, uint32_t L, size_t chunks, cudaStream_t st);
+cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
+                           const uint32_t* total, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
+                           void* head, void* tail, cudaStream_t st, int* launches);
+// Rounds to use for nD bucket entries over M buckets (0: the
 // XYZZ-only k_accumulate).
 uint32_t msm_affine_rounds(size_t nD, size_t M);
 

@@ -90,19 +90,40 @@ struct PinnedBuf {
     }
 };
 
+// Workspaces of the batch-affine accumulation (bucket_affine.cu): one set per
+// stream of the two its slices alternate between, and the second stream.
+struct AffWork {
+    struct Set {
+        DevBuf pts0, pts1, key0, key1, meta, pairpos, prefix, rest, gtot;
+    } set[2];
+    cudaStream_t stream = nullptr;                 // forked from and joined to the pipeline's stream
+    cudaEvent_t fork = nullptr, join = nullptr;
+    void release()
+    {
+        for (Set& w : set)
+            for (DevBuf* b : {&w.pts0, &w.pts1, &w.key0, &w.key1, &w.meta, &w.pairpos, &w.prefix, &w.rest, &w.gtot})
+                b->release();
+        for (cudaEvent_t* e : {&fork, &join}) {
+            if (*e) cudaEventDestroy(*e);
+            *e = nullptr;
+        }
+        if (stream) cudaStreamDestroy(stream);
+        stream = nullptr;
+    }
+};
+
 // Device workspaces of one MSM pipeline instance.
 struct MsmWork {
     DevBuf points, scalars, digits, ranks, counts, offsets, block_sums, sorted_pt, sorted_key,
         buckets, head, tail, seg, wins, total, status, misc, glv_pts, glv_sc, glv_sign;
-    // batch-affine accumulation rounds (bucket_affine.cu)
-    DevBuf aff_pts0, aff_pts1, aff_key0, aff_key1, aff_meta, aff_pairpos, aff_prefix, aff_rest, aff_gtot;
+    AffWork aff;
     void release()
     {
         for (DevBuf* b : {&points, &scalars, &digits, &ranks, &counts, &offsets, &block_sums, &sorted_pt,
                           &sorted_key, &buckets, &head, &tail, &seg, &wins, &total, &status, &misc, &glv_pts,
-                          &glv_sc, &glv_sign, &aff_pts0, &aff_pts1, &aff_key0, &aff_key1, &aff_meta, &aff_pairpos,
-                          &aff_prefix, &aff_rest, &aff_gtot})
+                          &glv_sc, &glv_sign})
             b->release();
+        aff.release();
     }
 };
 
@@ -135,9 +156,6 @@ struct Ctx {
     int affine_rounds = -1;   // batch-affine accumulation rounds (-1: by size; catmsm_msm_affine_rounds)
     cudaStream_t copy_stream = nullptr;    // host->device point copies that overlap the scalar stages
     cudaEvent_t points_ready = nullptr;
-    // second half of the batch-affine rounds (bucket_affine.cu), forked from and joined to `stream`
-    cudaStream_t aff_stream = nullptr;
-    cudaEvent_t aff_fork = nullptr, aff_join = nullptr;
 };
 
 // Per-thread context bound to the thread's current device.  A thread's

@@ -1182,10 +1182,11 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     mark(4);
     const uint32_t rounds = tile_window ? 0
                           : ctx->affine_rounds >= 0 ? (uint32_t)ctx->affine_rounds : msm_affine_rounds(nD, M);
-    if (rounds)
-        CATMSM_CHECK(msm_accumulate_affine(ctx, d_points, sorted_pt, sorted_key, total, L, chunks, rounds, buckets,
-                                           head, tail, st));
-    else
+    if (rounds) {
+        CATMSM_CHECK(aff_prepare(W.aff, L, chunks, st));
+        CATMSM_CHECK(aff_accumulate(W.aff, d_points, sorted_pt, sorted_key, total, L, chunks, rounds, buckets, head,
+                                    tail, st, &g_stats.launches));
+    } else
         k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)d_points, sorted_pt, sorted_key, total, L,
                                                           buckets, head, tail);
     mark(5);

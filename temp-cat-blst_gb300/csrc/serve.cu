@@ -132,7 +132,8 @@ size_t msm_mem(const Basis* b, size_t k)
     // a smaller MSM runs over the tables in a batch, or through the plain
     // pipeline alone: the larger of the two
     const size_t D = 256 / basis_window(b) + 1;
-    const size_t table = k * D * 24 + ((size_t)1 << (basis_window(b) - 1)) * 192 * 2 + k * 32 + (1 << 20);
+    // (index/key/rank words and the batch-affine lists of a window's entry: ~256 B)
+    const size_t table = k * D * 256 + ((size_t)1 << (basis_window(b) - 1)) * 192 * 2 + k * 32 + (1 << 20);
     return std::max(plain, table);
 }
 
