@@ -716,14 +716,38 @@ __device__ __forceinline__ bool fp_is_zero_raw(const fp& a)
 
 __device__ __forceinline__ void fp_dbl(fp& r, const fp& a) { fp_add(r, a, a); }
 
-// r = a^e for a public exponent given as 12 little-endian words
+// r = a^e for a public exponent e > 0 given as 12 little-endian words: sliding
+// windows of five bits over the odd powers a, a^3, ..., a^31 (~380 squarings and
+// ~80 multiplications for a 381-bit e; bit by bit it is ~190 multiplications).
+// The exponent is the same for every lane, so the windows do not diverge.
 __device__ __forceinline__ void fp_pow(fp& r, const fp& a, const uint32_t* e)
 {
-    fp acc;
-    fp_set_one(acc);
-    for (int i = 383; i >= 0; i--) {
-        fp_sqr(acc, acc);
-        if ((e[i >> 5] >> (i & 31)) & 1) fp_mul(acc, acc, a);
+    fp T[16], acc;
+    T[0] = a;
+    fp_sqr(acc, a);
+#pragma unroll 1
+    for (int i = 1; i < 16; i++) fp_mul(T[i], T[i - 1], acc);
+    bool started = false;
+    int i = 383;
+    while (i >= 0) {
+        if (!((e[i >> 5] >> (i & 31)) & 1)) {
+            if (started) fp_sqr(acc, acc);
+            i--;
+            continue;
+        }
+        int l = i < 4 ? 0 : i - 4;                    // the window: bits i .. l, l the lowest set bit in reach
+        while (!((e[l >> 5] >> (l & 31)) & 1)) l++;
+        uint32_t w = 0;
+        for (int b = i; b >= l; b--) w = (w << 1) | ((e[b >> 5] >> (b & 31)) & 1);
+        if (started) {
+#pragma unroll 1
+            for (int b = i; b >= l; b--) fp_sqr(acc, acc);
+            fp_mul(acc, acc, T[w >> 1]);
+        } else {
+            acc = T[w >> 1];
+            started = true;
+        }
+        i = l - 1;
     }
     r = acc;
 }
