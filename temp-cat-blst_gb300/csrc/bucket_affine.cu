@@ -37,6 +37,7 @@
 // affine) returns the other operand, x1 = x2 with y1 = y2 doubles
 // (l = 3 x1^2 / 2 y1), x1 = x2 with y1 = -y2 gives infinity; their batch
 // slots use the denominator 1 (or 2 y1 for the doubling).
+#define CATMSM_INLINE_SQR   // see field.cuh
 #include "common.cuh"
 #include "curve.cuh"
 #include "fpinv.cuh"

@@ -28,6 +28,8 @@
 // The inverse's 1/n scale is multiplied into the roots of a job's last pass.
 // Each butterfly is ~1.5k Fp multiplications (~0.9M IMAD) against 768 bytes of
 // traffic, so memory never binds.
+#define CATMSM_INLINE_SQR   // see field.cuh
+#define CATMSM_INLINE_MUL2   // see field.cuh
 #include "common.cuh"
 #include "curve.cuh"
 #include "fr.cuh"

@@ -107,6 +107,7 @@ __device__ __forceinline__ void chain_top(uint32_t* w, const uint32_t* x, uint32
         asm(CATMSM_CHAIN6(CATMSM_FIRST, "mov.u32 %12, 0;", "madc.hi.u32 %11, %18, %19, %11;\n\t")
             : CATMSM_ACC11(w), "+r"(w[11]), "=r"(unused)
             : CATMSM_IN6(x), "r"(b));
+    (void)unused;
 }
 
 // The Montgomery rows: A += m (p_0, p_2, ...) with the carry in its word 12, ...
@@ -128,6 +129,7 @@ __device__ __forceinline__ void mont_top(uint32_t* w, uint32_t m, uint32_t lo_a,
         : CATMSM_ACC11(w), "+r"(w[11]), "=&r"(dropped)
         : "n"(CATMSM_P1), "n"(CATMSM_P3), "n"(CATMSM_P5), "n"(CATMSM_P7), "n"(CATMSM_P9), "n"(CATMSM_P11), "r"(m),
           "r"(lo_a), "r"(lo_b));
+    (void)dropped;
 }
 
 // Row i's reduction: A, B as above.
@@ -203,7 +205,13 @@ __device__ __forceinline__ void fp_mul_impl(fp& r, const fp& a, const fp& b)
 // ~10 copies of ~750 instructions and the accumulation loop outgrows the
 // instruction cache (ncu: ~2 cycles of no_instruction stall per issue); out of
 // line the hot loop is one body plus call sites.  Measured on GB300: the 2^20
-// MSM 9.1 -> 8.0 ms, a 2^14 G1 FFT 39 -> 26 ms.
+// MSM 9.1 -> 8.0 ms, a 2^14 G1 FFT 39 -> 26 ms.  A call costs ~24 moves that the
+// compiler puts on the multiply pipe, so a translation unit may inline the
+// squaring (CATMSM_INLINE_SQR) and the two-product multiplication
+// (CATMSM_INLINE_MUL2), which have few call sites: accumulating mixed additions
+// 2.50 -> 2.45 ms (300007-point MSM without affine rounds), a 2^16 FFT 28.9 ->
+// 28.3.  Inlining the multiplication as well is slower again (2.59, 33.7 ms),
+// and decoding keeps the calls (300000 elements 13.8 -> 15.3 ms inlined).
 static __device__ __noinline__ fp fp_mul_call(const fp a, const fp b)
 {
     fp r;
@@ -531,7 +539,16 @@ static __device__ __noinline__ fp fp_sqr_call(const fp a)
     return r;
 }
 
-__device__ __forceinline__ void fp_sqr(fp& r, const fp& a) { r = fp_sqr_call(a); }
+__device__ __forceinline__ void fp_sqr(fp& r, const fp& a)
+{
+#ifdef CATMSM_INLINE_SQR
+    fp t;
+    fp_sqr_impl(t, a);
+    r = t;
+#else
+    r = fp_sqr_call(a);
+#endif
+}
 
 // r = (a * b + c * d) * 2^-384 mod p; inputs in [0, 2p), output in [0, 2p).
 // The rows of fp_mul_impl with both products added in each row
@@ -568,7 +585,13 @@ static __device__ __noinline__ fp fp_mul2_call(const fp a, const fp b, const fp 
 // r = a * b + c * d (Montgomery), one reduction
 __device__ __forceinline__ void fp_mul2(fp& r, const fp& a, const fp& b, const fp& c, const fp& d)
 {
+#ifdef CATMSM_INLINE_MUL2
+    fp t;
+    fp_mul2_impl(t, a, b, c, d);
+    r = t;
+#else
     r = fp_mul2_call(a, b, c, d);
+#endif
 }
 
 // r = a + b mod 2p (inputs < 2p)

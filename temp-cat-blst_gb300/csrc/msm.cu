@@ -38,6 +38,8 @@
 //                    and the last levels of every window in one launch.
 //   8. host          folds the D window sums: ret = 2^c ret + W_w, top first
 //                    (reference multi_scalar.cpp:913-922), then normalises.
+#define CATMSM_INLINE_SQR   // see field.cuh
+#define CATMSM_INLINE_MUL2   // see field.cuh
 #include "common.cuh"
 #include "curve.cuh"
 #include "fr.cuh"
