@@ -546,14 +546,7 @@ cudaError_t aff_prepare(AffWork& W, uint32_t L, size_t chunks, cudaStream_t st)
             !w.gtot.get(T / kAffGroup * sizeof(fp)))
             return cudaErrorMemoryAllocation;
     }
-    if (!W.stream) {
-        int prio = 0;
-        CATMSM_CHECK(cudaStreamGetPriority(st, &prio));     // the second stream runs at the pipeline stream's priority
-        CATMSM_CHECK(cudaStreamCreateWithPriority(&W.stream, cudaStreamNonBlocking, prio));
-    }
-    if (!W.fork) CATMSM_CHECK(cudaEventCreateWithFlags(&W.fork, cudaEventDisableTiming));
-    if (!W.join) CATMSM_CHECK(cudaEventCreateWithFlags(&W.join, cudaEventDisableTiming));
-    return cudaSuccess;
+    return W.aux.ensure(st);
 }
 
 cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
@@ -565,7 +558,7 @@ cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* so
     const AffSlices S = aff_slices(L, grid);
     constexpr uint32_t kGroups = kAffThreads / kAffGroup;      // per block
     AffArgs A[2];
-    cudaStream_t sts[2] = {st, W.stream};
+    cudaStream_t sts[2] = {st, W.aux.stream};
     for (int h = 0; h < 2; h++) {
         const AffWork::Set& w = W.set[h];
         A[h].pts = (const affine*)pts;
@@ -590,10 +583,7 @@ cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* so
         A[h].slice = 0;
         A[h].slices = S.count;
     }
-    if (S.count > 1) {
-        CATMSM_CHECK(cudaEventRecord(W.fork, st));
-        CATMSM_CHECK(cudaStreamWaitEvent(W.stream, W.fork, 0));
-    }
+    if (S.count > 1) CATMSM_CHECK(W.aux.begin(st));
     for (uint32_t s0 = 0; s0 < S.count; s0 += 2) {
         uint32_t nblk[2];
         for (uint32_t h = 0; h < 2; h++) {
@@ -618,11 +608,7 @@ cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* so
         }
     }
     CATMSM_CHECK(cudaGetLastError());
-    if (S.count > 1) {
-        CATMSM_CHECK(cudaEventRecord(W.join, W.stream));
-        CATMSM_CHECK(cudaStreamWaitEvent(st, W.join, 0));
-    }
-    return cudaSuccess;
+    return S.count > 1 ? W.aux.end(st) : cudaSuccess;
 }
 
 }  // namespace catmsm

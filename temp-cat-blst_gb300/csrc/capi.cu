@@ -28,7 +28,8 @@ static void ctx_destroy(Ctx* c)
     if (cudaSetDevice(c->device) == cudaSuccess) {
         if (c->stream) cudaStreamSynchronize(c->stream);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
-        if (c->msm.aff.stream) cudaStreamSynchronize(c->msm.aff.stream);
+        for (const AuxStream* a : {&c->msm.aff.aux, &c->fft.aux})
+            if (a->stream) cudaStreamSynchronize(a->stream);
         c->msm.release();
         c->fft.release();
         for (PinnedBuf* b : {&c->h_points, &c->h_scalars, &c->h_out, &c->h_values, &c->h_meta}) b->release();

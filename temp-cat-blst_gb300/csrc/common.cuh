@@ -90,25 +90,57 @@ struct PinnedBuf {
     }
 };
 
-// Workspaces of the batch-affine accumulation (bucket_affine.cu): one set per
-// stream of the two its slices alternate between, and the second stream.
-struct AffWork {
-    struct Set {
-        DevBuf pts0, pts1, key0, key1, meta, pairpos, prefix, rest, gtot;
-    } set[2];
-    cudaStream_t stream = nullptr;                 // forked from and joined to the pipeline's stream
+// A second stream of a pipeline, forked from and joined to its own.
+struct AuxStream {
+    cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    // created on first use, at the pipeline stream's priority
+    cudaError_t ensure(cudaStream_t st)
+    {
+        cudaError_t e = cudaSuccess;
+        if (!stream) {
+            int prio = 0;
+            e = cudaStreamGetPriority(st, &prio);
+            if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, prio);
+        }
+        if (e == cudaSuccess && !fork) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        if (e == cudaSuccess && !join) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+        return e;
+    }
+    cudaError_t begin(cudaStream_t st) const
+    {
+        const cudaError_t e = cudaEventRecord(fork, st);
+        return e == cudaSuccess ? cudaStreamWaitEvent(stream, fork, 0) : e;
+    }
+    cudaError_t end(cudaStream_t st) const
+    {
+        const cudaError_t e = cudaEventRecord(join, stream);
+        return e == cudaSuccess ? cudaStreamWaitEvent(st, join, 0) : e;
+    }
     void release()
     {
-        for (Set& w : set)
-            for (DevBuf* b : {&w.pts0, &w.pts1, &w.key0, &w.key1, &w.meta, &w.pairpos, &w.prefix, &w.rest, &w.gtot})
-                b->release();
         for (cudaEvent_t* e : {&fork, &join}) {
             if (*e) cudaEventDestroy(*e);
             *e = nullptr;
         }
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
+    }
+};
+
+// Workspaces of the batch-affine accumulation (bucket_affine.cu): one set per
+// stream of the two its slices alternate between, and the second stream.
+struct AffWork {
+    struct Set {
+        DevBuf pts0, pts1, key0, key1, meta, pairpos, prefix, rest, gtot;
+    } set[2];
+    AuxStream aux;
+    void release()
+    {
+        for (Set& w : set)
+            for (DevBuf* b : {&w.pts0, &w.pts1, &w.key0, &w.key1, &w.meta, &w.pairpos, &w.prefix, &w.rest, &w.gtot})
+                b->release();
+        aux.release();
     }
 };
 
@@ -129,8 +161,10 @@ struct MsmWork {
 
 struct FftWork {
     DevBuf values, roots, glv, scratch, prod, meta;
+    AuxStream aux;
     void release()
     {
+        aux.release();
         for (DevBuf* b : {&values, &roots, &glv, &scratch, &prod, &meta}) b->release();
     }
 };

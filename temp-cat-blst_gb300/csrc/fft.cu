@@ -415,17 +415,19 @@ static size_t fft_quad_wave()
 
 // One pass: levels s0 + 1 .. s0 + q.
 struct FftPass {
-    uint32_t s0 = 0, q = 1;
+    uint32_t s0 = 0, q = 1, group = 0;
     enum { kStage, kQuads, kLanes } kind = kStage;
     uint32_t off = 0, cnt = 0;          // its entries of the job lists
     uint32_t items = 0, outputs = 0;
 };
 
 // Items and outputs of a pass over every job that has its first level.
-static void pass_counts(const std::vector<FftJob>& jobs, uint32_t s0, uint32_t q, size_t& items, size_t& outputs)
+static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uint32_t q, size_t& items,
+                        size_t& outputs)
 {
     items = outputs = 0;
-    for (const FftJob& J : jobs) {
+    for (const FftJob* job : jobs) {
+        const FftJob& J = *job;
         if (J.logn <= s0) continue;
         const uint32_t qe = std::min(q, J.logn - s0);
         const size_t bf = (size_t)std::min(J.n >> (s0 + qe), J.xn) << s0;
@@ -457,24 +459,28 @@ static double stage_ms(size_t butterflies, size_t wave)
     return 0.5 + 2.3 * (double)butterflies / (double)(4 * wave);
 }
 
-static std::vector<FftPass> fft_plan(const std::vector<FftJob>& jobs, uint32_t maxlog)
+// Several levels a pass only where the jobs have the GPU to themselves (solo): next to
+// another group the launches add up, and one level at a time is the least work.
+static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, bool solo)
 {
     constexpr double kSumMs = 0.8e-6, kLaunchMs = 0.02;
     constexpr uint32_t kMaxQ = 4;
     constexpr size_t kMaxItems = size_t(1) << 18;    // 50 MB of products
     const size_t wave = fft_quad_wave();
+    uint32_t maxlog = 0;
+    for (const FftJob* J : jobs) maxlog = std::max(maxlog, J->logn);
     std::vector<double> best(maxlog + 1, 1e300);
     std::vector<FftPass> via(maxlog + 1);
     best[0] = 0;
     for (uint32_t s = 0; s < maxlog; s++) {
-        for (uint32_t q = 1; q <= kMaxQ && s + q <= maxlog; q++) {
+        for (uint32_t q = 1; q <= (solo ? kMaxQ : 1) && s + q <= maxlog; q++) {
             size_t items, outputs;
             pass_counts(jobs, s, q, items, outputs);
             FftPass p;
             p.s0 = s;
             p.q = q;
             double ms = q == 1 ? stage_ms(outputs / 2, wave) : 1e300;
-            if (items <= kMaxItems) {
+            if (solo && items <= kMaxItems) {
                 const size_t products = items - (outputs >> q);      // item 0 is a copy
                 const double sums = kLaunchMs * q + kSumMs * (double)outputs * (1u << q);
                 const double quads = quads_ms(products, wave) + sums;
@@ -505,7 +511,6 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
     std::vector<FftJob> jobs(count);
     std::vector<uint32_t> vpre(count + 1);
     size_t total = 0, glv_total = 0;
-    uint32_t maxlog = 0;
     for (size_t i = 0; i < count; i++) {
         const size_t n = specs[i].n;
         uint32_t lg = 0;
@@ -521,20 +526,42 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
         vpre[i] = (uint32_t)total;
         total += n;
         glv_total += n + n / 2 + 1;
-        maxlog = lg > maxlog ? lg : maxlog;
     }
     vpre[count] = (uint32_t)total;
     if (total >= 0x7fffffffu) return cudaErrorInvalidValue;
-    std::vector<FftPass> plan = fft_plan(jobs, maxlog);
+    // A batch of more than one wave of lanes runs as two groups of jobs on two
+    // streams: a level's last, partly filled wave (46080 butterflies are 1.18
+    // waves) overlaps a level of the other group.  Six transforms of 2^10 ..
+    // 2^16: 55.5 ms as one group, 46.9 as two.
+    const int groups = count > 1 && total / 2 > 4 * fft_quad_wave() ? 2 : 1;
+    std::vector<uint32_t> group(count, 0);
+    std::vector<const FftJob*> members[2];
+    if (groups == 2) {
+        std::vector<uint32_t> order(count);
+        for (size_t i = 0; i < count; i++) order[i] = (uint32_t)i;
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return jobs[a].n > jobs[b].n; });
+        size_t load[2] = {0, 0};
+        for (uint32_t i : order) {
+            group[i] = load[1] < load[0] ? 1 : 0;
+            load[group[i]] += (size_t)jobs[i].n * jobs[i].logn;
+        }
+    }
+    for (size_t i = 0; i < count; i++) members[group[i]].push_back(&jobs[i]);
+    std::vector<FftPass> plan;
+    for (int g = 0; g < groups; g++)
+        for (FftPass p : fft_plan(members[g], groups == 1)) {
+            p.group = (uint32_t)g;
+            plan.push_back(p);
+        }
     // per-pass lists of (job, first item, first output)
     std::vector<uint32_t> lst_job, lst_item, lst_out;
-    size_t max_items = 0;
+    size_t max_items[2] = {0, 0};
     bool stages = false;
     for (FftPass& p : plan) {
         p.off = (uint32_t)lst_job.size();
         for (size_t i = 0; i < count; i++) {
             const FftJob& J = jobs[i];
-            if (J.logn <= p.s0) continue;
+            if (group[i] != p.group || J.logn <= p.s0) continue;
             const uint32_t qe = std::min(p.q, J.logn - p.s0);
             const uint32_t bf = std::min(J.n >> (p.s0 + qe), J.xn) << p.s0;
             lst_job.push_back((uint32_t)i);
@@ -545,15 +572,16 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
         }
         p.cnt = (uint32_t)lst_job.size() - p.off;
         if (p.kind == FftPass::kStage) stages = true;
-        else max_items = std::max(max_items, (size_t)p.items);
+        else max_items[p.group] = std::max(max_items[p.group], (size_t)p.items);
     }
     const size_t meta_words = count * (sizeof(FftJob) / 4) + (count + 1) + 3 * lst_job.size() + 8;
     xyzz* tmp = (xyzz*)W.scratch.get(total * sizeof(xyzz));
-    xyzz* prod = (xyzz*)W.prod.get(max_items * sizeof(xyzz));
+    xyzz* prod = (xyzz*)W.prod.get((max_items[0] + max_items[1]) * sizeof(xyzz));
     uint32_t* glv = (uint32_t*)W.glv.get(stages ? glv_total * 32 : 0);
     uint32_t* meta = (uint32_t*)W.meta.get(meta_words * 4);
     uint32_t* hmeta = (uint32_t*)ctx->h_meta.get(meta_words * 4);
     if (!tmp || !prod || !glv || !meta || !hmeta) return cudaErrorMemoryAllocation;
+    if (groups == 2) CATMSM_CHECK(W.aux.ensure(st));
     uint32_t* hp = hmeta;
     std::memcpy(hp, jobs.data(), count * sizeof(FftJob));
     hp += count * (sizeof(FftJob) / 4);
@@ -582,29 +610,42 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
     k_bitrev_multi<<<div_up(total, 128), 128, 0, st>>>((const jac*)d_values, tmp, d_jobs, d_vpre, (uint32_t)count,
                                                        (uint32_t)total);
     g_stats.launches++;
-    for (const FftPass& p : plan) {
+    if (groups == 2) CATMSM_CHECK(W.aux.begin(st));
+    // launches alternate between the groups, so neither stream waits for the host
+    std::vector<const FftPass*> seq;
+    size_t next[2] = {0, plan.size()};
+    while (next[1] > 0 && plan[next[1] - 1].group == 1) next[1]--;
+    const size_t first1 = next[1];
+    while (next[0] < first1 || next[1] < plan.size()) {
+        if (next[0] < first1) seq.push_back(&plan[next[0]++]);
+        if (next[1] < plan.size()) seq.push_back(&plan[next[1]++]);
+    }
+    for (const FftPass* pass : seq) {
+        const FftPass& p = *pass;
+        cudaStream_t ps = p.group ? W.aux.stream : st;
+        xyzz* pp = prod + (p.group ? max_items[0] : 0);
         const uint32_t* lj = d_lst_job + p.off;
         const uint32_t* li = d_lst_item + p.off;
         if (p.kind == FftPass::kStage) {
             if (p.items <= 4 * fft_quad_wave())
-                k_fft_stage_multi<4><<<div_up(p.items, 64), 64, 0, st>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
+                k_fft_stage_multi<4><<<div_up(p.items, 64), 64, 0, ps>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
                                                                          2u << p.s0, glv);
             else
-                k_fft_stage_multi<6><<<div_up(p.items, 64), 64, 0, st>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
+                k_fft_stage_multi<6><<<div_up(p.items, 64), 64, 0, ps>>>(tmp, d_jobs, lj, li, p.cnt, p.items,
                                                                          2u << p.s0, glv);
             g_stats.launches++;
             continue;
         }
         if (p.kind == FftPass::kQuads)
-            k_fft_items<true><<<div_up(4 * (size_t)p.items, 64), 64, 0, st>>>(tmp, prod, d_jobs, lj, li, p.cnt,
-                                                                              p.items, p.s0, p.q);
+            k_fft_items<true><<<div_up(4 * (size_t)p.items, 64), 64, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items,
+                                                                              p.s0, p.q);
         else
-            k_fft_items<false><<<div_up(p.items, 64), 64, 0, st>>>(tmp, prod, d_jobs, lj, li, p.cnt, p.items, p.s0,
-                                                                   p.q);
-        k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1), 128), 128, 0, st>>>(
-            prod, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q);
+            k_fft_items<false><<<div_up(p.items, 64), 64, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+        k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1), 128), 128, 0, ps>>>(
+            pp, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q);
         g_stats.launches += 2;
     }
+    if (groups == 2) CATMSM_CHECK(W.aux.end(st));
     k_fft_finish_multi<<<div_up(total, 64), 64, 0, st>>>(tmp, (jac*)d_values, d_jobs, d_vpre, (uint32_t)count,
                                                          (uint32_t)total);
     g_stats.launches++;
