@@ -190,16 +190,15 @@ __device__ __forceinline__ void times_abs_z(jac& out, const fp& ax, const fp& ay
     }
 }
 
-// The same by a quad: zz in lane 2, zzz in lane 3.
-__device__ __forceinline__ void times_abs_z_quad(quad_acc& out, const fp& ax, const fp& ay, const quad_lane& q)
+// The same by a quad, distributed; lane k passes coordinate k mod 2.
+__device__ __forceinline__ void qd_times_abs_z(fp& out, const fp& a, const quad_lane& q)
 {
-    qacc_set(out, ax, ay);
+    qd_set_affine(out, a, q);
 #pragma unroll 1
     for (int r = 0; r < 6; r++) {
 #pragma unroll 1
-        for (int i = Z_RUNS[r]; i > 0; i--)
-            if (!out.inf) qacc_dbl(out, q);
-        if (r < 5) qacc_madd(out, ax, ay, q);
+        for (int i = Z_RUNS[r]; i > 0; i--) qd_dbl(out, q);
+        if (r < 5) qd_madd(out, a, q);
     }
 }
 
@@ -233,18 +232,22 @@ __device__ __forceinline__ bool in_subgroup(const affine& a)
 __device__ __forceinline__ bool in_subgroup_quad(const affine& a, const quad_lane& q)
 {
     if (fp_is_zero_raw(a.x) && fp_is_zero_raw(a.y)) return true;
-    quad_acc t0, t1;
-    times_abs_z_quad(t0, a.x, a.y, q);
-    if (t0.inf) return false;
-    times_abs_z_quad(t1, t0.x, t0.y, q);
-    if (t1.inf) return false;
-    const fp z = fp_mul_call(t1.z, t0.z);                   // lanes 2, 3: zz, zzz of z^2 P
+    const bool odd = (q.k & 1) != 0;
+    fp t0, t1;
+    qd_times_abs_z(t0, fp_sel(a.x, a.y, odd), q);
+    if (qd_is_inf(t0, q)) return false;
+    const fp base = fp_swap(t0, 2, q);                      // lanes 2, 3: X, Y
+    qd_times_abs_z(t1, fp_sel(base, t0, q.k < 2), q);
+    if (qd_is_inf(t1, q)) return false;
     fp b2, t;
     load_const(b2, FP_BETA2);
     fp_mul(b2, a.x, b2);
-    t = fp_mul_call(fp_sel(b2, a.y, 0u - (q.k & 1u)), z);   // lane 2: beta^2 x ZZ, lane 3: y ZZZ
-    fp_neg(t1.y, t1.y);
-    return eq_canon(fp_bcast(t, 2, q), t1.x) && eq_canon(fp_bcast(t, 3, q), t1.y);
+    t = fp_mul_call(t1, t0);                                // lanes 2, 3: zz, zzz of z^2 P
+    t = fp_mul_call(fp_sel(b2, a.y, odd), t);               // beta^2 x ZZ, y ZZZ
+    t = fp_swap(t, 2, q);
+    if (q.k == 1) fp_neg(t, t);
+    const bool eq = q.k >= 2 || eq_canon(t, t1);            // X, -Y
+    return quad_flag(eq, 0, q) && quad_flag(eq, 1, q);
 }
 
 // mode 0: uncompress (48-byte elements), 1: deserialize (96), 2: in_g1 only

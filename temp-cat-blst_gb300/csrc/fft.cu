@@ -315,8 +315,11 @@ __global__ void __launch_bounds__(64) k_fft_items(const xyzz* __restrict__ a, xy
         uint32_t kc[8], k12[8];
         fr_from_mont(kc, c);
         fr_glv_split(k12, k12 + 4, kc);
-        if (Quad) xyzz_mult_glv_quad(v, v, k12, k12 + 4, tabs + (threadIdx.x >> 2), ql);
-        else xyzz_mult_glv(v, v, k12, k12 + 4);
+        if (Quad) {
+            qd_store(prod + t, qd_mult_glv(v, k12, k12 + 4, tabs + (threadIdx.x >> 2), ql), ql);
+            return;
+        }
+        xyzz_mult_glv(v, v, k12, k12 + 4);
     }
     if (!Quad || ql.k == 0) store_xyzz(prod + t, v);
 }
@@ -337,8 +340,8 @@ __global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ pr
     const quad_lane ql = quad_of(threadIdx.x & 31);
     const uint32_t qi = (gt & ((1u << lw) - 1)) >> 2;
     uint32_t dst = 0;
-    xyzz acc, v;
-    xyzz_set_inf(acc);
+    fp acc;
+    fp_zero(acc);
     if (valid) {
         const uint32_t e = find_range(lst_out, cnt, o);
         const FftJob J = jobs[lst_job[e]];
@@ -350,22 +353,21 @@ __global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ pr
         const xyzz* p = prod + lst_pre[e] + bf;
         if (2 * qi < (1u << G.q)) {
             const uint32_t m0 = 2 * qi, m1 = m0 + 1;
-            load_xyzz(acc, p + (size_t)item_of(m0, k) * G.bf);
-            load_xyzz(v, p + (size_t)item_of(m1, k) * G.bf);
-            if (__popc(m0 & k) & 1) xyzz_neg(acc);
-            if (__popc(m1 & k) & 1) xyzz_neg(v);
-            xyzz_add_quad(acc, v, ql);
+            acc = qd_load(p + (size_t)item_of(m0, k) * G.bf, ql.k);
+            fp v = qd_load(p + (size_t)item_of(m1, k) * G.bf, ql.k);
+            if ((__popc(m0 & k) & 1) && ql.k == 1) fp_neg(acc, acc);
+            if ((__popc(m1 & k) & 1) && ql.k == 1) fp_neg(v, v);
+            qd_add(acc, v, ql);
         }
     }
     for (uint32_t d = 4; d < (1u << lw); d <<= 1) {
         __syncwarp();
-        const uint32_t* pv = reinterpret_cast<const uint32_t*>(&acc);
-        uint32_t* po = reinterpret_cast<uint32_t*>(&v);
+        fp v;
 #pragma unroll
-        for (int w = 0; w < 48; w++) po[w] = __shfl_down_sync(0xffffffffu, pv[w], d);
-        if (((4 * qi) & (2 * d - 1)) == 0) xyzz_add_quad(acc, v, ql);
+        for (int w = 0; w < 12; w++) v.v[w] = __shfl_down_sync(0xffffffffu, acc.v[w], d);
+        if (((4 * qi) & (2 * d - 1)) == 0) qd_add(acc, v, ql);
     }
-    if (valid && (gt & ((1u << lw) - 1)) == 0) store_xyzz(a + dst, acc);
+    if (valid && qi == 0) qd_store(a + dst, acc, ql);
 }
 
 // Jacobian with canonical coordinates; one-point jobs are scaled here (they

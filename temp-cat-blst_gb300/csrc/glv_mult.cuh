@@ -302,145 +302,52 @@ static __device__ __noinline__ void xyzz_mult_glv_shared(xyzz& out, const xyzz& 
 // ---------------------------------------------------------------------------
 // The quad form: four lanes on one multiplication (see the quad point
 // operations), for launches whose time is the chain of one of them.  XYZZ
-// throughout: a doubling is 3 dependent products and a mixed addition 4.  zz
-// lives in lane 2 and zzz in lane 3 only, the lanes that multiply them, so
-// neither is ever exchanged and most operands are the same expression in
-// several lanes: an operation broadcasts 7 or 8 products where the general quad
-// operations broadcast 9 or 10, and picks operands with a third of the selects.  The
+// throughout: a doubling is 3 dependent products and a mixed addition 4.  The
 // table lives in shared memory, one copy per quad.
 struct quad_table {
     fp x[8], y[8], bx[8], ny[8];  // ny: -y; while the table is built, the z ratios and their suffix products
 };
 
-struct quad_acc {
-    fp x, y;    // every lane
-    fp z;       // lane 2: zz, lane 3: zzz (other lanes: unused)
-    bool inf;
-};
-
-// m ? b : a, word by word (m all ones or zero)
-__device__ __forceinline__ fp fp_sel(const fp& a, const fp& b, uint32_t m)
+// Every lane of the quad passes the same point and scalar and its own
+// coordinate of the point (d = qd_load of it); returns the product, distributed.
+static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1, const uint32_t* k2, quad_table* tab,
+                                              const quad_lane q)
 {
-    fp r;
-#pragma unroll
-    for (int i = 0; i < 12; i++) r.v[i] = (a.v[i] & ~m) | (b.v[i] & m);
-    return r;
-}
-
-// dbl-2008-s: U^2, X^2 | U V, X V, ZZ V, M^2 | M (S - X3), Y W, -, ZZZ W
-__device__ __forceinline__ void qacc_dbl(quad_acc& p, const quad_lane& q)
-{
-    const uint32_t odd = 0u - (q.k & 1u), l2 = 0u - (q.k == 2), l3 = 0u - (q.k == 3);
-    fp U, M, t, r;
-    fp_dbl(U, p.y);
-    t = fp_sel(U, p.x, odd);
-    r = fp_mul_call(t, t);
-    const fp V = fp_bcast(r, 0, q);
-    M = fp_bcast(r, 1, q);
-    fp_dbl(t, M);
-    fp_add(M, t, M);
-    r = fp_mul_call(fp_sel(fp_sel(fp_sel(U, p.x, odd), p.z, l2), M, l3), fp_sel(V, M, l3));
-    p.z = fp_sel(p.z, r, l2);
-    const fp W = fp_bcast(r, 0, q), S = fp_bcast(r, 1, q);
-    t = fp_bcast(r, 3, q);
-    fp_sub(t, t, S);
-    fp_sub(p.x, t, S);
-    fp_sub(t, S, p.x);
-    r = fp_mul_call(fp_sel(fp_sel(M, p.y, odd), p.z, l3), fp_sel(t, W, odd));
-    p.z = fp_sel(p.z, r, l3);
-    const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
-    fp_sub(p.y, a, b);
-}
-
-// The part of a mixed addition after the differences P = U2 - X1 and R = S2 -
-// Y1: P^2, R^2 | P PP, X1 PP, ZZ PP | R (Q - X3), Y1 PPP, -, ZZZ PPP
-__device__ __forceinline__ void qacc_madd_core(quad_acc& p, const fp& P, const fp& R, const quad_lane& q)
-{
-    const uint32_t odd = 0u - (q.k & 1u), l2 = 0u - (q.k == 2), l3 = 0u - (q.k == 3);
-    fp t = fp_sel(P, R, odd);
-    fp r = fp_mul_call(t, t);
-    const fp PP = fp_bcast(r, 0, q), RR = fp_bcast(r, 1, q);
-    r = fp_mul_call(fp_sel(fp_sel(P, p.x, odd), p.z, l2), PP);
-    p.z = fp_sel(p.z, r, l2);
-    const fp PPP = fp_bcast(r, 0, q), Q = fp_bcast(r, 1, q);
-    fp_sub(t, RR, PPP);
-    fp_sub(t, t, Q);
-    fp_sub(p.x, t, Q);
-    fp_sub(t, Q, p.x);
-    r = fp_mul_call(fp_sel(fp_sel(R, p.y, odd), p.z, l3), fp_sel(t, PPP, odd));
-    p.z = fp_sel(p.z, r, l3);
-    const fp a = fp_bcast(r, 0, q), b = fp_bcast(r, 1, q);
-    fp_sub(p.y, a, b);
-}
-
-// The differences of (ax, ay) and p: lanes 2 and 3 multiply by zz and zzz.
-__device__ __forceinline__ void qacc_diff(fp& P, fp& R, const quad_acc& p, const fp& ax, const fp& ay,
-                                          const quad_lane& q)
-{
-    const fp r = fp_mul_call(fp_sel(ax, ay, 0u - (q.k & 1u)), p.z);
-    P = fp_bcast(r, 2, q);
-    R = fp_bcast(r, 3, q);
-    fp_sub(P, P, p.x);
-    fp_sub(R, R, p.y);
-}
-
-__device__ __forceinline__ void qacc_set(quad_acc& p, const fp& ax, const fp& ay)
-{
-    p.x = ax;
-    p.y = ay;
-    fp_set_one(p.z);
-    p.inf = false;
-}
-
-__device__ __forceinline__ void qacc_madd(quad_acc& p, const fp& ax, const fp& ay, const quad_lane& q)
-{
-    if (p.inf) {
-        qacc_set(p, ax, ay);
-        return;
-    }
-    fp P, R;
-    qacc_diff(P, R, p, ax, ay, q);
-    if (fp_is_zero(P)) {
-        if (fp_is_zero(R)) qacc_dbl(p, q);
-        else p.inf = true;
-        return;
-    }
-    qacc_madd_core(p, P, R, q);
-}
-
-// Every lane of the quad passes the same point and scalar and ends with the product.
-static __device__ __noinline__ void xyzz_mult_glv_quad(xyzz& out, const xyzz& P, const uint32_t* k1,
-                                                       const uint32_t* k2, quad_table* tab, const quad_lane q)
-{
-    if (xyzz_is_inf(P)) {
-        xyzz_set_inf(out);
-        return;
-    }
+    fp d;
+    fp_zero(d);
+    if (xyzz_is_inf(P)) return d;
+    const bool odd = (q.k & 1) != 0;
     // multiples 1 .. 8 of the affine (X, Y), z ratios to tab->ny
-    quad_acc c;
-    qacc_set(c, P.x, P.y);
-    fp h;
+    const fp a = fp_sel(P.x, P.y, odd);
+    fp c, h;
+    qd_set_affine(c, a, q);
     fp_dbl(h, P.y);               // z of 2 (X, Y)
-    qacc_dbl(c, q);
+    qd_dbl(c, q);
     if (q.k == 0) {
-        tab->x[0] = P.x; tab->y[0] = P.y;
-        tab->x[1] = c.x; tab->y[1] = c.y;
+        tab->x[0] = a;
+        tab->x[1] = c;
         tab->ny[1] = h;
+    } else if (q.k == 1) {
+        tab->y[0] = a;
+        tab->y[1] = c;
     }
 #pragma unroll 1
     for (int i = 2; i < 8; i++) {
-        fp R;
-        qacc_diff(h, R, c, P.x, P.y, q);
-        qacc_madd_core(c, h, R, q);
+        const fp PR = qd_madd_diff(c, a, q);
+        c = qd_add_core<true>(PR, c, c, c, q);
         if (q.k == 0) {
-            tab->x[i] = c.x; tab->y[i] = c.y;
-            tab->ny[i] = h;
+            tab->x[i] = c;
+            tab->ny[i] = PR;
+        } else if (q.k == 1) {
+            tab->y[i] = c;
         }
     }
     __syncwarp(q.mask);
-    if (fp_is_zero(fp_bcast(c.z, 2, q))) {       // zz of 8 P: zero if any ratio is
+    if (qd_is_inf(c, q)) {        // zz of 8 P: zero if any ratio is
+        xyzz out;
         xyzz_mult_plain(out, P, k1, k2);
-        return;
+        const fp lo = fp_sel(out.x, out.y, odd), hi = fp_sel(out.zz, out.zzz, odd);
+        return fp_sel(lo, hi, q.k >= 2);
     }
     // suffix products: ny[i] = product of the ratios i + 1 .. 7 (i < 7)
     fp s = tab->ny[7];
@@ -479,35 +386,26 @@ static __device__ __noinline__ void xyzz_mult_glv_quad(xyzz& out, const xyzz& P,
     int8_t d1[33], d2[33];
     booth4_128(d1, k1);
     booth4_128(d2, k2);
-    quad_acc acc;
-    qacc_set(acc, P.x, P.y);
-    acc.inf = true;
+    bool started = false;
 #pragma unroll 1
     for (int i = 32; i >= 0; i--) {
-        if (!acc.inf) {
+        if (started) {
 #pragma unroll 1
-            for (int k = 0; k < 4; k++) qacc_dbl(acc, q);
+            for (int k = 0; k < 4; k++) qd_dbl(d, q);
         }
 #pragma unroll 1
         for (int hh = 0; hh < 2; hh++) {
-            const int a = hh ? d2[i] : d1[i];
-            if (a) {
-                const int e = (a > 0 ? a : -a) - 1;
-                qacc_madd(acc, hh ? tab->bx[e] : tab->x[e], a > 0 ? tab->y[e] : tab->ny[e], q);
+            const int g = hh ? d2[i] : d1[i];
+            if (g) {
+                const int e = (g > 0 ? g : -g) - 1;
+                qd_madd(d, odd ? (g > 0 ? tab->y[e] : tab->ny[e]) : (hh ? tab->bx[e] : tab->x[e]), q);
+                started = true;
             }
         }
     }
-    if (acc.inf) {
-        xyzz_set_inf(out);
-        return;
-    }
-    // common z of the table (lanes 2 and 3 hold its zz and zzz), then P's own
-    fp r = fp_mul_call(acc.z, c.z);
-    r = fp_mul_call(r, fp_sel(P.zz, P.zzz, 0u - (q.k & 1u)));
-    out.x = acc.x;
-    out.y = acc.y;
-    out.zz = fp_bcast(r, 2, q);
-    out.zzz = fp_bcast(r, 3, q);
+    // common z of the table (c's zz, zzz), then P's own
+    const fp r = fp_mul_call(fp_mul_call(d, c), fp_sel(P.zz, P.zzz, odd));
+    return fp_sel(d, r, q.k >= 2);
 }
 
 }  // namespace catmsm

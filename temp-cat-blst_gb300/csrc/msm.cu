@@ -418,25 +418,25 @@ __device__ __forceinline__ void shfl_down_xyzz(xyzz& o, const xyzz& v, int d)
 
 // Sum of `span` partials of one bucket by one warp: the warp's eight quads
 // each add every 8th partial with quad point operations, then a tree over the quads as deep as the span needs: a span
-// of s <= 8 costs 1 + ceil(log2 s) quad additions (~10k cycles each against
-// ~26k for one lane's addition).  Lane 0 ends with the sum.
+// of s <= 8 costs 1 + ceil(log2 s) quad additions.  Quad 0 ends with the sum,
+// distributed.
 template <class PartAt>
-__device__ __forceinline__ void warp_join(xyzz& acc, uint32_t span, uint32_t lane, PartAt part_at)
+__device__ __forceinline__ fp warp_join(uint32_t span, uint32_t lane, PartAt part_at)
 {
     const quad_lane ql = quad_of(lane);
     const uint32_t qi = lane >> 2;
-    xyzz part;
-    xyzz_set_inf(acc);
-    for (uint32_t i = qi; i < span; i += 8) {
-        load_xyzz(part, part_at(i));
-        xyzz_add_quad(acc, part, ql);
-    }
+    fp acc;
+    fp_zero(acc);
+    for (uint32_t i = qi; i < span; i += 8) qd_add(acc, qd_load(part_at(i), ql.k), ql);
     const uint32_t width = min(span, 8u);
     for (uint32_t d = 1; d < width; d <<= 1) {
-        xyzz o;
-        shfl_down_xyzz(o, acc, (int)(4 * d));
-        if ((qi & (2 * d - 1)) == 0 && qi + d < width) xyzz_add_quad(acc, o, ql);
+        __syncwarp();
+        fp o;
+#pragma unroll
+        for (int k = 0; k < 12; k++) o.v[k] = __shfl_down_sync(0xffffffffu, acc.v[k], 4 * d);
+        if ((qi & (2 * d - 1)) == 0 && qi + d < width) qd_add(acc, o, ql);
     }
+    return acc;
 }
 
 // The same for a bucket too large for one warp (a narrow top window, one
@@ -483,9 +483,8 @@ __global__ void __launch_bounds__(kHotThreads) k_fixup_hot(uint2* __restrict__ h
         const uint32_t key = e.x, t0 = e.y;
         const uint32_t span = (offsets[key + 1] - 1) / L - t0 + 1;
         if (span > kWarpJoinMax) continue;
-        xyzz acc;
-        warp_join(acc, span, lane, [&](uint32_t i) { return i == 0 ? tail + t0 : head + t0 + i; });
-        if (lane == 0) store_xyzz(buckets + key, acc);
+        const fp acc = warp_join(span, lane, [&](uint32_t i) { return i == 0 ? tail + t0 : head + t0 + i; });
+        if (lane < 4) qd_store(buckets + key, acc, quad_of(lane));
     }
     for (uint32_t h = blockIdx.x; h < nh; h += gridDim.x) {
         const uint2 e = hot_list[h];
@@ -596,9 +595,8 @@ __global__ void __launch_bounds__(kHotThreads) k_fixup_hot_seg(uint2* __restrict
         const uint32_t t1 = (offsets[key + 1] - 1) / L;
         const uint32_t np = 2 + (t1 >> 5) - ((t0 + 1) >> 5);          // tail + pieces
         if (np > kWarpJoinMax) continue;
-        xyzz acc;
-        warp_join(acc, np, lane, [&](uint32_t i) { return piece(t0, i); });
-        if (lane == 0) store_xyzz(buckets + key, acc);
+        const fp acc = warp_join(np, lane, [&](uint32_t i) { return piece(t0, i); });
+        if (lane < 4) qd_store(buckets + key, acc, quad_of(lane));
     }
     for (uint32_t h = blockIdx.x; h < nh; h += gridDim.x) {
         const uint2 e = hot_list[h];
@@ -758,35 +756,35 @@ __global__ void __launch_bounds__(128) k_reduce_level(const xyzz* __restrict__ i
 // doubles A_0.  This is k_reduce_level's rule with fan-in 2.  Quad = true:
 // each of the two is a quad of lanes (quad point operations), for levels
 // too small to fill the GPU.
-template <bool Quad>
-__device__ __forceinline__ void add_op(xyzz& p, const xyzz& o, const quad_lane& q)
-{
-    if (Quad) xyzz_add_quad(p, o, q);
-    else xyzz_add(p, o);
-}
-
-template <bool Quad>
-__device__ __forceinline__ void pair_node(xyzz& out, const xyzz* a, const xyzz* q, uint32_t cnt, bool q_role,
-                                          const quad_lane& ql)
+__device__ __forceinline__ void pair_node(xyzz& out, const xyzz* a, const xyzz* q, uint32_t cnt, bool q_role)
 {
     xyzz b;
     if (q_role) {
         load_xyzz(out, q);
         if (cnt == 2) {
             load_xyzz(b, a + 1);
-            add_op<Quad>(out, b, ql);
+            xyzz_add(out, b);
             load_xyzz(b, q + 1);
-            add_op<Quad>(out, b, ql);
+            xyzz_add(out, b);
         }
     } else {
         load_xyzz(out, a);
         if (cnt == 2) {
             load_xyzz(b, a + 1);
-            add_op<Quad>(out, b, ql);
+            xyzz_add(out, b);
         }
-        if (Quad) xyzz_dbl_quad(out, ql);
-        else xyzz_dbl(out);
+        xyzz_dbl(out);
     }
+}
+
+__device__ __forceinline__ fp pair_node_quad(const xyzz* a, const xyzz* q, uint32_t cnt, bool q_role,
+                                             const quad_lane& ql)
+{
+    fp out = qd_load(q_role ? q : a, ql.k);
+    if (cnt == 2) qd_add(out, qd_load(a + 1, ql.k), ql);
+    if (!q_role) qd_dbl(out, ql);
+    else if (cnt == 2) qd_add(out, qd_load(q + 1, ql.k), ql);
+    return out;
 }
 
 // Thread g's node and role.  The role is uniform per warp (even warps Q, odd
@@ -813,9 +811,15 @@ __global__ void __launch_bounds__(128) k_reduce_pair(const xyzz* __restrict__ in
     const quad_lane ql = quad_of(threadIdx.x & 31);
     const uint32_t w = t / m_out, u = t % m_out;
     const size_t base = (size_t)w * m_in + 2 * u;
-    xyzz r;
-    pair_node<Quad>(r, inA + base, inQ + base, min(2u, m_in - 2 * u), q_role, ql);
-    if (!Quad || ql.k == 0) store_xyzz((q_role ? outQ : outA) + (size_t)w * m_out + u, r);
+    xyzz* dst = (q_role ? outQ : outA) + (size_t)w * m_out + u;
+    const uint32_t cnt = min(2u, m_in - 2 * u);
+    if (Quad) {
+        qd_store(dst, pair_node_quad(inA + base, inQ + base, cnt, q_role, ql), ql);
+    } else {
+        xyzz r;
+        pair_node(r, inA + base, inQ + base, cnt, q_role);
+        store_xyzz(dst, r);
+    }
 }
 
 // The last binary levels in one launch: block w reduces window w's m_in
@@ -846,11 +850,11 @@ __global__ void __launch_bounds__(kTailThreads) k_reduce_tail(const xyzz* __rest
     const xyzz* srcQ = inQ + (size_t)w * m_in;
     while (m > 1) {
         const uint32_t m_out = (m + 1) / 2;
-        xyzz r;
+        fp r;
         const bool act = t < m_out && (q_role || m_out > 1);
-        if (act) pair_node<true>(r, srcA + 2 * t, srcQ + 2 * t, min(2u, m - 2 * t), q_role, ql);
+        if (act) r = pair_node_quad(srcA + 2 * t, srcQ + 2 * t, min(2u, m - 2 * t), q_role, ql);
         __syncthreads();
-        if (act && ql.k == 0) (q_role ? shQ : shA)[t] = r;
+        if (act) qd_store((q_role ? shQ : shA) + t, r, ql);
         __syncthreads();
         srcA = shA;
         srcQ = shQ;
