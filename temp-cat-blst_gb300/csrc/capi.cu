@@ -158,9 +158,12 @@ static void msm_entry(blst_p1* ret, const blst_p1_affine* const points[], size_t
     // Scalars first on the pipeline stream; the points on the copy stream,
     // overlapping the digit, scan and scatter stages (which need only the
     // scalars).  The pipeline waits for points_ready before reading points.
+    // A small MSM needs both at once: one stream.
     cudaError_t err = cudaMemcpyAsync(ds, hs, npoints * nbytes, cudaMemcpyHostToDevice, ctx->stream);
     cudaEvent_t ready = nullptr;
-    if (err == cudaSuccess) err = copy_points_async(ctx, dp, hp, npoints * sizeof(blst_p1_affine), &ready);
+    if (err == cudaSuccess && msm_small_applies(2 * npoints, true))
+        err = cudaMemcpyAsync(dp, hp, npoints * sizeof(blst_p1_affine), cudaMemcpyHostToDevice, ctx->stream);
+    else if (err == cudaSuccess) err = copy_points_async(ctx, dp, hp, npoints * sizeof(blst_p1_affine), &ready);
     if (err == cudaSuccess)
         err = msm_device(ctx, dp, (const uint8_t*)ds, (uint32_t)nbytes, npoints, (uint32_t)nbits, 0, out, ready);
     if (ready) cudaStreamSynchronize(ctx->copy_stream);   // the caller's points are not read after return

@@ -40,6 +40,20 @@ void msm_plan(const Ctx* ctx, size_t n, uint32_t nbits, uint32_t* c, uint32_t* w
 // context.
 cudaError_t msm_setup_device();
 
+// The small MSM (msm_small.cu), for up to a few thousand pipeline points.  Window
+// sums (as the device wrote them) in wins after the stream is synchronised.
+struct SmallMsm {
+    const uint64_t* wins = nullptr;
+    const uint32_t* over = nullptr;     // nonzero: too skewed, nothing computed (run the general pipeline)
+    uint32_t D = 0, c = 0;
+};
+bool msm_small_applies(size_t pipeline_points, bool glv);
+uint32_t msm_small_window(size_t pipeline_points);
+uint32_t msm_small_windows(size_t pipeline_points, uint32_t bits, bool glv);
+cudaError_t msm_small_setup_device();
+cudaError_t msm_small(Ctx* ctx, const void* pts, const uint8_t* scalars, uint32_t stride, size_t n, uint32_t nbits,
+                      bool glv, uint32_t* entries, SmallMsm& out);
+
 // The fused last reduction levels for D independent sets of m (A, Q) XYZZ
 // pairs (m <= msm_reduce_tail_max(D)); roots to outQ[0..D).
 uint32_t msm_reduce_tail_max(uint32_t D);

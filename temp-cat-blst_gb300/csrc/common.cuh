@@ -147,12 +147,12 @@ struct AffWork {
 // Device workspaces of one MSM pipeline instance.
 struct MsmWork {
     DevBuf points, scalars, digits, ranks, counts, offsets, block_sums, sorted_pt, sorted_key,
-        buckets, head, tail, seg, wins, total, status, misc, glv_pts, glv_sc, glv_sign;
+        buckets, head, tail, seg, total, status, misc, glv_pts, glv_sc, glv_sign;
     AffWork aff;
     void release()
     {
         for (DevBuf* b : {&points, &scalars, &digits, &ranks, &counts, &offsets, &block_sums, &sorted_pt,
-                          &sorted_key, &buckets, &head, &tail, &seg, &wins, &total, &status, &misc, &glv_pts,
+                          &sorted_key, &buckets, &head, &tail, &seg, &total, &status, &misc, &glv_pts,
                           &glv_sc, &glv_sign})
             b->release();
         aff.release();

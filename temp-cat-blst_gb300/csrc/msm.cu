@@ -43,6 +43,7 @@
 #include "common.cuh"
 #include "curve.cuh"
 #include "fr.cuh"
+#include "scalar.cuh"
 #include "host_curve.hpp"
 #include "catmsm_internal.h"
 
@@ -55,30 +56,6 @@ namespace catmsm {
 thread_local LaunchStats g_stats;
 
 // ----------------------------------------------------------------- 1. digits
-// k = the low nbits bits of a little-endian scalar of `stride` bytes
-__device__ __forceinline__ void load_scalar(uint32_t* k, const uint8_t* s, uint32_t stride, uint32_t nbits)
-{
-#pragma unroll
-    for (int j = 0; j < 8; j++) k[j] = 0;
-    const uint32_t nbytes = (nbits + 7) >> 3;
-    if (stride == 32 && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(s));
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(s) + 1);
-        k[0] = a.x; k[1] = a.y; k[2] = a.z; k[3] = a.w;
-        k[4] = b.x; k[5] = b.y; k[6] = b.z; k[7] = b.w;
-    } else if (stride == 16 && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(s));
-        k[0] = a.x; k[1] = a.y; k[2] = a.z; k[3] = a.w;
-    } else {
-        for (uint32_t b = 0; b < nbytes; b++) k[b >> 2] |= (uint32_t)s[b] << (8 * (b & 3));
-    }
-#pragma unroll
-    for (uint32_t j = 0; j < 8; j++) {
-        if (nbits <= 32 * j) k[j] = 0;
-        else if (nbits < 32 * (j + 1)) k[j] &= (1u << (nbits - 32 * j)) - 1;
-    }
-}
-
 // ----------------------------------------------------------------- 0. GLV split
 // Thread i: k = k_i mod r = k1 + k2 lambda (0 <= k1 < lambda, k2 <= lambda + 1),
 // balanced to k = s1 m1 + s2 m2 lambda with m1, m2 <= (lambda + 1) / 2:
@@ -887,6 +864,7 @@ uint32_t msm_default_window(size_t n)
 // entries on this GPU).  Measured best: 16 for n2 = 2^21, 19 for n2 = 2^23.
 uint32_t msm_glv_window(size_t n2)
 {
+    if (msm_small_applies(n2, true)) return msm_small_window(n2);
     double best = 0;
     uint32_t bc = 0;
     for (uint32_t c = 2; c <= 20; c++) {
@@ -914,6 +892,7 @@ uint32_t msm_glv_window(size_t n2)
 // the grid-wide fixup).  1500003 points of 64 bits: c = 16 3.05 ms, 17 2.80 ms (262144 points: 0.98, 0.90).
 static uint32_t msm_plain_window(size_t n, uint32_t nbits)
 {
+    if (nbits <= 128 && msm_small_applies(n, false)) return msm_small_window(n);
     const uint32_t def = msm_default_window(n);
     if (n < (size_t(1) << 18)) return def;
     double best = 0;
@@ -930,6 +909,7 @@ static uint32_t msm_plain_window(size_t n, uint32_t nbits)
 
 cudaError_t msm_setup_device()
 {
+    CATMSM_CHECK(msm_small_setup_device());
     return cudaFuncSetAttribute(k_reduce_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(kTailThreads / 8 * 2 * sizeof(xyzz)));
 }
@@ -1051,6 +1031,12 @@ static uint32_t level1_fan_in(size_t M)
     return M >= kFanIn16MinBuckets ? 16 : M >= kFanIn8MinBuckets ? 8 : 2;
 }
 
+static uint32_t msm_windows(size_t np, uint32_t nbits, bool glv, uint32_t c)
+{
+    if ((glv || nbits <= 128) && msm_small_applies(np, glv)) return msm_small_windows(np, glv ? 127 : nbits, glv);
+    return (glv ? 127 : nbits) / c + 1;
+}
+
 // The plan without a context (host arithmetic only; off a GPU the chunk
 // model uses 152 SMs x 4 resident blocks, the GB300's figures): window,
 // windows, pipeline points, accumulate chunk length and level-1 fan-in.
@@ -1060,7 +1046,7 @@ void msm_plan_detail(size_t n, uint32_t nbits, bool glv, uint32_t* c, uint32_t* 
     const bool g = glv && nbits > 128 && n < (1u << 30);
     const size_t np = g ? 2 * n : n;
     *c = g ? msm_glv_window(np) : msm_plain_window(np, nbits);
-    *windows = (g ? 127 : nbits) / *c + 1;
+    *windows = msm_windows(np, nbits, g, *c);
     *points = np;
     *chunk = accumulate_chunk(np * *windows);
     *fan_in = level1_fan_in((size_t)*windows << (*c - 1));
@@ -1070,10 +1056,46 @@ void msm_plan(const Ctx* ctx, size_t n, uint32_t nbits, uint32_t* c, uint32_t* w
 {
     const bool g = use_glv(ctx, n, nbits);
     const size_t np = g ? 2 * n : n;
-    const uint32_t nb = g ? 127 : nbits;
     *c = g ? msm_glv_window(np) : msm_plain_window(np, nbits);
-    *windows = nb / *c + 1;
+    *windows = msm_windows(np, nbits, g, *c);
     *points = np;
+}
+
+// Adds a call's stage times and its bucket entries (a device counter).
+static cudaError_t profile_end(StageProfile& P, cudaStream_t st, const uint32_t* entries)
+{
+    CATMSM_CHECK(cudaEventRecord(P.ev[kMsmStages], st));
+    CATMSM_CHECK(cudaEventSynchronize(P.ev[kMsmStages]));
+    for (int i = 0; i < kMsmStages; i++) {
+        float ms = 0.f;
+        CATMSM_CHECK(cudaEventElapsedTime(&ms, P.ev[i], P.ev[i + 1]));
+        P.ms[i] += ms;
+    }
+    uint32_t E = 0;
+    CATMSM_CHECK(cudaMemcpy(&E, entries, 4, cudaMemcpyDeviceToHost));
+    P.entries += E;
+    P.calls++;
+    return cudaSuccess;
+}
+
+// out = sum_w 2^(c w) W_w (Jacobian, normalised), top window first
+// (reference multi_scalar.cpp:913-922); wins: the window sums as the device
+// wrote them.
+static void fold_windows(uint64_t* out, const uint64_t* wins, uint32_t D, uint32_t c)
+{
+    using namespace catmsm_host;
+    hjac ret;
+    std::memset(&ret, 0, sizeof(ret));
+    for (uint32_t w = D; w-- > 0;) {
+        hjac tile;
+        from_device_xyzz(tile, wins + (size_t)w * 24);
+        jac_add(ret, ret, tile);
+        if (w)
+            for (uint32_t i = 0; i < c; i++) jac_dbl(ret, ret);
+    }
+    hjac norm;
+    normalize(norm, ret);
+    std::memcpy(out, &norm, 144);
 }
 
 // Runs the device pipeline over device-resident points/scalars on the context
@@ -1095,6 +1117,31 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
         if (P.enabled) cudaEventRecord(P.ev[i], st);
     };
     mark(0);
+    // Few points (and no width or rounds asked for): one kernel for the buckets of
+    // all windows instead of the sort, accumulate, fixup and reduce launches
+    const bool glv_split = !tile_window && use_glv(ctx, n, nbits);
+    if (!tile_window && c == 0 && ctx->affine_rounds < 0 && (glv_split || nbits <= 128) &&
+        msm_small_applies(glv_split ? 2 * n : n, glv_split)) {
+        if (points_ready) CATMSM_CHECK(cudaStreamWaitEvent(st, points_ready, 0));
+        SmallMsm m;
+        uint32_t* entries = nullptr;
+        if (P.enabled) {
+            entries = (uint32_t*)W.status.get(256);
+            if (!entries) return cudaErrorMemoryAllocation;
+            CATMSM_CHECK(cudaMemsetAsync(entries, 0, 4, st));
+        }
+        for (int i = 1; i < 5; i++) mark(i);
+        CATMSM_CHECK(msm_small(ctx, (const affine*)d_points, d_scalars, stride, n, nbits, glv_split, entries, m));
+        mark(5);
+        mark(6);
+        mark(7);
+        CATMSM_CHECK(cudaStreamSynchronize(st));
+        if (!*m.over) {
+            fold_windows(out, m.wins, m.D, m.c);
+            if (P.enabled) CATMSM_CHECK(profile_end(P, st, entries));
+            return cudaSuccess;
+        }
+    }
     // The points are read only from the point stage on (after the scatter):
     // points_ready, if given, is an event on another stream (a host copy in
     // flight) that the pipeline waits for just before that stage.
@@ -1102,7 +1149,7 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     affine* gpts = nullptr;
     uint8_t* sgn = nullptr;
     const size_t n_in = n;
-    if (!tile_window && use_glv(ctx, n, nbits)) {
+    if (glv_split) {
         gpts = (affine*)W.glv_pts.get(2 * n * sizeof(affine));
         uint4* gsc = (uint4*)W.glv_sc.get(2 * n * sizeof(uint4));
         sgn = (uint8_t*)W.glv_sign.get(n);
@@ -1154,12 +1201,11 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     xyzz* head = (xyzz*)W.head.get(chunks * sizeof(xyzz));
     xyzz* tail = (xyzz*)W.tail.get(chunks * sizeof(xyzz));
     xyzz* seg = (xyzz*)W.seg.get(2 * (lvl1 + lvl2) * sizeof(xyzz));
-    xyzz* wins = (xyzz*)W.wins.get((size_t)D * sizeof(xyzz));
     uint64_t* h_wins = (uint64_t*)ctx->h_out.get((size_t)D * sizeof(xyzz));
     uint32_t* hot_count = (uint32_t*)W.status.get(256 + chunks * sizeof(uint2));
     uint2* hot_list = reinterpret_cast<uint2*>(hot_count + 64);
     if (!digits || !ranks || !counts || !offsets || !bsums || !sorted_pt || !sorted_key || !buckets ||
-        !head || !tail || !seg || !wins || !h_wins || !hot_count)
+        !head || !tail || !seg || !h_wins || !hot_count)
         return cudaErrorMemoryAllocation;
     uint32_t* total = offsets + M;
 
@@ -1225,10 +1271,10 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
         bool first = S != 2;
         while (m > 1) {
             if (!first && m <= msm_reduce_tail_max(D)) {
-                msm_reduce_tail(inA, inQ, m, D, bufQ[pp], st);
+                msm_reduce_tail(inA, inQ, m, D, h_wins, st);       // page-locked: the root goes straight there
                 g_stats.launches++;
-                inQ = bufQ[pp];
-                m = 1;
+                inQ = nullptr;
+                inA = nullptr;
                 break;
             }
             const uint32_t F = first ? S : 2;
@@ -1245,40 +1291,16 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
             m = m_out;
             first = false;
         }
-        CATMSM_CHECK(cudaMemcpyAsync(wins, inQ ? inQ : inA, (size_t)D * sizeof(xyzz), cudaMemcpyDeviceToDevice, st));
+        if (inA)
+            CATMSM_CHECK(cudaMemcpyAsync(h_wins, inQ ? inQ : inA, (size_t)D * sizeof(xyzz), cudaMemcpyDeviceToHost, st));
     }
     g_stats.launches += 8;
     CATMSM_CHECK(cudaGetLastError());
-    CATMSM_CHECK(cudaMemcpyAsync(h_wins, wins, (size_t)D * sizeof(xyzz), cudaMemcpyDeviceToHost, st));
     mark(7);
     CATMSM_CHECK(cudaStreamSynchronize(st));
 
-    using namespace catmsm_host;
-    hjac ret;
-    std::memset(&ret, 0, sizeof(ret));
-    for (uint32_t w = D; w-- > 0;) {
-        hjac tile;
-        from_device_xyzz(tile, h_wins + (size_t)w * 24);
-        jac_add(ret, ret, tile);
-        if (w)
-            for (uint32_t i = 0; i < c; i++) jac_dbl(ret, ret);
-    }
-    hjac norm;
-    normalize(norm, ret);
-    std::memcpy(out, &norm, 144);
-    if (P.enabled) {
-        CATMSM_CHECK(cudaEventRecord(P.ev[kMsmStages], st));
-        CATMSM_CHECK(cudaEventSynchronize(P.ev[kMsmStages]));
-        for (int i = 0; i < kMsmStages; i++) {
-            float ms = 0.f;
-            CATMSM_CHECK(cudaEventElapsedTime(&ms, P.ev[i], P.ev[i + 1]));
-            P.ms[i] += ms;
-        }
-        uint32_t E = 0;
-        CATMSM_CHECK(cudaMemcpy(&E, total, 4, cudaMemcpyDeviceToHost));
-        P.entries += E;
-        P.calls++;
-    }
+    fold_windows(out, h_wins, D, c);
+    if (P.enabled) CATMSM_CHECK(profile_end(P, st, total));
     return cudaSuccess;
 }
 
