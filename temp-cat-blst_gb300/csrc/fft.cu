@@ -255,25 +255,29 @@ __device__ __forceinline__ PassGeom pass_geom(const FftJob& J, uint32_t s0, uint
 }
 
 // The products of a pass: item-major per job (all items of one kind are
-// adjacent, so trivial ones do not share warps with multiplications).
-// Quad: a quad of lanes per item.
-template <bool Quad>
-__global__ void __launch_bounds__(64) k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod,
-                                                  const FftJob* __restrict__ jobs,
-                                                  const uint32_t* __restrict__ lst_job,
-                                                  const uint32_t* __restrict__ lst_pre, uint32_t cnt, uint32_t total,
-                                                  uint32_t s0, uint32_t q)
+// adjacent, so trivial ones do not share warps with multiplications).  Lanes per
+// item: 1, 2 (the pair form) or 4 (the quad form).  Split: the halves k1 x and
+// k2 phi(x) of a product are two items (item 2 i + half), with half the additions
+// each; the combine adds twice as many.
+constexpr uint32_t kItemThreads = 64;
+
+template <int Lanes, bool Split>
+__global__ void __launch_bounds__(kItemThreads, Lanes == 2 ? 6 : 4)
+k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* __restrict__ jobs,
+            const uint32_t* __restrict__ lst_job, const uint32_t* __restrict__ lst_pre, uint32_t cnt, uint32_t total,
+            uint32_t s0, uint32_t q)
 {
-    __shared__ quad_table tabs[Quad ? 16 : 1];
-    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t t = Quad ? gt >> 2 : gt;
+    __shared__ __align__(16) unsigned char tabs[Lanes == 1   ? 16
+                                                : Lanes == 2 ? kItemThreads / 2 * sizeof(pair_table)
+                                                             : kItemThreads / 4 * sizeof(quad_table)];
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / Lanes;
     if (t >= total) return;
-    const quad_lane ql = quad_of(threadIdx.x & 31);
     const uint32_t e = find_range(lst_pre, cnt, t);
     const FftJob J = jobs[lst_job[e]];
     const PassGeom G = pass_geom(J, s0, q);
     const uint32_t b = t - lst_pre[e];
-    const uint32_t it = b / G.bf, bf = b % G.bf;
+    const uint32_t bf = b % G.bf, half = Split ? b / G.bf & 1 : 0;
+    const uint32_t it = b / G.bf >> (Split ? 1 : 0);
     const uint32_t h = 1u << s0, j = bf & (h - 1);
     const uint32_t g = active_group(bf >> s0, G.active, G.groups);
     uint32_t m = 0, k = 0;
@@ -311,29 +315,47 @@ __global__ void __launch_bounds__(64) k_fft_items(const xyzz* __restrict__ a, xy
             fr_mul(c, c, r);
         }
     }
-    if (!one) {
-        uint32_t kc[8], k12[8];
-        fr_from_mont(kc, c);
-        fr_glv_split(k12, k12 + 4, kc);
-        if (Quad) {
-            qd_store(prod + t, qd_mult_glv(v, k12, k12 + 4, tabs + (threadIdx.x >> 2), ql), ql);
-            return;
-        }
-        xyzz_mult_glv(v, v, k12, k12 + 4);
+    if (one) {
+        if (half) xyzz_set_inf(v);
+        if (threadIdx.x % Lanes == 0) store_xyzz(prod + t, v);
+        return;
     }
-    if (!Quad || ql.k == 0) store_xyzz(prod + t, v);
+    uint32_t kc[8], k12[8];
+    fr_from_mont(kc, c);
+    fr_glv_split(k12, k12 + 4, kc);
+    if (Lanes == 1) {
+        xyzz_mult_glv(v, v, k12, k12 + 4);
+        store_xyzz(prod + t, v);
+    } else if (Lanes == 2) {
+        const pair_lane l{(threadIdx.x & 1) != 0, 3u << (threadIdx.x & 30)};
+        fp lo, hi;
+        pd_mult_glv(lo, hi, v, k12, k12 + 4, reinterpret_cast<pair_table*>(tabs) + threadIdx.x / 2, l);
+        const quad_lane w0{l.odd ? 1u : 0u, 0}, w1{l.odd ? 3u : 2u, 0};     // the coordinates this lane holds
+        qd_store(prod + t, lo, w0);
+        qd_store(prod + t, hi, w1);
+    } else {
+        const quad_lane ql = quad_of(threadIdx.x & 31);
+        if (half) {
+            fp beta;
+#pragma unroll
+            for (int w = 0; w < 12; w++) beta.v[w] = FP_BETA[w];
+            fp_mul(v.x, v.x, beta);
+        }
+        qd_store(prod + t, qd_mult_glv<Split>(v, half ? k12 + 4 : k12, k12 + 4,
+                                              reinterpret_cast<quad_table*>(tabs) + threadIdx.x / 4, ql), ql);
+    }
 }
 
-// The sums of a pass: `width` = 4 * 2^(q - 1) lanes per output, each quad adds
-// two products, then a tree over the output's quads.
+// The sums of a pass: 4 * 2^(q - 1) lanes per output (twice that if split), each
+// quad adds two products (the halves of one), then a tree over the output's quads.
 __global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ prod, xyzz* __restrict__ a,
                                                      const FftJob* __restrict__ jobs,
                                                      const uint32_t* __restrict__ lst_job,
                                                      const uint32_t* __restrict__ lst_pre,
                                                      const uint32_t* __restrict__ lst_out, uint32_t cnt,
-                                                     uint32_t total, uint32_t s0, uint32_t q)
+                                                     uint32_t total, uint32_t s0, uint32_t q, uint32_t split)
 {
-    const uint32_t lw = q + 1;                       // log2 of the lanes per output
+    const uint32_t lw = q + 1 + split;               // log2 of the lanes per output
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t o = gt >> lw;
     const bool valid = o < total;
@@ -351,10 +373,10 @@ __global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ pr
         const uint32_t h = 1u << s0;
         dst = J.val_off + (active_group(bf >> s0, G.active, G.groups) << (s0 + G.q)) + (bf & (h - 1)) + k * h;
         const xyzz* p = prod + lst_pre[e] + bf;
-        if (2 * qi < (1u << G.q)) {
-            const uint32_t m0 = 2 * qi, m1 = m0 + 1;
-            acc = qd_load(p + (size_t)item_of(m0, k) * G.bf, ql.k);
-            fp v = qd_load(p + (size_t)item_of(m1, k) * G.bf, ql.k);
+        if (2 * qi < (1u << (G.q + split))) {
+            const uint32_t m0 = 2 * qi >> split, m1 = (2 * qi + 1) >> split;
+            acc = qd_load(p + ((size_t)item_of(m0, k) << split) * G.bf, ql.k);
+            fp v = qd_load(p + (((size_t)item_of(m1, k) << split) + split) * G.bf, ql.k);
             if ((__popc(m0 & k) & 1) && ql.k == 1) fp_neg(acc, acc);
             if ((__popc(m1 & k) & 1) && ql.k == 1) fp_neg(v, v);
             qd_add(acc, v, ql);
@@ -397,7 +419,7 @@ __global__ void __launch_bounds__(64) k_fft_finish_multi(const xyzz* __restrict_
     store_jac(out + t, o);
 }
 
-// Scalar multiplications that run at once as quads (one wave of k_fft_items<true>).
+// Scalar multiplications that run at once as quads (one wave of k_fft_items).
 static size_t fft_quad_wave()
 {
     static std::atomic<size_t> by_dev[64];          // shared by every calling thread
@@ -409,7 +431,7 @@ static size_t fft_quad_wave()
     }
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_items<true>, 64, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_fft_items<4, false>), kItemThreads, 0);
     size_t v = (sms > 0 && per_sm > 0) ? (size_t)sms * per_sm * 16 : (size_t)device_sms() * 64;
     if (dev >= 0 && dev < 64) by_dev[dev].store(v, std::memory_order_relaxed);
     return v;
@@ -418,35 +440,63 @@ static size_t fft_quad_wave()
 // One pass: levels s0 + 1 .. s0 + q.
 struct FftPass {
     uint32_t s0 = 0, q = 1, group = 0;
-    enum { kStage, kQuads, kLanes } kind = kStage;
+    uint32_t split = 0;
+    enum { kStage, kQuads, kPairs, kLanes } kind = kStage;
     uint32_t off = 0, cnt = 0;          // its entries of the job lists
     uint32_t items = 0, outputs = 0;
 };
 
-// Items and outputs of a pass over every job that has its first level.
-static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uint32_t q, size_t& items,
-                        size_t& outputs)
+// Products of a butterfly of a pass that are multiplications: all of its items
+// but x_0, less (first pass, j = 0 throughout) those without a root.
+static size_t pass_products(uint32_t s0, uint32_t q)
 {
-    items = outputs = 0;
+    if (s0) return pass_items(q) - 1;
+    size_t c = 0;
+    for (uint32_t m = 1; m < (1u << q); m++) {
+        const uint32_t top = 1u << (31 - __builtin_clz(m));
+        for (uint32_t k = 0; k < top; k++) {
+            bool root = false;
+            for (uint32_t i = 1; i < q; i++) root |= ((m >> i) & 1u) && (k & ((1u << i) - 1));
+            c += root;
+        }
+    }
+    return c;
+}
+
+// Items, multiplications and outputs of a pass over every job that has its first level.
+static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uint32_t q, size_t& items,
+                        size_t& products, size_t& outputs)
+{
+    items = products = outputs = 0;
     for (const FftJob* job : jobs) {
         const FftJob& J = *job;
         if (J.logn <= s0) continue;
         const uint32_t qe = std::min(q, J.logn - s0);
         const size_t bf = (size_t)std::min(J.n >> (s0 + qe), J.xn) << s0;
         items += bf * pass_items(qe);
+        products += bf * pass_products(s0, qe);
         outputs += bf << qe;
     }
 }
 
 // The cheapest sequence of passes by a model of their times (ms), fitted on
-// GB300 (wave = 9728 quads, 4 blocks of 16 on each of 152 SMs; four waves' worth of
-// lanes are resident at once).  Both forms last one multiplication's latency as
-// long as a warp has its scheduler to itself, more when two share it, and
-// add up beyond a wave; a sum costs kSumMs per product.
-static double quads_ms(size_t items, size_t wave)
+// GB300 (wave = 9728 quads, 4 blocks of 16 on each of 152 SMs; three waves' worth of
+// pairs and four of lanes are resident at once).  Every form lasts one
+// multiplication's latency as long as a warp has its scheduler to itself (quads
+// 0.75 ms, the halves of a split product 0.64, pairs 0.98, lanes 1.65), more when
+// two share it, and adds up beyond a wave; a sum costs kSumMs per product.
+static double quads_ms(size_t items, size_t wave, bool split)
 {
+    const double part = split ? 0.65 : 0.76, full = split ? 0.95 : 1.03;
     const size_t rem = items % wave;
-    return 1.05 * (double)(items / wave) + (rem == 0 ? 0.0 : rem <= 3 * wave / 10 ? 0.76 : 1.05);
+    return full * (double)(items / wave) + (rem == 0 ? 0.0 : rem <= 3 * wave / 10 ? part : full);
+}
+
+static double pairs_ms(size_t items, size_t wave)
+{
+    const size_t rem = items % (3 * wave);
+    return 2.05 * (double)(items / (3 * wave)) +
+           (rem == 0 ? 0.0 : rem <= 6 * wave / 10 ? 1.0 : rem <= 5 * wave / 4 ? 1.33 : 2.05);
 }
 
 static double lanes_ms(size_t items, size_t wave)
@@ -476,21 +526,28 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
     best[0] = 0;
     for (uint32_t s = 0; s < maxlog; s++) {
         for (uint32_t q = 1; q <= (solo ? kMaxQ : 1) && s + q <= maxlog; q++) {
-            size_t items, outputs;
-            pass_counts(jobs, s, q, items, outputs);
+            size_t items, products, outputs;
+            pass_counts(jobs, s, q, items, products, outputs);
             FftPass p;
             p.s0 = s;
             p.q = q;
             double ms = q == 1 ? stage_ms(outputs / 2, wave) : 1e300;
             if (solo && items <= kMaxItems) {
-                const size_t products = items - (outputs >> q);      // item 0 is a copy
                 const double sums = kLaunchMs * q + kSumMs * (double)outputs * (1u << q);
-                const double quads = quads_ms(products, wave) + sums;
-                const double lanes = lanes_ms(products, wave) + sums;
-                if (std::min(quads, lanes) < ms) {
-                    p.kind = quads <= lanes ? FftPass::kQuads : FftPass::kLanes;
-                    ms = std::min(quads, lanes);
-                }
+                const struct {
+                    decltype(p.kind) kind;
+                    uint32_t split;
+                    double ms;
+                } forms[] = {{FftPass::kLanes, 0, lanes_ms(products, wave) + sums},
+                             {FftPass::kPairs, 0, pairs_ms(products, wave) + sums},
+                             {FftPass::kQuads, 0, quads_ms(products, wave, false) + sums},
+                             {FftPass::kQuads, 1, q <= 3 ? quads_ms(2 * products, wave, true) + 2 * sums : 1e300}};
+                for (const auto& f : forms)
+                    if (f.ms < ms) {
+                        p.kind = f.kind;
+                        p.split = f.split;
+                        ms = f.ms;
+                    }
             }
             if (best[s] + ms < best[s + q]) {
                 best[s + q] = best[s] + ms;
@@ -569,7 +626,7 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
             lst_job.push_back((uint32_t)i);
             lst_item.push_back(p.items);
             lst_out.push_back(p.outputs);
-            p.items += p.kind == FftPass::kStage ? bf : bf * pass_items(qe);
+            p.items += p.kind == FftPass::kStage ? bf : bf * pass_items(qe) << p.split;
             p.outputs += bf << qe;
         }
         p.cnt = (uint32_t)lst_job.size() - p.off;
@@ -638,13 +695,18 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
             g_stats.launches++;
             continue;
         }
-        if (p.kind == FftPass::kQuads)
-            k_fft_items<true><<<div_up(4 * (size_t)p.items, 64), 64, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items,
-                                                                              p.s0, p.q);
+        const uint32_t lanes = p.kind == FftPass::kQuads ? 4 : p.kind == FftPass::kPairs ? 2 : 1;
+        const unsigned grid = div_up((size_t)lanes * p.items, kItemThreads);
+        if (p.split)
+            k_fft_items<4, true><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+        else if (lanes == 4)
+            k_fft_items<4, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+        else if (lanes == 2)
+            k_fft_items<2, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
         else
-            k_fft_items<false><<<div_up(p.items, 64), 64, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
-        k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1), 128), 128, 0, ps>>>(
-            pp, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q);
+            k_fft_items<1, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+        k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1 + p.split), 128), 128, 0, ps>>>(
+            pp, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q, p.split);
         g_stats.launches += 2;
     }
     if (groups == 2) CATMSM_CHECK(W.aux.end(st));

@@ -308,8 +308,9 @@ struct quad_table {
     fp x[8], y[8], bx[8], ny[8];  // ny: -y; while the table is built, the z ratios and their suffix products
 };
 
-// Every lane of the quad passes the same point and scalar and its own
-// coordinate of the point (d = qd_load of it); returns the product, distributed.
+// Every lane of the quad passes the same point and scalar; returns the product,
+// distributed.  Half: k1 P only.
+template <bool Half>
 static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1, const uint32_t* k2, quad_table* tab,
                                               const quad_lane q)
 {
@@ -344,8 +345,9 @@ static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1,
     }
     __syncwarp(q.mask);
     if (qd_is_inf(c, q)) {        // zz of 8 P: zero if any ratio is
+        const uint32_t zero[4] = {0, 0, 0, 0};
         xyzz out;
-        xyzz_mult_plain(out, P, k1, k2);
+        xyzz_mult_plain(out, P, k1, Half ? zero : k2);
         const fp lo = fp_sel(out.x, out.y, odd), hi = fp_sel(out.zz, out.zzz, odd);
         return fp_sel(lo, hi, q.k >= 2);
     }
@@ -385,7 +387,7 @@ static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1,
     __syncwarp(q.mask);
     int8_t d1[33], d2[33];
     booth4_128(d1, k1);
-    booth4_128(d2, k2);
+    if (!Half) booth4_128(d2, k2);
     bool started = false;
 #pragma unroll 1
     for (int i = 32; i >= 0; i--) {
@@ -394,7 +396,7 @@ static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1,
             for (int k = 0; k < 4; k++) qd_dbl(d, q);
         }
 #pragma unroll 1
-        for (int hh = 0; hh < 2; hh++) {
+        for (int hh = 0; hh < (Half ? 1 : 2); hh++) {
             const int g = hh ? d2[i] : d1[i];
             if (g) {
                 const int e = (g > 0 ? g : -g) - 1;
@@ -406,6 +408,217 @@ static __device__ __noinline__ fp qd_mult_glv(const xyzz& P, const uint32_t* k1,
     // common z of the table (c's zz, zzz), then P's own
     const fp r = fp_mul_call(fp_mul_call(d, c), fp_sel(P.zz, P.zzz, odd));
     return fp_sel(d, r, q.k >= 2);
+}
+
+// ---------------------------------------------------------------------------
+// The pair form: two lanes on one multiplication, between the quad (whose four
+// lanes idle in a third of their products) and the single lane (whose chain of
+// 7 and 11 products a doubling and an addition is twice as long).  Jacobian: lane
+// 0 holds x, lane 1 holds y and z; a doubling is 4 dependent products (two of
+// them squarings), a mixed addition 6.  5.4 k of them 0.98 ms (quads 1.03), 12 k
+// 1.33 (lanes 1.65, quads two waves), from 20 k no faster than lanes: 2^12 FFT
+// 6.2 -> 5.4 ms, 2^13 9.9 -> 8.1.
+struct pair_table {
+    fp x[8], y[8], bx[8];         // bx: while the table is built, the z ratios and their suffix products
+};
+
+struct pair_lane {
+    bool odd;
+    uint32_t mask;
+};
+
+struct pair_acc {
+    fp c, z;                      // lane 0: x, -; lane 1: y, z
+};
+
+__device__ __forceinline__ fp pd_swap(const fp& v, const pair_lane& l)
+{
+    fp r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = __shfl_xor_sync(l.mask, v.v[i], 1, 2);
+    return r;
+}
+
+__device__ __forceinline__ fp pd_bcast(const fp& v, int src, const pair_lane& l)
+{
+    fp r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = __shfl_sync(l.mask, v.v[i], src, 2);
+    return r;
+}
+
+// dbl-2009-l: X^2, Y^2 | (X + B)^2, B^2 | E^2, Y Z | E (D - X3), -
+__device__ __forceinline__ void pd_dbl(pair_acc& p, const pair_lane& l)
+{
+    fp s, w, t, E, X3;
+    fp_sqr(s, p.c);                                       // A, B
+    fp_add(t, p.c, pd_swap(s, l));                        // lane 0: X + B
+    fp_sqr(w, fp_sel(t, s, l.odd));                       // (X + B)^2, C
+    fp_dbl(E, s);
+    fp_add(E, E, s);                                      // lane 0: E = 3A
+    fp r, D;
+    fp_mul(r, fp_sel(E, p.c, l.odd), fp_sel(E, p.z, l.odd));
+    fp_sub(t, w, s);
+    fp_sub(t, t, pd_swap(w, l));
+    fp_dbl(D, t);
+    fp_sub(t, r, D);
+    fp_sub(X3, t, D);
+    fp_sub(t, D, X3);
+    fp_mul(t, E, t);                                      // lane 0: E (D - X3)
+    fp_dbl(w, w);
+    fp_dbl(w, w);
+    fp_dbl(w, w);                                         // lane 1: 8C
+    fp_sub(t, pd_swap(t, l), w);                          // lane 1: Y3
+    p.c = fp_sel(X3, t, l.odd);
+    fp_dbl(p.z, r);                                       // lane 1: 2YZ
+}
+
+// h = the difference H = U2 - X1 (both lanes), r = S2 - Y1 (lane 1), hh = H^2
+// (lane 0) of (ax, ay) and p: Z^2 | U2, Z^3 | H^2, S2
+__device__ __forceinline__ void pd_diff(fp& h, fp& r, fp& hh, const pair_acc& p, const fp& a, const pair_lane& l)
+{
+    fp t, u;
+    fp_sqr(t, p.z);
+    t = pd_bcast(t, 1, l);
+    fp_mul(u, fp_sel(a, p.z, l.odd), t);
+    fp_sub(t, u, p.c);
+    h = pd_bcast(t, 0, l);
+    fp_mul(hh, fp_sel(h, a, l.odd), fp_sel(h, u, l.odd));
+    fp_sub(r, hh, p.c);
+}
+
+// The rest of the addition: H HH, Z H | X HH, R^2 | R (V - X3), Y HHH
+__device__ __forceinline__ void pd_core(pair_acc& p, const fp& h, const fp& r, const fp& hh, const pair_lane& l)
+{
+    fp z, v, t, X3, u;
+    fp_mul(z, fp_sel(hh, p.z, l.odd), h);                 // HHH, Z3
+    fp_mul(v, fp_sel(p.c, r, l.odd), fp_sel(hh, r, l.odd));   // V, RR
+    const fp R = pd_swap(r, l), o = pd_swap(fp_sel(z, v, l.odd), l);   // lane 0: R, RR; lane 1: -, HHH
+    fp_sub(t, o, z);
+    fp_sub(t, t, v);
+    fp_sub(X3, t, v);                                     // lane 0: RR - HHH - 2V
+    fp_sub(u, v, X3);
+    fp_mul(t, fp_sel(R, p.c, l.odd), fp_sel(u, o, l.odd));
+    fp_sub(t, pd_swap(t, l), t);                          // lane 1: R (V - X3) - Y HHH
+    p.c = fp_sel(X3, t, l.odd);
+    p.z = z;
+}
+
+__device__ __forceinline__ void pd_set(pair_acc& p, const fp& a)
+{
+    p.c = a;
+    fp_set_one(p.z);
+}
+
+// Both lanes of the pair pass the same point and scalar; the product's x and zz
+// in lane 0 (lo, hi), y and zzz in lane 1.
+static __device__ __noinline__ void pd_mult_glv(fp& lo, fp& hi, const xyzz& P, const uint32_t* k1, const uint32_t* k2,
+                                                pair_table* tab, const pair_lane l)
+{
+    fp_zero(lo);
+    fp_zero(hi);
+    if (xyzz_is_inf(P)) return;
+    const fp a = fp_sel(P.x, P.y, l.odd);
+    pair_acc p;
+    pd_set(p, a);
+    (l.odd ? tab->y : tab->x)[0] = a;
+#pragma unroll 1
+    for (int i = 1; i < 8; i++) {
+        if (i == 1) {
+            pd_dbl(p, l);
+            if (l.odd) tab->bx[1] = p.z;                  // 2Y
+        } else {
+            fp h, r, hh;
+            pd_diff(h, r, hh, p, a, l);
+            pd_core(p, h, r, hh, l);
+            if (l.odd) tab->bx[i] = h;
+        }
+        (l.odd ? tab->y : tab->x)[i] = p.c;
+    }
+    const fp zg = pd_bcast(p.z, 1, l);                    // z of 8 P: zero if any ratio is
+    if (fp_is_zero(zg)) {
+        xyzz out;
+        xyzz_mult_plain(out, P, k1, k2);
+        lo = fp_sel(out.x, out.y, l.odd);
+        hi = fp_sel(out.zz, out.zzz, l.odd);
+        return;
+    }
+    __syncwarp(l.mask);
+    // suffix products: bx[i] = product of the ratios i + 1 .. 7 (i < 7)
+    fp s = tab->bx[7];
+#pragma unroll 1
+    for (int i = 5; i >= 0; i--) {
+        fp t;
+        fp_mul(t, s, tab->bx[i + 1]);
+        __syncwarp(l.mask);
+        if (!l.odd) tab->bx[i + 1] = s;
+        s = t;
+    }
+    if (!l.odd) tab->bx[0] = s;
+    __syncwarp(l.mask);
+    fp beta;
+#pragma unroll
+    for (int k = 0; k < 12; k++) beta.v[k] = FP_BETA[k];
+    // a lane rescales every second entry (entry 7 has the common z already)
+#pragma unroll 1
+    for (int i = l.odd ? 1 : 0; i < 8; i += 2) {
+        fp one;
+        fp_set_one(one);
+        const fp si = i < 7 ? tab->bx[i] : one;
+        fp s2, x;
+        fp_sqr(s2, si);
+        fp_mul(x, tab->x[i], s2);
+        tab->x[i] = x;
+        fp_mul(x, x, beta);
+        tab->bx[i] = x;
+        fp_mul(s2, s2, si);
+        fp_mul(x, tab->y[i], s2);
+        tab->y[i] = x;
+    }
+    __syncwarp(l.mask);
+    int8_t d1[33], d2[33];
+    booth4_128(d1, k1);
+    booth4_128(d2, k2);
+    bool inf = true;
+#pragma unroll 1
+    for (int i = 32; i >= 0; i--) {
+        if (!inf) {
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) pd_dbl(p, l);
+        }
+#pragma unroll 1
+        for (int w = 0; w < 2; w++) {
+            const int g = w ? d2[i] : d1[i];
+            if (!g) continue;
+            const int e = (g > 0 ? g : -g) - 1;
+            fp b = l.odd ? tab->y[e] : w ? tab->bx[e] : tab->x[e], n;
+            fp_neg(n, b);
+            b = fp_sel(b, n, l.odd && g < 0);
+            if (inf) {
+                pd_set(p, b);
+                inf = false;
+                continue;
+            }
+            fp h, r, hh;
+            pd_diff(h, r, hh, p, b, l);
+            if (fp_is_zero(h)) {
+                const bool same = __shfl_sync(l.mask, (int)fp_is_zero(r), 1, 2) != 0;
+                if (same) pd_dbl(p, l);
+                else inf = true;
+                continue;
+            }
+            pd_core(p, h, r, hh, l);
+        }
+    }
+    if (inf) return;
+    // Z zg, then its square (lane 0) and cube (lane 1), times P's own
+    fp z, zz, t;
+    fp_mul(z, p.z, zg);
+    z = pd_bcast(z, 1, l);
+    fp_sqr(zz, z);
+    fp_mul(t, zz, z);
+    fp_mul(hi, fp_sel(zz, t, l.odd), fp_sel(P.zz, P.zzz, l.odd));
+    lo = p.c;
 }
 
 }  // namespace catmsm
