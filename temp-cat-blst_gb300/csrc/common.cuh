@@ -129,7 +129,8 @@ struct AuxStream {
 };
 
 // Workspaces of the batch-affine accumulation (bucket_affine.cu): one set per
-// stream of the two its slices alternate between, and the second stream.
+// stream of the two its slices alternate between, and the second stream (which
+// runs the second half of a large decode too).
 struct AffWork {
     struct Set {
         DevBuf pts0, pts1, key0, key1, meta, pairpos, prefix, rest, gtot;

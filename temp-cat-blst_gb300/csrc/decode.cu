@@ -250,45 +250,119 @@ __device__ __forceinline__ bool in_subgroup_quad(const affine& a, const quad_lan
     return quad_flag(eq, 0, q) && quad_flag(eq, 1, q);
 }
 
-// mode 0: uncompress (48-byte elements), 1: deserialize (96), 2: in_g1 only
-// (96-byte affine Montgomery points in `out`).  Quad: four lanes an element, for
-// calls that do not fill the GPU: they last as long as one element's chain,
-// whose doublings a quad does in half the time (the square root's chain
-// stays).  2111 checked elements: 1.50 -> 0.93 ms; a full launch keeps one lane:
-// 100003 checked elements, 6.21 -> 5.33 ms (square root by windows, mixed
-// additions, four warps per scheduler instead of two), the multiply pipe 88% busy.
+constexpr int kLaneThreads = 64, kLaneBlocks = 8;    // one lane an element: four warps per scheduler
+
+// mode 0: uncompress (48-byte elements), 1: deserialize (96).  Points go to `pts`
+// (which may be `in`, element over element) and codes to errs.  A kernel of its
+// own, so that the squarings of the square root can be inlined in its loop
+// without the membership test's code growing past the instruction cache: 300000
+// checked elements 13.76 -> 13.57 ms (14.33 with the squarings inlined in both).
+__global__ void __launch_bounds__(kLaneThreads, kLaneBlocks) k_decode(const uint8_t* in, uint32_t n, int mode,
+                                                                      affine* pts, int32_t* __restrict__ errs)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    affine a;
+    const int err = mode == 0 ? uncompress48(a, in + 48 * (size_t)i) : deserialize96(a, in + 96 * (size_t)i);
+    if (err == kOk) pts[i] = a;
+    errs[i] = err;
+}
+
+// Membership.  Decoded points (result false): the points of `pts` whose code is
+// kOk go to `out` or change the code.  Otherwise errs is the result, 1 for a
+// member, and a point may be off the curve.
+// Quad: four lanes an element, for calls that do not fill the GPU: they last as
+// long as one element's chain, whose doublings a quad does in half the time.
+// 2111 checked elements: 1.50 -> 0.92 ms.  A full launch keeps one lane: 77824
+// checked elements (one wave) 3.58 ms, the multiply pipe 88% busy.
 template <bool Quad>
-__global__ void __launch_bounds__(Quad ? 128 : 64, Quad ? 2 : 8) k_decode(const uint8_t* __restrict__ in, uint32_t n, int mode,
-                                                              int check_group, affine* __restrict__ out,
-                                                              int32_t* __restrict__ errs)
+__global__ void __launch_bounds__(Quad ? 128 : kLaneThreads, Quad ? 2 : kLaneBlocks) k_members(const affine* __restrict__ pts, uint32_t n,
+                                                                           bool result, affine* __restrict__ out,
+                                                                           int32_t* __restrict__ errs)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = Quad ? t >> 2 : t;
     if (i >= n) return;
     const quad_lane q = quad_of(threadIdx.x & 31);
-    const bool writes = !Quad || q.k == 0;
-    affine a;
-    int err = kOk;
-    bool check = check_group != 0;
-    if (mode == 2) {
-        a = out[i];
-        check = (fp_is_zero_raw(a.x) && fp_is_zero_raw(a.y)) || on_curve_xy(a.x, a.y);
-        if (!check) err = kNotOnCurve;
-    } else {
-        err = mode == 0 ? uncompress48(a, in + 48 * (size_t)i) : deserialize96(a, in + 96 * (size_t)i);
-    }
-    if (err == kOk && check && !(Quad ? in_subgroup_quad(a, q) : in_subgroup(a))) err = kNotInGroup;
-    if (!writes) return;
-    if (mode == 2) {
-        errs[i] = err == kOk ? 1 : 0;
+    if (!result && errs[i] != kOk) return;
+    const affine a = pts[i];
+    bool ok = true;
+    if (result) ok = (fp_is_zero_raw(a.x) && fp_is_zero_raw(a.y)) || on_curve_xy(a.x, a.y);
+    if (ok) ok = Quad ? in_subgroup_quad(a, q) : in_subgroup(a);
+    if (Quad) __syncwarp(q.mask);
+    if (Quad && q.k != 0) return;
+    if (result) {
+        errs[i] = ok ? 1 : 0;
         return;
     }
-    if (err == kOk) out[i] = a;
-    errs[i] = err;
+    if (ok) out[i] = a;
+    else errs[i] = kNotInGroup;
 }
 
-// Elements up to which a launch takes quads: one wave of them.
+// Elements up to which the membership test takes quads: one wave of them.
 constexpr size_t kQuadBlocksPerSm = 2;
+
+// Elements [lo, lo + m) of a call, on one stream.
+struct DecodeSlice {
+    const uint8_t* in;
+    uint8_t* din;
+    blst_p1_affine* out;
+    affine *dout, *pts;
+    int* errs;
+    int32_t* derr;
+    uint32_t m;
+    cudaStream_t st;
+};
+
+static cudaError_t decode_upload(const DecodeSlice& s, size_t elem)
+{
+    if (s.din) CATMSM_CHECK(cudaMemcpyAsync(s.din, s.in, s.m * elem, cudaMemcpyHostToDevice, s.st));
+    return cudaMemcpyAsync(s.dout, s.out, s.m * sizeof(affine), cudaMemcpyHostToDevice, s.st);
+}
+
+static cudaError_t decode_kernels(const DecodeSlice& s, int mode, bool check, bool quads)
+{
+    if (mode != 2) {
+        k_decode<<<div_up(s.m, kLaneThreads), kLaneThreads, 0, s.st>>>(s.din, s.m, mode, s.pts, s.derr);
+        g_stats.launches++;
+        CATMSM_CHECK(cudaGetLastError());
+    }
+    if (check) {
+        if (quads)
+            k_members<true><<<div_up(4 * (size_t)s.m, 128), 128, 0, s.st>>>(s.pts, s.m, mode == 2, s.dout, s.derr);
+        else
+            k_members<false><<<div_up(s.m, kLaneThreads), kLaneThreads, 0, s.st>>>(s.pts, s.m, mode == 2, s.dout,
+                                                                                   s.derr);
+        g_stats.launches++;
+        CATMSM_CHECK(cudaGetLastError());
+    }
+    return cudaSuccess;
+}
+
+static cudaError_t decode_download(const DecodeSlice& s, int mode)
+{
+    if (mode != 2) CATMSM_CHECK(cudaMemcpyAsync(s.out, s.dout, s.m * sizeof(affine), cudaMemcpyDeviceToHost, s.st));
+    return cudaMemcpyAsync(s.errs, s.derr, s.m * sizeof(int32_t), cudaMemcpyDeviceToHost, s.st);
+}
+
+// More elements than one wave run as two halves on two streams: the kernels of
+// one half fill the SMs that the last wave of the other's leave idle, and the
+// second half's upload and the first one's download run beside kernels.  One
+// stream -> two, checked uncompressing: 100003 elements 5.23 -> 4.95 ms, 200000
+// 9.44 -> 9.02, 300000 13.59 -> 13.13.  Three or more slices queue behind their own
+// streams' tails: 100003 elements 4.99 with three, 5.44 with four.  The caller's
+// arrays are read to the end before any of them is written.
+static cudaError_t decode_halves(DecodeSlice* s, AuxStream& aux, size_t elem, int mode, bool check)
+{
+    CATMSM_CHECK(aux.begin(s[0].st));
+    CATMSM_CHECK(decode_upload(s[0], elem));
+    CATMSM_CHECK(decode_kernels(s[0], mode, check, false));
+    CATMSM_CHECK(decode_upload(s[1], elem));
+    CATMSM_CHECK(aux.end(s[0].st));
+    CATMSM_CHECK(decode_kernels(s[1], mode, check, false));
+    CATMSM_CHECK(decode_download(s[0], mode));
+    return decode_download(s[1], mode);
+}
 
 static int decode_run(const uint8_t* in, size_t elem, int mode, size_t n, blst_p1_affine* out, int* errs,
                       int check_group)
@@ -298,27 +372,45 @@ static int decode_run(const uint8_t* in, size_t elem, int mode, size_t n, blst_p
     Ctx* ctx = get_ctx();
     if (!ctx) return (int)cudaErrorInitializationError;
     cudaStream_t st = ctx->stream;
+    AuxStream& aux = ctx->msm.aff.aux;
+    const bool check = mode == 2 || check_group;
     uint8_t* din = mode == 2 ? nullptr : (uint8_t*)ctx->msm.scalars.get(n * elem);
     affine* dout = (affine*)ctx->msm.points.get(n * sizeof(affine));
     int32_t* derr = (int32_t*)ctx->msm.digits.get(n * 4);
-    if ((mode != 2 && !din) || !dout || !derr) return (int)cudaErrorMemoryAllocation;
-    cudaError_t err = cudaSuccess;
-    if (mode != 2) err = cudaMemcpyAsync(din, in, n * elem, cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(dout, out, n * sizeof(affine), cudaMemcpyHostToDevice, st);
+    affine* pts = dout;                              // the decoded points, before the membership test:
+    if (mode == 0 && check) pts = (affine*)ctx->msm.buckets.get(n * sizeof(affine));
+    if (mode == 1 && check) pts = (affine*)din;      // each thread over its own 96 bytes
+    if ((mode != 2 && !din) || !dout || !derr || !pts) return (int)cudaErrorMemoryAllocation;
+    const size_t sms = (size_t)device_sms();
+    const bool halves = n > kLaneThreads * kLaneBlocks * sms;
+    const size_t cut = halves ? n / 2 / kLaneThreads * kLaneThreads : n;
+    cudaError_t err = halves ? aux.ensure(st) : cudaSuccess;
     if (err == cudaSuccess) {
-        const bool quads = (mode == 2 || check_group) && n <= kQuadBlocksPerSm * 32 * (size_t)device_sms();
-        if (quads)
-            k_decode<true><<<div_up(4 * n, 128), 128, 0, st>>>(din, (uint32_t)n, mode, check_group, dout, derr);
-        else
-            k_decode<false><<<div_up(n, 64), 64, 0, st>>>(din, (uint32_t)n, mode, check_group, dout, derr);
-        g_stats.launches++;
-        err = cudaGetLastError();
+        DecodeSlice s[2];
+        for (int k = 0; k < 2; k++) {
+            const size_t lo = k ? cut : 0;
+            s[k] = DecodeSlice{mode == 2 ? nullptr : in + lo * elem,
+                               mode == 2 ? nullptr : din + lo * elem,
+                               out + lo,
+                               dout + lo,
+                               pts + lo,
+                               errs + lo,
+                               derr + lo,
+                               (uint32_t)(k ? n - cut : cut),
+                               k ? aux.stream : st};
+        }
+        if (halves) {
+            err = decode_halves(s, aux, elem, mode, check);
+            const cudaError_t e = cudaStreamSynchronize(aux.stream);
+            if (err == cudaSuccess) err = e;
+        } else {
+            err = decode_upload(s[0], elem);
+            if (err == cudaSuccess) err = decode_kernels(s[0], mode, check, n <= kQuadBlocksPerSm * 32 * sms);
+            if (err == cudaSuccess) err = decode_download(s[0], mode);
+        }
     }
-    if (err == cudaSuccess && mode != 2)
-        err = cudaMemcpyAsync(out, dout, n * sizeof(affine), cudaMemcpyDeviceToHost, st);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(errs, derr, n * 4, cudaMemcpyDeviceToHost, st);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-    return (int)err;
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return (int)(err == cudaSuccess ? e : err);
 }
 
 }  // namespace catmsm

@@ -211,7 +211,8 @@ __device__ __forceinline__ void fp_mul_impl(fp& r, const fp& a, const fp& b)
 // (CATMSM_INLINE_MUL2), which have few call sites: accumulating mixed additions
 // 2.50 -> 2.45 ms (300007-point MSM without affine rounds), a 2^16 FFT 28.9 ->
 // 28.3.  Inlining the multiplication as well is slower again (2.59, 33.7 ms),
-// and decoding keeps the calls (300000 elements 13.8 -> 15.3 ms inlined).
+// and decoding keeps the calls (300000 elements 13.8 -> 14.3 ms inlined) but for
+// the loop of fp_pow, which inlines its squaring everywhere (-> 13.6).
 static __device__ __noinline__ fp fp_mul_call(const fp a, const fp b)
 {
     fp r;
@@ -539,12 +540,17 @@ static __device__ __noinline__ fp fp_sqr_call(const fp a)
     return r;
 }
 
-__device__ __forceinline__ void fp_sqr(fp& r, const fp& a)
+__device__ __forceinline__ void fp_sqr_inline(fp& r, const fp& a)
 {
-#ifdef CATMSM_INLINE_SQR
     fp t;
     fp_sqr_impl(t, a);
     r = t;
+}
+
+__device__ __forceinline__ void fp_sqr(fp& r, const fp& a)
+{
+#ifdef CATMSM_INLINE_SQR
+    fp_sqr_inline(r, a);
 #else
     r = fp_sqr_call(a);
 #endif
@@ -754,7 +760,7 @@ __device__ __forceinline__ void fp_pow(fp& r, const fp& a, const uint32_t* e)
     int i = 383;
     while (i >= 0) {
         if (!((e[i >> 5] >> (i & 31)) & 1)) {
-            if (started) fp_sqr(acc, acc);
+            if (started) fp_sqr_inline(acc, acc);
             i--;
             continue;
         }
@@ -764,7 +770,7 @@ __device__ __forceinline__ void fp_pow(fp& r, const fp& a, const uint32_t* e)
         for (int b = i; b >= l; b--) w = (w << 1) | ((e[b >> 5] >> (b & 31)) & 1);
         if (started) {
 #pragma unroll 1
-            for (int b = i; b >= l; b--) fp_sqr(acc, acc);
+            for (int b = i; b >= l; b--) fp_sqr_inline(acc, acc);
             fp_mul(acc, acc, T[w >> 1]);
         } else {
             acc = T[w >> 1];

@@ -31,3 +31,31 @@ def test_decode_same_at_every_size(gpu, oracle, synth):
         assert out == (aff * reps)[:96 * n]
         rc, member = gpu.p1s_affine_in_g1(out, n)
         assert rc == 0 and all(member)                         # failed elements keep the zero bytes: the identity
+
+
+@pytest.mark.parametrize("extra", [0, 1, 64, 65])
+def test_decode_halves_same_codes_and_bytes(gpu, oracle, synth, extra):
+    # one wave of lanes (512 elements per SM) is the line to two halves; every entry point
+    import torch
+    n = 512 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    base = 61
+    pts = gpu.points_from_scalars(synth.point_scalars(9, base), base)
+    one = ((1 << 384) % P).to_bytes(48, "little")
+    comp = bytearray(b"".join(oracle.compress(pts[96 * i:96 * i + 96] + one) for i in range(base)))
+    for i in range(0, base, 4):
+        comp[48 * i + 7] ^= 0x3c
+    flat = bytearray()
+    for i in range(base):                                      # big-endian x, y; every fifth y changed
+        c = [int.from_bytes(pts[96 * i + 48 * k:96 * i + 48 * k + 48], "little") * pow(1 << 384, -1, P) % P
+             for k in (0, 1)]
+        flat += c[0].to_bytes(48, "big") + ((c[1] + (i % 5 == 0)) % P).to_bytes(48, "big")
+    reps = n // base + 1
+    for data, elem, compressed in ((bytes(comp), 48, True), (bytes(flat), 96, False)):
+        for check in (True, False):
+            rc, ref, aff = gpu.p1s_decode(data, base, compressed, check_group=check)
+            assert rc == 0 and len(set(ref)) > 1 and ref[1] == 0
+            rc, errs, out = gpu.p1s_decode((data * reps)[:elem * n], n, compressed, check_group=check)
+            assert rc == 0 and errs == (ref * reps)[:n] and out == (aff * reps)[:96 * n]
+    rc, ref = gpu.p1s_affine_in_g1(aff, base)
+    rc, member = gpu.p1s_affine_in_g1((aff * reps)[:96 * n], n)
+    assert rc == 0 and list(member) == (list(ref) * reps)[:n]
