@@ -47,12 +47,12 @@
 
 namespace catmsm {
 
-constexpr int kAffThreads = 128;
+constexpr int kAffThreads = 64;         // 128: 2^20 points 5.57 -> 5.53 ms, 300007 2.337 -> 2.325 (shorter last waves)
 constexpr uint32_t kAffGroup = 16;      // lanes that share an inversion
 // Resident blocks per SM the round kernels are compiled for (register limit
-// 65536 / (128 x this)).
+// 65536 / (64 x this)).
 #ifndef CATMSM_AFF_MIN_BLOCKS
-#define CATMSM_AFF_MIN_BLOCKS 4
+#define CATMSM_AFF_MIN_BLOCKS 8
 #endif
 
 // 48 bytes (one coordinate) from a 16-byte aligned address.  Mutable: data
