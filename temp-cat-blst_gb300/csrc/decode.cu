@@ -38,9 +38,6 @@ __device__ __constant__ static const uint32_t FP_SQRT_E[12] = { // (p + 1) / 4
 __device__ __constant__ static const uint32_t FP_HALF[12] = {   // (p - 1) / 2
     0xffffd555u, 0xdcff7fffu, 0x58a9ffffu, 0x0f55ffffu, 0x7b587b12u, 0xb3986950u,
     0x79c2895fu, 0xb23ba5c2u, 0x21a5d66bu, 0x258dd3dbu, 0x1cbff34du, 0x0d0088f5u};
-__device__ __constant__ static const uint32_t FP_BETA2[12] = {  // beta^2 (Montgomery)
-    0x798a64e8u, 0x30f1361bu, 0x7ece5a2au, 0xf3b8ddabu, 0xc61577f7u, 0x16a8ca3au,
-    0x74fd029bu, 0xc26a2ff8u, 0x60701c6eu, 0x3636b766u, 0x241b6160u, 0x051ba4abu};
 
 __device__ __forceinline__ void fp_from_be(fp& r, const uint8_t* b)
 {
@@ -170,36 +167,6 @@ __device__ int deserialize96(affine& out, const uint8_t* in)
         return kOk;
     }
     return kBadEncoding;
-}
-
-// |z| = 0xd201000000010000 as runs of doublings, each but the last followed by
-// one addition (the reference's addition chain)
-__device__ __constant__ static const uint8_t Z_RUNS[6] = {1, 2, 3, 9, 32, 16};
-
-// out = |z| (ax, ay)
-__device__ __forceinline__ void times_abs_z(jac& out, const fp& ax, const fp& ay)
-{
-    out.x = ax;
-    out.y = ay;
-    fp_set_one(out.z);
-#pragma unroll 1
-    for (int r = 0; r < 6; r++) {
-#pragma unroll 1
-        for (int i = Z_RUNS[r]; i > 0; i--) jac_dbl(out);
-        if (r < 5) jac_madd(out, ax, ay);
-    }
-}
-
-// The same by a quad, distributed; lane k passes coordinate k mod 2.
-__device__ __forceinline__ void qd_times_abs_z(fp& out, const fp& a, const quad_lane& q)
-{
-    qd_set_affine(out, a, q);
-#pragma unroll 1
-    for (int r = 0; r < 6; r++) {
-#pragma unroll 1
-        for (int i = Z_RUNS[r]; i > 0; i--) qd_dbl(out, q);
-        if (r < 5) qd_madd(out, a, q);
-    }
 }
 
 // Whether a point of the curve is in G1: phi^2(P) == -z^2 P.  Both products by |z|

@@ -15,15 +15,19 @@
 //                      the GPU: the multiply pipe bounds it (~80% busy), so it
 //                      takes the fewest multiplications: n/2 scalar
 //                      multiplications a level.
-//   k_fft_items + k_fft_combine  q levels at once, for batches that do not:
-//                      there a level lasts as long as ONE scalar multiplication
-//                      (~0.7 ms), whatever its count, so q levels are rewritten as
-//                      sums over products of roots.  Every output of a 2^q-point
+//   k_fft_items + k_fft_quarter + k_fft_combine  q levels at once: a level lasts as
+//                      long as ONE scalar multiplication (0.6 to 1.5 ms) while it
+//                      does not fill the GPU, so q levels are rewritten as sums over
+//                      products of roots.  Every output of a 2^q-point
 //                      block is sum_m +- (root product) x_m, each product
 //                      of a point by a root product is an item of its own
 //                      ((4^q - 1) / 3 of them per block, all independent), and
-//                      the combine adds them up.  Twice (q = 2) to 2.7 times (q = 4) the
-//                      scalar multiplications per level, q times fewer in sequence.
+//                      the combine adds them up.  Products by roots a quarter of
+//                      the circle apart are one product and a quarter turn, which
+//                      costs a third: for q = 2 three products and a turn where
+//                      two levels of butterflies have four.  2^14 points, inverse:
+//                      14.47 -> 11.52 ms, 2^10: 2.76 -> 2.66, six transforms of
+//                      2^10 .. 2^16: 46.7 -> 43.7.
 //   k_fft_finish_multi Jacobian, canonical coordinates.
 // The inverse's 1/n scale is multiplied into the roots of a job's last pass.
 // Each butterfly is ~1.5k Fp multiplications (~0.9M IMAD) against 768 bytes of
@@ -254,6 +258,73 @@ __device__ __forceinline__ PassGeom pass_geom(const FftJob& J, uint32_t s0, uint
     return g;
 }
 
+// Butterfly bf of a job's pass: block g (position-wise) and j < 2^s0.  With a
+// multiple of 32 active blocks they run fastest, so the lanes of a warp share
+// their roots (true is returned).
+__device__ __forceinline__ bool pass_pos(const PassGeom& G, uint32_t s0, uint32_t bf, uint32_t& g, uint32_t& j)
+{
+    const bool shared = (G.active & 31u) == 0;
+    g = active_group(shared ? bf % G.active : bf >> s0, G.active, G.groups);
+    j = shared ? bf / G.active : bf & ((1u << s0) - 1);
+    return shared;
+}
+
+__device__ __constant__ static const uint32_t FR_Z3[8] = {       // z^3 (Montgomery)
+    0x55763050u, 0x0c4fa98au, 0x9ff7a200u, 0x4c8ea2c2u,
+    0xe43b5ddfu, 0x649fca48u, 0xfc43f9d3u, 0x26c0c34du};
+
+// Quarter turns.  z = -0xd201000000010000 is a 12th root of unity mod r, so the
+// roots of order 4 are +-z^3, and z^3 P = |z| phi^2(P) costs 63 doublings and 5
+// additions, about a third of a product.  In a table of powers the root of level
+// t (from 0, t >= 1) at j + h (k + 2^(t - 1)), k < 2^(t - 1), is +-z^3 times its root at j + h k.
+// So of the items with top bit t only those with k < 2^(t - 1) are multiplied, and
+//   V = +-z^3 sum over those m of (-1)^popc(m & u) (item (m, k)),  u = k + 2^(t - 1),
+// stands for all the items (m, u): 3, 11, 43 products and 1, 3, 7 quarter turns for q
+// = 2, 3, 4 instead of 5, 21, 85 products.  The table is the caller's and may hold
+// anything: each use compares the two roots, and without the relation the items are
+// multiplied.
+// Returns 0 (no relation), or +-1: the sign of z^3.
+__device__ __forceinline__ int quarter_sign(const FftJob& J, uint32_t s0, uint32_t t, uint32_t pos)
+{
+    const uint32_t i2 = pos * (J.n >> (s0 + t + 1)), i3 = i2 + (J.n >> 2);   // i3 < n / 2
+    uint32_t e[8], r[8];
+    for (int w = 0; w < 8; w++) {
+        e[w] = FR_Z3[w];
+        r[w] = J.roots[8 * (size_t)(J.inv_from_fwd ? J.n - i3 : i3) + w];
+    }
+    if (pos) {
+        uint32_t r2[8];
+        for (int w = 0; w < 8; w++) r2[w] = J.roots[8 * (size_t)(J.inv_from_fwd ? J.n - i2 : i2) + w];
+        fr_mul(e, e, r2);
+    }
+    uint32_t d = 0, s[8], z = 0;
+    fr_add(s, e, r);
+    for (int w = 0; w < 8; w++) {
+        d |= e[w] ^ r[w];
+        z |= s[w];
+    }
+    return d == 0 ? 1 : z == 0 ? -1 : 0;
+}
+
+// Product `it` of `items` in the order that a pass starts them.  With quarter turns:
+// the ones that are multiplied, x_0 (multiplied if the pass scales), the ones a turn
+// stands for; so the blocks with work come first and spread evenly over the SMs.
+__host__ __device__ __forceinline__ void item_order(uint32_t it, uint32_t items, bool turns, uint32_t& m, uint32_t& k)
+{
+    const uint32_t x0 = turns ? items / 2 : items - 1;
+    m = k = 0;
+    if (it == x0) return;
+    const bool late = it > x0;
+    uint32_t rem = late ? it - x0 : it, top = 1, wide = 1;               // wide: the k of one m
+    while (rem >= top * wide) {
+        rem -= top * wide;
+        top <<= 1;
+        wide = turns ? top >> 1 : top;
+    }
+    m = top + rem / wide;
+    k = rem % wide + (late ? wide : 0);
+}
+
 // The products of a pass: item-major per job (all items of one kind are
 // adjacent, so trivial ones do not share warps with multiplications).  Lanes per
 // item: 1, 2 (the pair form) or 4 (the quad form).  Split: the halves k1 x and
@@ -265,7 +336,7 @@ template <int Lanes, bool Split>
 __global__ void __launch_bounds__(kItemThreads, Lanes == 2 ? 6 : 4)
 k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* __restrict__ jobs,
             const uint32_t* __restrict__ lst_job, const uint32_t* __restrict__ lst_pre, uint32_t cnt, uint32_t total,
-            uint32_t s0, uint32_t q)
+            uint32_t s0, uint32_t q, uint32_t turns)
 {
     __shared__ __align__(16) unsigned char tabs[Lanes == 1   ? 16
                                                 : Lanes == 2 ? kItemThreads / 2 * sizeof(pair_table)
@@ -278,17 +349,21 @@ k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* _
     const uint32_t b = t - lst_pre[e];
     const uint32_t bf = b % G.bf, half = Split ? b / G.bf & 1 : 0;
     const uint32_t it = b / G.bf >> (Split ? 1 : 0);
-    const uint32_t h = 1u << s0, j = bf & (h - 1);
-    const uint32_t g = active_group(bf >> s0, G.active, G.groups);
-    uint32_t m = 0, k = 0;
-    if (it) {
-        uint32_t top = 1, rem = it - 1;              // rem in [0, top^2) at top = 2^t
-        while (rem >= top * top) {
-            rem -= top * top;
-            top <<= 1;
+    const uint32_t h = 1u << s0;
+    uint32_t g, j, m, k;
+    const bool shared = pass_pos(G, s0, bf, g, j);
+    item_order(it, pass_items(G.q), turns != 0, m, k);
+    xyzz* dst = prod + lst_pre[e] + (((size_t)item_of(m, k) << (Split ? 1 : 0)) + half) * G.bf + bf;
+    if (turns && k) {
+        const uint32_t top = 31 - __clz(m), turn = 1u << (top - 1);
+        if ((k & turn) && quarter_sign(J, s0, top, j + h * (k - turn))) {    // k_fft_quarter writes V at m = 2^top
+            if ((m != 2 * turn || half) && threadIdx.x % Lanes == 0) {
+                xyzz o;
+                xyzz_set_inf(o);
+                store_xyzz(dst, o);
+            }
+            return;
         }
-        m = top + rem / top;
-        k = rem & (top - 1);
     }
     xyzz v;
     load_xyzz(v, a + J.val_off + ((size_t)g << (s0 + G.q)) + j + m * h);
@@ -317,22 +392,23 @@ k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* _
     }
     if (one) {
         if (half) xyzz_set_inf(v);
-        if (threadIdx.x % Lanes == 0) store_xyzz(prod + t, v);
+        if (threadIdx.x % Lanes == 0) store_xyzz(dst, v);
         return;
     }
     uint32_t kc[8], k12[8];
     fr_from_mont(kc, c);
     fr_glv_split(k12, k12 + 4, kc);
     if (Lanes == 1) {
-        xyzz_mult_glv(v, v, k12, k12 + 4);
-        store_xyzz(prod + t, v);
+        if (shared) xyzz_mult_glv_shared(v, v, k12, k12 + 4);
+        else xyzz_mult_glv(v, v, k12, k12 + 4);
+        store_xyzz(dst, v);
     } else if (Lanes == 2) {
         const pair_lane l{(threadIdx.x & 1) != 0, 3u << (threadIdx.x & 30)};
         fp lo, hi;
         pd_mult_glv(lo, hi, v, k12, k12 + 4, reinterpret_cast<pair_table*>(tabs) + threadIdx.x / 2, l);
         const quad_lane w0{l.odd ? 1u : 0u, 0}, w1{l.odd ? 3u : 2u, 0};     // the coordinates this lane holds
-        qd_store(prod + t, lo, w0);
-        qd_store(prod + t, hi, w1);
+        qd_store(dst, lo, w0);
+        qd_store(dst, hi, w1);
     } else {
         const quad_lane ql = quad_of(threadIdx.x & 31);
         if (half) {
@@ -341,8 +417,77 @@ k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* _
             for (int w = 0; w < 12; w++) beta.v[w] = FP_BETA[w];
             fp_mul(v.x, v.x, beta);
         }
-        qd_store(prod + t, qd_mult_glv<Split>(v, half ? k12 + 4 : k12, k12 + 4,
+        qd_store(dst, qd_mult_glv<Split>(v, half ? k12 + 4 : k12, k12 + 4,
                                               reinterpret_cast<quad_table*>(tabs) + threadIdx.x / 4, ql), ql);
+    }
+}
+
+// The V of a pass: one lane or a quad per (butterfly, u), u < 2^(q - 1), u-major per
+// job, which is half a job's outputs; u = 0, the last, has none.
+template <bool Quad>
+__global__ void __launch_bounds__(64, 4)
+k_fft_quarter(xyzz* prod, const FftJob* __restrict__ jobs, const uint32_t* __restrict__ lst_job,
+              const uint32_t* __restrict__ lst_pre, const uint32_t* __restrict__ lst_out, uint32_t cnt, uint32_t total,
+              uint32_t s0, uint32_t q, uint32_t split)
+{
+    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = Quad ? gt >> 2 : gt;
+    if (t >= total) return;
+    const uint32_t e = find_range(lst_out, cnt, 2 * t);
+    const FftJob J = jobs[lst_job[e]];
+    const PassGeom G = pass_geom(J, s0, q);
+    const uint32_t b = t - lst_out[e] / 2;
+    const uint32_t bf = b % G.bf, u = (1u << (G.q - 1)) - 1 - b / G.bf;
+    if (u == 0) return;
+    const uint32_t turn = 1u << (31 - __clz(u)), k = u - turn, top = 2 * turn;
+    uint32_t g, j;
+    pass_pos(G, s0, bf, g, j);
+    const int sign = quarter_sign(J, s0, 32 - __clz(u), j + (k << s0));
+    if (!sign) return;
+    xyzz* p = prod + lst_pre[e] + bf;
+    xyzz* dst = p + ((size_t)item_of(top, u) << split) * G.bf;
+    fp b2;
+#pragma unroll
+    for (int w = 0; w < 12; w++) b2.v[w] = FP_BETA2[w];
+    if (Quad) {
+        const quad_lane ql = quad_of(threadIdx.x & 31);
+        fp d;
+        fp_zero(d);
+#pragma unroll 1
+        for (uint32_t i = 0; i < top << split; i++) {
+            const uint32_t m = top + (i >> split);
+            fp v = qd_load(p + (((size_t)item_of(m, k) << split) + (i & split)) * G.bf, ql.k);
+            if (((__popc(m & u) & 1) != 0) != (sign < 0) && ql.k == 1) fp_neg(v, v);
+            qd_add(d, v, ql);
+        }
+        const fp x = fp_mul_call(d, b2);
+        d = fp_sel(d, x, ql.k == 0);
+        const fp base = fp_swap(d, 2, ql);
+        fp o;
+        qd_times_abs_z(o, fp_sel(base, d, ql.k < 2), ql);
+        const fp zz = fp_mul_call(o, d);                 // lanes 2, 3: back from the curve scaled by d's z
+        qd_store(dst, fp_sel(o, zz, ql.k >= 2), ql);
+    } else {
+        xyzz d, v;
+        xyzz_set_inf(d);
+#pragma unroll 1
+        for (uint32_t i = 0; i < top << split; i++) {
+            const uint32_t m = top + (i >> split);
+            load_xyzz(v, p + (((size_t)item_of(m, k) << split) + (i & split)) * G.bf);
+            if (((__popc(m & u) & 1) != 0) != (sign < 0)) fp_neg(v.y, v.y);
+            xyzz_add(d, v);
+        }
+        fp_mul(d.x, d.x, b2);
+        jac o;
+        times_abs_z(o, d.x, d.y);
+        fp zz;
+        fp_sqr(zz, o.z);
+        fp_mul(d.zz, d.zz, zz);
+        fp_mul(zz, zz, o.z);
+        fp_mul(d.zzz, d.zzz, zz);
+        d.x = o.x;
+        d.y = o.y;
+        store_xyzz(dst, d);
     }
 }
 
@@ -370,8 +515,9 @@ __global__ void __launch_bounds__(128) k_fft_combine(const xyzz* __restrict__ pr
         const PassGeom G = pass_geom(J, s0, q);
         const uint32_t b = o - lst_out[e];
         const uint32_t k = b / G.bf, bf = b % G.bf;
-        const uint32_t h = 1u << s0;
-        dst = J.val_off + (active_group(bf >> s0, G.active, G.groups) << (s0 + G.q)) + (bf & (h - 1)) + k * h;
+        uint32_t g, j;
+        pass_pos(G, s0, bf, g, j);
+        dst = J.val_off + (g << (s0 + G.q)) + j + (k << s0);
         const xyzz* p = prod + lst_pre[e] + bf;
         if (2 * qi < (1u << (G.q + split))) {
             const uint32_t m0 = 2 * qi >> split, m1 = (2 * qi + 1) >> split;
@@ -440,22 +586,21 @@ static size_t fft_quad_wave()
 // One pass: levels s0 + 1 .. s0 + q.
 struct FftPass {
     uint32_t s0 = 0, q = 1, group = 0;
-    uint32_t split = 0;
+    uint32_t split = 0, turns = 0;
     enum { kStage, kQuads, kPairs, kLanes } kind = kStage;
     uint32_t off = 0, cnt = 0;          // its entries of the job lists
     uint32_t items = 0, outputs = 0;
 };
 
-// Products of a butterfly of a pass that are multiplications: all of its items
-// but x_0, less (first pass, j = 0 throughout) those without a root.
-static size_t pass_products(uint32_t s0, uint32_t q)
+// Products of a butterfly of a pass that are multiplications: without x_0, items that
+// quarter turns stand for and (first pass, j = 0 throughout) those without a root.
+static size_t pass_products(uint32_t s0, uint32_t q, bool turns)
 {
-    if (s0) return pass_items(q) - 1;
     size_t c = 0;
     for (uint32_t m = 1; m < (1u << q); m++) {
         const uint32_t top = 1u << (31 - __builtin_clz(m));
-        for (uint32_t k = 0; k < top; k++) {
-            bool root = false;
+        for (uint32_t k = 0; k < (turns && top > 1 ? top / 2 : top); k++) {
+            bool root = s0 != 0;
             for (uint32_t i = 1; i < q; i++) root |= ((m >> i) & 1u) && (k & ((1u << i) - 1));
             c += root;
         }
@@ -463,18 +608,20 @@ static size_t pass_products(uint32_t s0, uint32_t q)
     return c;
 }
 
-// Items, multiplications and outputs of a pass over every job that has its first level.
+// Items, multiplications (without and with quarter turns) and outputs of a pass over
+// every job that has its first level.
 static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uint32_t q, size_t& items,
-                        size_t& products, size_t& outputs)
+                        size_t products[2], size_t& outputs)
 {
-    items = products = outputs = 0;
+    items = products[0] = products[1] = outputs = 0;
     for (const FftJob* job : jobs) {
         const FftJob& J = *job;
         if (J.logn <= s0) continue;
         const uint32_t qe = std::min(q, J.logn - s0);
         const size_t bf = (size_t)std::min(J.n >> (s0 + qe), J.xn) << s0;
         items += bf * pass_items(qe);
-        products += bf * pass_products(s0, qe);
+        const bool scaled = J.scale && s0 + qe == J.logn;          // x_0 as well
+        for (int t = 0; t < 2; t++) products[t] += bf * (pass_products(s0, qe, t != 0) + (scaled ? 1 : 0));
         outputs += bf << qe;
     }
 }
@@ -483,26 +630,32 @@ static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uin
 // GB300 (wave = 9728 quads, 4 blocks of 16 on each of 152 SMs; three waves' worth of
 // pairs and four of lanes are resident at once).  Every form lasts one
 // multiplication's latency as long as a warp has its scheduler to itself (quads
-// 0.75 ms, the halves of a split product 0.64, pairs 0.98, lanes 1.65), more when
-// two share it, and adds up beyond a wave; a sum costs kSumMs per product.
+// 0.78 ms, the halves of a split product 0.64, pairs 0.99, lanes 1.5; a quarter
+// turn by a quad 0.25), more when two share it, and adds up beyond a wave; a sum
+// costs kSumMs per product.
 static double quads_ms(size_t items, size_t wave, bool split)
 {
-    const double part = split ? 0.65 : 0.76, full = split ? 0.95 : 1.03;
-    const size_t rem = items % wave;
-    return full * (double)(items / wave) + (rem == 0 ? 0.0 : rem <= 3 * wave / 10 ? part : full);
+    if (items <= wave / 2) return items == 0 ? 0.0 : split ? 0.64 : 0.78;
+    return (split ? 0.83 : 1.0) * (double)((items + wave - 1) / wave);
 }
 
 static double pairs_ms(size_t items, size_t wave)
 {
     const size_t rem = items % (3 * wave);
-    return 2.05 * (double)(items / (3 * wave)) +
-           (rem == 0 ? 0.0 : rem <= 6 * wave / 10 ? 1.0 : rem <= 5 * wave / 4 ? 1.33 : 2.05);
+    return 2.03 * (double)(items / (3 * wave)) +
+           (rem == 0 ? 0.0 : rem <= wave ? 0.99 : rem <= 3 * wave / 2 ? 1.32 : 2.03);
 }
 
 static double lanes_ms(size_t items, size_t wave)
 {
     const size_t rem = items % (4 * wave);
-    return 2.4 * (double)(items / (4 * wave)) + (rem == 0 ? 0.0 : rem <= 2 * wave ? 1.65 : 1.95);
+    return 2.3 * (double)(items / (4 * wave)) + (rem == 0 ? 0.0 : rem <= 2 * wave ? 1.5 : 2.07);
+}
+
+static double quarter_ms(size_t turns, size_t wave)
+{
+    if (turns <= wave) return turns <= wave / 2 ? 0.26 : turns <= 7 * wave / 10 ? 0.34 : 0.49;
+    return 0.62 + 0.8 * (double)(turns / (4 * wave));
 }
 
 static double stage_ms(size_t butterflies, size_t wave)
@@ -511,11 +664,12 @@ static double stage_ms(size_t butterflies, size_t wave)
     return 0.5 + 2.3 * (double)butterflies / (double)(4 * wave);
 }
 
-// Several levels a pass only where the jobs have the GPU to themselves (solo): next to
-// another group the launches add up, and one level at a time is the least work.
+// Next to another group of jobs (not solo) the launches share the GPU: there a pass
+// costs its part of a full wave, and its forms are a level of butterflies or two levels
+// by lanes with quarter turns, the least work.
 static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, bool solo)
 {
-    constexpr double kSumMs = 0.8e-6, kLaunchMs = 0.02;
+    constexpr double kSumMs = 0.5e-6, kSumsMs = 0.03, kFullMs = 0.57;     // kFullMs: wave products of a full launch
     constexpr uint32_t kMaxQ = 4;
     constexpr size_t kMaxItems = size_t(1) << 18;    // 50 MB of products
     const size_t wave = fft_quad_wave();
@@ -525,28 +679,43 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
     std::vector<FftPass> via(maxlog + 1);
     best[0] = 0;
     for (uint32_t s = 0; s < maxlog; s++) {
-        for (uint32_t q = 1; q <= (solo ? kMaxQ : 1) && s + q <= maxlog; q++) {
-            size_t items, products, outputs;
+        for (uint32_t q = 1; q <= (solo ? kMaxQ : 2) && s + q <= maxlog; q++) {
+            size_t items, products[2], outputs;
             pass_counts(jobs, s, q, items, products, outputs);
             FftPass p;
             p.s0 = s;
             p.q = q;
-            double ms = q == 1 ? stage_ms(outputs / 2, wave) : 1e300;
-            if (solo && items <= kMaxItems) {
-                const double sums = kLaunchMs * q + kSumMs * (double)outputs * (1u << q);
+            double ms = 1e300;
+            if (q == 1) {
+                const double bf = (double)outputs / 2, scaled = (double)products[0] - (s ? bf : 0);
+                ms = (solo ? stage_ms(outputs / 2, wave) : kFullMs / (double)wave * bf) * (1 + 0.85 * scaled / bf);
+            }
+            for (uint32_t turns = solo ? 0 : 1; items <= kMaxItems && turns < (q > 1 ? 2u : 1u); turns++) {
+                // the products of a first pass are not adjacent: its SMs have uneven shares
+                const size_t n = s || turns ? products[turns] : products[turns] * 3 / 2;
+                const size_t v = outputs / 2 - (outputs >> q);
+                const double sums = kSumsMs + kSumMs * (double)outputs * (1u << q);
+                const double turn = turns ? quarter_ms(v, wave) : 0.0;
+                if (!solo) {
+                    ms = kFullMs / (double)wave * ((double)n + (double)v / 3) + sums;
+                    p.kind = FftPass::kLanes;
+                    p.turns = 1;
+                    continue;
+                }
                 const struct {
                     decltype(p.kind) kind;
                     uint32_t split;
                     double ms;
-                } forms[] = {{FftPass::kLanes, 0, lanes_ms(products, wave) + sums},
-                             {FftPass::kPairs, 0, pairs_ms(products, wave) + sums},
-                             {FftPass::kQuads, 0, quads_ms(products, wave, false) + sums},
-                             {FftPass::kQuads, 1, q <= 3 ? quads_ms(2 * products, wave, true) + 2 * sums : 1e300}};
+                } forms[] = {{FftPass::kLanes, 0, lanes_ms(n, wave) + sums},
+                             {FftPass::kPairs, 0, pairs_ms(n, wave) + sums},
+                             {FftPass::kQuads, 0, quads_ms(n, wave, false) + sums},
+                             {FftPass::kQuads, 1, q <= 3 ? quads_ms(2 * n, wave, true) + 2 * sums : 1e300}};
                 for (const auto& f : forms)
-                    if (f.ms < ms) {
+                    if (f.ms + turn < ms) {
                         p.kind = f.kind;
                         p.split = f.split;
-                        ms = f.ms;
+                        p.turns = turns;
+                        ms = f.ms + turn;
                     }
             }
             if (best[s] + ms < best[s + q]) {
@@ -698,13 +867,23 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
         const uint32_t lanes = p.kind == FftPass::kQuads ? 4 : p.kind == FftPass::kPairs ? 2 : 1;
         const unsigned grid = div_up((size_t)lanes * p.items, kItemThreads);
         if (p.split)
-            k_fft_items<4, true><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+            k_fft_items<4, true><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q, p.turns);
         else if (lanes == 4)
-            k_fft_items<4, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+            k_fft_items<4, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q, p.turns);
         else if (lanes == 2)
-            k_fft_items<2, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+            k_fft_items<2, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q, p.turns);
         else
-            k_fft_items<1, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q);
+            k_fft_items<1, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q, p.turns);
+        if (p.turns) {
+            const uint32_t turns = p.outputs / 2;
+            if (turns <= 2 * fft_quad_wave())
+                k_fft_quarter<true><<<div_up(4 * (size_t)turns, 64), 64, 0, ps>>>(
+                    pp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, turns, p.s0, p.q, p.split);
+            else
+                k_fft_quarter<false><<<div_up(turns, 64), 64, 0, ps>>>(pp, d_jobs, lj, li, d_lst_out + p.off, p.cnt,
+                                                                       turns, p.s0, p.q, p.split);
+            g_stats.launches++;
+        }
         k_fft_combine<<<div_up((size_t)p.outputs << (p.q + 1 + p.split), 128), 128, 0, ps>>>(
             pp, tmp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, p.outputs, p.s0, p.q, p.split);
         g_stats.launches += 2;

@@ -621,4 +621,38 @@ static __device__ __noinline__ void pd_mult_glv(fp& lo, fp& hi, const xyzz& P, c
     lo = p.c;
 }
 
+__device__ __constant__ static const uint32_t FP_BETA2[12] = {  // beta^2 (Montgomery)
+    0x798a64e8u, 0x30f1361bu, 0x7ece5a2au, 0xf3b8ddabu, 0xc61577f7u, 0x16a8ca3au,
+    0x74fd029bu, 0xc26a2ff8u, 0x60701c6eu, 0x3636b766u, 0x241b6160u, 0x051ba4abu};
+
+// |z| = 0xd201000000010000 as runs of doublings, each but the last followed by
+// one addition (the reference's addition chain)
+__device__ __constant__ static const uint8_t Z_RUNS[6] = {1, 2, 3, 9, 32, 16};
+
+// out = |z| (ax, ay)
+__device__ __forceinline__ void times_abs_z(jac& out, const fp& ax, const fp& ay)
+{
+    out.x = ax;
+    out.y = ay;
+    fp_set_one(out.z);
+#pragma unroll 1
+    for (int r = 0; r < 6; r++) {
+#pragma unroll 1
+        for (int i = Z_RUNS[r]; i > 0; i--) jac_dbl(out);
+        if (r < 5) jac_madd(out, ax, ay);
+    }
+}
+
+// The same by a quad, distributed; lane k passes coordinate k mod 2.
+__device__ __forceinline__ void qd_times_abs_z(fp& out, const fp& a, const quad_lane& q)
+{
+    qd_set_affine(out, a, q);
+#pragma unroll 1
+    for (int r = 0; r < 6; r++) {
+#pragma unroll 1
+        for (int i = Z_RUNS[r]; i > 0; i--) qd_dbl(out, q);
+        if (r < 5) qd_madd(out, a, q);
+    }
+}
+
 }  // namespace catmsm

@@ -127,3 +127,85 @@ def test_passes_match_oracle(gpu, oracle, n, mode):
     for i in range(n):
         s = slice(144 * i, 144 * i + 144)
         assert oracle.serialize(got[1][s]) == oracle.serialize(ref[1][s]), i
+
+
+def item_order(it, items, turns):
+    """Started `it`-th -> (m, k mod 2^t), as k_fft_items numbers them."""
+    x0 = items // 2 if turns else items - 1
+    if it == x0:
+        return 0, 0
+    late, top, wide = it > x0, 1, 1
+    rem = it - x0 if late else it
+    while rem >= top * wide:
+        rem -= top * wide
+        top *= 2
+        wide = top // 2 if turns else top
+    return top + rem // wide, rem % wide + (wide if late else 0)
+
+
+Z3 = pow(-0xd201000000010000, 3, R)
+
+
+@pytest.mark.parametrize("n,q", [(4, 2), (16, 2), (16, 4), (64, 3), (64, 2)])
+@pytest.mark.parametrize("broken", [False, True])
+def test_quarter_turns_equal_the_products(n, q, broken):
+    # per butterfly: the items a turn stands for against the sum that replaces them
+    assert Z3 * Z3 % R == R - 1
+    assert {item_order(i, items_of(q), t) for i in range(items_of(q)) for t in (0, 1)} == \
+        {decode(i) for i in range(items_of(q))}
+    w = pow(7, (R - 1) // n, R)
+    rnd = random.Random(n + q)
+    roots = [pow(w, i, R) for i in range(n)]
+    if broken:
+        for i in range(1, n, 3):
+            roots[i] = rnd.randrange(R)
+    turned = 0
+    for s0 in range(0, n.bit_length() - q):
+        h = 1 << s0
+        for j in range(h):
+            def root(t, pos):
+                return roots[pos * (n >> (s0 + t + 1))] if pos else 1
+
+            def coeff(m, k):
+                c = 1
+                for i in range(q):
+                    if m >> i & 1:
+                        c = c * root(i, j + h * (k & ((1 << i) - 1))) % R
+                return c
+            x = [rnd.randrange(R) for _ in range(1 << q)]
+            for u in range(1, 1 << (q - 1)):
+                t = u.bit_length()
+                turn = 1 << (t - 1)
+                k = u - turn
+                e = Z3 * root(t, j + h * k) % R
+                r3 = roots[(j + h * k) * (n >> (s0 + t + 1)) + n // 4]
+                assert r3 == root(t, j + h * u)
+                if r3 not in (e, R - e):
+                    assert broken
+                    continue
+                turned += 1
+                sign = 1 if r3 == e else -1
+                ms = range(1 << t, 2 << t)
+                want = sum((-1) ** bin(m & u).count("1") * coeff(m, u) * x[m] for m in ms) % R
+                got = sign * Z3 * sum((-1) ** bin(m & u).count("1") * coeff(m, k) * x[m] for m in ms) % R
+                assert want == got
+    assert turned or broken
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4, 16, 64, 256])
+@pytest.mark.parametrize("mode", ["fwd", "inv"])
+def test_turns_where_only_some_roots_are_powers(gpu, oracle, n, mode):
+    rnd = random.Random(7 + n)
+    jac = oracle.jacobian_randomize(n, n, oracle.gen_points(n, n))
+    ok, d = gpu.fr_fft_domain_init(n)
+    assert ok
+    d = bytearray(d)
+    for i in range(1, n):
+        if i > n // 4 and rnd.random() < 0.3:
+            d[32 * i:32 * i + 32] = (rnd.randrange(R) * (1 << 256) % R).to_bytes(32, "little")
+    got, ref = (x.p1_fft_with_domain(bytes(jac), n, bytes(d), n + 2, mode == "inv") for x in (gpu, oracle))
+    assert got[0] and ref[0]
+    for i in range(n):
+        s = slice(144 * i, 144 * i + 144)
+        assert oracle.serialize(got[1][s]) == oracle.serialize(ref[1][s]), i
