@@ -664,6 +664,11 @@ static double stage_ms(size_t butterflies, size_t wave)
     return 0.5 + 2.3 * (double)butterflies / (double)(4 * wave);
 }
 
+// Products of a pass of q levels: 50 MB; two levels, the form for large launches (1.5 products
+// per output), 805 MB.  64 transforms of 2^10 .. 2^16 (1.4 M points): 110.1 transforms/s at
+// one level a pass, 143.9 at two.
+static size_t pass_max_items(uint32_t q) { return size_t(1) << (q <= 2 ? 22 : 18); }
+
 // Next to another group of jobs (not solo) the launches share the GPU: there a pass
 // costs its part of a full wave, and its forms are a level of butterflies or two levels
 // by lanes with quarter turns, the least work.
@@ -671,7 +676,6 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
 {
     constexpr double kSumMs = 0.5e-6, kSumsMs = 0.03, kFullMs = 0.57;     // kFullMs: wave products of a full launch
     constexpr uint32_t kMaxQ = 4;
-    constexpr size_t kMaxItems = size_t(1) << 18;    // 50 MB of products
     const size_t wave = fft_quad_wave();
     uint32_t maxlog = 0;
     for (const FftJob* J : jobs) maxlog = std::max(maxlog, J->logn);
@@ -690,7 +694,7 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
                 const double bf = (double)outputs / 2, scaled = (double)products[0] - (s ? bf : 0);
                 ms = (solo ? stage_ms(outputs / 2, wave) : kFullMs / (double)wave * bf) * (1 + 0.85 * scaled / bf);
             }
-            for (uint32_t turns = solo ? 0 : 1; items <= kMaxItems && turns < (q > 1 ? 2u : 1u); turns++) {
+            for (uint32_t turns = solo ? 0 : 1; items <= pass_max_items(q) && turns < (q > 1 ? 2u : 1u); turns++) {
                 // the products of a first pass are not adjacent: its SMs have uneven shares
                 const size_t n = s || turns ? products[turns] : products[turns] * 3 / 2;
                 const size_t v = outputs / 2 - (outputs >> q);

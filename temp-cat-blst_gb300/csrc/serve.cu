@@ -137,7 +137,12 @@ size_t msm_mem(const Basis* b, size_t k)
     return std::max(plain, table);
 }
 
-size_t fft_mem(size_t n) { return n * 144 * 2 + n * 64 + (1 << 20); }
+// values, scratch, prepared and given roots, and the products of a pass
+size_t fft_mem(size_t n)
+{
+    const size_t products = std::max(std::min(6 * n, size_t(1) << 18), std::min(n + n / 2, size_t(1) << 22));
+    return n * (144 + 192 + 48 + 32) + products * 192 + (1 << 20);
+}
 
 // A large MSM through the plain pipeline over the basis points: the scalars
 // are copied to the worker context's device buffer first.
