@@ -199,8 +199,9 @@ int catmsm_p1_fft_device(void *d_values, size_t n, const void *d_domain, int mod
 /* A batch of G1 FFTs in one pass (no reference counterpart): transform i is
  * blst_p1_fft_with_domain(values[i], ns[i], domains[i], ns[i] + 2, ...) with
  * modes[i] = 0 forward, 1 inverse (scaled by domain[n]), 2 inverse unscaled
- * (as blst_p1_ifft_unscaled_with_domain).  Sizes may differ; every stage
- * level runs as one launch over all transforms that have it.  Any invalid
+ * (as blst_p1_ifft_unscaled_with_domain).  Sizes may differ; every pass
+ * (one or several levels) runs as one launch over all transforms that have it;
+ * large batches run as two groups of transforms on two streams.  Any invalid
  * entry (NULL values, bad size, domain length or tag, bad mode) returns
  * cudaErrorInvalidValue before anything is written.  Host buffers; returns 0
  * on success or a cudaError_t value (values untouched on failure). */
