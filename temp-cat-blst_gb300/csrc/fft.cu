@@ -11,23 +11,23 @@
 // (192 B) between the passes; a job descriptor per transform.
 //   k_bitrev_multi     Jacobian input -> XYZZ in bit-reversed order.
 //   then passes over the levels, each chosen by fft_plan for the whole batch:
-//   k_fft_stage_multi  one level, one lane per butterfly, for batches that fill
-//                      the GPU: the multiply pipe bounds it (~80% busy), so it
-//                      takes the fewest multiplications: n/2 scalar
-//                      multiplications a level.
-//   k_fft_items + k_fft_quarter + k_fft_combine  q levels at once: a level lasts as
-//                      long as ONE scalar multiplication (0.6 to 1.5 ms) while it
-//                      does not fill the GPU, so q levels are rewritten as sums over
-//                      products of roots.  Every output of a 2^q-point
-//                      block is sum_m +- (root product) x_m, each product
+//   k_fft_stage_multi  one level, one lane per butterfly: n/2 scalar multiplications,
+//                      one launch.  For sizes whose levels are a whole wave or less
+//                      (2^16 points) and for more products than a pass may hold.
+//   k_fft_items + k_fft_quarter + k_fft_combine  q levels at once.  Every output of
+//                      a 2^q-point block is sum_m +- (root product) x_m; each product
 //                      of a point by a root product is an item of its own
 //                      ((4^q - 1) / 3 of them per block, all independent), and
-//                      the combine adds them up.  Products by roots a quarter of
-//                      the circle apart are one product and a quarter turn, which
-//                      costs a third: for q = 2 three products and a turn where
-//                      two levels of butterflies have four.  2^14 points, inverse:
-//                      14.47 -> 11.52 ms, 2^10: 2.76 -> 2.66, six transforms of
-//                      2^10 .. 2^16: 46.7 -> 43.7.
+//                      the combine adds them up.  A launch that does not fill the GPU
+//                      lasts as long as ONE scalar multiplication (0.6 to 1.5
+//                      ms), so small transforms take q = 3 and 4.  Products by roots a
+//                      quarter of the circle apart are one product and a quarter
+//                      turn, which costs a third: for q = 2 three products and a turn
+//                      where two levels of butterflies have four, the least work
+//                      for launches that fill the GPU (the multiply pipe bounds them).
+//                      With turns against without: 2^14 points, inverse, 14.47 -> 11.52 ms,
+//                      2^10 2.76 -> 2.66, 2^20 514 -> 414, 64 transforms of 2^10 .. 2^16
+//                      581 -> 436 ms.
 //   k_fft_finish_multi Jacobian, canonical coordinates.
 // The inverse's 1/n scale is multiplied into the roots of a job's last pass.
 // Each butterfly is ~1.5k Fp multiplications (~0.9M IMAD) against 768 bytes of
@@ -423,7 +423,10 @@ k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* _
 }
 
 // The V of a pass: one lane or a quad per (butterfly, u), u < 2^(q - 1), u-major per
-// job, which is half a job's outputs; u = 0, the last, has none.
+// job, which is half a job's outputs; u = 0, the last, has none.  A chain of 63
+// doublings: a quad's lasts 0.25 ms up to two blocks per SM and 0.49 at 8192 turns, a lane's
+// 0.60 at 16384 (2^16 points, q = 2), so quads take up to a wave of turns (two of slots) and
+// lanes, with less work in all, the rest.
 template <bool Quad>
 __global__ void __launch_bounds__(64, 4)
 k_fft_quarter(xyzz* prod, const FftJob* __restrict__ jobs, const uint32_t* __restrict__ lst_job,
