@@ -321,6 +321,7 @@ __global__ void k_batch_out(const xyzz* __restrict__ roots, uint32_t nmsm, jac* 
 struct BatchGraph {
     cudaGraphExec_t exec = nullptr;
     uint32_t nmsm = 0, c = 0, L = 0, rounds = 0;
+    uint32_t moves = 0;      // BatchWork::moves() at the capture: the graph holds the buffers' addresses
     size_t cap = 0;
 };
 
@@ -332,14 +333,27 @@ struct BatchWork {
     PinnedBuf h_scal, h_off, h_out;
     AffWork aff;
     BatchGraph graph;
-    void release()
+    std::array<DevBuf*, 17> bufs()
+    {
+        return {&scal, &off, &digits, &ranks, &pidx, &base, &counts, &offsets, &bsums, &sorted_pt,
+                &sorted_key, &buckets, &head, &tail, &hot, &seg, &out};
+    }
+    uint32_t moves()
+    {
+        uint32_t m = aff.moves();
+        for (const DevBuf* d : bufs()) m += d->moves;
+        return m;
+    }
+    void drop_graph()
     {
         if (graph.exec) cudaGraphExecDestroy(graph.exec);
         graph = BatchGraph();
+    }
+    void release()
+    {
+        drop_graph();
         aff.release();
-        DevBuf* bufs[] = {&scal, &off, &digits, &ranks, &pidx, &base, &counts, &offsets, &bsums, &sorted_pt,
-                          &sorted_key, &buckets, &head, &tail, &hot, &seg, &out};
-        for (DevBuf* d : bufs) d->release();
+        for (DevBuf* d : bufs()) d->release();
         PinnedBuf* hb[] = {&h_scal, &h_off, &h_out};
         for (PinnedBuf* h : hb) {
             if (h->p) cudaFreeHost(h->p);
@@ -373,10 +387,7 @@ static cudaError_t build_tables(Basis* b, uint32_t c)
     b->tmp.release();
     b->c = c;
     b->D = D;
-    if (b->work.graph.exec) {
-        cudaGraphExecDestroy(b->work.graph.exec);
-        b->work.graph = BatchGraph();
-    }
+    b->work.drop_graph();
     return cudaSuccess;
 }
 
@@ -544,7 +555,9 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
         const size_t step = (full + 15) / 16;
         cap = std::min(full, (P / step + 1) * step);
         const BatchGraph& g = w->graph;
-        if (use_graph && g.exec && g.nmsm == nmsm && g.c == b->c && g.L == b->L && g.cap >= P) cap = g.cap;
+        if (use_graph && g.exec && g.moves == w->moves() && g.nmsm == nmsm && g.c == b->c && g.L == b->L &&
+            g.cap >= P)
+            cap = g.cap;
     }
     CATMSM_CHECK(ensure_work(b, w, nmsm, cap));
     uint32_t* off = (uint32_t*)w->h_off.p;
@@ -572,10 +585,12 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     CATMSM_CHECK(copy_scalars(w, scalars, P * 32, st));
     CATMSM_CHECK(cudaMemcpyAsync(w->off.p, off, (nmsm + 2 + 2 * (size_t)np) * 4, cudaMemcpyHostToDevice, st));
     if (use_graph) {
+        // A buffer that moved since the capture (a larger batch, another chunk length,
+        // an allocation that failed half-way) leaves the graph with freed addresses.
         BatchGraph& g = w->graph;
-        if (!g.exec || g.nmsm != nmsm || g.c != b->c || g.L != b->L || g.cap != cap || g.rounds != rounds) {
-            if (g.exec) cudaGraphExecDestroy(g.exec);
-            g = BatchGraph();
+        if (!g.exec || g.moves != w->moves() || g.nmsm != nmsm || g.c != b->c || g.L != b->L || g.cap != cap ||
+            g.rounds != rounds) {
+            w->drop_graph();
             cudaGraph_t graph;
             CATMSM_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             enqueue_batch(b, w, st, nmsm, cap, rounds);
@@ -588,6 +603,7 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
             g.L = b->L;
             g.cap = cap;
             g.rounds = rounds;
+            g.moves = w->moves();
         }
         CATMSM_CHECK(cudaGraphLaunch(g.exec, st));
         g_stats.launches += 1;

@@ -3,6 +3,7 @@
 // error helpers.  All public entry points are synchronous and fail closed.
 #pragma once
 #include <cuda_runtime.h>
+#include <array>
 #include <atomic>
 #include <cstring>
 #include <cstddef>
@@ -41,13 +42,13 @@ inline int device_sms()
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    uint32_t moves = 0;      // times the address changed: what holds it (a captured graph) is stale after that
     void* get(size_t bytes)
     {
         if (bytes == 0) bytes = 256;
         if (bytes > cap) {
-            if (p) cudaFree(p);
-            p = nullptr;
-            cap = 0;
+            release();
+            moves++;
             if (cudaMalloc(&p, bytes) != cudaSuccess) {
                 p = nullptr;
                 return nullptr;
@@ -58,9 +59,11 @@ struct DevBuf {
     }
     void release()
     {
-        if (p) cudaFree(p);
+        if (!p) return;
+        cudaFree(p);
         p = nullptr;
         cap = 0;
+        moves++;
     }
 };
 
@@ -134,13 +137,23 @@ struct AuxStream {
 struct AffWork {
     struct Set {
         DevBuf pts0, pts1, key0, key1, meta, pairpos, prefix, rest, gtot;
+        std::array<DevBuf*, 9> bufs()
+        {
+            return {&pts0, &pts1, &key0, &key1, &meta, &pairpos, &prefix, &rest, &gtot};
+        }
     } set[2];
     AuxStream aux;
+    uint32_t moves()
+    {
+        uint32_t m = 0;
+        for (Set& w : set)
+            for (const DevBuf* b : w.bufs()) m += b->moves;
+        return m;
+    }
     void release()
     {
         for (Set& w : set)
-            for (DevBuf* b : {&w.pts0, &w.pts1, &w.key0, &w.key1, &w.meta, &w.pairpos, &w.prefix, &w.rest, &w.gtot})
-                b->release();
+            for (DevBuf* b : w.bufs()) b->release();
         aux.release();
     }
 };

@@ -1,0 +1,81 @@
+"""CPU check of the batched commitments' captured graph against its buffers.
+
+A captured graph holds device addresses, so it may be replayed only while no
+buffer that existed at its capture has been freed.  The library's host code
+runs over a fake CUDA runtime that logs allocations, frees and replays (see
+fake_cuda); the sequences are the ones in which a workspace moves between two
+batches that would use the same graph.
+"""
+import pytest
+
+import fake_cuda
+
+SEQUENCES = {
+    # a larger batch of the same number of MSMs, without the graph
+    "more_pairs": """
+b.batch([300] * 8, True)
+b.batch([4096] * 8, False)
+b.batch([300] * 8, True)
+""",
+    # more MSMs
+    "more_msms": """
+b.batch([300] * 8, True)
+b.batch([300] * 64, False)
+b.batch([300] * 8, True)
+""",
+    # a shorter chunk (more chunk carries), and back
+    "chunk": """
+b.batch([300] * 8, True)
+b.config(10, 4)
+b.batch([300] * 8, False)
+b.config(10, 96)
+b.batch([300] * 8, True)
+""",
+    # the affine rounds' lists: 64 x 4096 pairs run rounds
+    "rounds": """
+b.batch([4096] * 60 + [1] * 4, True)
+b.config(10, 16)
+b.batch([4096] * 64, False)
+b.config(10, 96)
+b.batch([4096] * 60 + [1] * 4, True)
+""",
+    # a larger batch that runs out of memory half-way
+    "no_memory": """
+b.batch([300] * 8, True)
+limit(F.fake_used() + (1 << 22))
+assert b.batch([4096] * 8, False) != 0
+limit(0)
+b.batch([300] * 8, True)
+""",
+}
+
+PRELUDE = "b = Basis(4096, 10)\nclear()\n"
+
+
+@pytest.mark.parametrize("name", sorted(SEQUENCES))
+def test_no_replay_over_freed_buffers(gpu_binding, name):
+    gpu_binding.load()
+    ops = fake_cuda.run(gpu_binding.LIB_PATH, PRELUDE + SEQUENCES[name] + "done(log())")
+    stale, replays = {}, 0
+    for op in ops:
+        if op[0] == "instantiate":
+            stale[op[1]] = None
+        elif op[0] == "free":
+            for g in stale:
+                stale[g] = stale[g] or op[1]
+        elif op[0] == "destroy":
+            stale.pop(op[1])
+        elif op[0] == "replay":
+            replays += 1
+            assert stale[op[2]] is None, "graph replayed after a buffer was freed"
+    assert replays == 2
+
+
+def test_graph_is_kept_while_nothing_moves(gpu_binding):
+    gpu_binding.load()
+    ops = fake_cuda.run(gpu_binding.LIB_PATH, PRELUDE + """
+for k in (300, 280, 300, 1, 299):
+    b.batch([k] * 8, True)
+done(log())
+""")
+    assert [o[0] for o in ops].count("instantiate") == 1 and [o[0] for o in ops].count("replay") == 5
