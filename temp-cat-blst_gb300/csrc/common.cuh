@@ -50,6 +50,7 @@ struct DevBuf {
             release();
             moves++;
             if (cudaMalloc(&p, bytes) != cudaSuccess) {
+                cudaGetLastError();      // the null pointer reports it; the next call's launches must not
                 p = nullptr;
                 return nullptr;
             }
@@ -78,6 +79,7 @@ struct PinnedBuf {
             p = nullptr;
             cap = 0;
             if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();
                 p = nullptr;
                 return nullptr;
             }
