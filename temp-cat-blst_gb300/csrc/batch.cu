@@ -367,6 +367,7 @@ struct Basis {
     int device = -1;
     size_t n = 0;
     uint32_t c = 0, D = 0, L = 16;
+    bool tables = false;   // the tables of window c are built (not after a failed rebuild: batches fail)
     cudaStream_t stream = nullptr;
     DevBuf points, table, tmp;
     BatchWork work;
@@ -377,6 +378,7 @@ struct Basis {
 static cudaError_t build_tables(Basis* b, uint32_t c)
 {
     const uint32_t D = 256 / c + 1;
+    b->tables = false;
     affine* table = (affine*)b->table.get((size_t)D * b->n * sizeof(affine));
     xyzz* tmp = (xyzz*)b->tmp.get((size_t)D * b->n * (sizeof(xyzz) + sizeof(fp)));
     if (!table || !tmp) return cudaErrorMemoryAllocation;
@@ -387,6 +389,7 @@ static cudaError_t build_tables(Basis* b, uint32_t c)
     b->tmp.release();
     b->c = c;
     b->D = D;
+    b->tables = true;
     b->work.drop_graph();
     return cudaSuccess;
 }
@@ -543,6 +546,7 @@ static cudaError_t copy_scalars(BatchWork* w, const uint8_t* scalars, size_t byt
 static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* out, uint32_t nmsm,
                              const size_t* counts, const uint8_t* scalars, bool use_graph, bool exact_cap)
 {
+    if (!b->tables) return cudaErrorMemoryAllocation;
     size_t P = 0;
     for (uint32_t j = 0; j < nmsm; j++) {
         if (counts[j] > b->n) return cudaErrorInvalidValue;
@@ -755,7 +759,7 @@ static int set_config_locked(Basis* b, size_t window, size_t chunk)
 {
     if (window < 2 || window > 20 || chunk < 2 || chunk > 256) return (int)cudaErrorInvalidValue;
     b->L = (uint32_t)chunk;
-    if (window != b->c) return (int)build_tables(b, (uint32_t)window);
+    if (window != b->c || !b->tables) return (int)build_tables(b, (uint32_t)window);
     return 0;
 }
 

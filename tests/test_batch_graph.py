@@ -79,3 +79,21 @@ for k in (300, 280, 300, 1, 299):
 done(log())
 """)
     assert [o[0] for o in ops].count("instantiate") == 1 and [o[0] for o in ops].count("replay") == 5
+
+
+def test_no_batch_over_freed_tables(gpu_binding):
+    """A reconfiguration that runs out of memory has given up the old tables:
+    batches fail until a configuration succeeds, whichever window it asks for."""
+    gpu_binding.load()
+    got = fake_cuda.run(gpu_binding.LIB_PATH, """
+b = Basis(4096, 13)
+b.batch([300] * 8, True)
+limit(F.fake_used() + (1 << 20))
+bad = [b.config(4, 96), b.batch([300] * 8, True), b.batch([300] * 8, False), b.config(4, 96)]
+limit(0)
+again = b.config(13, 96)
+clear()
+done([bad, again, b.batch([300] * 8, True), [l[0] for l in log()].count("instantiate")])
+""")
+    bad, again, ok, captures = got
+    assert all(bad) and again == 0 and ok == 0 and captures == 1
