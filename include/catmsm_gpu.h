@@ -228,7 +228,8 @@ void *catmsm_stream(void);
 long catmsm_launch_count(void);
 
 /* The window width the GPU MSM uses for n points of scalars of at most 128
- * bits (no GLV split). */
+ * bits (no GLV split); from 2^18 points on the width depends on the bits too,
+ * and this is the one for 128 (catmsm_msm_plan has the others). */
 size_t catmsm_msm_window(size_t npoints);
 
 /* The plan of the calling thread's next MSM of n points with nbits-bit

@@ -476,7 +476,7 @@ void* catmsm_stream(void)
 
 long catmsm_launch_count(void) { return g_stats.launches; }
 
-size_t catmsm_msm_window(size_t npoints) { return msm_default_window(npoints); }
+size_t catmsm_msm_window(size_t npoints) { return msm_plain_window(npoints, 128); }
 
 int catmsm_msm_glv(int enable)
 {

@@ -6,6 +6,7 @@
 namespace catmsm {
 
 uint32_t msm_default_window(size_t n);
+uint32_t msm_plain_window(size_t n, uint32_t nbits);
 
 // Bucket-count scan (k_scan_local / k_scan_top / k_scan_add in msm.cu): a
 // block of kScanThreads threads scans a tile of kScanTile counts, so M counts

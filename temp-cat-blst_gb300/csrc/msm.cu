@@ -890,7 +890,7 @@ uint32_t msm_glv_window(size_t n2)
 // of c bits: the plain heuristic's width may leave a top window of nothing but
 // the recoding's carry (64 = 4 x 16: half of all points in ONE bucket, joined by
 // the grid-wide fixup).  1500003 points of 64 bits: c = 16 3.05 ms, 17 2.80 ms (262144 points: 0.98, 0.90).
-static uint32_t msm_plain_window(size_t n, uint32_t nbits)
+uint32_t msm_plain_window(size_t n, uint32_t nbits)
 {
     if (nbits <= 128 && msm_small_applies(n, false)) return msm_small_window(n);
     const uint32_t def = msm_default_window(n);
