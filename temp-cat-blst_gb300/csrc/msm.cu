@@ -1031,9 +1031,15 @@ static uint32_t level1_fan_in(size_t M)
     return M >= kFanIn16MinBuckets ? 16 : M >= kFanIn8MinBuckets ? 8 : 2;
 }
 
-static uint32_t msm_windows(size_t np, uint32_t nbits, bool glv, uint32_t c)
+// Whether an MSM of np pipeline points (no window asked for) takes the small path.
+static bool takes_small(int affine_rounds, size_t np, uint32_t nbits, bool glv)
 {
-    if ((glv || nbits <= 128) && msm_small_applies(np, glv)) return msm_small_windows(np, glv ? 127 : nbits, glv);
+    return affine_rounds < 0 && (glv || nbits <= 128) && msm_small_applies(np, glv);
+}
+
+static uint32_t msm_windows(int affine_rounds, size_t np, uint32_t nbits, bool glv, uint32_t c)
+{
+    if (takes_small(affine_rounds, np, nbits, glv)) return msm_small_windows(np, glv ? 127 : nbits, glv);
     return (glv ? 127 : nbits) / c + 1;
 }
 
@@ -1046,7 +1052,7 @@ void msm_plan_detail(size_t n, uint32_t nbits, bool glv, uint32_t* c, uint32_t* 
     const bool g = glv && nbits > 128 && n < (1u << 30);
     const size_t np = g ? 2 * n : n;
     *c = g ? msm_glv_window(np) : msm_plain_window(np, nbits);
-    *windows = msm_windows(np, nbits, g, *c);
+    *windows = msm_windows(-1, np, nbits, g, *c);
     *points = np;
     *chunk = accumulate_chunk(np * *windows);
     *fan_in = level1_fan_in((size_t)*windows << (*c - 1));
@@ -1057,7 +1063,7 @@ void msm_plan(const Ctx* ctx, size_t n, uint32_t nbits, uint32_t* c, uint32_t* w
     const bool g = use_glv(ctx, n, nbits);
     const size_t np = g ? 2 * n : n;
     *c = g ? msm_glv_window(np) : msm_plain_window(np, nbits);
-    *windows = msm_windows(np, nbits, g, *c);
+    *windows = msm_windows(ctx->affine_rounds, np, nbits, g, *c);
     *points = np;
 }
 
@@ -1120,8 +1126,7 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     // Few points (and no width or rounds asked for): one kernel for the buckets of
     // all windows instead of the sort, accumulate, fixup and reduce launches
     const bool glv_split = !tile_window && use_glv(ctx, n, nbits);
-    if (!tile_window && c == 0 && ctx->affine_rounds < 0 && (glv_split || nbits <= 128) &&
-        msm_small_applies(glv_split ? 2 * n : n, glv_split)) {
+    if (!tile_window && c == 0 && takes_small(ctx->affine_rounds, glv_split ? 2 * n : n, nbits, glv_split)) {
         if (points_ready) CATMSM_CHECK(cudaStreamWaitEvent(st, points_ready, 0));
         SmallMsm m;
         uint32_t* entries = nullptr;

@@ -41,6 +41,9 @@ def buf(n):
     b = (C.c_char * n)()
     _keep.append(b)
     return C.c_void_p(C.addressof(b))
+def aligned(n):
+    b = buf(n + 64)
+    return C.c_void_p((b.value + 63) & ~63)
 def pin(b, n):
     F.fake_pin(b, S(n))
     return b
