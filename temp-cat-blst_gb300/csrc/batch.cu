@@ -426,10 +426,10 @@ static cudaError_t ensure_work(const Basis* b, BatchWork* w, uint32_t nmsm, size
 }
 
 // The device sequence of one batch (everything after the input copies), with
-// `rounds` batch-affine accumulation rounds.  Returns the number of kernels it
+// `rounds` batch-affine accumulation rounds.  *kernels: the number of kernels it
 // launched.
-static uint32_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
-                              uint32_t rounds)
+static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
+                                 uint32_t rounds, uint32_t* kernels)
 {
     const uint32_t c = b->c, D = b->D, L = b->L, B = 1u << (c - 1);
     const size_t M = (size_t)nmsm * B;
@@ -477,8 +477,8 @@ static uint32_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uin
                                                         (uint32_t)nD, sorted_pt, sorted_key);
     int aff_launches = 0;
     if (rounds)
-        aff_accumulate(w->aff, b->table.p, sorted_pt, sorted_key, total, L,
-                       chunks, rounds, buckets, head, tail, st, &aff_launches);
+        CATMSM_CHECK(aff_accumulate(w->aff, b->table.p, sorted_pt, sorted_key, total, L,
+                                    chunks, rounds, buckets, head, tail, st, &aff_launches));
     else
         k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)b->table.p, sorted_pt,
                                                           sorted_key, total, L, buckets, head,
@@ -516,11 +516,38 @@ static uint32_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uin
         first = false;
     }
     k_batch_out<<<div_up(nmsm, 128), 128, 0, st>>>(inQ ? inQ : inA, nmsm, (jac*)w->out.p);
-    return launches;
+    *kernels = launches;
+    return cudaGetLastError();
 }
 
-// H2D of the batch's scalars.  Page-locked caller memory is read in place (the
-// call returns after the copy); anything else goes through pinned staging, by
+// Captures enqueue_batch as w->graph.  The capture is ended whatever fails.
+static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
+                                 uint32_t rounds)
+{
+    w->drop_graph();
+    CATMSM_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    uint32_t kernels = 0;
+    const cudaError_t queued = enqueue_batch(b, w, st, nmsm, cap, rounds, &kernels);
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    cudaError_t e = cudaStreamEndCapture(st, &graph);
+    if (queued != cudaSuccess) e = queued;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    CATMSM_CHECK(e);
+    BatchGraph& g = w->graph;
+    g.exec = exec;
+    g.nmsm = nmsm;
+    g.c = b->c;
+    g.L = b->L;
+    g.cap = cap;
+    g.rounds = rounds;
+    g.moves = w->moves();
+    return cudaSuccess;
+}
+
+// H2D of the batch's scalars.  Page-locked caller memory is read in place (run_batch
+// waits for the stream, also after a failure); anything else goes through pinned staging, by
 // several host threads (a copy of 44 MB: ~1 ms of a 14 ms batch).
 static cudaError_t copy_scalars(BatchWork* w, const uint8_t* scalars, size_t bytes, cudaStream_t st)
 {
@@ -538,6 +565,30 @@ static cudaError_t copy_scalars(BatchWork* w, const uint8_t* scalars, size_t byt
     if (!w->h_scal.get(bytes)) return cudaErrorMemoryAllocation;
     host_copy(w->h_scal.p, scalars, bytes);
     return cudaMemcpyAsync(w->scal.p, w->h_scal.p, bytes, cudaMemcpyHostToDevice, st);
+}
+
+// Queues the copies of a batch (`bytes` of scalars, np parts) and its device sequence.
+static cudaError_t queue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
+                               uint32_t rounds, const uint8_t* scalars, size_t bytes, uint32_t np, bool use_graph)
+{
+    CATMSM_CHECK(copy_scalars(w, scalars, bytes, st));
+    CATMSM_CHECK(cudaMemcpyAsync(w->off.p, w->h_off.p, (nmsm + 2 + 2 * (size_t)np) * 4, cudaMemcpyHostToDevice, st));
+    if (use_graph) {
+        // A buffer that moved since the capture (a larger batch, another chunk length,
+        // an allocation that failed half-way) leaves the graph with freed addresses.
+        const BatchGraph& g = w->graph;
+        if (!g.exec || g.moves != w->moves() || g.nmsm != nmsm || g.c != b->c || g.L != b->L || g.cap != cap ||
+            g.rounds != rounds)
+            CATMSM_CHECK(capture_batch(b, w, st, nmsm, cap, rounds));
+        CATMSM_CHECK(cudaGraphLaunch(g.exec, st));
+        g_stats.launches += 1;
+    } else {
+        uint32_t kernels = 0;
+        CATMSM_CHECK(enqueue_batch(b, w, st, nmsm, cap, rounds, &kernels));
+        g_stats.launches += kernels;
+    }
+    CATMSM_CHECK(cudaGetLastError());
+    return cudaMemcpyAsync(w->h_out.p, w->out.p, (size_t)nmsm * sizeof(jac), cudaMemcpyDeviceToHost, st);
 }
 
 // exact_cap: size the work for exactly the pairs of this batch (serving);
@@ -586,39 +637,13 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
         cudaGetLastError();
         rounds = 0;
     }
-    CATMSM_CHECK(copy_scalars(w, scalars, P * 32, st));
-    CATMSM_CHECK(cudaMemcpyAsync(w->off.p, off, (nmsm + 2 + 2 * (size_t)np) * 4, cudaMemcpyHostToDevice, st));
-    if (use_graph) {
-        // A buffer that moved since the capture (a larger batch, another chunk length,
-        // an allocation that failed half-way) leaves the graph with freed addresses.
-        BatchGraph& g = w->graph;
-        if (!g.exec || g.moves != w->moves() || g.nmsm != nmsm || g.c != b->c || g.L != b->L || g.cap != cap ||
-            g.rounds != rounds) {
-            w->drop_graph();
-            cudaGraph_t graph;
-            CATMSM_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            enqueue_batch(b, w, st, nmsm, cap, rounds);
-            CATMSM_CHECK(cudaStreamEndCapture(st, &graph));
-            cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
-            cudaGraphDestroy(graph);
-            CATMSM_CHECK(e);
-            g.nmsm = nmsm;
-            g.c = b->c;
-            g.L = b->L;
-            g.cap = cap;
-            g.rounds = rounds;
-            g.moves = w->moves();
-        }
-        CATMSM_CHECK(cudaGraphLaunch(g.exec, st));
-        g_stats.launches += 1;
-    } else {
-        g_stats.launches += enqueue_batch(b, w, st, nmsm, cap, rounds);
-    }
-    CATMSM_CHECK(cudaGetLastError());
-    CATMSM_CHECK(cudaMemcpyAsync(w->h_out.p, w->out.p, (size_t)nmsm * sizeof(jac), cudaMemcpyDeviceToHost, st));
-    CATMSM_CHECK(cudaStreamSynchronize(st));
-    std::memcpy(out, w->h_out.p, (size_t)nmsm * sizeof(jac));
-    return cudaSuccess;
+    cudaError_t err = queue_batch(b, w, st, nmsm, cap, rounds, scalars, P * 32, np, use_graph);
+    if (err != cudaSuccess && w->aff.aux.stream) cudaStreamSynchronize(w->aff.aux.stream);
+    const cudaError_t done = cudaStreamSynchronize(st);      // the caller's scalars are not read after return
+    if (err == cudaSuccess) err = done;
+    if (err == cudaSuccess) std::memcpy(out, w->h_out.p, (size_t)nmsm * sizeof(jac));
+    else cudaGetLastError();                                 // err reports it
+    return err;
 }
 
 BatchWork* batch_work_new() { return new (std::nothrow) BatchWork(); }

@@ -318,10 +318,11 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t st, enum cudaStreamCaptureMode)
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t st, cudaGraph_t* g)
 {
-    ENTER;
+    std::unique_lock<std::mutex> lk(mu);
     line("end %ld", id(st));
     if (!capturing[st]) return err(cudaErrorIllegalState);
-    capturing[st] = false;
+    capturing[st] = false;           // a capture that fails has ended too
+    if (fails(__func__)) return err(cudaErrorUnknown);
     *g = (cudaGraph_t)next_id++;
     return cudaSuccess;
 }

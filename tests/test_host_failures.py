@@ -22,3 +22,28 @@ limit(0)
 done([first, call(1 << 16)])
 """)
     assert first != 0 and second == 0
+
+
+@pytest.mark.parametrize("name,nth", [("cudaMemcpyAsync", 2), ("cudaMemcpyAsync", 3), ("cudaStreamBeginCapture", 1),
+                                      ("cudaStreamEndCapture", 1), ("cudaGraphInstantiate", 1),
+                                      ("cudaGraphLaunch", 1), ("cudaEventRecord", 1), ("cudaEventRecord", 2)])
+def test_failed_batch_reads_nothing_after_return(host, name, nth):
+    """A batch whose scalars are page-locked (read in place) and that fails after
+    their copy was queued: the stream is waited for before the call returns, no
+    capture stays open, and the next batch works."""
+    rc, ops, again = host("""
+b = Basis(4096, 10)
+counts = [4096] * 60                       # 60 x 4096 pairs: affine rounds, on two streams
+sc = pin(buf(32 * sum(counts)), 32 * sum(counts))
+clear()
+fail(%r, %d)
+rc = b.batch(counts, True, sc)
+ops = log()
+done([rc, ops, b.batch(counts, True, sc)])
+""" % (name, nth))
+    assert rc != 0 and again == 0 and ["failed", name] in ops
+    copies = [i for i, o in enumerate(ops) if o[0] == "copy"]
+    stream = ops[copies[0]][1]
+    assert ["sync", stream] in ops[copies[-1]:]
+    begun = [o for o in ops if o[0] == "begin"]
+    assert len(begun) == len([o for o in ops if o[0] == "end"])
