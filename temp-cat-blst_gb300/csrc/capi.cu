@@ -167,7 +167,11 @@ static void msm_entry(blst_p1* ret, const blst_p1_affine* const points[], size_t
     if (err == cudaSuccess)
         err = msm_device(ctx, dp, (const uint8_t*)ds, (uint32_t)nbytes, npoints, (uint32_t)nbits, 0, out, ready);
     if (ready) cudaStreamSynchronize(ctx->copy_stream);   // the caller's points are not read after return
-    if (err != cudaSuccess) { write_inf(ret); return; }
+    if (err != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);               // nor, after a failure, what else is queued
+        write_inf(ret);
+        return;
+    }
     std::memcpy(ret, out, sizeof(*ret));
 }
 

@@ -47,3 +47,20 @@ done([rc, ops, b.batch(counts, True, sc)])
     assert ["sync", stream] in ops[copies[-1]:]
     begun = [o for o in ops if o[0] == "begin"]
     assert len(begun) == len([o for o in ops if o[0] == "end"])
+
+
+@pytest.mark.parametrize("n", [64, 4096, 20000])
+@pytest.mark.parametrize("nth", [3, 4])
+def test_failed_msm_reads_nothing_after_return(host, n, nth):
+    """A host MSM whose workspaces cannot be had after its inputs' copies were
+    queued (the first two allocations are the inputs') waits for them."""
+    ops = host("""
+n = %d
+ptr = (P * 2)(buf(96 * n).value, None), (P * 2)(buf(32 * n).value, None)
+fail("cudaMalloc", %d)
+L.blst_p1s_mult_pippenger(buf(144), ptr[0], S(n), ptr[1], S(255), buf(64))
+done(log())
+""" % (n, nth))
+    assert ["failed", "cudaMalloc"] in ops
+    at = {o[1]: i for i, o in enumerate(ops) if o[0] == "copy"}
+    assert at and all(["sync", stream] in ops[i:] for stream, i in at.items())
