@@ -543,8 +543,10 @@ cudaError_t aff_prepare(AffWork& W, uint32_t L, size_t chunks, cudaStream_t st)
         if (!w.pts0.get(T * L * sizeof(affine)) || !w.pts1.get(T * L * sizeof(affine)) || !w.key0.get(T * L * 4) ||
             !w.key1.get(T * L * 4) || !w.meta.get(T * 4) || !w.pairpos.get(T * H * 4) ||
             !w.prefix.get(T * H * sizeof(fp)) || !w.rest.get(T * sizeof(fp)) ||
-            !w.gtot.get(T / kAffGroup * sizeof(fp)))
+            !w.gtot.get(T / kAffGroup * sizeof(fp))) {
+            W.release_lists();       // the caller goes on without the rounds: the others may need what was got
             return cudaErrorMemoryAllocation;
+        }
     }
     return W.aux.ensure(st);
 }

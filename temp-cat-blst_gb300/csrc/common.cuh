@@ -152,10 +152,14 @@ struct AffWork {
             for (const DevBuf* b : w.bufs()) m += b->moves;
         return m;
     }
-    void release()
+    void release_lists()
     {
         for (Set& w : set)
             for (DevBuf* b : w.bufs()) b->release();
+    }
+    void release()
+    {
+        release_lists();
         aux.release();
     }
 };

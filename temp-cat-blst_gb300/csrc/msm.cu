@@ -1237,10 +1237,15 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
         g_stats.launches++;
     }
     mark(4);
-    const uint32_t rounds = tile_window ? 0
-                          : ctx->affine_rounds >= 0 ? (uint32_t)ctx->affine_rounds : msm_affine_rounds(nD, M);
+    // Without the memory for their lists (about 230 B per entry of a slice) the mixed
+    // additions of every entry, which need none.
+    uint32_t rounds = tile_window ? 0
+                    : ctx->affine_rounds >= 0 ? (uint32_t)ctx->affine_rounds : msm_affine_rounds(nD, M);
+    if (rounds && aff_prepare(W.aff, L, chunks, st) != cudaSuccess) {
+        cudaGetLastError();
+        rounds = 0;
+    }
     if (rounds) {
-        CATMSM_CHECK(aff_prepare(W.aff, L, chunks, st));
         CATMSM_CHECK(aff_accumulate(W.aff, d_points, sorted_pt, sorted_key, total, L, chunks, rounds, buckets, head,
                                     tail, st, &g_stats.launches));
     } else

@@ -64,3 +64,27 @@ done(log())
     assert ["failed", "cudaMalloc"] in ops
     at = {o[1]: i for i, o in enumerate(ops) if o[0] == "copy"}
     assert at and all(["sync", stream] in ops[i:] for stream, i in at.items())
+
+
+def test_msm_without_memory_for_the_affine_rounds(host):
+    """An MSM that would run affine rounds and has memory for everything but their
+    lists runs without them, keeps none of the lists, and runs them again later."""
+    full, kept, rc, ran, later = host("""
+n = 1 << 18
+pts, sc = aligned(96 * n), buf(32 * n)
+def call():
+    clear()
+    rc = L.catmsm_p1s_mult_pippenger_device(buf(144), pts, sc, S(32), S(n), S(255), S(0))
+    return rc, ["k_aff_first" in kernels(), "k_accumulate" in kernels()]
+L.catmsm_msm_affine_rounds(0)
+call()
+base = F.fake_used()
+limit(base + (256 << 20))
+L.catmsm_msm_affine_rounds(-1)
+rc, ran = call()
+kept = F.fake_used() - base
+limit(0)
+done([F.fake_used(), kept, rc, ran, call()])
+""")
+    assert rc == 0 and ran == [False, True] and kept == 0
+    assert later == [0, [True, False]]
