@@ -674,8 +674,9 @@ static size_t pass_max_items(uint32_t q) { return size_t(1) << (q <= 2 ? 22 : 18
 
 // Next to another group of jobs (not solo) the launches share the GPU: there a pass
 // costs its part of a full wave, and its forms are a level of butterflies or two levels
-// by lanes with quarter turns, the least work.
-static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, bool solo)
+// by lanes with quarter turns, the least work.  Without memory for products, a level
+// of butterflies a pass.
+static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, bool solo, bool with_products)
 {
     constexpr double kSumMs = 0.5e-6, kSumsMs = 0.03, kFullMs = 0.57;     // kFullMs: wave products of a full launch
     constexpr uint32_t kMaxQ = 4;
@@ -686,7 +687,7 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
     std::vector<FftPass> via(maxlog + 1);
     best[0] = 0;
     for (uint32_t s = 0; s < maxlog; s++) {
-        for (uint32_t q = 1; q <= (solo ? kMaxQ : 2) && s + q <= maxlog; q++) {
+        for (uint32_t q = 1; q <= (!with_products ? 1 : solo ? kMaxQ : 2) && s + q <= maxlog; q++) {
             size_t items, products[2], outputs;
             pass_counts(jobs, s, q, items, products, outputs);
             FftPass p;
@@ -697,7 +698,8 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
                 const double bf = (double)outputs / 2, scaled = (double)products[0] - (s ? bf : 0);
                 ms = (solo ? stage_ms(outputs / 2, wave) : kFullMs / (double)wave * bf) * (1 + 0.85 * scaled / bf);
             }
-            for (uint32_t turns = solo ? 0 : 1; items <= pass_max_items(q) && turns < (q > 1 ? 2u : 1u); turns++) {
+            const bool fits = with_products && items <= pass_max_items(q);
+            for (uint32_t turns = solo ? 0 : 1; fits && turns < (q > 1 ? 2u : 1u); turns++) {
                 // the products of a first pass are not adjacent: its SMs have uneven shares
                 const size_t n = s || turns ? products[turns] : products[turns] * 3 / 2;
                 const size_t v = outputs / 2 - (outputs >> q);
@@ -783,35 +785,46 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
     }
     for (size_t i = 0; i < count; i++) members[group[i]].push_back(&jobs[i]);
     std::vector<FftPass> plan;
-    for (int g = 0; g < groups; g++)
-        for (FftPass p : fft_plan(members[g], groups == 1)) {
-            p.group = (uint32_t)g;
-            plan.push_back(p);
-        }
     // per-pass lists of (job, first item, first output)
     std::vector<uint32_t> lst_job, lst_item, lst_out;
-    size_t max_items[2] = {0, 0};
-    bool stages = false;
-    for (FftPass& p : plan) {
-        p.off = (uint32_t)lst_job.size();
-        for (size_t i = 0; i < count; i++) {
-            const FftJob& J = jobs[i];
-            if (group[i] != p.group || J.logn <= p.s0) continue;
-            const uint32_t qe = std::min(p.q, J.logn - p.s0);
-            const uint32_t bf = std::min(J.n >> (p.s0 + qe), J.xn) << p.s0;
-            lst_job.push_back((uint32_t)i);
-            lst_item.push_back(p.items);
-            lst_out.push_back(p.outputs);
-            p.items += p.kind == FftPass::kStage ? bf : bf * pass_items(qe) << p.split;
-            p.outputs += bf << qe;
+    size_t max_items[2];
+    bool stages;
+    auto make_plan = [&](bool with_products) {
+        plan.clear();
+        for (std::vector<uint32_t>* l : {&lst_job, &lst_item, &lst_out}) l->clear();
+        max_items[0] = max_items[1] = 0;
+        stages = false;
+        for (int g = 0; g < groups; g++)
+            for (FftPass p : fft_plan(members[g], groups == 1, with_products)) {
+                p.group = (uint32_t)g;
+                plan.push_back(p);
+            }
+        for (FftPass& p : plan) {
+            p.off = (uint32_t)lst_job.size();
+            for (size_t i = 0; i < count; i++) {
+                const FftJob& J = jobs[i];
+                if (group[i] != p.group || J.logn <= p.s0) continue;
+                const uint32_t qe = std::min(p.q, J.logn - p.s0);
+                const uint32_t bf = std::min(J.n >> (p.s0 + qe), J.xn) << p.s0;
+                lst_job.push_back((uint32_t)i);
+                lst_item.push_back(p.items);
+                lst_out.push_back(p.outputs);
+                p.items += p.kind == FftPass::kStage ? bf : bf * pass_items(qe) << p.split;
+                p.outputs += bf << qe;
+            }
+            p.cnt = (uint32_t)lst_job.size() - p.off;
+            if (p.kind == FftPass::kStage) stages = true;
+            else max_items[p.group] = std::max(max_items[p.group], (size_t)p.items);
         }
-        p.cnt = (uint32_t)lst_job.size() - p.off;
-        if (p.kind == FftPass::kStage) stages = true;
-        else max_items[p.group] = std::max(max_items[p.group], (size_t)p.items);
+    };
+    make_plan(true);
+    xyzz* prod = (xyzz*)W.prod.get((max_items[0] + max_items[1]) * sizeof(xyzz));
+    if (!prod) {                                     // up to 805 MB a group: butterflies need none of it
+        make_plan(false);
+        prod = (xyzz*)W.prod.get(0);
     }
     const size_t meta_words = count * (sizeof(FftJob) / 4) + (count + 1) + 3 * lst_job.size() + 8;
     xyzz* tmp = (xyzz*)W.scratch.get(total * sizeof(xyzz));
-    xyzz* prod = (xyzz*)W.prod.get((max_items[0] + max_items[1]) * sizeof(xyzz));
     uint32_t* glv = (uint32_t*)W.glv.get(stages ? glv_total * 32 : 0);
     uint32_t* meta = (uint32_t*)W.meta.get(meta_words * 4);
     uint32_t* hmeta = (uint32_t*)ctx->h_meta.get(meta_words * 4);

@@ -49,6 +49,12 @@ def pin(b, n):
     return b
 def sizes(v):
     return (S * len(v))(*v)
+def domain(n):
+    """A domain of n zero roots with the tag that the library asks for (n, Montgomery)."""
+    b = buf(32 * (n + 2))
+    r = 0x73eda753299d7d483339d80809a1d80553bda402fffe5bfeffffffff00000001
+    C.memmove(b.value + 32 * (n + 1), (n * 2**256 % r).to_bytes(32, "little"), 32)
+    return b
 def kernels():
     return [l[2] for l in log() if l[0] == "launch"]
 class Basis:

@@ -88,3 +88,30 @@ done([F.fake_used(), kept, rc, ran, call()])
 """)
     assert rc == 0 and ran == [False, True] and kept == 0
     assert later == [0, [True, False]]
+
+
+@pytest.mark.parametrize("ns", [[1 << 12], [1 << 17], [1 << 15] * 3, [4, 1 << 10, 1 << 14]])
+def test_fft_without_memory_for_products(host, ns):
+    """Transforms that have memory for everything but a pass's products run a level
+    of butterflies a pass, and several levels again later."""
+    rc, ran, stages, later = host("""
+ns = %r
+dom = {n: domain(n) for n in set(ns)}
+vals = (P * len(ns))(*[buf(144 * n).value for n in ns])
+doms = (P * len(ns))(*[dom[n].value for n in ns])
+modes = (C.c_int * len(ns))(*[i %% 3 for i in range(len(ns))])
+def call():
+    clear()
+    rc = L.catmsm_p1_fft_batch(vals, sizes(ns), doms, modes, S(len(ns)))
+    return rc, log()
+total = sum(ns)
+limit(total * (144 + 192 + 32 + 48) + 200 * 1024)
+rc, ops = call()
+names = [o[2] for o in ops if o[0] == "launch"]
+limit(0)
+rc2, ops2 = call()
+done([rc, any("k_fft_items" in k for k in names), sum("k_fft_stage" in k for k in names),
+      rc2 == 0 and any("k_fft_items" in o[2] for o in ops2 if o[0] == "launch")])
+""" % ns)
+    assert rc == 0 and not ran and later
+    assert stages >= max(ns).bit_length() - 1
