@@ -318,11 +318,13 @@ static cudaError_t decode_download(const DecodeSlice& s, int mode)
 // stream -> two, checked uncompressing: 100003 elements 5.23 -> 4.95 ms, 200000
 // 9.44 -> 9.02, 300000 13.59 -> 13.13.  Three or more slices queue behind their own
 // streams' tails: 100003 elements 4.99 with three, 5.44 with four.  The caller's
-// arrays are read to the end before any of them is written.
+// arrays are read to the end before any of them is written (they may overlap): the
+// second stream starts after the first half's upload, and the first half's download
+// waits for the second's upload.
 static cudaError_t decode_halves(DecodeSlice* s, AuxStream& aux, size_t elem, int mode, bool check)
 {
-    CATMSM_CHECK(aux.begin(s[0].st));
     CATMSM_CHECK(decode_upload(s[0], elem));
+    CATMSM_CHECK(aux.begin(s[0].st));
     CATMSM_CHECK(decode_kernels(s[0], mode, check, false));
     CATMSM_CHECK(decode_upload(s[1], elem));
     CATMSM_CHECK(aux.end(s[0].st));
