@@ -48,3 +48,10 @@ def test_arrays_are_read_before_they_are_written(host, call, check, n):
     down = [i for i, o in enumerate(ops) if o[0] == "copy" and o[5] == "2"]
     assert up and down
     assert all(before(i, j) for i in up for j in down)
+
+
+@pytest.mark.parametrize("call,check,streams", [("deserialize", 0, 1), ("deserialize", 1, 2), ("uncompress", 0, 2)])
+def test_two_streams_only_with_work(host, call, check, streams):
+    """A large deserialization without the membership test is its copies: one stream."""
+    ops = host("n = 100003\nassert %s == 0\ndone(log())" % (DECODES[call] % check))
+    assert len({o[1] for o in ops if o[0] == "launch"}) == streams
