@@ -22,6 +22,8 @@
 #include "catmsm_internal.h"
 #include "catmsm_gpu.h"
 
+#include <algorithm>
+
 namespace catmsm {
 
 enum { kOk = 0, kBadEncoding = 1, kNotOnCurve = 2, kNotInGroup = 3 };
@@ -348,13 +350,16 @@ static int decode_run(const uint8_t* in, size_t elem, int mode, size_t n, blst_p
     affine* dout = (affine*)ctx->msm.points.get(n * sizeof(affine));
     int32_t* derr = (int32_t*)ctx->msm.digits.get(n * 4);
     affine* pts = dout;                              // the decoded points, before the membership test:
-    if (mode == 0 && check) pts = (affine*)ctx->msm.buckets.get(n * sizeof(affine));
+    // without memory for all of them, the elements go through a smaller buffer in turn
+    size_t piece = n;
+    if (mode == 0 && check)
+        while (!(pts = (affine*)ctx->msm.buckets.get(piece * sizeof(affine))) && piece > 4096) piece = (piece + 1) / 2;
     if (mode == 1 && check) pts = (affine*)din;      // each thread over its own 96 bytes
     if ((mode != 2 && !din) || !dout || !derr || !pts) return (int)cudaErrorMemoryAllocation;
     const size_t sms = (size_t)device_sms();
     // A deserialization without the membership test is its copies: 77825 elements
     // 184 us on one stream, 206 on two.
-    const bool halves = n > kLaneThreads * kLaneBlocks * sms && (mode == 0 || check);
+    const bool halves = n > kLaneThreads * kLaneBlocks * sms && (mode == 0 || check) && piece == n;
     const size_t cut = halves ? n / 2 / kLaneThreads * kLaneThreads : n;
     cudaError_t err = halves ? aux.ensure(st) : cudaSuccess;
     if (err == cudaSuccess) {
@@ -377,7 +382,14 @@ static int decode_run(const uint8_t* in, size_t elem, int mode, size_t n, blst_p
             if (err == cudaSuccess) err = e;
         } else {
             err = decode_upload(s[0], elem);
-            if (err == cudaSuccess) err = decode_kernels(s[0], mode, check, n <= kQuadBlocksPerSm * 32 * sms);
+            for (size_t lo = 0; lo < n && err == cudaSuccess; lo += piece) {
+                DecodeSlice t = s[0];
+                t.din = mode == 2 ? nullptr : t.din + lo * elem;
+                t.dout += lo;
+                t.derr += lo;
+                t.m = (uint32_t)std::min(piece, n - lo);
+                err = decode_kernels(t, mode, check, t.m <= kQuadBlocksPerSm * 32 * sms);
+            }
             if (err == cudaSuccess) err = decode_download(s[0], mode);
         }
     }

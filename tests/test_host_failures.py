@@ -115,3 +115,19 @@ done([rc, any("k_fft_items" in k for k in names), sum("k_fft_stage" in k for k i
 """ % ns)
     assert rc == 0 and not ran and later
     assert stages >= max(ns).bit_length() - 1
+
+
+@pytest.mark.parametrize("n", [9000, 100003])
+def test_checked_decode_without_memory_for_the_points(host, n):
+    """Checked uncompressing with memory for its inputs and results but not for all
+    the points between its two kernels: every element goes through both, in pieces."""
+    rc, ops = host("""
+n = %d
+limit(n * (48 + 96 + 4) + (1 << 19))
+rc = L.catmsm_p1s_uncompress(buf(96 * n), buf(48 * n), S(n), buf(4 * n), 1)
+done([rc, log()])
+""" % n)
+    run = [o for o in ops if o[0] == "launch"]
+    assert rc == 0 and len({o[1] for o in run}) == 1
+    assert [o[2].split("<")[0] for o in run] == ["k_decode", "k_members"] * (len(run) // 2) and len(run) > 2
+    assert sum(int(o[3]) for o in run if o[2].startswith("k_decode")) * 64 >= n
