@@ -318,12 +318,17 @@ __global__ void k_batch_out(const xyzz* __restrict__ roots, uint32_t nmsm, jac* 
 }
 
 // ---------------------------------------------------------------- basis object
+// The captured graphs of a workspace, one per number of affine rounds: batches of one
+// size whose entries lie on both sides of a rounds threshold alternate between them.
 struct BatchGraph {
-    cudaGraphExec_t exec = nullptr;
-    uint32_t nmsm = 0, c = 0, L = 0, rounds = 0;
-    uint32_t moves = 0;      // BatchWork::moves() at the capture: the graph holds the buffers' addresses
+    static constexpr uint32_t kKinds = 4;
+    cudaGraphExec_t exec[kKinds] = {};
+    uint32_t nmsm = 0, c = 0, L = 0;
+    uint32_t moves = 0;      // BatchWork::moves() at the capture: the graphs hold the buffers' addresses
     size_t cap = 0;
 };
+
+struct Basis;
 
 // Device/pinned workspace of one batch pipeline instance (a basis has one;
 // a server worker has its own, sharing the basis tables).
@@ -344,9 +349,12 @@ struct BatchWork {
         for (const DevBuf* d : bufs()) m += d->moves;
         return m;
     }
+    // Whether the graphs are of nmsm MSMs over b's tables and address the buffers as they are.
+    bool graph_fits(const Basis* b, uint32_t nmsm);
     void drop_graph()
     {
-        if (graph.exec) cudaGraphExecDestroy(graph.exec);
+        for (cudaGraphExec_t e : graph.exec)
+            if (e) cudaGraphExecDestroy(e);
         graph = BatchGraph();
     }
     void release()
@@ -374,6 +382,13 @@ struct Basis {
     std::mutex mu;     // serialises the direct calls (batches, reconfiguration, autotuning): they share the
                        // basis's workspace and stream, and a rebuild replaces the tables a batch reads
 };
+
+// A buffer that moved since the capture (a larger batch, another chunk length, an
+// allocation that failed half-way) leaves the graphs with freed addresses.
+bool BatchWork::graph_fits(const Basis* b, uint32_t nmsm)
+{
+    return graph.moves == moves() && graph.nmsm == nmsm && graph.c == b->c && graph.L == b->L;
+}
 
 static cudaError_t build_tables(Basis* b, uint32_t c)
 {
@@ -520,11 +535,19 @@ static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
     return cudaGetLastError();
 }
 
-// Captures enqueue_batch as w->graph.  The capture is ended whatever fails.
+// Captures enqueue_batch as one of w->graph's.  The capture is ended whatever fails.
 static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
                                  uint32_t rounds)
 {
-    w->drop_graph();
+    BatchGraph& g = w->graph;
+    if (!w->graph_fits(b, nmsm) || g.cap != cap) {
+        w->drop_graph();
+        g.nmsm = nmsm;
+        g.c = b->c;
+        g.L = b->L;
+        g.moves = w->moves();
+        g.cap = cap;
+    }
     CATMSM_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     uint32_t kernels = 0;
     const cudaError_t queued = enqueue_batch(b, w, st, nmsm, cap, rounds, &kernels);
@@ -535,14 +558,7 @@ static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     CATMSM_CHECK(e);
-    BatchGraph& g = w->graph;
-    g.exec = exec;
-    g.nmsm = nmsm;
-    g.c = b->c;
-    g.L = b->L;
-    g.cap = cap;
-    g.rounds = rounds;
-    g.moves = w->moves();
+    g.exec[rounds] = exec;
     return cudaSuccess;
 }
 
@@ -574,13 +590,10 @@ static cudaError_t queue_batch(const Basis* b, BatchWork* w, cudaStream_t st, ui
     CATMSM_CHECK(copy_scalars(w, scalars, bytes, st));
     CATMSM_CHECK(cudaMemcpyAsync(w->off.p, w->h_off.p, (nmsm + 2 + 2 * (size_t)np) * 4, cudaMemcpyHostToDevice, st));
     if (use_graph) {
-        // A buffer that moved since the capture (a larger batch, another chunk length,
-        // an allocation that failed half-way) leaves the graph with freed addresses.
         const BatchGraph& g = w->graph;
-        if (!g.exec || g.moves != w->moves() || g.nmsm != nmsm || g.c != b->c || g.L != b->L || g.cap != cap ||
-            g.rounds != rounds)
+        if (!w->graph_fits(b, nmsm) || g.cap != cap || !g.exec[rounds])
             CATMSM_CHECK(capture_batch(b, w, st, nmsm, cap, rounds));
-        CATMSM_CHECK(cudaGraphLaunch(g.exec, st));
+        CATMSM_CHECK(cudaGraphLaunch(g.exec[rounds], st));
         g_stats.launches += 1;
     } else {
         uint32_t kernels = 0;
@@ -609,10 +622,7 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     if (!exact_cap) {
         const size_t step = (full + 15) / 16;
         cap = std::min(full, (P / step + 1) * step);
-        const BatchGraph& g = w->graph;
-        if (use_graph && g.exec && g.moves == w->moves() && g.nmsm == nmsm && g.c == b->c && g.L == b->L &&
-            g.cap >= P)
-            cap = g.cap;
+        if (use_graph && w->graph_fits(b, nmsm) && w->graph.cap >= P) cap = w->graph.cap;
     }
     CATMSM_CHECK(ensure_work(b, w, nmsm, cap));
     uint32_t* off = (uint32_t*)w->h_off.p;
@@ -632,7 +642,7 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     // Batch-affine rounds by the entries this batch holds (the plain MSM's rule;
     // 1024 MSMs, 33 M entries, 32 a bucket: 15.4 ms without, 14.1 with).  Without
     // the memory for their lists the batch keeps the mixed additions.
-    uint32_t rounds = msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1));
+    uint32_t rounds = std::min(msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1)), BatchGraph::kKinds - 1);
     if (rounds && aff_prepare(w->aff, b->L, (cap * b->D + b->L - 1) / b->L + 1, st) != cudaSuccess) {
         cudaGetLastError();
         rounds = 0;

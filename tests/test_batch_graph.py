@@ -97,3 +97,18 @@ done([bad, again, b.batch([300] * 8, True), [l[0] for l in log()].count("instant
 """)
     bad, again, ok, captures = got
     assert all(bad) and again == 0 and ok == 0 and captures == 1
+
+
+def test_batches_around_a_rounds_threshold_share_the_captures(gpu_binding):
+    """48 x 4096 pairs of 26 windows run one affine round, 30 x fewer none: batches of
+    one size that alternate between the two are captured once each."""
+    gpu_binding.load()
+    ops = fake_cuda.run(gpu_binding.LIB_PATH, PRELUDE + """
+for i in range(6):
+    b.batch([4096] * 48 if i % 2 == 0 else [4096] * 30 + [1] * 18, True)
+done(log())
+""")
+    kinds = [o[0] for o in ops]
+    assert any("k_aff_first" in o[2] for o in ops if o[0] == "launch")
+    assert any("k_accumulate" in o[2] for o in ops if o[0] == "launch")
+    assert kinds.count("instantiate") == 2 and kinds.count("replay") == 6
