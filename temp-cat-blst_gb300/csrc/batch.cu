@@ -152,10 +152,16 @@ __device__ __forceinline__ void load_scalar32(uint32_t* k, const uint8_t* s)
 // No digit, rank or index arrays (400 MB written and read again for 33 M entries) and
 // ~24 times fewer global atomics, which bounded the per-pair form below: 1.11 ->
 // 0.28 ms for 1024 MSMs of 33 M entries in all (single-word scattered writes: 0.81).
-// For MSMs of at most kPartMaxB buckets whose part fits shared memory.
+// For MSMs of at most kPartMaxB buckets whose part fits shared memory, in batches
+// of at least kPartMinFill entries per bucket of an MSM: with fewer the launches
+// last as long as one block, whose copies go over all buckets.  Sort per pair
+// against by parts, us: 12 bits, 8 x 4096 pairs (352 a bucket) 44 / 62, 16 x 4096 (704)
+// 75 / 62; 13 bits, 24 x 4096 (480) 85 / 91, 32 x 4096 (640) 113 / 92; 11 bits, 8 x 4096
+// (768) 49 / 50, 256 x 100 (600) 45 / 45; 9 bits, 64 x 100 (725) 41 / 30.
 constexpr uint32_t kPartPairs = 1024;
 constexpr uint32_t kPartThreads = 512;
 constexpr uint32_t kPartMaxB = 4096;
+constexpr size_t kPartMinFill = 600;
 constexpr size_t kPartMaxSmem = 220 * 1024;
 
 static size_t part_smem(uint32_t c, uint32_t D) { return ((size_t)2 << (c - 1)) * 4 + 128 + (size_t)kPartPairs * D * 4; }
@@ -318,10 +324,18 @@ __global__ void k_batch_out(const xyzz* __restrict__ roots, uint32_t nmsm, jac* 
 }
 
 // ---------------------------------------------------------------- basis object
-// The captured graphs of a workspace, one per number of affine rounds: batches of one
-// size whose entries lie on both sides of a rounds threshold alternate between them.
+// How a batch of one size runs, by its entries: the affine rounds of its accumulation
+// and the form of its sort (by parts wherever there are rounds).
+struct BatchRoute {
+    uint32_t rounds = 0;
+    bool parts = false;
+    uint32_t kind() const { return rounds ? 1 + rounds : parts ? 1 : 0; }
+};
+
+// The captured graphs of a workspace, one per route: batches of one size whose
+// entries lie on both sides of a threshold alternate between them.
 struct BatchGraph {
-    static constexpr uint32_t kKinds = 4;
+    static constexpr uint32_t kMaxRounds = 3, kKinds = 2 + kMaxRounds;
     cudaGraphExec_t exec[kKinds] = {};
     uint32_t nmsm = 0, c = 0, L = 0;
     uint32_t moves = 0;      // BatchWork::moves() at the capture: the graphs hold the buffers' addresses
@@ -409,16 +423,17 @@ static cudaError_t build_tables(Basis* b, uint32_t c)
     return cudaSuccess;
 }
 
-// Workspace for batches of up to nmsm MSMs and cap pairs.
-// Whether a batch takes the part sort, and the most parts it can have.
-static bool part_sort(const Basis* b)
+// Whether a batch of that many entries takes the part sort, and the most parts it can have.
+static bool part_sort(const Basis* b, size_t entries)
 {
-    return (1u << (b->c - 1)) <= kPartMaxB && part_smem(b->c, b->D) <= kPartMaxSmem;
+    const size_t B = (size_t)1 << (b->c - 1);
+    return B <= kPartMaxB && part_smem(b->c, b->D) <= kPartMaxSmem && entries >= kPartMinFill * B;
 }
 
 static size_t max_parts(uint32_t nmsm, size_t cap) { return cap / kPartPairs + nmsm; }
 
-static cudaError_t ensure_work(const Basis* b, BatchWork* w, uint32_t nmsm, size_t cap)
+// Workspace for batches of up to nmsm MSMs and cap pairs.
+static cudaError_t ensure_work(const Basis* b, BatchWork* w, uint32_t nmsm, size_t cap, bool parts)
 {
     const uint32_t B = 1u << (b->c - 1);
     const size_t M = (size_t)nmsm * B;
@@ -427,7 +442,7 @@ static cudaError_t ensure_work(const Basis* b, BatchWork* w, uint32_t nmsm, size
     const size_t lvl1 = (size_t)nmsm * ((B + 7) / 8);
     const size_t lvl2 = (size_t)nmsm * ((B + 15) / 16) + nmsm;
     const size_t meta = (nmsm + 2 + 2 * max_parts(nmsm, cap)) * 4;      // off, number of parts, parts
-    const bool sorts = part_sort(b) ? w->base.get(max_parts(nmsm, cap) * B * sizeof(uint2)) != nullptr
+    const bool sorts = parts ? w->base.get(max_parts(nmsm, cap) * B * sizeof(uint2)) != nullptr
                                     : w->digits.get(nD * 4) && w->ranks.get(nD * 4) && w->pidx.get(nD * 4);
     bool ok = sorts && w->scal.get(cap * 32) && w->off.get(meta) && w->counts.get(M * 4) &&
               w->offsets.get((M + 1) * 4) &&
@@ -440,12 +455,13 @@ static cudaError_t ensure_work(const Basis* b, BatchWork* w, uint32_t nmsm, size
     return ok ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 
-// The device sequence of one batch (everything after the input copies), with
-// `rounds` batch-affine accumulation rounds.  *kernels: the number of kernels it
-// launched.
+// The device sequence of one batch (everything after the input copies).  *kernels:
+// the number of kernels it launched.
 static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
-                                 uint32_t rounds, uint32_t* kernels)
+                                 BatchRoute route, uint32_t* kernels)
 {
+    const uint32_t rounds = route.rounds;
+    const bool parts = route.parts;
     const uint32_t c = b->c, D = b->D, L = b->L, B = 1u << (c - 1);
     const size_t M = (size_t)nmsm * B;
     const size_t nD = cap * D;
@@ -466,7 +482,6 @@ static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
     cudaMemsetAsync(counts, 0, M * 4, st);
     cudaMemsetAsync(buckets, 0, M * sizeof(xyzz), st);
     cudaMemsetAsync(hot_count, 0, 12, st);
-    const bool parts = part_sort(b);
     const uint32_t* nparts = off + nmsm + 1;
     const unsigned pgrid = (unsigned)max_parts(nmsm, cap);
     uint32_t* sorted_pt = (uint32_t*)w->sorted_pt.p;
@@ -537,7 +552,7 @@ static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
 
 // Captures enqueue_batch as one of w->graph's.  The capture is ended whatever fails.
 static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
-                                 uint32_t rounds)
+                                 BatchRoute route)
 {
     BatchGraph& g = w->graph;
     if (!w->graph_fits(b, nmsm) || g.cap != cap) {
@@ -550,7 +565,7 @@ static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
     }
     CATMSM_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     uint32_t kernels = 0;
-    const cudaError_t queued = enqueue_batch(b, w, st, nmsm, cap, rounds, &kernels);
+    const cudaError_t queued = enqueue_batch(b, w, st, nmsm, cap, route, &kernels);
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
@@ -558,7 +573,7 @@ static cudaError_t capture_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     CATMSM_CHECK(e);
-    g.exec[rounds] = exec;
+    g.exec[route.kind()] = exec;
     return cudaSuccess;
 }
 
@@ -585,19 +600,19 @@ static cudaError_t copy_scalars(BatchWork* w, const uint8_t* scalars, size_t byt
 
 // Queues the copies of a batch (`bytes` of scalars, np parts) and its device sequence.
 static cudaError_t queue_batch(const Basis* b, BatchWork* w, cudaStream_t st, uint32_t nmsm, size_t cap,
-                               uint32_t rounds, const uint8_t* scalars, size_t bytes, uint32_t np, bool use_graph)
+                               BatchRoute route, const uint8_t* scalars, size_t bytes, uint32_t np, bool use_graph)
 {
     CATMSM_CHECK(copy_scalars(w, scalars, bytes, st));
     CATMSM_CHECK(cudaMemcpyAsync(w->off.p, w->h_off.p, (nmsm + 2 + 2 * (size_t)np) * 4, cudaMemcpyHostToDevice, st));
     if (use_graph) {
         const BatchGraph& g = w->graph;
-        if (!w->graph_fits(b, nmsm) || g.cap != cap || !g.exec[rounds])
-            CATMSM_CHECK(capture_batch(b, w, st, nmsm, cap, rounds));
-        CATMSM_CHECK(cudaGraphLaunch(g.exec[rounds], st));
+        if (!w->graph_fits(b, nmsm) || g.cap != cap || !g.exec[route.kind()])
+            CATMSM_CHECK(capture_batch(b, w, st, nmsm, cap, route));
+        CATMSM_CHECK(cudaGraphLaunch(g.exec[route.kind()], st));
         g_stats.launches += 1;
     } else {
         uint32_t kernels = 0;
-        CATMSM_CHECK(enqueue_batch(b, w, st, nmsm, cap, rounds, &kernels));
+        CATMSM_CHECK(enqueue_batch(b, w, st, nmsm, cap, route, &kernels));
         g_stats.launches += kernels;
     }
     CATMSM_CHECK(cudaGetLastError());
@@ -624,7 +639,9 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
         cap = std::min(full, (P / step + 1) * step);
         if (use_graph && w->graph_fits(b, nmsm) && w->graph.cap >= P) cap = w->graph.cap;
     }
-    CATMSM_CHECK(ensure_work(b, w, nmsm, cap));
+    BatchRoute route;
+    route.parts = part_sort(b, P * b->D);
+    CATMSM_CHECK(ensure_work(b, w, nmsm, cap, route.parts));
     uint32_t* off = (uint32_t*)w->h_off.p;
     uint32_t* parts = off + nmsm + 2;
     uint32_t np = 0, f = 0;
@@ -642,12 +659,12 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     // Batch-affine rounds by the entries this batch holds (the plain MSM's rule;
     // 1024 MSMs, 33 M entries, 32 a bucket: 15.4 ms without, 14.1 with).  Without
     // the memory for their lists the batch keeps the mixed additions.
-    uint32_t rounds = std::min(msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1)), BatchGraph::kKinds - 1);
-    if (rounds && aff_prepare(w->aff, b->L, (cap * b->D + b->L - 1) / b->L + 1, st) != cudaSuccess) {
+    route.rounds = std::min(msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1)), BatchGraph::kMaxRounds);
+    if (route.rounds && aff_prepare(w->aff, b->L, (cap * b->D + b->L - 1) / b->L + 1, st) != cudaSuccess) {
         cudaGetLastError();
-        rounds = 0;
+        route.rounds = 0;
     }
-    cudaError_t err = queue_batch(b, w, st, nmsm, cap, rounds, scalars, P * 32, np, use_graph);
+    cudaError_t err = queue_batch(b, w, st, nmsm, cap, route, scalars, P * 32, np, use_graph);
     if (err != cudaSuccess && w->aff.aux.stream) cudaStreamSynchronize(w->aff.aux.stream);
     const cudaError_t done = cudaStreamSynchronize(st);      // the caller's scalars are not read after return
     if (err == cudaSuccess) err = done;

@@ -112,3 +112,27 @@ done(log())
     assert any("k_aff_first" in o[2] for o in ops if o[0] == "launch")
     assert any("k_accumulate" in o[2] for o in ops if o[0] == "launch")
     assert kinds.count("instantiate") == 2 and kinds.count("replay") == 6
+
+
+@pytest.mark.parametrize("window,pairs,parts", [(13, 4096 * 29, False), (13, 4096 * 32, True), (11, 25599, False),
+                                                (11, 25600, True), (9, 64 * 80, False), (9, 64 * 100, True),
+                                                (14, 4096 * 32, False)])
+def test_sort_follows_the_entries(gpu_binding, window, pairs, parts):
+    """The sort by parts runs from 600 entries per bucket of an MSM on, up to 13-bit
+    windows, with and without the graph, whatever ran before."""
+    gpu_binding.load()
+    got = fake_cuda.run(gpu_binding.LIB_PATH, """
+b = Basis(4096, %d)
+counts = [%d // 64] * 63 + [%d - %d // 64 * 63]
+seen = []
+for graph in (False, True):
+    for c in (counts, [1] * 64, counts, [1] * 64, counts):
+        clear()
+        assert b.batch(c, graph) == 0
+        seen.append(["k_part_scatter" in kernels(), "k_scatter_batch" in kernels(), any(l[0] == "replay" for l in log())])
+done(seen)
+""" % (window, pairs, pairs, pairs))
+    assert got[0] == got[2] == got[4] == [parts, not parts, False] and got[1] == got[3] == [False, True, False]
+    assert got[5] == [parts, not parts, True]
+    # both routes' graphs are kept (the second route's buffers may move once)
+    assert got[8] == got[9] == [False, False, True]
