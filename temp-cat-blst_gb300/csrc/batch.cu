@@ -59,9 +59,6 @@ __global__ void k_fixup_join(const uint32_t* __restrict__ sorted_key, const uint
 __global__ void k_fixup_hot_seg(uint2* __restrict__ hot_list, uint32_t* __restrict__ hot_count,
                                 const uint32_t* __restrict__ offsets, uint32_t L, xyzz* __restrict__ buckets,
                                 const xyzz* __restrict__ head, const xyzz* __restrict__ tail);
-__global__ void k_reduce_level(const xyzz* __restrict__ inA, const xyzz* __restrict__ inQ, uint32_t m_in,
-                               uint32_t F, uint32_t lgF, uint32_t D, int first, xyzz* __restrict__ outA,
-                               xyzz* __restrict__ outQ);
 
 constexpr int kScanTileB = 1024 * 4;
 
@@ -324,18 +321,19 @@ __global__ void k_batch_out(const xyzz* __restrict__ roots, uint32_t nmsm, jac* 
 }
 
 // ---------------------------------------------------------------- basis object
-// How a batch of one size runs, by its entries: the affine rounds of its accumulation
-// and the form of its sort (by parts wherever there are rounds).
+// How a batch of one size runs, by its entries: the affine rounds of its accumulation,
+// the form of its sort, and whether its buckets hold two entries or more (with rounds
+// they do, and the window alone gives the sort).
 struct BatchRoute {
     uint32_t rounds = 0;
-    bool parts = false;
-    uint32_t kind() const { return rounds ? 1 + rounds : parts ? 1 : 0; }
+    bool parts = false, dense = false;
+    uint32_t kind() const { return rounds ? 3 + rounds : (parts ? 1 : 0) + (dense ? 2 : 0); }
 };
 
 // The captured graphs of a workspace, one per route: batches of one size whose
 // entries lie on both sides of a threshold alternate between them.
 struct BatchGraph {
-    static constexpr uint32_t kMaxRounds = 3, kKinds = 2 + kMaxRounds;
+    static constexpr uint32_t kMaxRounds = 3, kKinds = 4 + kMaxRounds;
     cudaGraphExec_t exec[kKinds] = {};
     uint32_t nmsm = 0, c = 0, L = 0;
     uint32_t moves = 0;      // BatchWork::moves() at the capture: the graphs hold the buffers' addresses
@@ -535,8 +533,7 @@ static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
         const uint32_t F = first ? 8 : 2;
         const uint32_t m_out = (m + F - 1) / F;
         if (first)
-            k_reduce_level<<<div_up((size_t)nmsm * m_out, 128), 128, 0, st>>>(inA, inQ, m, F, 3, nmsm, 1, bufA[pp],
-                                                                              bufQ[pp]);
+            msm_reduce_level(inA, m, F, nmsm, route.dense, bufA[pp], bufQ[pp], st);
         else
             msm_reduce_pair(inA, inQ, m, nmsm, bufA[pp], bufQ[pp], st);
         inA = bufA[pp];
@@ -641,6 +638,7 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     }
     BatchRoute route;
     route.parts = part_sort(b, P * b->D);
+    route.dense = P * b->D >= 2 * ((size_t)nmsm << (b->c - 1));
     CATMSM_CHECK(ensure_work(b, w, nmsm, cap, route.parts));
     uint32_t* off = (uint32_t*)w->h_off.p;
     uint32_t* parts = off + nmsm + 2;

@@ -66,6 +66,15 @@ void fixup_giants(const void* hot_list, const uint32_t* hot_count, const uint32_
 // One binary reduction level (fan-in 2) over D sets of m (A, Q) pairs.
 void msm_reduce_pair(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outA, void* outQ,
                      cudaStream_t st);
+// Level 1 of the reduction: D sets of m buckets to D x ceil(m / fan_in) pairs (fan-in
+// a power of two).  dense: at least two entries a bucket.  reduce_level_calls and
+// reduce_pair_lanes: its and msm_reduce_pair's form of field operation calls.
+void msm_reduce_level(const void* in, uint32_t m, uint32_t fan_in, uint32_t D, bool dense, void* outA, void* outQ,
+                      cudaStream_t st);
+void reduce_level_calls(const void* inA, const void* inQ, uint32_t m, uint32_t fan_in, uint32_t lg, uint32_t D,
+                        bool first, void* outA, void* outQ, cudaStream_t st);
+void reduce_pair_lanes(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outA, void* outQ,
+                       cudaStream_t st);
 
 // Bucket accumulation with `rounds` (>= 1) rounds of batch-affine additions
 // (Montgomery batch inversion) before the XYZZ fold; same outputs as

@@ -43,6 +43,7 @@
 #include "common.cuh"
 #include "curve.cuh"
 #include "fr.cuh"
+#include "reduce.cuh"
 #include "scalar.cuh"
 #include "host_curve.hpp"
 #include "catmsm_internal.h"
@@ -689,71 +690,16 @@ void fixup_giants(const void* hot_list, const uint32_t* hot_count, const uint32_
 // with fan-in 8: a 2-addition-per-bucket running sum that keeps every SM
 // busy.  Upper levels use fan-in 2 (one addition, one doubling, two Q
 // additions), keeping the dependent chain per level short: with few threads
-// the cost of a level is its serial latency, not its work.
-__global__ void __launch_bounds__(128) k_reduce_level(const xyzz* __restrict__ inA, const xyzz* __restrict__ inQ,
-                                                      uint32_t m_in, uint32_t F, uint32_t lgF, uint32_t D,
-                                                      int first, xyzz* __restrict__ outA, xyzz* __restrict__ outQ)
-{
-    const uint32_t m_out = (m_in + F - 1) / F;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= D * m_out) return;
-    const uint32_t w = t / m_out, u = t % m_out;
-    const uint32_t c0 = u * F;
-    const uint32_t cnt = min(F, m_in - c0);
-    const xyzz* a = inA + (size_t)w * m_in + c0;
-    xyzz r, tt, b;
-    xyzz_set_inf(r);
-    xyzz_set_inf(tt);
-    for (int j = (int)cnt - 1; j >= 1; j--) {
-        load_xyzz(b, a + j);
-        xyzz_add(r, b);
-        xyzz_add(tt, r);
-    }
-    load_xyzz(b, a);
-    xyzz_add(r, b);
-    if (first) xyzz_add(tt, r);
-    if (inQ) {
-        const xyzz* q = inQ + (size_t)w * m_in + c0;
-        for (uint32_t j = 0; j < cnt; j++) {
-            load_xyzz(b, q + j);
-            xyzz_add(tt, b);
-        }
-    }
-    if (m_out > 1) {
-        for (uint32_t k = 0; k < lgF; k++) xyzz_dbl(r);
-        store_xyzz(outA + (size_t)w * m_out + u, r);
-    }
-    store_xyzz(outQ + (size_t)w * m_out + u, tt);
-}
+// the cost of a level is its serial latency, not its work.  (k_reduce_level and the
+// binary levels by lanes: reduce.cuh.)
 
 // Binary levels with two threads per node: the Q thread computes
 // Q = A_1 + Q_0 + Q_1 and the A thread A = 2 (A_0 + A_1), concurrently (one
 // thread doing both ran 3 additions and a doubling back to back; the level's
 // dependent chain is now 2 additions).  A node with one child keeps Q_0 and
-// doubles A_0.  This is k_reduce_level's rule with fan-in 2.  Quad = true:
-// each of the two is a quad of lanes (quad point operations), for levels
-// too small to fill the GPU.
-__device__ __forceinline__ void pair_node(xyzz& out, const xyzz* a, const xyzz* q, uint32_t cnt, bool q_role)
-{
-    xyzz b;
-    if (q_role) {
-        load_xyzz(out, q);
-        if (cnt == 2) {
-            load_xyzz(b, a + 1);
-            xyzz_add(out, b);
-            load_xyzz(b, q + 1);
-            xyzz_add(out, b);
-        }
-    } else {
-        load_xyzz(out, a);
-        if (cnt == 2) {
-            load_xyzz(b, a + 1);
-            xyzz_add(out, b);
-        }
-        xyzz_dbl(out);
-    }
-}
-
+// doubles A_0.  This is k_reduce_level's rule with fan-in 2.  Each of the two is
+// a lane, or a quad of lanes (quad point operations) for levels too small to fill
+// the GPU.
 __device__ __forceinline__ fp pair_node_quad(const xyzz* a, const xyzz* q, uint32_t cnt, bool q_role,
                                              const quad_lane& ql)
 {
@@ -764,45 +710,28 @@ __device__ __forceinline__ fp pair_node_quad(const xyzz* a, const xyzz* q, uint3
     return out;
 }
 
-// Thread g's node and role.  The role is uniform per warp (even warps Q, odd
-// warps A): lanes of one warp taking different roles would run both paths one
-// after the other.  A warp covers 32 nodes, or 8 with quads.
-template <bool Quad>
-__device__ __forceinline__ void pair_slot(uint32_t g, uint32_t& node, bool& q_role)
-{
-    node = Quad ? (g >> 6) * 8 + ((g >> 2) & 7) : (g >> 6) * 32 + (g & 31);
-    q_role = ((g >> 5) & 1) == 0;
-}
-
-// One binary level over D windows of m_in (A, Q) pairs.
-template <bool Quad>
-__global__ void __launch_bounds__(128) k_reduce_pair(const xyzz* __restrict__ inA, const xyzz* __restrict__ inQ,
-                                                     uint32_t m_in, uint32_t D, xyzz* __restrict__ outA,
-                                                     xyzz* __restrict__ outQ)
+// One binary level over D windows of m_in (A, Q) pairs, by quads (k_reduce_pair_lanes:
+// by lanes).
+__global__ void __launch_bounds__(128) k_reduce_pair_quads(const xyzz* __restrict__ inA, const xyzz* __restrict__ inQ,
+                                                           uint32_t m_in, uint32_t D, xyzz* __restrict__ outA,
+                                                           xyzz* __restrict__ outQ)
 {
     const uint32_t m_out = (m_in + 1) / 2;
     uint32_t t;
     bool q_role;
-    pair_slot<Quad>(blockIdx.x * blockDim.x + threadIdx.x, t, q_role);
+    pair_slot<true>(blockIdx.x * blockDim.x + threadIdx.x, t, q_role);
     if (t >= D * m_out || (!q_role && m_out == 1)) return;
     const quad_lane ql = quad_of(threadIdx.x & 31);
     const uint32_t w = t / m_out, u = t % m_out;
     const size_t base = (size_t)w * m_in + 2 * u;
-    xyzz* dst = (q_role ? outQ : outA) + (size_t)w * m_out + u;
-    const uint32_t cnt = min(2u, m_in - 2 * u);
-    if (Quad) {
-        qd_store(dst, pair_node_quad(inA + base, inQ + base, cnt, q_role, ql), ql);
-    } else {
-        xyzz r;
-        pair_node(r, inA + base, inQ + base, cnt, q_role);
-        store_xyzz(dst, r);
-    }
+    qd_store((q_role ? outQ : outA) + (size_t)w * m_out + u,
+             pair_node_quad(inA + base, inQ + base, min(2u, m_in - 2 * u), q_role, ql), ql);
 }
 
 // The last binary levels in one launch: block w reduces window w's m_in
 // (A, Q) pairs (m_in <= kTailThreads / 4) to its root Q in shared memory with
 // one barrier per level, instead of one launch and a global round trip per
-// level.  Quads placed as in k_reduce_pair<true>; the block is sized to the
+// level.  Quads placed as in k_reduce_pair_quads; the block is sized to the
 // first level so that many windows fit on an SM.
 constexpr int kTailThreads = 256;
 constexpr size_t kFanIn8MinBuckets = size_t(1) << 18;   // all windows' buckets
@@ -930,18 +859,36 @@ void msm_reduce_tail(const void* inA, const void* inQ, uint32_t m, uint32_t D, v
     k_reduce_tail<<<D, T, T / 8 * 2 * sizeof(xyzz), st>>>((const xyzz*)inA, (const xyzz*)inQ, m, (xyzz*)outQ);
 }
 
+// Level 1 of the reduction over D sets of m buckets.  dense: at least two entries a
+// bucket on average.  With fewer, and below a full launch, the form whose field
+// operations are all calls is faster, by up to a third where most buckets are empty
+// (inlined, a warp's few busy lanes walk far more code); a full dense launch gains from
+// the inlined one.  Calls against inlined, us: 256 x 4096 buckets, 0.02 entries a bucket 837 / 1222,
+// 0.5 1430 / 1544, 1 1340 / 1394, 2 1252 / 1243, 4 1199 / 1181, 20 1165 / 1102; 8192 nodes (64 x 1024
+// buckets, 96 a bucket) 230 / 246, 32768 nodes 298 / 288.
+void msm_reduce_level(const void* in, uint32_t m, uint32_t fan_in, uint32_t D, bool dense, void* outA, void* outQ,
+                      cudaStream_t st)
+{
+    const size_t nodes = (size_t)D * ((m + fan_in - 1) / fan_in);
+    uint32_t lg = 0;
+    while ((1u << lg) < fan_in) lg++;
+    if (dense && nodes >= 32768)
+        k_reduce_level<true><<<div_up(nodes, 128), 128, 0, st>>>((const xyzz*)in, nullptr, m, fan_in, lg, D, 1,
+                                                                 (xyzz*)outA, (xyzz*)outQ);
+    else
+        reduce_level_calls(in, nullptr, m, fan_in, lg, D, true, outA, outQ, st);
+}
+
 void msm_reduce_pair(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outA, void* outQ,
                      cudaStream_t st)
 {
     const size_t nodes = (size_t)D * ((m + 1) / 2);
     if (nodes <= kQuadMaxNodes) {
         const size_t threads = (nodes + 7) / 8 * 64;
-        k_reduce_pair<true><<<div_up(threads, 128), 128, 0, st>>>((const xyzz*)inA, (const xyzz*)inQ, m, D,
+        k_reduce_pair_quads<<<div_up(threads, 128), 128, 0, st>>>((const xyzz*)inA, (const xyzz*)inQ, m, D,
                                                                   (xyzz*)outA, (xyzz*)outQ);
     } else {
-        const size_t threads = (nodes + 31) / 32 * 64;
-        k_reduce_pair<false><<<div_up(threads, 128), 128, 0, st>>>((const xyzz*)inA, (const xyzz*)inQ, m, D,
-                                                                   (xyzz*)outA, (xyzz*)outQ);
+        reduce_pair_lanes(inA, inQ, m, D, outA, outQ, st);
     }
 }
 
@@ -1289,11 +1236,8 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
             }
             const uint32_t F = first ? S : 2;
             const uint32_t m_out = (m + F - 1) / F;
-            if (first)
-                k_reduce_level<<<div_up((size_t)D * m_out, 128), 128, 0, st>>>(inA, inQ, m, F, S == 16 ? 4 : 3, D, 1,
-                                                                              bufA[pp], bufQ[pp]);
-            else
-                msm_reduce_pair(inA, inQ, m, D, bufA[pp], bufQ[pp], st);
+            if (first) msm_reduce_level(inA, m, F, D, nD >= 2 * M, bufA[pp], bufQ[pp], st);
+            else msm_reduce_pair(inA, inQ, m, D, bufA[pp], bufQ[pp], st);
             g_stats.launches++;
             inA = bufA[pp];
             inQ = bufQ[pp];

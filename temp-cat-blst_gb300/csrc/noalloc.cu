@@ -68,9 +68,6 @@ __global__ void k_fixup_rest(const uint2* __restrict__ hot_list, const uint32_t*
 __global__ void k_fixup_hot(uint2* __restrict__ hot_list, uint32_t* __restrict__ hot_count,
                             const uint32_t* __restrict__ offsets, uint32_t L, xyzz* __restrict__ buckets,
                             const xyzz* __restrict__ head, const xyzz* __restrict__ tail);
-__global__ void k_reduce_level(const xyzz* __restrict__ inA, const xyzz* __restrict__ inQ, uint32_t m_in,
-                               uint32_t F, uint32_t lgF, uint32_t D, int first, xyzz* __restrict__ outA,
-                               xyzz* __restrict__ outQ);
 
 namespace {
 
@@ -189,13 +186,11 @@ static cudaError_t noalloc_queue(unsigned char* base, const blst_p1_affine* poin
     bool first = true;
     while (m > 1) {
         const uint32_t F = first ? 8 : 2, lgF = first ? 3 : 1;
-        const uint32_t m_out = (m + F - 1) / F;
-        k_reduce_level<<<div_up((size_t)D * m_out, 128), 128, 0, st>>>(inA, inQ, m, F, lgF, D, first ? 1 : 0,
-                                                                      bufA[pp], bufQ[pp]);
+        reduce_level_calls(inA, inQ, m, F, lgF, D, first, bufA[pp], bufQ[pp], st);
         inA = bufA[pp];
         inQ = bufQ[pp];
         pp ^= 1;
-        m = m_out;
+        m = (m + F - 1) / F;
         first = false;
     }
     CATMSM_CHECK(cudaMemcpyAsync(wins, inQ, (size_t)D * sizeof(xyzz), cudaMemcpyDeviceToDevice, st));

@@ -74,7 +74,7 @@ def test_no_replay_over_freed_buffers(gpu_binding, name):
 def test_graph_is_kept_while_nothing_moves(gpu_binding):
     gpu_binding.load()
     ops = fake_cuda.run(gpu_binding.LIB_PATH, PRELUDE + """
-for k in (300, 280, 300, 1, 299):
+for k in (300, 280, 300, 150, 299):
     b.batch([k] * 8, True)
 done(log())
 """)
@@ -136,3 +136,17 @@ done(seen)
     assert got[5] == [parts, not parts, True]
     # both routes' graphs are kept (the second route's buffers may move once)
     assert got[8] == got[9] == [False, False, True]
+
+
+@pytest.mark.parametrize("nmsm,pairs,inlined", [(256, 4, False), (256, 399, False), (256, 410, True), (32, 4096, False)])
+def test_level_form_follows_the_fill(gpu_binding, nmsm, pairs, inlined):
+    """The reduction's first level: inlined field operations in full launches over at
+    least two entries a bucket, calls elsewhere."""
+    gpu_binding.load()
+    got = fake_cuda.run(gpu_binding.LIB_PATH, """
+b = Basis(4096, 13)
+clear()
+b.batch([%d] * %d, False)
+done([k for k in kernels() if k.startswith("k_reduce_level")])
+""" % (pairs, nmsm))
+    assert len(got) == 1 and ("true" in got[0]) == inlined
