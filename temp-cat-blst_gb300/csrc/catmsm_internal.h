@@ -45,7 +45,8 @@ cudaError_t msm_setup_device();
 // sums (as the device wrote them) in wins after the stream is synchronised.
 struct SmallMsm {
     const uint64_t* wins = nullptr;
-    const uint32_t* over = nullptr;     // nonzero: too skewed, nothing computed (run the general pipeline)
+    const uint32_t* over = nullptr;     // nonzero: too skewed, no sums (run the general pipeline, on W.glv_pts and
+                                        // W.glv_sc if the scalars were split)
     uint32_t D = 0, c = 0;
 };
 bool msm_small_applies(size_t pipeline_points, bool glv);
@@ -56,9 +57,11 @@ cudaError_t msm_small(Ctx* ctx, const void* pts, const uint8_t* scalars, uint32_
                       bool glv, uint32_t* entries, SmallMsm& out);
 
 // The fused last reduction levels for D independent sets of m (A, Q) XYZZ
-// pairs (m <= msm_reduce_tail_max(D)); roots to outQ[0..D).
+// pairs (m <= msm_reduce_tail_max(D)); roots to outQ[0..D).  stop: a device word that
+// leaves the launch without work when it is set, or null.
 uint32_t msm_reduce_tail_max(uint32_t D);
-void msm_reduce_tail(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outQ, cudaStream_t st);
+void msm_reduce_tail(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outQ, cudaStream_t st,
+                     const uint32_t* stop = nullptr);
 // Joins of buckets whose carries span more than 1024 partials, by the whole
 // grid (after k_fixup_hot / k_fixup_hot_seg; seg = the segmented fixup).
 void fixup_giants(const void* hot_list, const uint32_t* hot_count, const uint32_t* offsets, uint32_t L,

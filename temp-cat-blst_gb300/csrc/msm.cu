@@ -740,9 +740,11 @@ constexpr uint32_t kQuadMaxNodes = 8192;                  // a level of at most 
 
 __global__ void __launch_bounds__(kTailThreads) k_reduce_tail(const xyzz* __restrict__ inA,
                                                               const xyzz* __restrict__ inQ, uint32_t m_in,
-                                                              xyzz* __restrict__ outQ)
+                                                              xyzz* __restrict__ outQ,
+                                                              const uint32_t* __restrict__ stop)
 {
     extern __shared__ __align__(16) unsigned char tail_smem[];
+    if (stop && *stop) return;
     const uint32_t nodes = blockDim.x / 8;
     xyzz* shA = reinterpret_cast<xyzz*>(tail_smem);
     xyzz* shQ = shA + nodes;
@@ -791,9 +793,8 @@ uint32_t msm_default_window(size_t n)
 // its entries in a few hot buckets), the c in [2, 20] minimising bucket
 // entries + 4 x buckets (reducing a bucket costs about four accumulated
 // entries on this GPU).  Measured best: 16 for n2 = 2^21, 19 for n2 = 2^23.
-uint32_t msm_glv_window(size_t n2)
+static uint32_t glv_model_window(size_t n2)
 {
-    if (msm_small_applies(n2, true)) return msm_small_window(n2);
     double best = 0;
     uint32_t bc = 0;
     for (uint32_t c = 2; c <= 20; c++) {
@@ -812,6 +813,11 @@ uint32_t msm_glv_window(size_t n2)
     while ((size_t(2) << lg) <= n2) lg++;
     if (n2 <= (size_t(1) << 15)) bc = std::min(bc, std::max(8u, lg - 5));
     return bc;
+}
+
+uint32_t msm_glv_window(size_t n2)
+{
+    return msm_small_applies(n2, true) ? msm_small_window(n2) : glv_model_window(n2);
 }
 
 // Window for n points of nbits-bit scalars without the GLV split.  From 2^18 points
@@ -853,10 +859,12 @@ constexpr uint32_t kTailMaxSets = 64;
 
 uint32_t msm_reduce_tail_max(uint32_t D) { return D > kTailMaxSets ? 1 : kTailThreads / 4; }
 
-void msm_reduce_tail(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outQ, cudaStream_t st)
+void msm_reduce_tail(const void* inA, const void* inQ, uint32_t m, uint32_t D, void* outQ, cudaStream_t st,
+                     const uint32_t* stop)
 {
     const uint32_t T = ((m + 1) / 2 + 7) / 8 * 64;   // a Q warp and an A warp per 8 first-level nodes
-    k_reduce_tail<<<D, T, T / 8 * 2 * sizeof(xyzz), st>>>((const xyzz*)inA, (const xyzz*)inQ, m, (xyzz*)outQ);
+    k_reduce_tail<<<D, T, T / 8 * 2 * sizeof(xyzz), st>>>((const xyzz*)inA, (const xyzz*)inQ, m, (xyzz*)outQ,
+                                                       stop);
 }
 
 // Level 1 of the reduction over D sets of m buckets.  dense: at least two entries a
@@ -1073,6 +1081,7 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     // Few points (and no width or rounds asked for): one kernel for the buckets of
     // all windows instead of the sort, accumulate, fixup and reduce launches
     const bool glv_split = !tile_window && use_glv(ctx, n, nbits);
+    bool split_done = false;             // the small path has written the halves and the signed points
     if (!tile_window && c == 0 && takes_small(ctx->affine_rounds, glv_split ? 2 * n : n, nbits, glv_split)) {
         if (points_ready) CATMSM_CHECK(cudaStreamWaitEvent(st, points_ready, 0));
         SmallMsm m;
@@ -1093,6 +1102,7 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
             if (P.enabled) CATMSM_CHECK(profile_end(P, st, entries));
             return cudaSuccess;
         }
+        split_done = glv_split;
     }
     // The points are read only from the point stage on (after the scatter):
     // points_ready, if given, is an event on another stream (a host copy in
@@ -1106,14 +1116,16 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
         uint4* gsc = (uint4*)W.glv_sc.get(2 * n * sizeof(uint4));
         sgn = (uint8_t*)W.glv_sign.get(n);
         if (!gpts || !gsc || !sgn) return cudaErrorMemoryAllocation;
-        k_glv_scalars<<<div_up(n, 128), 128, 0, st>>>(d_scalars, stride, (uint32_t)n, nbits, gsc, sgn);
-        g_stats.launches++;
+        if (!split_done) {
+            k_glv_scalars<<<div_up(n, 128), 128, 0, st>>>(d_scalars, stride, (uint32_t)n, nbits, gsc, sgn);
+            g_stats.launches++;
+        }
         d_points = gpts;
         d_scalars = reinterpret_cast<const uint8_t*>(gsc);
         stride = 16;
         n *= 2;
         nbits = 127;
-        if (c == 0) c = msm_glv_window(n);
+        if (c == 0) c = split_done ? glv_model_window(n) : msm_glv_window(n);
     }
     uint32_t D;
     if (tile_window) {
@@ -1179,7 +1191,7 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
     k_scatter<<<div_up(nD, 256), 256, 0, st>>>(digits, ranks, offsets, (uint32_t)n, (uint32_t)nD, sorted_pt,
                                               sorted_key);
     if (points_ready) CATMSM_CHECK(cudaStreamWaitEvent(st, points_ready, 0));
-    if (gpts) {
+    if (gpts && !split_done) {
         k_glv_points<<<div_up(n_in, 128), 128, 0, st>>>(src_points, sgn, (uint32_t)n_in, gpts);
         g_stats.launches++;
     }

@@ -14,10 +14,10 @@
 //   sums     about 368 threads, each with up to L entries of ONE bucket (a bucket of
 //            m entries gets ceil(m / L) threads, so one hot bucket still uses them all),
 //            then a quad tree over each bucket's threads.
-//            A block of more than twice its share and 2048 entries (equal scalars:
-//            all of a window in one block) stops, and the general pipeline, which
-//            spreads a bucket over the whole GPU, runs instead (4096 equal scalars:
-//            372 us there, 626 here);
+//            A block with too many entries (kSmallMaxEntries; equal scalars: all of a
+//            window in one block) raises a flag, the others leave before their sums,
+//            and the general pipeline, which spreads a bucket over the whole GPU, runs
+//            instead, on the split that is there already;
 //   reduce   sum_b (b + 1) S_b of the range by binary (A, Q) levels (the rule of
 //            the general reduction), the ranges of a window by k_reduce_tail.
 #define CATMSM_INLINE_SQR   // see field.cuh
@@ -38,6 +38,13 @@ constexpr uint32_t kSmallNarrow = 512;         // up to this many: 4-bit windows
 constexpr uint32_t kSmallThreads = 512;
 constexpr uint32_t kSmallSums = 368;           // threads with entries, before one more per bucket
 constexpr uint32_t kSmallMaxR = 16;            // buckets per block
+// Entries of a block: at most this many, or 7/4 of its share of a window (the top
+// window of GLV halves below 2^126.4 has 1.49 of it in a block), and of one bucket
+// kSmallMaxBucket.  Above, the general pipeline is faster although the attempt comes
+// before it (about 15 us).  Twice the share, no bound on a bucket and every block at work
+// to its end: 8192 scalars below 2^64 649 us, 461 now; eight values 890, 540; 12288 zeros and
+// ones 469, 345; 8192 scalars of 129 bits 743, 530.
+constexpr uint32_t kSmallMaxEntries = 2048, kSmallMaxBucket = 2560;
 
 // Measured against the general pipeline (host call, us): 255 bits 64 points 170 / 308,
 // 4096 306 / 405, 12288 497 / 521, 16384 611 / 553; 64 bits 2048 points 237 / 348,
@@ -65,10 +72,12 @@ uint32_t msm_small_windows(size_t pipeline_points, uint32_t bits, bool glv)
 // k_glv_points; thread i < n writes s1 P_i, thread n + i s2 phi(P_i).
 __global__ void __launch_bounds__(128) k_small_glv(const uint8_t* __restrict__ scalars, uint32_t stride, uint32_t n,
                                                    uint32_t nbits, const affine* __restrict__ pts,
-                                                   uint4* __restrict__ mag, affine* __restrict__ gpts)
+                                                   uint4* __restrict__ mag, affine* __restrict__ gpts,
+                                                   uint32_t* __restrict__ stop)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 2 * n) return;
+    if (t == 0) *stop = 0;
     const uint32_t i = t < n ? t : t - n;
     uint32_t k[8], m1[4], m2[4];
     bool s1, s2;
@@ -91,10 +100,12 @@ __global__ void __launch_bounds__(128) k_small_glv(const uint8_t* __restrict__ s
 
 // Scalars of at most 128 bits as 16-byte magnitudes (no split).
 __global__ void __launch_bounds__(128) k_small_scalars(const uint8_t* __restrict__ scalars, uint32_t stride, uint32_t n,
-                                                       uint32_t nbits, uint4* __restrict__ mag)
+                                                       uint32_t nbits, uint4* __restrict__ mag,
+                                                       uint32_t* __restrict__ stop)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i == 0) *stop = 0;
     uint32_t k[8];
     load_scalar(k, scalars + (size_t)i * stride, stride, nbits);
     mag[i] = make_uint4(k[0], k[1], k[2], k[3]);
@@ -109,7 +120,8 @@ struct SmallArgs {
     xyzz* outQ;                 // per (window, range): sum (b + 1) S_b
     uint32_t* entries;          // counter of nonzero digits, or null
     uint32_t limit;             // most entries of a block
-    uint32_t* over;             // page-locked: set when a block has more
+    uint32_t* stop;             // set when a block has more (zeroed by the kernel before)
+    uint32_t* over;             // page-locked: the same for the host
 };
 
 // Signed digit of window w (bits [c w, c w + c) of k + bias, minus 2^(c - 1)).
@@ -147,7 +159,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
     xyzz* acc = reinterpret_cast<xyzz*>(small_smem);          // a partial sum per thread
     xyzz* lev = acc + kSmallAcc;                              // bucket sums, then (Q | A) of the levels
     uint32_t* list = reinterpret_cast<uint32_t*>(lev + 3 * kSmallMaxR);
-    __shared__ uint32_t cnt[kSmallMaxR], start[kSmallMaxR + 1], ts[kSmallMaxR + 1], shape[3];
+    __shared__ uint32_t cnt[kSmallMaxR], start[kSmallMaxR + 1], ts[kSmallMaxR + 1], shape[4];
     const uint32_t tid = threadIdx.x, R = A.R;
     const uint32_t w = blockIdx.x / A.nb, b0 = blockIdx.x % A.nb * R;
     if (tid < kSmallMaxR) cnt[tid] = 0;
@@ -155,7 +167,10 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
     for (uint32_t i = tid; i < A.n; i += blockDim.x) {
         const int32_t d = small_digit(__ldg(A.mag + i), A, w);
         const uint32_t b = (uint32_t)(d < 0 ? -d : d) - 1 - b0;          // d = 0 wraps past R
-        if (d != 0 && b < R) atomicAdd(&cnt[b], 1u);
+        if (d != 0 && b < R && atomicAdd(&cnt[b], 1u) == kSmallMaxBucket) {      // one bucket is too many already
+            *(volatile uint32_t*)A.stop = 1;
+            *A.over = 1;
+        }
     }
     __syncthreads();
     if (tid == 0) {
@@ -178,7 +193,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
         shape[0] = L;
         shape[1] = most;
         shape[2] = s > A.limit;
-        if (s > A.limit) *A.over = 1;
+        if (shape[2]) {
+            *(volatile uint32_t*)A.stop = 1;
+            *A.over = 1;
+        }
+        if (*(volatile uint32_t*)A.stop) shape[2] = 1;
         if (A.entries) atomicAdd(A.entries, s);
     }
     __syncthreads();
@@ -189,7 +208,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
         const uint32_t b = (uint32_t)(d < 0 ? -d : d) - 1 - b0;
         if (d != 0 && b < R) list[atomicAdd(&cnt[b], 1u)] = i | (d < 0 ? 0x80000000u : 0u);
     }
+    // Some block has raised the flag: no sums here either.  A block that read it too early
+    // computes in vain (its results are not used); nothing waits for it.
+    if (tid == 0) shape[3] = *(volatile uint32_t*)A.stop;
     __syncthreads();
+    if (shape[3]) return;
     if (tid < ts[R]) {
         uint32_t b = 0;
         while (ts[b + 1] <= tid) b++;
@@ -292,17 +315,19 @@ cudaError_t msm_small(Ctx* ctx, const void* pts, const uint8_t* scalars, uint32_
     }
     uint4* mag = (uint4*)W.glv_sc.get(np * sizeof(uint4));
     affine* gpts = glv ? (affine*)W.glv_pts.get(np * sizeof(affine)) : nullptr;
-    xyzz* seg = (xyzz*)W.seg.get(2 * (size_t)D * A.nb * sizeof(xyzz));
+    xyzz* seg = (xyzz*)W.seg.get((2 * (size_t)D * A.nb + 1) * sizeof(xyzz));
     xyzz* wins = (xyzz*)ctx->h_out.get((size_t)(D + 1) * sizeof(xyzz));
     if (!mag || (glv && !gpts) || !seg || !wins) return cudaErrorMemoryAllocation;
+    A.stop = (uint32_t*)(seg + 2 * (size_t)D * A.nb);
     if (glv)
-        k_small_glv<<<div_up(np, 64), 64, 0, st>>>(scalars, stride, (uint32_t)n, nbits, (const affine*)pts, mag, gpts);
+        k_small_glv<<<div_up(np, 64), 64, 0, st>>>(scalars, stride, (uint32_t)n, nbits, (const affine*)pts, mag, gpts,
+                                                   A.stop);
     else
-        k_small_scalars<<<div_up(np, 128), 128, 0, st>>>(scalars, stride, (uint32_t)n, nbits, mag);
+        k_small_scalars<<<div_up(np, 128), 128, 0, st>>>(scalars, stride, (uint32_t)n, nbits, mag, A.stop);
     A.pts = glv ? gpts : (const affine*)pts;
     A.mag = mag;
     A.entries = entries;
-    A.limit = std::max(2048u, 2 * (A.n + A.nb - 1) / A.nb);
+    A.limit = std::max(kSmallMaxEntries, 7 * (A.n / A.nb) / 4);
     A.over = (uint32_t*)(wins + D);
     *A.over = 0;
     A.outA = A.nb > 1 ? seg : nullptr;
@@ -310,7 +335,7 @@ cudaError_t msm_small(Ctx* ctx, const void* pts, const uint8_t* scalars, uint32_
     k_small_buckets<<<D * A.nb, kSmallThreads, kSmallFixed + np * 4, st>>>(A);
     g_stats.launches += 2;
     if (A.nb > 1) {
-        msm_reduce_tail(A.outA, A.outQ, A.nb, D, wins, st);
+        msm_reduce_tail(A.outA, A.outQ, A.nb, D, wins, st, A.stop);
         g_stats.launches++;
     }
     out.wins = (const uint64_t*)wins;
