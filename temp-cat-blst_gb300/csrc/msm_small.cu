@@ -42,8 +42,8 @@ constexpr uint32_t kSmallMaxR = 16;            // buckets per block
 // window of GLV halves below 2^126.4 has 1.49 of it in a block), and of one bucket
 // kSmallMaxBucket.  Above, the general pipeline is faster although the attempt comes
 // before it (about 15 us).  Twice the share, no bound on a bucket and every block at work
-// to its end: 8192 scalars below 2^64 649 us, 461 now; eight values 890, 540; 12288 zeros and
-// ones 469, 345; 8192 scalars of 129 bits 743, 530.
+// to its end: 8192 scalars below 2^64 649 us, 477 now; eight values 890, 569; 12288 zeros and
+// ones 469, 345; 8192 scalars of 129 bits 743, 540.
 constexpr uint32_t kSmallMaxEntries = 2048, kSmallMaxBucket = 2560;
 
 // Measured against the general pipeline (host call, us): 255 bits 64 points 170 / 308,
