@@ -616,11 +616,13 @@ static cudaError_t queue_batch(const Basis* b, BatchWork* w, cudaStream_t st, ui
     return cudaMemcpyAsync(w->h_out.p, w->out.p, (size_t)nmsm * sizeof(jac), cudaMemcpyDeviceToHost, st);
 }
 
+// rounds false: no affine rounds, whatever the entries (their memory is not to be had).
 // exact_cap: size the work for exactly the pairs of this batch (serving);
 // otherwise for its pairs rounded up to a sixteenth of full-basis MSMs, or for
 // the captured graph's if they fit it, so one graph serves batches of one size.
 static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* out, uint32_t nmsm,
-                             const size_t* counts, const uint8_t* scalars, bool use_graph, bool exact_cap)
+                             const size_t* counts, const uint8_t* scalars, bool use_graph, bool exact_cap,
+                             bool rounds = true)
 {
     if (!b->tables) return cudaErrorMemoryAllocation;
     size_t P = 0;
@@ -657,7 +659,8 @@ static cudaError_t run_batch(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* o
     // Batch-affine rounds by the entries this batch holds (the plain MSM's rule;
     // 1024 MSMs, 33 M entries, 32 a bucket: 15.4 ms without, 14.1 with).  Without
     // the memory for their lists the batch keeps the mixed additions.
-    route.rounds = std::min(msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1)), BatchGraph::kMaxRounds);
+    if (rounds)
+        route.rounds = std::min(msm_affine_rounds(P * b->D, (size_t)nmsm << (b->c - 1)), BatchGraph::kMaxRounds);
     if (route.rounds && aff_prepare(w->aff, b->L, (cap * b->D + b->L - 1) / b->L + 1, st) != cudaSuccess) {
         cudaGetLastError();
         route.rounds = 0;
@@ -681,9 +684,9 @@ void batch_work_free(BatchWork* w)
 }
 
 cudaError_t batch_run(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* out, uint32_t nmsm, const size_t* counts,
-                      const uint8_t* scalars)
+                      const uint8_t* scalars, bool rounds)
 {
-    return run_batch(b, w, st, out, nmsm, counts, scalars, false, true);
+    return run_batch(b, w, st, out, nmsm, counts, scalars, false, true, rounds);
 }
 
 size_t basis_points(const Basis* b) { return b->n; }

@@ -21,9 +21,10 @@ struct BatchWork;
 BatchWork* batch_work_new();
 void batch_work_free(BatchWork* w);
 // nmsm MSMs over the basis prefixes counts[j] with 32-byte scalars
-// (concatenated); Jacobian results to host `out`; synchronous on stream st.
+// (concatenated); Jacobian results to host `out`; synchronous on stream st.  rounds
+// false: no affine rounds, whatever the entries.
 cudaError_t batch_run(Basis* b, BatchWork* w, cudaStream_t st, blst_p1* out, uint32_t nmsm,
-                      const size_t* counts, const uint8_t* scalars);
+                      const size_t* counts, const uint8_t* scalars, bool rounds);
 size_t basis_points(const Basis* b);
 uint32_t basis_window(const Basis* b);
 int basis_device(const Basis* b);

@@ -132,9 +132,18 @@ size_t msm_mem(const Basis* b, size_t k)
     // a smaller MSM runs over the tables in a batch, or through the plain
     // pipeline alone: the larger of the two
     const size_t D = 256 / basis_window(b) + 1;
-    // (index/key/rank words and the batch-affine lists of a window's entry: ~256 B)
-    const size_t table = k * D * 256 + ((size_t)1 << (basis_window(b) - 1)) * 192 * 2 + k * 32 + (1 << 20);
+    const size_t table = k * D * 24 + ((size_t)1 << (basis_window(b) - 1)) * 192 * 2 + k * 32 + (1 << 20);
     return std::max(plain, table);
+}
+
+// What the affine rounds of a batch over the tables take besides (0: it would run
+// none): ~232 B of lists and prefix products an entry, two slices of 2^25 at most.
+// The batch runs without them where the budget has no room for that.
+size_t rounds_mem(const Basis* b, size_t points, size_t msms)
+{
+    const size_t entries = points * (256 / basis_window(b) + 1);
+    if (!msm_affine_rounds(entries, msms << (basis_window(b) - 1))) return 0;
+    return std::min(entries, (size_t)1 << 26) * 232;
 }
 
 // values, scratch, prepared and given roots, and the products of a pass
@@ -176,7 +185,7 @@ void worker_main(Worker* wk)
     for (;;) {
         std::vector<Request*> batch;
         size_t mem = 0;
-        bool large = false;
+        bool large = false, rounds = true;
         {
             std::unique_lock<std::mutex> lk(s->mu);
             const Request* head = nullptr;
@@ -219,6 +228,11 @@ void worker_main(Worker* wk)
                 mem += r->mem;
                 it = s->queue.erase(it);
             }
+            if (type == 0 && batch.size() > 1 && batch[0]->k < kPlainMinPoints) {
+                const size_t more = rounds_mem(s->basis, pts, batch.size());
+                rounds = s->inflight + mem + more <= s->budget;
+                if (rounds) mem += more;
+            }
             s->inflight += mem;
             s->batches++;
             s->batched_reqs += (long)batch.size();
@@ -252,7 +266,7 @@ void worker_main(Worker* wk)
             }
             std::vector<blst_p1> out(batch.size());
             rc = (int)batch_run(s->basis, wk->work, ctx->stream, out.data(), (uint32_t)batch.size(), counts.data(),
-                                sc.data());
+                                sc.data(), rounds);
             for (size_t j = 0; j < batch.size(); j++) batch[j]->result = out[j];
         } else {
             std::vector<blst_p1*> vals;
