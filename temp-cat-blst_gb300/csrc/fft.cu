@@ -425,8 +425,9 @@ k_fft_items(const xyzz* __restrict__ a, xyzz* __restrict__ prod, const FftJob* _
 // The V of a pass: one lane or a quad per (butterfly, u), u < 2^(q - 1), u-major per
 // job, which is half a job's outputs; u = 0, the last, has none.  A chain of 63
 // doublings: a quad's lasts 0.25 ms up to two blocks per SM and 0.49 at 8192 turns, a lane's
-// 0.60 at 16384 (2^16 points, q = 2), so quads take up to a wave of turns (two of slots) and
-// lanes, with less work in all, the rest.
+// 0.60 at 16384 (2^16 points, q = 2), so quads take up to a wave of turns and lanes, with
+// less work in all, the rest (1.3 waves, q = 3, a batch of 2^15, 2^6 and 2^2: 19.33 ms with
+// quads, 19.20 with lanes).
 template <bool Quad>
 __global__ void __launch_bounds__(64, 4)
 k_fft_quarter(xyzz* prod, const FftJob* __restrict__ jobs, const uint32_t* __restrict__ lst_job,
@@ -590,6 +591,7 @@ static size_t fft_quad_wave()
 struct FftPass {
     uint32_t s0 = 0, q = 1, group = 0;
     uint32_t split = 0, turns = 0;
+    bool quad_turns = false;            // the turns by quads
     enum { kStage, kQuads, kPairs, kLanes } kind = kStage;
     uint32_t off = 0, cnt = 0;          // its entries of the job lists
     uint32_t items = 0, outputs = 0;
@@ -705,6 +707,7 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
                 const size_t v = outputs / 2 - (outputs >> q);
                 const double sums = kSumsMs + kSumMs * (double)outputs * (1u << q);
                 const double turn = turns ? quarter_ms(v, wave) : 0.0;
+                p.quad_turns = v <= wave;
                 if (!solo) {
                     ms = kFullMs / (double)wave * ((double)n + (double)v / 3) + sums;
                     p.kind = FftPass::kLanes;
@@ -896,7 +899,7 @@ cudaError_t fft_run_multi(Ctx* ctx, void* d_values, const FftSpec* specs, size_t
             k_fft_items<1, false><<<grid, kItemThreads, 0, ps>>>(tmp, pp, d_jobs, lj, li, p.cnt, p.items, p.s0, p.q, p.turns);
         if (p.turns) {
             const uint32_t turns = p.outputs / 2;
-            if (turns <= 2 * fft_quad_wave())
+            if (p.quad_turns)
                 k_fft_quarter<true><<<div_up(4 * (size_t)turns, 64), 64, 0, ps>>>(
                     pp, d_jobs, lj, li, d_lst_out + p.off, p.cnt, turns, p.s0, p.q, p.split);
             else

@@ -1,0 +1,59 @@
+"""Which kernels the G1 FFT's pass planner takes, on the CPU over a fake CUDA runtime
+(see fake_cuda), and transforms of every form against the oracle with root tables in
+which only some entries are powers of one root."""
+import json
+import math
+import random
+
+import pytest
+
+R = 0x73eda753299d7d483339d80809a1d80553bda402fffe5bfeffffffff00000001
+WAVE = 152 * 4 * 16             # quads that are resident at once
+
+
+def _launches(gpu_binding, shapes, mode):
+    """Per shape (log sizes of a batch), per stream: (kernel, threads) of the passes."""
+    import fake_cuda
+    gpu_binding.load()
+    ops = fake_cuda.run(gpu_binding.LIB_PATH, """
+out = []
+for logs in json.loads(%r):
+    ns = [1 << k for k in logs]
+    dom = {n: domain(n) for n in set(ns)}
+    vals = (P * len(ns))(*[buf(144 * n).value for n in ns])
+    doms = (P * len(ns))(*[dom[n].value for n in ns])
+    clear()
+    assert L.catmsm_p1_fft_batch(vals, sizes(ns), doms, (C.c_int * len(ns))(*[%d] * len(ns)), S(len(ns))) == 0
+    out.append([(l[1], l[2], int(l[3]) * int(l[4])) for l in log() if l[0] == "launch"])
+    _keep.clear()
+done(out)
+""" % (json.dumps(shapes), mode))
+    res = []
+    for launches in ops:
+        streams = {}
+        for st, k, threads in launches:
+            if "items" in k or "quarter" in k or "combine" in k or "stage" in k:
+                streams.setdefault(st, []).append((k, threads))
+        res.append(streams)
+    return res
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_turns_run_in_the_form_that_was_priced(gpu_binding, mode):
+    """Quarter turns by quads up to a wave of turns, by lanes above, for every number of
+    levels a pass has."""
+    shapes = [[15, 6, 2], [15, 3], [15, 11], [14, 14, 10, 9, 5], [12] * 3, [13], [16], [16] * 4]
+    seen = set()
+    for streams in _launches(gpu_binding, shapes, mode):
+        for seq in streams.values():
+            for i, (k, threads) in enumerate(seq):
+                if "quarter" not in k:
+                    continue
+                quads = "true" in k
+                slots = threads // (4 if quads else 1)               # two outputs each
+                split = "true" in seq[i - 1][0]
+                q = round(math.log2(seq[i + 1][1] / (2 * slots))) - 1 - split
+                turns = slots - 2 * slots // 2 ** q
+                seen.add((q, quads))
+                assert quads == (turns <= WAVE), (q, slots, turns)
+    assert {(2, True), (2, False)} <= seen and any(q > 2 for q, _ in seen)
