@@ -57,3 +57,58 @@ def test_turns_run_in_the_form_that_was_priced(gpu_binding, mode):
                 seen.add((q, quads))
                 assert quads == (turns <= WAVE), (q, slots, turns)
     assert {(2, True), (2, False)} <= seen and any(q > 2 for q, _ in seen)
+
+
+# Batches of the same transform that take every form with turns (the small sizes' forms
+# meet such tables in test_fft_passes.py).
+BATCHES = {"pairs": [12], "lanes": [12] * 3, "lane_turns_two_groups": [12] * 32, "stages": [10] * 3 + [15]}
+
+
+def test_batches_reach_every_form(gpu_binding):
+    """The batches below and the golden sizes take, between them, every kind of pass."""
+    shapes = list(BATCHES.values()) + [[3], [9], [17]]
+    seen, streams = set(), {}
+    for mode in (0, 1):
+        for name, s in zip(list(BATCHES) + [None] * 3, _launches(gpu_binding, shapes, mode)):
+            seen |= {k.replace("_", "") for seq in s.values() for k, _ in seq}
+            streams[name] = len(s)
+    want = {"kfftitems<1,false>", "kfftitems<2,false>", "kfftitems<4,false>", "kfftitems<4,true>",
+            "kfftquarter<true>", "kfftquarter<false>", "kfftstagemulti<4>", "kfftstagemulti<6>", "kfftcombine"}
+    assert want <= seen, want - seen
+    assert streams["lane_turns_two_groups"] == 2 and streams["pairs"] == 1
+
+
+@pytest.fixture(scope="module")
+def broken(gpu, oracle):
+    """2^12 points, a root table with a tenth of its entries replaced, and the oracle's
+    forward and inverse transforms over it."""
+    n = 1 << 12
+    rnd = random.Random(12)
+    jac = oracle.jacobian_randomize(5, n, oracle.gen_points(5, n))
+    ok, d = gpu.fr_fft_domain_init(n)
+    assert ok
+    d = bytearray(d)
+    for i in range(1, n):
+        if rnd.random() < 0.1:
+            d[32 * i:32 * i + 32] = (rnd.randrange(R) * (1 << 256) % R).to_bytes(32, "little")
+    d, want = bytes(d), []
+    for inverse in (False, True):
+        ok, out = oracle.p1_fft_with_domain(jac, n, d, n + 2, inverse)
+        assert ok
+        want.append([oracle.serialize(out[144 * i:144 * i + 144]) for i in range(n)])
+    return n, jac, d, want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("batch", ["pairs", "lanes", "lane_turns_two_groups"])
+def test_partly_broken_tables(gpu, oracle, broken, batch, mode):
+    n, jac, d, want = broken
+    count = len(BATCHES[batch])
+    rc, out = gpu.p1_fft_batch([jac] * count, [n] * count, [d] * count, [mode] * count)
+    assert rc == 0
+    first = bytes(out[0])
+    assert [oracle.serialize(first[144 * i:144 * i + 144]) for i in range(n)] == want[mode]
+    for other in out[1:]:
+        for i in range(0, n, 37 if count > 4 else 1):
+            assert oracle.serialize(bytes(other[144 * i:144 * i + 144])) == want[mode][i]
