@@ -623,11 +623,15 @@ static void pass_counts(const std::vector<const FftJob*>& jobs, uint32_t s0, uin
         const FftJob& J = *job;
         if (J.logn <= s0) continue;
         const uint32_t qe = std::min(q, J.logn - s0);
-        const size_t bf = (size_t)std::min(J.n >> (s0 + qe), J.xn) << s0;
+        const uint32_t groups = J.n >> (s0 + qe);
+        const size_t bf = (size_t)std::min(groups, J.xn) << s0;
         items += bf * pass_items(qe);
-        const bool scaled = J.scale && s0 + qe == J.logn;          // x_0 as well
-        for (int t = 0; t < 2; t++) products[t] += bf * (pass_products(s0, qe, t != 0) + (scaled ? 1 : 0));
         outputs += bf << qe;
+        const bool scaled = J.scale && s0 + qe == J.logn;          // x_0 as well
+        // a block with one non-identity input or none (a truncated prefix): that input is x_0
+        const bool only_x0 = J.xn <= groups;
+        for (int t = 0; t < 2; t++)
+            products[t] += bf * ((only_x0 ? 0 : pass_products(s0, qe, t != 0)) + (scaled ? 1 : 0));
     }
 }
 
@@ -697,7 +701,7 @@ static std::vector<FftPass> fft_plan(const std::vector<const FftJob*>& jobs, boo
             p.q = q;
             double ms = 1e300;
             if (q == 1) {
-                const double bf = (double)outputs / 2, scaled = (double)products[0] - (s ? bf : 0);
+                const double bf = (double)outputs / 2, scaled = std::max(0.0, (double)products[0] - (s ? bf : 0));
                 ms = (solo ? stage_ms(outputs / 2, wave) : kFullMs / (double)wave * bf) * (1 + 0.85 * scaled / bf);
             }
             const bool fits = with_products && items <= pass_max_items(q);

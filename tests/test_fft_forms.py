@@ -112,3 +112,22 @@ def test_partly_broken_tables(gpu, oracle, broken, batch, mode):
     for other in out[1:]:
         for i in range(0, n, 37 if count > 4 else 1):
             assert oracle.serialize(bytes(other[144 * i:144 * i + 144])) == want[mode][i]
+
+
+@pytest.mark.parametrize("n,xn,turns", [(4, 1, 0), (64, 1, 0), (4, 2, 1)])
+def test_passes_without_products_are_not_priced_as_products(gpu_binding, n, xn, turns):
+    """Where every block of a pass has one non-identity input (a truncated prefix) there is
+    nothing to multiply: no quarter turns are launched for it."""
+    import fake_cuda
+    gpu_binding.load()
+    names = fake_cuda.run(gpu_binding.LIB_PATH, """
+n, xn = %d, %d
+v, d = buf(144 * n), domain(n)
+for i in range(xn):
+    C.memset(v.value + 144 * i, 1, 144)
+L.catmsm_p1_fft_truncated_prefix.restype = C.c_bool
+assert L.catmsm_p1_fft_truncated_prefix(v, S(n), S(xn), d, S(n + 2))
+done(kernels())
+""" % (n, xn))
+    assert any("k_fft_items" in k or "k_fft_stage" in k for k in names)
+    assert sum("quarter" in k for k in names) == turns
