@@ -149,16 +149,18 @@ __device__ __forceinline__ void load_scalar32(uint32_t* k, const uint8_t* s)
 // No digit, rank or index arrays (400 MB written and read again for 33 M entries) and
 // ~24 times fewer global atomics, which bounded the per-pair form below: 1.11 ->
 // 0.28 ms for 1024 MSMs of 33 M entries in all (single-word scattered writes: 0.81).
-// For MSMs of at most kPartMaxB buckets whose part fits shared memory, in batches
-// of at least kPartMinFill entries per bucket of an MSM: with fewer the launches
-// last as long as one block, whose copies go over all buckets.  Sort per pair
+// For MSMs of at most kPartMaxB buckets whose part fits shared memory: up to
+// kPartAnyB buckets always, above in batches of at least kPartMinFill entries per
+// bucket of an MSM.  With fewer the launches last as long as one block, whose copies
+// go over all buckets; the form per pair lasts as long as a thread's D digits.  Per pair
 // against by parts, us: 12 bits, 8 x 4096 pairs (352 a bucket) 44 / 62, 16 x 4096 (704)
 // 75 / 62; 13 bits, 24 x 4096 (480) 85 / 91, 32 x 4096 (640) 113 / 92; 11 bits, 8 x 4096
-// (768) 49 / 50, 256 x 100 (600) 45 / 45; 9 bits, 64 x 100 (725) 41 / 30.
+// (768) 49 / 50, 256 x 100 (600) 45 / 45; 9 bits, 64 x 100 (725) 41 / 30; 8 bits, one MSM of
+// 500 (129) 40 / 30, of 2000 (516) 39 / 45.
 constexpr uint32_t kPartPairs = 1024;
 constexpr uint32_t kPartThreads = 512;
 constexpr uint32_t kPartMaxB = 4096;
-constexpr size_t kPartMinFill = 600;
+constexpr size_t kPartMinFill = 600, kPartAnyB = 512;
 constexpr size_t kPartMaxSmem = 220 * 1024;
 
 static size_t part_smem(uint32_t c, uint32_t D) { return ((size_t)2 << (c - 1)) * 4 + 128 + (size_t)kPartPairs * D * 4; }
@@ -425,7 +427,8 @@ static cudaError_t build_tables(Basis* b, uint32_t c)
 static bool part_sort(const Basis* b, size_t entries)
 {
     const size_t B = (size_t)1 << (b->c - 1);
-    return B <= kPartMaxB && part_smem(b->c, b->D) <= kPartMaxSmem && entries >= kPartMinFill * B;
+    return B <= kPartMaxB && part_smem(b->c, b->D) <= kPartMaxSmem &&
+           (B <= kPartAnyB || entries >= kPartMinFill * B);
 }
 
 static size_t max_parts(uint32_t nmsm, size_t cap) { return cap / kPartPairs + nmsm; }

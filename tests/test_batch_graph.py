@@ -115,11 +115,11 @@ done(log())
 
 
 @pytest.mark.parametrize("window,pairs,parts", [(13, 4096 * 29, False), (13, 4096 * 32, True), (11, 25599, False),
-                                                (11, 25600, True), (9, 64 * 80, False), (9, 64 * 100, True),
+                                                (11, 25600, True), (12, 55855, True), (12, 55854, False),
                                                 (14, 4096 * 32, False)])
 def test_sort_follows_the_entries(gpu_binding, window, pairs, parts):
-    """The sort by parts runs from 600 entries per bucket of an MSM on, up to 13-bit
-    windows, with and without the graph, whatever ran before."""
+    """The sort by parts runs from 600 entries per bucket of an MSM on, for windows of 11
+    to 13 bits, with and without the graph, whatever ran before."""
     gpu_binding.load()
     got = fake_cuda.run(gpu_binding.LIB_PATH, """
 b = Basis(4096, %d)
@@ -150,3 +150,17 @@ b.batch([%d] * %d, False)
 done([k for k in kernels() if k.startswith("k_reduce_level")])
 """ % (pairs, nmsm))
     assert len(got) == 1 and ("true" in got[0]) == inlined
+
+
+@pytest.mark.parametrize("window", [2, 8, 10])
+def test_narrow_windows_sort_by_parts(gpu_binding, window):
+    """Up to 512 buckets an MSM, where its parts fit shared memory (not 2 bits), always."""
+    gpu_binding.load()
+    got = fake_cuda.run(gpu_binding.LIB_PATH, """
+b = Basis(4096, %d)
+clear()
+b.batch([1] * 8, False)
+b.batch([4096] * 8, False)
+done([k for k in kernels() if "scatter" in k])
+""" % window)
+    assert got == [("k_part_scatter" if window > 2 else "k_scatter_batch")] * 2
