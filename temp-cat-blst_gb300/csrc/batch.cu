@@ -40,7 +40,7 @@ __global__ void k_scan_local(const uint32_t* __restrict__ in, uint32_t* __restri
 __global__ void k_scan_top(uint32_t* __restrict__ block_sums, uint32_t nb, uint32_t* __restrict__ total_out);
 __global__ void k_scan_add(uint32_t* __restrict__ out, const uint32_t* __restrict__ block_sums, uint32_t M);
 __global__ void k_accumulate(const affine* __restrict__ pts, const uint32_t* __restrict__ sorted_pt,
-                             const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ total_ptr,
+                             const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ total_ptr, uint32_t below,
                              uint32_t L, xyzz* __restrict__ buckets, xyzz* __restrict__ head,
                              xyzz* __restrict__ tail);
 __global__ void k_fixup(const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ offsets,
@@ -508,12 +508,11 @@ static cudaError_t enqueue_batch(const Basis* b, BatchWork* w, cudaStream_t st, 
                                                         (uint32_t)nD, sorted_pt, sorted_key);
     int aff_launches = 0;
     if (rounds)
-        CATMSM_CHECK(aff_accumulate(w->aff, b->table.p, sorted_pt, sorted_key, total, L,
+        CATMSM_CHECK(aff_accumulate(w->aff, b->table.p, sorted_pt, sorted_key, total, msm_affine_min_entries(rounds), L,
                                     chunks, rounds, buckets, head, tail, st, &aff_launches));
     else
-        k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)b->table.p, sorted_pt,
-                                                          sorted_key, total, L, buckets, head,
-                                                          tail);
+        k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)b->table.p, sorted_pt, sorted_key, total,
+                                                          0xffffffffu, L, buckets, head, tail);
     k_fixup_seg<<<div_up(chunks, 128), 128, 0, st>>>(sorted_key, total, L, head);
     k_fixup_join<<<div_up(chunks, 128), 128, 0, st>>>(sorted_key, offsets, total, L, buckets,
                                                       head, tail, hot_list, hot_count);

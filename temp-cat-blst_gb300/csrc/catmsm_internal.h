@@ -85,14 +85,18 @@ void reduce_pair_lanes(const void* inA, const void* inQ, uint32_t m, uint32_t D,
 // k_accumulate (buckets / head / tail per chunk of L sorted entries), so the
 // fixup stage is unchanged.  aff_prepare sizes W for up to `chunks` chunks
 // (bounded: the chunks run in slices); aff_accumulate only launches, so it can
-// be captured.  *launches is increased by the kernels launched.
+// be captured.  With fewer than `least` entries (*total, on the device) the rounds are
+// left out and k_accumulate runs.
+// *launches is increased by the kernels launched.
 cudaError_t aff_prepare(AffWork& W, uint32_t L, size_t chunks, cudaStream_t st);
 cudaError_t aff_accumulate(const AffWork& W, const void* pts, const uint32_t* sorted_pt, const uint32_t* sorted_key,
-                           const uint32_t* total, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
+                           const uint32_t* total, uint32_t least, uint32_t L, size_t chunks, uint32_t rounds, void* buckets,
                            void* head, void* tail, cudaStream_t st, int* launches);
 // Rounds to use for nD bucket entries over M buckets (0: the
 // XYZZ-only k_accumulate).
 uint32_t msm_affine_rounds(size_t nD, size_t M);
+// The entries from which that many rounds (> 0) pay.
+uint32_t msm_affine_min_entries(uint32_t rounds);
 
 // H2D of `bytes` from src to dst on the context's copy stream, after the work
 // already queued on its pipeline stream; *ready is an event recorded after

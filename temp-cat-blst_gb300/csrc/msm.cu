@@ -285,14 +285,14 @@ __device__ __forceinline__ void madd_entry(xyzz& acc, const affine* __restrict__
 __global__ void __launch_bounds__(128, 4) k_accumulate(const affine* __restrict__ pts,
                                                     const uint32_t* __restrict__ sorted_pt,
                                                     const uint32_t* __restrict__ sorted_key,
-                                                    const uint32_t* __restrict__ total_ptr, uint32_t L,
-                                                    xyzz* __restrict__ buckets, xyzz* __restrict__ head,
-                                                    xyzz* __restrict__ tail)
+                                                    const uint32_t* __restrict__ total_ptr, uint32_t below,
+                                                    uint32_t L, xyzz* __restrict__ buckets,
+                                                    xyzz* __restrict__ head, xyzz* __restrict__ tail)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t E = *total_ptr;
     const size_t start = (size_t)t * L;
-    if (start >= E) return;
+    if (start >= E || E >= below) return;
     const uint32_t end = (uint32_t)min((size_t)E, start + L);
     uint32_t cur = sorted_key[start];
     const bool starts_before = start > 0 && sorted_key[start - 1] == cur;
@@ -969,6 +969,20 @@ static uint32_t accumulate_chunk(size_t nD)
 // (4.2 M); 300007 2.49 / 2.43 / 2.47 / 2.58 (4.8 M); 2^19 3.68 / 3.55 / 3.39 / 3.45
 // (8.4 M); 700001 4.63 / 4.38 / 4.17 / 4.22 (11.2 M); 2^20 6.51 / 6.18 / 5.75 / 5.65
 // (16.8 M); 2^22 22.5 / 22.2 / 20.6 / 20.3 (58.7 M); a fourth round is slower at all.
+//
+// nD counts every digit, and sparse scalars (zeros, values of few bits) may leave far
+// fewer entries, which only the device knows.  Below the rounds' least entries
+// (msm_affine_min_entries) their launches leave at once and k_accumulate, which
+// leaves at once otherwise, does them all.  Whole MSM, ms, with the rounds /
+// without: one round, 1.2 M entries (2^18 points below 2^64) 1.60 / 1.53, 1.8 M 1.99 / 1.96, 2.4 M
+// 1.97 / 1.99, 3.2 M 2.37 / 2.46; two, 0.8 M (2^19 points, nine in ten zero) 1.71 / 1.50, 3.2 M 2.32
+// / 2.37, 4.2 M (every second zero) 2.40 / 2.20, 5.6 M 2.88 / 2.70; three, 1.7 M 2.12 / 1.86, 2.9 M 2.62 /
+// 2.55, 4.7 M 2.79 / 2.84, 6.8 M 3.30 / 3.46.
+uint32_t msm_affine_min_entries(uint32_t rounds)
+{
+    return rounds == 1 ? 9u << 18 : rounds == 2 ? 13u << 19 : 3u << 20;
+}
+
 uint32_t msm_affine_rounds(size_t nD, size_t M)
 {
     const double per = (double)nD / (double)(M ? M : 1);
@@ -1204,12 +1218,13 @@ static cudaError_t msm_run(Ctx* ctx, const void* d_points, const uint8_t* d_scal
         cudaGetLastError();
         rounds = 0;
     }
-    if (rounds) {
-        CATMSM_CHECK(aff_accumulate(W.aff, d_points, sorted_pt, sorted_key, total, L, chunks, rounds, buckets, head,
-                                    tail, st, &g_stats.launches));
-    } else
-        k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)d_points, sorted_pt, sorted_key, total, L,
-                                                          buckets, head, tail);
+    const uint32_t least = rounds && ctx->affine_rounds < 0 ? msm_affine_min_entries(rounds) : 0;
+    if (rounds)
+        CATMSM_CHECK(aff_accumulate(W.aff, d_points, sorted_pt, sorted_key, total, least, L, chunks, rounds, buckets,
+                                    head, tail, st, &g_stats.launches));
+    else
+        k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>((const affine*)d_points, sorted_pt, sorted_key, total,
+                                                          0xffffffffu, L, buckets, head, tail);
     mark(5);
     if (nD > 2 * (size_t)L * M) {
         // buckets average more than two chunks: tree over each warp's chunks

@@ -55,7 +55,7 @@ __global__ void k_scatter(const uint32_t* __restrict__ digits, const uint32_t* _
                           const uint32_t* __restrict__ offsets, uint32_t n, uint32_t nD,
                           uint32_t* __restrict__ sorted_pt, uint32_t* __restrict__ sorted_key);
 __global__ void k_accumulate(const affine* __restrict__ pts, const uint32_t* __restrict__ sorted_pt,
-                             const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ total_ptr,
+                             const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ total_ptr, uint32_t below,
                              uint32_t L, xyzz* __restrict__ buckets, xyzz* __restrict__ head,
                              xyzz* __restrict__ tail);
 __global__ void k_fixup(const uint32_t* __restrict__ sorted_key, const uint32_t* __restrict__ offsets,
@@ -173,7 +173,8 @@ static cudaError_t noalloc_queue(unsigned char* base, const blst_p1_affine* poin
     k_scan_add<<<div_up(M, 256), 256, 0, st>>>(offsets, bsums, (uint32_t)M);
     k_scatter<<<div_up(nD, 256), 256, 0, st>>>(digits, ranks, offsets, (uint32_t)n, (uint32_t)nD, sorted_pt,
                                               sorted_key);
-    k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>(d_pts, sorted_pt, sorted_key, total, kL, buckets, head, tail);
+    k_accumulate<<<div_up(chunks, 128), 128, 0, st>>>(d_pts, sorted_pt, sorted_key, total, 0xffffffffu, kL, buckets,
+                                                      head, tail);
     k_fixup<<<div_up(chunks, 128), 128, 0, st>>>(sorted_key, offsets, total, kL, buckets, head, tail, hot_list,
                                                  hot_count, (uint32_t)kChunks);
     k_fixup_hot<<<device_sms(), 128, 0, st>>>(hot_list, hot_count, offsets, kL, buckets, head, tail);
