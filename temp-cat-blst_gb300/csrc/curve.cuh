@@ -232,8 +232,6 @@ __device__ __forceinline__ void xyzz_add_sub(xyzz& p, xyzz& d, const xyzz& q)
     fp_mul2(d.y, t, R, S1, PPP);
 }
 
-__device__ __forceinline__ void xyzz_neg(xyzz& p) { fp_neg(p.y, p.y); }
-
 // Jacobian (X, Y, Z) = (x*zz, y*zzz, zz); reference point.cpp:2109
 __device__ __forceinline__ void xyzz_to_jac(jac& o, const xyzz& p)
 {
@@ -305,43 +303,6 @@ __device__ __forceinline__ void jac_dbl(jac& p)
     fp_dbl(C, C);
     fp_sub(p.y, t, C);
 }
-
-// p += q, add-2007-bl style with explicit infinity / doubling / opposite cases
-__device__ __forceinline__ void jac_add(jac& p, const jac& q)
-{
-    if (jac_is_inf(q)) return;
-    if (jac_is_inf(p)) { p = q; return; }
-    fp z1z1, z2z2, u1, h, s1, r, t;
-    fp_sqr(z1z1, p.z);
-    fp_sqr(z2z2, q.z);
-    fp_mul(u1, p.x, z2z2);
-    fp_mul(h, q.x, z1z1);
-    fp_sub(h, h, u1);
-    fp_mul(s1, p.y, q.z);
-    fp_mul(s1, s1, z2z2);
-    fp_mul(r, q.y, p.z);
-    fp_mul(r, r, z1z1);
-    fp_sub(r, r, s1);
-    if (fp_is_zero(h)) {
-        if (fp_is_zero(r)) jac_dbl(p);
-        else jac_set_inf(p);
-        return;
-    }
-    fp_mul(p.z, p.z, q.z);
-    fp_mul(p.z, p.z, h);
-    fp_sqr(t, h);                 // HH
-    fp_mul(u1, u1, t);            // V = U1 HH
-    fp_mul(t, t, h);              // HHH
-    fp_sqr(z1z1, r);
-    fp_sub(z1z1, z1z1, t);
-    fp_sub(z1z1, z1z1, u1);
-    fp_sub(p.x, z1z1, u1);        // X3 = R^2 - HHH - 2V
-    fp_sub(u1, u1, p.x);
-    fp_neg(t, t);
-    fp_mul2(p.y, u1, r, s1, t);   // Y3 = R (V - X3) - S1 HHH, one reduction
-}
-
-__device__ __forceinline__ void jac_neg(jac& p) { fp_neg(p.y, p.y); }
 
 // GLV endomorphism of G1: phi(x, y) = (beta x, y) = lambda (x, y) for
 // lambda = z^2 - 1 = 0xac45a4010001a40200000000ffffffff (lambda^2 + lambda + 1 = r)
@@ -505,9 +466,7 @@ __device__ __forceinline__ void qd_add(fp& d, const fp& e, const quad_lane& q)
     d = qd_add_core<false>(PR, r, d, e, q);
 }
 
-// d += an affine point (not infinity): lane k passes coordinate k mod 2 of it.
-// h: the difference P (every even lane), the ratio of the new z to the old.
-// madd-2008-s with the complete special cases.
+// d = an affine point (not infinity): lane k passes coordinate k mod 2 of it.
 __device__ __forceinline__ void qd_set_affine(fp& d, const fp& a, const quad_lane& q)
 {
     fp one;
@@ -515,6 +474,7 @@ __device__ __forceinline__ void qd_set_affine(fp& d, const fp& a, const quad_lan
     d = fp_sel(a, one, q.k >= 2);
 }
 
+// The differences P (even lanes: the ratio of the sum's z to d's) and R (odd lanes).
 __device__ __forceinline__ fp qd_madd_diff(const fp& d, const fp& a, const quad_lane& q)
 {
     const fp r = fp_sel(fp_mul_call(d, a), d, q.k < 2);    // X1, Y1, U2, S2
@@ -524,6 +484,7 @@ __device__ __forceinline__ fp qd_madd_diff(const fp& d, const fp& a, const quad_
     return PR;
 }
 
+// d += an affine point, as above: madd-2008-s with the complete special cases.
 __device__ __forceinline__ void qd_madd(fp& d, const fp& a, const quad_lane& q)
 {
     if (qd_is_inf(d, q)) {
