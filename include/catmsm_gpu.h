@@ -87,7 +87,9 @@ bool blst_fr_fft_domain_init(blst_fr *domain, size_t domain_len, size_t n);
 /* Replaces blst_p1_fft (bindings/blst_fft.h:109, blst/fft_c_api.cpp:184 -> :51-66):
  * in-place natural-order G1 DFT with powers of the primitive n-th root
  * (inverse: of its reciprocal, then scaled by 1/n).  false before writing on
- * NULL values or invalid n; false with values untouched on a device failure. */
+ * NULL values or invalid n; false with values untouched on a device failure.
+ * Values are elements of G1, the prime-order subgroup (not checked), here and in
+ * every FFT below. */
 bool blst_p1_fft(blst_p1 *values, size_t n, bool inverse);
 
 /* Replaces blst_p1_fft_with_domain (bindings/blst_fft.h:111, blst/fft_c_api.cpp:194 ->
