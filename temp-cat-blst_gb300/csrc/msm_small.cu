@@ -14,7 +14,7 @@
 //   sums     about 368 threads, each with up to L entries of ONE bucket (a bucket of
 //            m entries gets ceil(m / L) threads, so one hot bucket still uses them all),
 //            then a quad tree over each bucket's threads.
-//            A block with too many entries (kSmallMaxEntries; equal scalars: all of a
+//            A block with too many entries (small_limit; equal scalars: all of a
 //            window in one block) raises a flag, the others leave before their sums,
 //            and the general pipeline, which spreads a bucket over the whole GPU, runs
 //            instead, on the split that is there already;
@@ -38,13 +38,8 @@ constexpr uint32_t kSmallNarrow = 512;         // up to this many: 4-bit windows
 constexpr uint32_t kSmallThreads = 512;
 constexpr uint32_t kSmallSums = 368;           // threads with entries, before one more per bucket
 constexpr uint32_t kSmallMaxR = 16;            // buckets per block
-// Entries of a block: at most this many, or 7/4 of its share of a window (the top
-// window of GLV halves below 2^126.4 has 1.49 of it in a block), and of one bucket
-// kSmallMaxBucket.  Above, the general pipeline is faster although the attempt comes
-// before it (about 15 us).  Twice the share, no bound on a bucket and every block at work
-// to its end: 8192 scalars below 2^64 649 us, 477 now; eight values 890, 569; 12288 zeros and
-// ones 469, 345; 8192 scalars of 129 bits 743, 540.
-constexpr uint32_t kSmallMaxEntries = 2048, kSmallMaxBucket = 2560;
+// Most entries of a block, and of one bucket: see small_limit.
+constexpr uint32_t kSmallAny = 2048, kSmallDense = 5400, kSmallHot = 3600, kSmallMaxBucket = 4000;
 
 // Measured against the general pipeline (host call, us): 255 bits 64 points 170 / 308,
 // 4096 306 / 405, 12288 497 / 521, 16384 611 / 553; 64 bits 2048 points 237 / 348,
@@ -119,8 +114,7 @@ struct SmallArgs {
     xyzz* outA;                 // per (window, range): 2^log2(R) S, null with one range
     xyzz* outQ;                 // per (window, range): sum (b + 1) S_b
     uint32_t* entries;          // counter of nonzero digits, or null
-    uint32_t limit;             // most entries of a block
-    uint32_t* stop;             // set when a block has more (zeroed by the kernel before)
+    uint32_t* stop;             // set when a block has too many entries (zeroed by the kernel before)
     uint32_t* over;             // page-locked: the same for the host
 };
 
@@ -150,6 +144,20 @@ __device__ __forceinline__ int32_t small_digit(const uint4& k, const SmallArgs& 
     return (int32_t)raw - (int32_t)(1u << (A.c - 1));
 }
 
+// The most entries of a block for which the small kernel runs, out of W of its window:
+// kSmallAny; twice its even share, up to kSmallDense; or, if it has most of the window (0/1
+// vectors, the carries of short scalars: where the general pipeline has little to do
+// elsewhere), 9/40 of the points up to kSmallHot.  Above, the general pipeline is faster although the attempt
+// comes before it (about 15 us).  The top window of uniform GLV halves, below 2^126.4, has
+// 1.49 shares in a block.  Small kernel against general pipeline, us: 6000 points, 43%
+// ones (2580 entries) 289 / 322; 8192, 43% (3522) 330 / 362; 12288, 43% (5284) 432 / 350; 6000, a
+// quarter ones and the rest random (1.75 shares) 388 / 470; 10000 scalars of 127 bits (1.8) 494 / 554, 12288 (1.8,
+// 5542 entries) 556 / 509.
+__device__ __forceinline__ uint32_t small_limit(uint32_t s, uint32_t W, const SmallArgs& A)
+{
+    return max(kSmallAny, 2 * s > W ? min(A.n * 9 / 40, kSmallHot) : min(2 * ((A.n + A.nb - 1) / A.nb), kSmallDense));
+}
+
 constexpr uint32_t kSmallAcc = kSmallSums + kSmallMaxR;
 constexpr size_t kSmallFixed = (kSmallAcc + 3 * kSmallMaxR) * sizeof(xyzz);
 
@@ -159,19 +167,24 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
     xyzz* acc = reinterpret_cast<xyzz*>(small_smem);          // a partial sum per thread
     xyzz* lev = acc + kSmallAcc;                              // bucket sums, then (Q | A) of the levels
     uint32_t* list = reinterpret_cast<uint32_t*>(lev + 3 * kSmallMaxR);
-    __shared__ uint32_t cnt[kSmallMaxR], start[kSmallMaxR + 1], ts[kSmallMaxR + 1], shape[4];
+    __shared__ uint32_t cnt[kSmallMaxR], start[kSmallMaxR + 1], ts[kSmallMaxR + 1], shape[4], W;
     const uint32_t tid = threadIdx.x, R = A.R;
     const uint32_t w = blockIdx.x / A.nb, b0 = blockIdx.x % A.nb * R;
     if (tid < kSmallMaxR) cnt[tid] = 0;
+    if (tid == 0) W = 0;
     __syncthreads();
+    uint32_t nonzero = 0;
     for (uint32_t i = tid; i < A.n; i += blockDim.x) {
         const int32_t d = small_digit(__ldg(A.mag + i), A, w);
         const uint32_t b = (uint32_t)(d < 0 ? -d : d) - 1 - b0;          // d = 0 wraps past R
+        nonzero += d != 0;
         if (d != 0 && b < R && atomicAdd(&cnt[b], 1u) == kSmallMaxBucket) {      // one bucket is too many already
             *(volatile uint32_t*)A.stop = 1;
             *A.over = 1;
         }
     }
+    nonzero = __reduce_add_sync(0xffffffffu, nonzero);
+    if ((tid & 31) == 0) atomicAdd(&W, nonzero);
     __syncthreads();
     if (tid == 0) {
         uint32_t s = 0;
@@ -192,7 +205,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_buckets(SmallArgs A)
         ts[R] = t;
         shape[0] = L;
         shape[1] = most;
-        shape[2] = s > A.limit;
+        shape[2] = s > small_limit(s, W, A);
         if (shape[2]) {
             *(volatile uint32_t*)A.stop = 1;
             *A.over = 1;
@@ -327,7 +340,6 @@ cudaError_t msm_small(Ctx* ctx, const void* pts, const uint8_t* scalars, uint32_
     A.pts = glv ? gpts : (const affine*)pts;
     A.mag = mag;
     A.entries = entries;
-    A.limit = std::max(kSmallMaxEntries, 7 * (A.n / A.nb) / 4);
     A.over = (uint32_t*)(wins + D);
     *A.over = 0;
     A.outA = A.nb > 1 ? seg : nullptr;
