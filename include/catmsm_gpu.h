@@ -323,7 +323,8 @@ int catmsm_p1s_mult_pippenger_noalloc(blst_p1 *ret, const blst_p1_affine *points
  * little-endian 256-bit scalars, concatenated MSM by MSM; counts[j] <= n.
  * Results are Jacobian blst_p1 (not normalised; z = 0 for infinity), as the
  * reference MSM returns them.  use_graph != 0 replays the batch's device
- * sequence as one CUDA graph launch (captured on first use per batch size).
+ * sequence as one CUDA graph launch (captured on first use per batch size, and
+ * again after a workspace has grown).
  * A basis has one stream and one workspace: calls on it from several host
  * threads (batches, set_config, config, autotune) are serialised by the
  * library and must be made with the basis's device current
