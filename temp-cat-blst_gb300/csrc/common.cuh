@@ -117,10 +117,13 @@ struct AuxStream {
         const cudaError_t e = cudaEventRecord(fork, st);
         return e == cudaSuccess ? cudaStreamWaitEvent(stream, fork, 0) : e;
     }
+    // Failing, it waits: the pipeline's next work must not meet what is queued here.
     cudaError_t end(cudaStream_t st) const
     {
-        const cudaError_t e = cudaEventRecord(join, stream);
-        return e == cudaSuccess ? cudaStreamWaitEvent(st, join, 0) : e;
+        cudaError_t e = cudaEventRecord(join, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, join, 0);
+        if (e != cudaSuccess) cudaStreamSynchronize(stream);
+        return e;
     }
     void release()
     {

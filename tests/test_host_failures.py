@@ -131,3 +131,32 @@ done([rc, log()])
     assert rc == 0 and len({o[1] for o in run}) == 1
     assert [o[2].split("<")[0] for o in run] == ["k_decode", "k_members"] * (len(run) // 2) and len(run) > 2
     assert sum(int(o[3]) for o in run if o[2].startswith("k_decode")) * 64 >= n
+
+
+@pytest.mark.parametrize("name,nth", [("cudaEventRecord", 2), ("cudaStreamWaitEvent", 2)])
+@pytest.mark.parametrize("call", ["msm", "fft"])
+def test_failed_join_waits_for_the_second_stream(host, call, name, nth):
+    """A call that forked a second stream and cannot join it waits for it: its buffers are
+    the next call's."""
+    rc, ops = host("""
+if %r == "msm":
+    n = 1 << 18
+    pts, sc = aligned(96 * n), buf(32 * n)
+    call = lambda: L.catmsm_p1s_mult_pippenger_device(buf(144), pts, sc, S(32), S(n), S(255), S(0))
+else:
+    n, k = 1 << 14, 6
+    v, d = (P * k)(*[buf(144 * n).value for _ in range(k)]), domain(n)
+    call = lambda: L.catmsm_p1_fft_batch(v, sizes([n] * k), (P * k)(*[d.value] * k), (C.c_int * k)(*[0] * k), S(k))
+assert call() == 0
+clear()
+fail(%r, %d)
+rc = call()
+done([rc, log()])
+""" % (call, name, nth))
+    assert rc != 0 and ["failed", name] in ops
+    launches = [(i, o[1]) for i, o in enumerate(ops) if o[0] == "launch"]
+    assert len({st for _, st in launches}) == 2
+    for st in {st for _, st in launches}:
+        last = max(i for i, s in launches if s == st)
+        if st != launches[0][1]:                              # the forked one
+            assert ["sync", st] in ops[last:]
