@@ -217,7 +217,7 @@ static bool fft_entry(blst_p1* values, size_t n, const blst_fr* domain, bool inv
         if (!hstage) err = cudaErrorMemoryAllocation;
     }
     if (err == cudaSuccess) err = cudaMemcpyAsync(hstage, dv, n * sizeof(blst_p1), cudaMemcpyDeviceToHost, st);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+    err = wait_stream(st, err);
     if (err != cudaSuccess) return false;
     host_copy(values, hstage, n * sizeof(blst_p1));
     return true;
@@ -296,6 +296,7 @@ void blst_p1s_tile_pippenger(blst_p1* ret, const blst_p1_affine* const points[],
             err = msm_tile_device(ctx, dp, (const uint8_t*)ds, (uint32_t)nbytes, npoints, (uint32_t)nbits,
                                   (uint32_t)bit0, (uint32_t)window, out);
         if (err == cudaSuccess) std::memcpy(ret, out, sizeof(*ret));
+        else cudaStreamSynchronize(ctx->stream);          // the caller's memory is not read after return
     } catch (...) {
         if (ret) write_inf(ret);
     }
@@ -318,7 +319,7 @@ bool blst_fr_fft_domain_init(blst_fr* domain, size_t domain_len, size_t n)
         if (err == cudaSuccess) err = fft_root_powers(ctx, dr + 8 * n, n, dr);
         if (err == cudaSuccess)
             err = cudaMemcpyAsync(domain, dr, n * sizeof(blst_fr), cudaMemcpyDeviceToHost, ctx->stream);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
+        err = wait_stream(ctx->stream, err);
         if (err != cudaSuccess) return false;
         hfr nn = fr_from_u64(n);
         hfr inv = fr_inv(nn);
@@ -427,7 +428,7 @@ int catmsm_p1_fft_batch(blst_p1* const values[], const size_t ns[], const blst_f
         if (err == cudaSuccess) err = fft_run_multi(ctx, dv, specs.data(), count);
         if (err == cudaSuccess)
             err = cudaMemcpyAsync(hstage, dv, total * sizeof(blst_p1), cudaMemcpyDeviceToHost, st);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+        err = wait_stream(st, err);
         if (err != cudaSuccess) return (int)err;
         off = 0;
         for (size_t i = 0; i < count; i++) {
@@ -468,8 +469,7 @@ int catmsm_p1_fft_device(void* d_values, size_t n, const void* d_domain, int mod
     if (!ctx) return (int)cudaErrorInitializationError;
     const uint32_t* dr = (const uint32_t*)d_domain;
     cudaError_t err = fft_run(ctx, d_values, n, dr, mode != 0, mode == 1 ? dr + 8 * n : nullptr);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    return (int)err;
+    return (int)wait_stream(ctx->stream, err);
 }
 
 void* catmsm_stream(void)
@@ -544,8 +544,7 @@ int catmsm_p1_affines_from_scalars_device(void* d_out, const void* d_k32, size_t
     Ctx* ctx = get_ctx();
     if (!ctx) return (int)cudaErrorInitializationError;
     cudaError_t err = points_from_scalars_device(ctx, (const uint8_t*)d_k32, n, d_out);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    return (int)err;
+    return (int)wait_stream(ctx->stream, err);
 }
 
 int catmsm_p1_affines_from_scalars(blst_p1_affine* out, const blst_byte* k32, size_t n)
@@ -561,8 +560,7 @@ int catmsm_p1_affines_from_scalars(blst_p1_affine* out, const blst_byte* k32, si
     if (err == cudaSuccess) err = points_from_scalars_device(ctx, (const uint8_t*)dk, n, dp);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(out, dp, sizeof(blst_p1_affine) * n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    return (int)err;
+    return (int)wait_stream(ctx->stream, err);
 }
 
 int catmsm_fp_inv(blst_fp* out, const blst_fp* a, size_t n)
@@ -577,8 +575,7 @@ int catmsm_fp_inv(blst_fp* out, const blst_fp* a, size_t n)
     if (err == cudaSuccess) err = fp_inv_test_device(ctx, d, d + 6 * n, n);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(out, d + 6 * n, n * sizeof(blst_fp), cudaMemcpyDeviceToHost, ctx->stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    return (int)err;
+    return (int)wait_stream(ctx->stream, err);
 }
 
 int catmsm_host_fp_inv(blst_fp* out, const blst_fp* a, size_t n)
@@ -633,8 +630,7 @@ int catmsm_fp_mul(blst_fp* out, const blst_fp* a, const blst_fp* b, size_t n)
     if (err == cudaSuccess) err = fp_mul_test_device(ctx, d, d + 6 * n, d + 12 * n, n, a == b);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(out, d + 12 * n, n * sizeof(blst_fp), cudaMemcpyDeviceToHost, ctx->stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
-    return (int)err;
+    return (int)wait_stream(ctx->stream, err);
 }
 
 }  // extern "C"

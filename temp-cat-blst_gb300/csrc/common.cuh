@@ -233,6 +233,14 @@ extern thread_local LaunchStats g_stats;
         if (e__ != cudaSuccess) return e__; \
     } while (0)
 
+// Waits for the stream, also after a failure: nothing that is queued uses the
+// caller's memory after the return.
+inline cudaError_t wait_stream(cudaStream_t st, cudaError_t err)
+{
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return err == cudaSuccess ? e : err;
+}
+
 inline unsigned div_up(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
 // Host copy between caller memory and pinned staging.  Large copies are

@@ -203,7 +203,7 @@ static bool fr_fft_entry(blst_fr* values, size_t n, const blst_fr* domain, bool 
     if (err == cudaSuccess) err = cudaMemcpyAsync(dv, values, n * 32, cudaMemcpyHostToDevice, st);
     if (err == cudaSuccess) err = fr_fft_run(st, dv, dv + 8 * n, n, dr, domain != nullptr && inverse, scale);
     if (err == cudaSuccess) err = cudaMemcpyAsync(hstage, dv, n * 32, cudaMemcpyDeviceToHost, st);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+    err = wait_stream(st, err);
     if (err != cudaSuccess) return false;
     host_copy(values, hstage, n * 32);
     return true;
@@ -308,7 +308,10 @@ static bool fr_msm_run(blst_p1* ret, const blst_p1_affine points[], const blst_f
     uint64_t out[18];
     if (err == cudaSuccess) err = msm_device(ctx, dp, (const uint8_t*)ds, 32, npoints, 255, 0, out, ready);
     if (ready) cudaStreamSynchronize(ctx->copy_stream);   // the caller's points are not read after return
-    if (err != cudaSuccess) return false;
+    if (err != cudaSuccess) {
+        cudaStreamSynchronize(st);                        // nor, after a failure, what else is queued
+        return false;
+    }
     std::memcpy(ret, out, sizeof(*ret));
     return true;
 }

@@ -162,7 +162,10 @@ int run_plain_msm(Server* s, Ctx* ctx, Request* r)
     cudaError_t err = cudaMemcpyAsync(d_sc, r->scalars, r->k * 32, cudaMemcpyHostToDevice, ctx->stream);
     uint64_t out[18];
     if (err == cudaSuccess) err = msm_device(ctx, basis_points_device(s->basis), d_sc, 32, r->k, 256, 0, out);
-    if (err != cudaSuccess) return (int)err;
+    if (err != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);              // the request's scalars are not read after its wait returns
+        return (int)err;
+    }
     std::memcpy(&r->result, out, sizeof(blst_p1));
     return 0;
 }

@@ -150,7 +150,7 @@ void blst_p1s_mult_wbits_precompute(blst_p1_affine table[], size_t wbits, const 
             if (err == cudaSuccess)
                 err = cudaMemcpyAsync(table + r0 * m, dt, rows * m * sizeof(affine), cudaMemcpyDeviceToHost, st);
         }
-        if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+        wait_stream(st, err);
     } catch (...) {
     }
 }
@@ -186,6 +186,7 @@ void blst_p1s_mult_wbits(blst_p1* ret, const blst_p1_affine table[], size_t wbit
         if (err == cudaSuccess)
             err = msm_device(ctx, dp, (const uint8_t*)ds, (uint32_t)nbytes, npoints, (uint32_t)nbits, 0, out);
         if (err != cudaSuccess) {
+            cudaStreamSynchronize(st);                    // the caller's memory is not read after return
             std::memset(ret, 0, sizeof(*ret));
             return;
         }

@@ -160,3 +160,27 @@ done([rc, log()])
         last = max(i for i, s in launches if s == st)
         if st != launches[0][1]:                              # the forked one
             assert ["sync", st] in ops[last:]
+
+
+ENTRIES = {
+    "fft": "L.blst_p1_fft_with_domain(buf(144 * n), S(n), domain(n), S(n + 2), C.c_bool(False))",
+    "fft_oneshot": "L.blst_p1_fft(buf(144 * n), S(n), C.c_bool(True))",
+    "fft_batch": "L.catmsm_p1_fft_batch((P * 1)(buf(144 * n).value), sizes([n]), (P * 1)(domain(n).value), "
+                 "(C.c_int * 1)(1), S(1))",
+    "fr_fft": "L.blst_fr_fft_with_domain(buf(32 * n), S(n), domain(n), S(n + 2), C.c_bool(False))",
+    "tile": "L.blst_p1s_tile_pippenger(buf(144), (P * 2)(buf(96 * n).value, None), S(n), (P * 2)(buf(32 * n).value, None), "
+            "S(255), buf(64), S(8), S(8))",
+    "mult_fr": "L.blst_p1s_mult_pippenger_fr(buf(144), aligned(96 * n), buf(32 * n), S(n), buf(1 << 20), S(1 << 20))",
+    "wbits": "L.blst_p1s_mult_wbits(buf(144), buf(96 * 8 * n), S(4), S(n), (P * 2)(buf(32 * n).value, None), S(255), buf(64))",
+}
+
+
+@pytest.mark.parametrize("name,nth", [("cudaMemcpyAsync", 2), ("cudaMalloc", 3)])
+@pytest.mark.parametrize("entry", sorted(ENTRIES))
+def test_failed_call_uses_nothing_after_return(host, entry, name, nth):
+    """Every host entry that fails after a copy was queued waits for it."""
+    ops = host("n = 1024\nfail(%r, %d)\n%s\ndone(log())" % (name, nth, ENTRIES[entry]))
+    if ["failed", name] not in ops:
+        pytest.skip("the call makes fewer of them")
+    at = {o[1]: i for i, o in enumerate(ops) if o[0] == "copy"}
+    assert all(["sync", stream] in ops[i:] for stream, i in at.items())
